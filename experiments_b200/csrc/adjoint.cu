@@ -115,6 +115,13 @@ __device__ void dplane_space(D3 n, D3& p, D3& q) {
 // ---------------------------------------------------------------------------
 // Adjoint buffers
 // ---------------------------------------------------------------------------
+// Row adjoints, float4 streams: 1..3 the header's (invMassA, invMassB, mu),
+// invInertiaA, invInertiaB; then three per row, of (axis, rhs), (angular part
+// A, 1/diag) and (angular part B, -): normal row j at kNormal0 + 3j, friction
+// row r at kFric0 + 3r.
+constexpr int kAdjSlots = 40;
+constexpr int kNormal0 = 4;
+constexpr int kFric0 = 16;
 constexpr int kContrib = 5;  // float4 per (manifold, side): (gx, gim), (gth, gmu), gv, gw, gii
 
 struct AdjView {
@@ -122,10 +129,10 @@ struct AdjView {
     float4 *gDv, *gDw;            // per body: adjoint of the solver's velocity change
     float* gInvMass;              // per body accumulators over all steps
     float* gMu;
-    float4* rowAdj;               // [kRowSlots][cap], layout of the rows
-    float4 *gInLin, *gInAng;      // [2 parity][2 sides][cap]: adjoint of each phase's inputs
+    float4* rowAdj;               // [kAdjSlots][cap]: adjoint of the header and the rows
+    float4* gIn;                  // [2 parity][2 cap][2]: adjoint of each phase's inputs, copies sorted by body
     float4* gLam;                 // [3][cap]: adjoint of the row impulses
-    float4* contrib;              // [kContrib][2 sides][cap]
+    float4* contrib;              // [kContrib][2 cap], copies sorted by body
     int cap;
 };
 
@@ -216,42 +223,29 @@ __global__ void k_adj_integrate(int n, const float* __restrict__ invMass, const 
 // ---------------------------------------------------------------------------
 // Jacobi adjoint: persistent cooperative kernel, phases in reverse
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void adj_average(const SolverView& V, const float4* gl, const float4* ga, int b, int buf,
-                                            float3& lin, float3& ang) {
-    const uint32_t s = V.incStart[b], e = V.incEnd[b];
-    float3 sl = make_float3(0.f, 0.f, 0.f), sa = sl;
-    for (uint32_t i = s; i < e; ++i) {
-        const uint32_t cid = V.incVals[i];
-        const size_t at = (size_t)(buf * 2 + (int)(cid & 1u)) * V.cap + (cid >> 1);
-        sl += f3(gl[at]);
-        sa += f3(ga[at]);
-    }
-    const float factor = 1.f / (float)(e - s);
-    lin = sl * factor;
-    ang = sa * factor;
-}
-
 __device__ __forceinline__ void add4(float4& a, float3 v, float w = 0.f) {
     a.x += v.x; a.y += v.y; a.z += v.z; a.w += w;
 }
 
 __device__ void reverse_phase(const SolverView& V, const b3::JacobiTape& T, const AdjView& A, int m, int p,
                               int phases) {
-    const float4 h0 = R(V, 0, m);
-    const int nRows = __float_as_int(h0.z);
-    const int bA = __float_as_int(h0.x), bB = __float_as_int(h0.y);
-    const int dyn = __float_as_int(h0.w);
+    const float4 ids = R(V, kIds, m), hd0 = R(V, kHead0, m), hd1 = R(V, kHead1, m);
+    const int bA = __float_as_int(ids.x), bB = __float_as_int(ids.y);
+    const uint32_t sA = __float_as_uint(hd0.x), eA = __float_as_uint(hd0.y), pA = __float_as_uint(hd0.z);
+    const uint32_t sB = __float_as_uint(hd0.w), eB = __float_as_uint(hd1.x), pB = __float_as_uint(hd1.y);
+    const int nRows = __float_as_int(hd1.z) & 0xffff, dyn = __float_as_int(hd1.z) >> 16;
+    const float mu = hd1.w;
     const bool friction = (p & 1) != 0;
     const bool last = p == phases - 1;
     // adjoint of this phase's copy outputs
     float3 gvA = make_float3(0.f, 0.f, 0.f), gwA = gvA, gvB = gvA, gwB = gvA;
     if (dyn & 1) {
         if (last) { gvA = f3(A.gDv[bA]); gwA = f3(A.gDw[bA]); }
-        else adj_average(V, A.gInLin, A.gInAng, bA, (p + 1) & 1, gvA, gwA);
+        else copy_average<4>(A.gIn + (size_t)((p + 1) & 1) * 4 * V.cap, sA, eA, gvA, gwA);
     }
     if (dyn & 2) {
         if (last) { gvB = f3(A.gDv[bB]); gwB = f3(A.gDw[bB]); }
-        else adj_average(V, A.gInLin, A.gInAng, bB, (p + 1) & 1, gvB, gwB);
+        else copy_average<4>(A.gIn + (size_t)((p + 1) & 1) * 4 * V.cap, sB, eB, gvB, gwB);
     }
     const size_t cap = (size_t)V.cap;
     float4 gLam0 = last ? make_float4(0.f, 0.f, 0.f, 0.f) : A.gLam[m];
@@ -259,20 +253,18 @@ __device__ void reverse_phase(const SolverView& V, const b3::JacobiTape& T, cons
     float4 gLam2 = last ? make_float4(0.f, 0.f, 0.f, 0.f) : A.gLam[2 * cap + m];
     if (last) {
         // first touch of this manifold in this step's reverse sweep
-        for (int s = 0; s < kRowSlots; ++s) A.rowAdj[(size_t)s * cap + m] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s = 0; s < kAdjSlots; ++s) A.rowAdj[(size_t)s * cap + m] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (nRows > 0) {
-        const float4 h1 = R(V, 1, m), h2 = R(V, 2, m), h3 = R(V, 3, m);
-        const float imA = h1.x, imB = h1.y, mu = h1.z;
-        const float3 iiA = f3(h2), iiB = f3(h3);
+        const float4 ia = R(V, kInA, m), ib = R(V, kInB, m);
+        const float imA = R(V, kNorm, m).w, imB = ia.w;
+        const float3 iiA = f3(ia), iiB = f3(ib);
         // inputs of the phase
         float3 dvA = make_float3(0.f, 0.f, 0.f), dwA = dvA, dvB = dvA, dwB = dvA;
         if (p > 0) {
-            SolverView Vt = V;
-            Vt.copyLin = T.copyLin;
-            Vt.copyAng = T.copyAng;
-            if (dyn & 1) body_average(Vt, bA, p - 1, dvA, dwA);
-            if (dyn & 2) body_average(Vt, bB, p - 1, dvB, dwB);
+            const float4* tape = T.copies + (size_t)(p - 1) * 4 * cap;
+            if (dyn & 1) copy_average<4>(tape, sA, eA, dvA, dwA);
+            if (dyn & 2) copy_average<4>(tape, sB, eB, dvB, dwB);
         }
         const int it = p >> 1;
         float lam[8], lamN[4] = {0.f, 0.f, 0.f, 0.f};
@@ -300,10 +292,9 @@ __device__ void reverse_phase(const SolverView& V, const b3::JacobiTape& T, cons
                 hi = mu * lamN[j];
                 lo = -hi;
             }
-            const int s = friction ? kFric0 + 3 * r : kNormal0 + 3 * r;
-            const float4 r0 = R(V, s, m), r1 = R(V, s + 1, m), r2 = R(V, s + 2, m);
-            const float3 n = f3(r0), t1 = f3(r1), t2 = f3(r2);
-            const float rhs = r0.w, jac = r1.w;
+            const RowData row = load_row(V, m, friction, r);
+            const float3 n = row.n, t1 = row.t1, t2 = row.t2;
+            const float rhs = row.rhs, jac = row.jac;
             const float dv1 = dot(n, dvA) + dot(t1, dwA);
             const float dv2 = -dot(n, dvB) + dot(t2, dwB);
             jdv[r] = dv1 + dv2;
@@ -337,9 +328,9 @@ __device__ void reverse_phase(const SolverView& V, const b3::JacobiTape& T, cons
             if (st[r] < 0) continue;
             const int j = friction ? (r >> 1) : r;
             const int s = friction ? kFric0 + 3 * r : kNormal0 + 3 * r;
-            const float4 r0 = R(V, s, m), r1 = R(V, s + 1, m), r2 = R(V, s + 2, m);
-            const float3 n = f3(r0), t1 = f3(r1), t2 = f3(r2);
-            const float jac = r1.w;
+            const RowData row = load_row(V, m, friction, r);
+            const float3 n = row.n, t1 = row.t1, t2 = row.t2;
+            const float jac = row.jac;
             const float d = dpr[r];
             const float3 ktA = mulv(iiA, t1), ktB = mulv(iiB, t2);
             // inputs of this row (step back through its update)
@@ -400,20 +391,20 @@ __device__ void reverse_phase(const SolverView& V, const b3::JacobiTape& T, cons
     A.gLam[2 * cap + m] = gLam2;
     // adjoint of the phase inputs (the averages read at its start)
     if (p > 0) {
-        const size_t a0 = (size_t)((p & 1) * 2 + 0) * cap + m, a1 = (size_t)((p & 1) * 2 + 1) * cap + m;
-        if (dyn & 1) { A.gInLin[a0] = f4(gvA); A.gInAng[a0] = f4(gwA); }
-        if (dyn & 2) { A.gInLin[a1] = f4(gvB); A.gInAng[a1] = f4(gwB); }
+        float4* g = A.gIn + (size_t)(p & 1) * 4 * cap;
+        if (dyn & 1) { g[2 * (size_t)pA] = f4(gvA); g[2 * (size_t)pA + 1] = f4(gwA); }
+        if (dyn & 2) { g[2 * (size_t)pB] = f4(gvB); g[2 * (size_t)pB + 1] = f4(gwB); }
     }
 }
 
 __global__ void __launch_bounds__(256)
 k_jacobi_adjoint(SolverView V, b3::JacobiTape T, AdjView A, int iterations, uint32_t* bar, int32_t* err,
                  b3Counters* counters) {
+    GridBarrier barrier(bar, err, counters, b3dev::kSpinLimit);
     const int M = *V.numManifolds;
-    const uint32_t nb = gridDim.x;
     const int phases = 2 * iterations;
     for (int p = phases - 1; p >= 0; --p) {
-        if (p < phases - 1 && !grid_barrier(bar, bar + 1, nb, err, counters)) return;
+        if (p < phases - 1 && !barrier.wait()) return;
         for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x)
             reverse_phase(V, T, A, m, p, phases);
     }
@@ -802,11 +793,10 @@ k_adj_manifold(SolverView V, AdjView A, ManifoldArgs MA, StepParams P) {
     const int M = *V.numManifolds;
     const size_t cap = (size_t)V.cap;
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
-        const float4 h0 = R(V, 0, m);
-        const int bA = __float_as_int(h0.x), bB = __float_as_int(h0.y);
-        const int dyn = __float_as_int(h0.w);
-        const float4 h1 = R(V, 1, m), h2 = R(V, 2, m), h3 = R(V, 3, m);
-        const float kA = h2.w, kB = h3.w;
+        const float4 ids = R(V, kIds, m), nn = R(V, kNorm, m), ia = R(V, kInA, m), ib = R(V, kInB, m);
+        const int bA = __float_as_int(ids.x), bB = __float_as_int(ids.y);
+        const int dyn = __float_as_int(R(V, kHead1, m).z) >> 16;
+        const float kA = ids.z, kB = ids.w;
         const b3Contact4 c = MA.contacts[MA.manifoldPair[m]];
         const int npts = (int)c.worldNormal[3];
         const bool dynA = dyn & 1, dynB = dyn & 2;
@@ -818,8 +808,8 @@ k_adj_manifold(SolverView V, AdjView A, ManifoldArgs MA, StepParams P) {
         const float3 wA = dynA ? f3(MA.angVel[bA]) : make_float3(0.f, 0.f, 0.f);
         const float3 vB = dynB ? f3(MA.linVel[bB]) + g : make_float3(0.f, 0.f, 0.f);
         const float3 wB = dynB ? f3(MA.angVel[bB]) : make_float3(0.f, 0.f, 0.f);
-        const float3 iiA = f3(h2), iiB = f3(h3);
-        const float imA = h1.x, imB = h1.y;
+        const float3 iiA = f3(ia), iiB = f3(ib);
+        const float imA = nn.w, imB = ia.w;
         const float3 n0 = normalize(make_float3(-c.worldNormal[0], -c.worldNormal[1], -c.worldNormal[2]));
         float3 p0[4];
         float dep0[4];
@@ -921,7 +911,7 @@ k_adj_manifold(SolverView V, AdjView A, ManifoldArgs MA, StepParams P) {
         // --- per-copy contributions --------------------------------------
         for (int side = 0; side < 2; ++side) {
             if (!(dyn & (1 << side))) continue;
-            const size_t slot = (size_t)(2 * m + side);
+            const size_t slot = V.incPos[2 * m + side];
             const size_t stride = 2 * cap;
             float4* C = A.contrib;
             if (side == 0) {
@@ -951,7 +941,7 @@ __global__ void k_adj_gather(int n, const float* __restrict__ invMass, const flo
     float4 sx = make_float4(0.f, 0.f, 0.f, 0.f), sth = sx, sv = sx, sw = sx, sii = sx;
     const size_t stride = 2 * (size_t)V.cap;
     for (uint32_t k = s; k < e; ++k) {
-        const uint32_t slot = V.incVals[k];
+        const size_t slot = k;
         const float4 a = A.contrib[slot], b = A.contrib[stride + slot], c = A.contrib[2 * stride + slot];
         const float4 d = A.contrib[3 * stride + slot], f = A.contrib[4 * stride + slot];
         sx.x += a.x; sx.y += a.y; sx.z += a.z; sx.w += a.w;
@@ -985,7 +975,7 @@ struct b3Adjoint_t {
     b3::JacobiTape tape{};
     float4 *gX = nullptr, *gTh = nullptr, *gV = nullptr, *gW = nullptr, *gDv = nullptr, *gDw = nullptr;
     float *gInvMass = nullptr, *gMu = nullptr;
-    float4 *rowAdj = nullptr, *gInLin = nullptr, *gInAng = nullptr, *gLam = nullptr, *contrib = nullptr;
+    float4 *rowAdj = nullptr, *gIn = nullptr, *gLam = nullptr, *contrib = nullptr;
     float4* seedQ = nullptr;
     int* unclassified = nullptr;
     bool forwardDone = false, backwardDone = false;
@@ -1019,7 +1009,7 @@ AdjView adj_view(b3Adjoint_t* a) {
     A.gX = a->gX; A.gTh = a->gTh; A.gV = a->gV; A.gW = a->gW;
     A.gDv = a->gDv; A.gDw = a->gDw;
     A.gInvMass = a->gInvMass; A.gMu = a->gMu;
-    A.rowAdj = a->rowAdj; A.gInLin = a->gInLin; A.gInAng = a->gInAng; A.gLam = a->gLam;
+    A.rowAdj = a->rowAdj; A.gIn = a->gIn; A.gLam = a->gLam;
     A.contrib = a->contrib;
     A.cap = a->cap;
     return A;
@@ -1128,7 +1118,7 @@ extern "C" int b3_adjoint_create(b3World w, int numSteps, int checkpointEvery, b
     {
         const size_t f4 = sizeof(float4);
         const size_t need = f4 * ((size_t)a->numCkpt * 4 * N + (size_t)a->K * 4 * N + phases * 4 * cap +
-                                  (size_t)a->iterations * 3 * cap + 7 * N + (size_t)kRowSlots * cap + 8 * cap +
+                                  (size_t)a->iterations * 3 * cap + 7 * N + (size_t)kAdjSlots * cap + 8 * cap +
                                   3 * cap + (size_t)kContrib * 2 * cap) +
                             2 * sizeof(float) * N;
         size_t freeB = 0, totalB = 0;
@@ -1146,8 +1136,7 @@ extern "C" int b3_adjoint_create(b3World w, int numSteps, int checkpointEvery, b
     if ((rc = aalloc(a, a->ckpt, (size_t)a->numCkpt * 4 * N)) != B3_OK) return fail(rc);
     if ((rc = aalloc(a, a->seg, (size_t)a->K * 4 * N)) != B3_OK) return fail(rc);
     if (phases > 0) {
-        if ((rc = aalloc(a, a->tape.copyLin, phases * 2 * cap)) != B3_OK) return fail(rc);
-        if ((rc = aalloc(a, a->tape.copyAng, phases * 2 * cap)) != B3_OK) return fail(rc);
+        if ((rc = aalloc(a, a->tape.copies, phases * 4 * cap)) != B3_OK) return fail(rc);
         if ((rc = aalloc(a, a->tape.lamN, (size_t)a->iterations * cap)) != B3_OK) return fail(rc);
         if ((rc = aalloc(a, a->tape.lamF, (size_t)a->iterations * 2 * cap)) != B3_OK) return fail(rc);
     }
@@ -1156,9 +1145,8 @@ extern "C" int b3_adjoint_create(b3World w, int numSteps, int checkpointEvery, b
         if ((rc = aalloc(a, *p, N)) != B3_OK) return fail(rc);
     if ((rc = aalloc(a, a->gInvMass, N)) != B3_OK) return fail(rc);
     if ((rc = aalloc(a, a->gMu, N)) != B3_OK) return fail(rc);
-    if ((rc = aalloc(a, a->rowAdj, (size_t)kRowSlots * cap)) != B3_OK) return fail(rc);
-    if ((rc = aalloc(a, a->gInLin, 4 * cap)) != B3_OK) return fail(rc);
-    if ((rc = aalloc(a, a->gInAng, 4 * cap)) != B3_OK) return fail(rc);
+    if ((rc = aalloc(a, a->rowAdj, (size_t)kAdjSlots * cap)) != B3_OK) return fail(rc);
+    if ((rc = aalloc(a, a->gIn, 8 * cap)) != B3_OK) return fail(rc);
     if ((rc = aalloc(a, a->gLam, 3 * cap)) != B3_OK) return fail(rc);
     if ((rc = aalloc(a, a->contrib, (size_t)kContrib * 2 * cap)) != B3_OK) return fail(rc);
     if ((rc = aalloc(a, a->unclassified, 1)) != B3_OK) return fail(rc);

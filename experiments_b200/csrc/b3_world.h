@@ -111,9 +111,8 @@ struct DevBuffers {
     uint32_t *incKeys = nullptr, *incVals = nullptr, *incKeysAlt = nullptr, *incValsAlt = nullptr;
     uint32_t *bodyIncStart = nullptr, *bodyIncEnd = nullptr;
     float4* rows = nullptr;           // constraint rows, see solver.cu
-    float4* manifoldHdr = nullptr;    // per manifold header
-    float4 *incLin = nullptr, *incAng = nullptr;   // per manifold side increments
-    float4 *avgLin = nullptr, *avgAng = nullptr;   // per body averaged delta velocity
+    uint32_t* incPos = nullptr;       // manifold side -> its copy in the body-sorted copy list
+    float4* copies = nullptr;         // solver-body copies, [2 buffers][2 sides][capacity][linear, angular]
     // scalars (device): [0] numSmall, [1] numPairs, [2] numManifolds, [3] numInc,
     // [4] stamp, [5] sort error flag, [6..7] barrier, [8] tile counter
     int32_t* scalars = nullptr;
@@ -229,10 +228,11 @@ struct b3World_t {
     int solverOccCap = 4;      // Jacobi persistent blocks per SM (at most)
     int solverMode = 0;        // Jacobi: 0 = grid barriers, 1 = one block per world (batched);
                                // batched Gauss-Seidel: grid width 0 = manifolds / 8, 1 = manifolds / 64
-    int solverGather = 0;      // Jacobi body averages: 0 = one copy at a time, 1 = four loads in flight
+    int solverGather = 0;      // Jacobi body averages: 0 = gathered by every manifold, 1 = a pass over the bodies
     int pairSearchMode = 0;    // grid pair search: 0 = thread per body, 1 = warp per body
     int clipGroups = 1;        // clip and float-float stages: 0 = a warp per pair, 1 = 8-lane groups
                                // (a warp per pair for what does not fit)
+    bool tuned = false;        // launch shapes set by the autotuner or by b3_set_tuning
     int tunedTrials = 0;       // configurations the autotuner timed
     int npSmemAttr = 0;        // dynamic shared memory attribute set on the narrowphase kernels
     int npGroupSmemAttr = 0;   // the same for the lane-group clip
@@ -244,6 +244,7 @@ struct b3World_t {
     int waitSpinLimit = b3::kDefaultSpinLimit;
     int waitHoldMicros = 0;
 
+    void defaultShapes();      // launch shapes by the number of bodies, until they are tuned
     b3::BodiesDev bodiesDev() const;
     b3::ShapesDev shapesDev() const;
 };
@@ -252,13 +253,13 @@ namespace b3 {
 // slots of the narrowphase candidate store (pairs queued for float-float
 // axis ranking beyond this recompute their FP32 sweep)
 constexpr int kNpCandSlots = 1 << 20;
+constexpr int kSolverRowSlots = 27;  // float4 streams of a manifold's constraint rows (solver_common.cuh)
 constexpr int kGsMaxBatch = 1024;  // batches per parity class (batched Gauss-Seidel)
 
 // Record of one Jacobi solve for the reverse sweep: every phase's solver-body
-// copies (both sides of every manifold) and the row impulses after it.
+// copies (dynamic sides) and the row impulses after it.
 struct JacobiTape {
-    float4* copyLin;   // [2 * iterations][2 sides][maxPairs]
-    float4* copyAng;
+    float4* copies;    // [2 * iterations][2 maxPairs][linear, angular], sorted by body
     float4* lamN;      // [iterations][maxPairs]: normal rows 0..3 after each normal phase
     float4* lamF;      // [iterations][2][maxPairs]: friction rows 0..7 after each friction phase
 };

@@ -38,7 +38,7 @@
 #include "solver_common.cuh"
 
 using namespace b3m;
-using b3solver::grid_barrier;
+using b3solver::GridBarrier;
 
 namespace {
 
@@ -107,12 +107,11 @@ __global__ void __launch_bounds__(256) k_gs_colour(ColourView V) {
     const int N = V.numBodies;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int stride = gridDim.x * blockDim.x;
-    uint32_t* cnt = V.bar;
-    uint32_t* gen = V.bar + 1;
+    GridBarrier barrier(V.bar, V.err, V.counters, b3dev::kSpinLimit);
     for (int s = tid; s < M; s += stride) V.slotBatch[s] = -1;
     if (tid < 4) V.batchCount[tid] = 0;
     if (tid < 5) V.roundCount[tid] = 0;
-    if (!grid_barrier(cnt, gen, gridDim.x, V.err, V.counters)) return;
+    if (!barrier.wait()) return;
     int round = 0;
     for (int batch = 0;; ++batch) {
         if (batch >= V.maxBatch) {
@@ -129,7 +128,7 @@ __global__ void __launch_bounds__(256) k_gs_colour(ColourView V) {
                 if (a >= 0) atomicMin(&V.minRank[cls * N + a], s);
                 if (b >= 0) atomicMin(&V.minRank[cls * N + b], s);
             }
-            if (!grid_barrier(cnt, gen, gridDim.x, V.err, V.counters)) return;
+            if (!barrier.wait()) return;
             // B: join where first on every dynamic body
             for (int s = tid; s < M; s += stride) {
                 if (__ldcg(&V.slotBatch[s]) != -1) continue;
@@ -142,7 +141,7 @@ __global__ void __launch_bounds__(256) k_gs_colour(ColourView V) {
                     atomicMax(&V.batchCount[cls], batch + 1);
                 }
             }
-            if (!grid_barrier(cnt, gen, gridDim.x, V.err, V.counters)) return;
+            if (!barrier.wait()) return;
             // C: wait when a body was taken; clear the ranks; count the rest
             int undecided = 0;
             for (int s = tid; s < M; s += stride) {
@@ -161,7 +160,7 @@ __global__ void __launch_bounds__(256) k_gs_colour(ColourView V) {
                 }
             }
             if (undecided) atomicAdd(&V.roundCount[round % 3], undecided);
-            if (!grid_barrier(cnt, gen, gridDim.x, V.err, V.counters)) return;
+            if (!barrier.wait()) return;
             if (__ldcg(&V.roundCount[round % 3]) == 0) {
                 ++round;
                 break;
@@ -176,7 +175,7 @@ __global__ void __launch_bounds__(256) k_gs_colour(ColourView V) {
                 ++waiting;
             }
         if (waiting) atomicAdd(&V.roundCount[3 + (batch & 1)], waiting);
-        if (!grid_barrier(cnt, gen, gridDim.x, V.err, V.counters)) return;
+        if (!barrier.wait()) return;
         if (__ldcg(&V.roundCount[3 + (batch & 1)]) == 0) return;
     }
 }
@@ -497,6 +496,7 @@ __device__ __forceinline__ int group_of(int j, const int nb[4], int maxBatch) {
 }
 
 __global__ void __launch_bounds__(256) k_gs_solve(SolveView V) {
+    GridBarrier barrier(V.bar, V.err, V.counters, b3dev::kSpinLimit);
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int stride = gridDim.x * blockDim.x;
     int nb[4];
@@ -525,7 +525,7 @@ __global__ void __launch_bounds__(256) k_gs_solve(SolveView V) {
             q1 = (int)V.groupOffset[g + 1];
             fetch(V, q0 + tid < q1 ? q0 + tid : -1, P);
         }
-        if (!grid_barrier(V.bar, V.bar + 1, gridDim.x, V.err, V.counters)) return;
+        if (!barrier.wait()) return;
     }
 }
 

@@ -78,11 +78,15 @@ __global__ void k_manifold_emit(const uint32_t* __restrict__ flag, const uint32_
     if (pts) atomicAdd(&counters->numContactPoints, pts);
 }
 
-__global__ void k_body_ranges(const uint32_t* __restrict__ keys, const int32_t* __restrict__ nDev,
-                              uint32_t* __restrict__ start, uint32_t* __restrict__ end, int numBodies) {
+// Ranges of the sorted copy list per body, and where each manifold's copies
+// lie in it (a static side's place is past every body's range).
+__global__ void k_body_ranges(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
+                              const int32_t* __restrict__ nDev, uint32_t* __restrict__ start,
+                              uint32_t* __restrict__ end, uint32_t* __restrict__ incPos, int numBodies) {
     const int n = *nDev;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t k = keys[i];
+        incPos[vals[i]] = (uint32_t)i;
         if (k >= (uint32_t)numBodies) continue;
         if (i == 0 || keys[i - 1] != k) start[k] = (uint32_t)i;
         if (i == n - 1 || keys[i + 1] != k) end[k] = (uint32_t)(i + 1);
@@ -99,10 +103,10 @@ struct SetupParams {
     float slopOffset;
 };
 
-__device__ __forceinline__ void setup_friction_row(const SolverView& V, int slot, int m, float3 dir,
-                                                   float3 r1, float3 r2, float imA, float imB,
-                                                   float3 iiA, float3 iiB, float cA, float cB,
-                                                   float3 vA, float3 wA, float3 vB, float3 wB) {
+// Friction row along dir: (dir, rhs) to its stream, 1/diag returned.
+__device__ __forceinline__ float setup_friction_row(const SolverView& V, int slot, int m, float3 dir, float3 r1,
+                                                    float3 r2, float imA, float imB, float3 iiA, float3 iiB,
+                                                    float cA, float cB, float3 vA, float3 wA, float3 vB, float3 wB) {
     const float3 t1 = cross(r1, dir);
     const float3 t2 = cross(r2, -dir);
     const float3 angA = mulv(iiA, t1);
@@ -113,9 +117,8 @@ __device__ __forceinline__ void setup_friction_row(const SolverView& V, int slot
     const float scaled = 1.f / (d0 * cA + d1 * cB);
     const float relv = (dot(dir, vA) + dot(t1, wA)) + (-dot(dir, vB) + dot(t2, wB));
     const float rhs = (0.f - relv) * scaled;
-    R(V, slot + 0, m) = make_float4(dir.x, dir.y, dir.z, rhs);
-    R(V, slot + 1, m) = make_float4(t1.x, t1.y, t1.z, denom);
-    R(V, slot + 2, m) = make_float4(t2.x, t2.y, t2.z, 0.f);
+    R(V, slot, m) = make_float4(dir.x, dir.y, dir.z, rhs);
+    return denom;
 }
 
 __global__ void k_setup_rows(b3::BodiesDev Bd, SolverView V, const int* __restrict__ manifoldPair,
@@ -126,8 +129,10 @@ __global__ void k_setup_rows(b3::BodiesDev Bd, SolverView V, const int* __restri
         const int A = abs(c.bodyAPtrAndSignBit), B = abs(c.bodyBPtrAndSignBit);
         const float imA = Bd.invMass[A], imB = Bd.invMass[B];
         const bool dynA = imA != 0.f, dynB = imB != 0.f;
-        const float kA = dynA ? (float)(V.incEnd[A] - V.incStart[A]) : 1.f;
-        const float kB = dynB ? (float)(V.incEnd[B] - V.incStart[B]) : 1.f;
+        const uint32_t sA = dynA ? V.incStart[A] : 0u, eA = dynA ? V.incEnd[A] : 0u;
+        const uint32_t sB = dynB ? V.incStart[B] : 0u, eB = dynB ? V.incEnd[B] : 0u;
+        const float kA = dynA ? (float)(eA - sA) : 1.f;
+        const float kB = dynB ? (float)(eB - sB) : 1.f;
         const float3 iiA = dynA ? f3(Bd.invInertia[A]) : make_float3(0.f, 0.f, 0.f);
         const float3 iiB = dynB ? f3(Bd.invInertia[B]) : make_float3(0.f, 0.f, 0.f);
         const float3 pA = f3(Bd.pos[A]), pB = f3(Bd.pos[B]);
@@ -139,6 +144,7 @@ __global__ void k_setup_rows(b3::BodiesDev Bd, SolverView V, const int* __restri
         const float restitution = Bd.restitution[A] * Bd.restitution[B];
         const float mu = c.friction;
         int nRows = 0;
+        float fjac[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         const int npts = (int)c.worldNormal[3];
         const bool solve = dynA || dynB;
         float3 n = normalize(make_float3(-c.worldNormal[0], -c.worldNormal[1], -c.worldNormal[2]));
@@ -176,10 +182,9 @@ __global__ void k_setup_rows(b3::BodiesDev Bd, SolverView V, const int* __restri
                 posErr = -penetration * SP.erp / SP.dt;
             }
             const float rhs = posErr * scaled + velErr * scaled;
-            const int s = kNormal0 + 3 * nRows;
-            R(V, s + 0, m) = make_float4(n.x, n.y, n.z, rhs);
-            R(V, s + 1, m) = make_float4(t0.x, t0.y, t0.z, denom);
-            R(V, s + 2, m) = make_float4(-t1.x, -t1.y, -t1.z, 0.f);
+            const int s = kPoint0 + 4 * nRows;
+            R(V, s + 0, m) = make_float4(r1.x, r1.y, r1.z, rhs);
+            R(V, s + 1, m) = make_float4(r2.x, r2.y, r2.z, denom);
             // friction directions (convertContact :1015-1049)
             float3 d1v = vel - n * relv0;
             const float lat = dot(d1v, d1v);
@@ -190,149 +195,256 @@ __global__ void k_setup_rows(b3::BodiesDev Bd, SolverView V, const int* __restri
             } else {
                 plane_space(n, d1v, d2v);
             }
-            const int fs = kFric0 + 3 * (2 * nRows);
-            setup_friction_row(V, fs, m, d2v, r1, r2, imA, imB, iiA, iiB, kA, kB, vA, wA, vB, wB);
-            setup_friction_row(V, fs + 3, m, d1v, r1, r2, imA, imB, iiA, iiB, kA, kB, vA, wA, vB, wB);
+            const float q2 = setup_friction_row(V, s + 2, m, d2v, r1, r2, imA, imB, iiA, iiB, kA, kB, vA, wA, vB, wB);
+            const float q1 = setup_friction_row(V, s + 3, m, d1v, r1, r2, imA, imB, iiA, iiB, kA, kB, vA, wA, vB, wB);
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (q == nRows) {
+                    fjac[2 * q] = q2;
+                    fjac[2 * q + 1] = q1;
+                }
             ++nRows;
         }
-        R(V, 0, m) = make_float4(__int_as_float(A), __int_as_float(B), __int_as_float(nRows),
-                                 __int_as_float((dynA ? 1 : 0) | (dynB ? 2 : 0)));
-        R(V, 1, m) = make_float4(imA, imB, mu, 0.f);
-        R(V, 2, m) = make_float4(iiA.x, iiA.y, iiA.z, kA);
-        R(V, 3, m) = make_float4(iiB.x, iiB.y, iiB.z, kB);
+        const int dyn = (dynA ? 1 : 0) | (dynB ? 2 : 0);
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        R(V, kHead0, m) = make_float4(__uint_as_float(sA), __uint_as_float(eA), __uint_as_float(V.incPos[2 * m]),
+                                      __uint_as_float(sB));
+        R(V, kHead1, m) = make_float4(__uint_as_float(eB), __uint_as_float(V.incPos[2 * m + 1]),
+                                      __int_as_float(nRows | dyn << 16), mu);
+        R(V, kNorm, m) = f4(n, imA);
+        R(V, kInA, m) = f4(iiA, imB);
+        R(V, kInB, m) = f4(iiB);
+        R(V, kIds, m) = make_float4(__int_as_float(A), __int_as_float(B), kA, kB);
+        R(V, kFJac, m) = make_float4(fjac[0], fjac[1], fjac[2], fjac[3]);
+        R(V, kFJac + 1, m) = make_float4(fjac[4], fjac[5], fjac[6], fjac[7]);
+        R(V, kLamN, m) = zero;
+        R(V, kLamF, m) = zero;
+        R(V, kLamF + 1, m) = zero;
     }
 }
 
 // ---------------------------------------------------------------------------
-// Persistent Jacobi kernel
+// Persistent Jacobi kernels
 // ---------------------------------------------------------------------------
-constexpr int kJacobiHeads = 4;         // manifolds per thread whose headers stay in shared memory
-constexpr int kJacobiMaxThreads = 256;  // k_jacobi's largest CTA
-
-// What a manifold's solve reads that no phase changes: its header (bodies,
-// row count, dynamic flags) and its bodies' incidence ranges.
-struct MHead {
-    int A, B, nRows, dyn;
-    uint32_t sA, eA, sB, eB;
+// Streams of one manifold: in global memory (slot major, stride cap) or in
+// the block's shared memory (slot major, stride blockDim), where a thread
+// keeps the manifolds that it solves in every phase.
+struct GlobalRows {
+    float4* at;
+    size_t stride;
+    __device__ __forceinline__ float4& operator()(int slot) const { return at[(size_t)slot * stride]; }
 };
+struct SharedRows {
+    float4* at;
+    int stride;
+    __device__ __forceinline__ float4& operator()(int slot) const { return at[slot * stride]; }
+};
+// streams a phase reads or writes (all but kIds)
+constexpr int kPhaseSlots = kIds;
+static_assert(kIds == kRowSlots - 1, "the ids are the last stream");
 
-__device__ __forceinline__ void load_head(const SolverView& V, int m, MHead& H) {
-    const float4 h0 = R(V, 0, m);
-    H.nRows = __float_as_int(h0.z);
-    H.A = __float_as_int(h0.x);
-    H.B = __float_as_int(h0.y);
-    H.dyn = __float_as_int(h0.w);
-    H.sA = H.eA = H.sB = H.eB = 0u;
+struct Heads {
+    uint32_t sA, eA, pA, sB, eB, pB;
+    int nRows, dyn;
+    float mu;
+};
+template <class Rows>
+__device__ __forceinline__ Heads load_heads(const Rows& S) {
+    const float4 a = S(kHead0), b = S(kHead1);
+    const int f = __float_as_int(b.z);
+    return Heads{__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z), __float_as_uint(a.w),
+                 __float_as_uint(b.x), __float_as_uint(b.y), f & 0xffff, f >> 16, b.w};
+}
+
+// Both bodies' averages, the first K copies of each side in flight at once
+// (past a range's end the last record again, which the sum leaves out).
+template <int K>
+__device__ __forceinline__ void gather_averages(const float4* __restrict__ copies, const Heads& H, float3& vA,
+                                                float3& wA, float3& vB, float3& wB) {
+    float4 l[2][K], a[2][K];
+    const uint32_t s[2] = {H.sA, H.sB}, e[2] = {H.eA, H.eB};
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int u = 0; u < K; ++u) {
+            const float4* r = copies + 2 * (size_t)min(s[h] + u, max(e[h], 1u) - 1u);
+            l[h][u] = __ldcg(r);
+            a[h][u] = __ldcg(r + 1);
+        }
+    float3 sl[2], sa[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        sl[h] = sa[h] = make_float3(0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < K; ++u)
+            if (s[h] + u < e[h]) {
+                sl[h] += f3(l[h][u]);
+                sa[h] += f3(a[h][u]);
+            }
+        for (uint32_t i0 = s[h] + K; i0 < e[h]; i0 += K) {
+#pragma unroll
+            for (int u = 0; u < K; ++u) {
+                const float4* r = copies + 2 * (size_t)min(i0 + u, e[h] - 1u);
+                l[h][u] = __ldcg(r);
+                a[h][u] = __ldcg(r + 1);
+            }
+#pragma unroll
+            for (int u = 0; u < K; ++u)
+                if (i0 + u < e[h]) {
+                    sl[h] += f3(l[h][u]);
+                    sa[h] += f3(a[h][u]);
+                }
+        }
+    }
     if (H.dyn & 1) {
-        H.sA = V.incStart[H.A];
-        H.eA = V.incEnd[H.A];
+        const float f = 1.f / (float)(H.eA - H.sA);
+        vA = scaled(sl[0], f);
+        wA = scaled(sa[0], f);
     }
     if (H.dyn & 2) {
-        H.sB = V.incStart[H.B];
-        H.eB = V.incEnd[H.B];
+        const float f = 1.f / (float)(H.eB - H.sB);
+        vB = scaled(sl[1], f);
+        wB = scaled(sa[1], f);
     }
 }
 
-// One phase for one manifold: start each copy from its body's average of
-// the previous phase (zero in the first phase), solve the manifold's normal
-// or friction rows in order, store both copies in buffer outBuf. A copy of a
-// manifold without rows keeps the average, as in the reference.
-template <bool TAPE, bool GATHER4>
-__device__ __forceinline__ void solve_manifold_h(const SolverView& V, int m, const MHead& H, bool friction,
-                                                 bool first, int inBuf, int outBuf, const b3::JacobiTape& T,
-                                                 int phase) {
-    {
-        const int nRows = H.nRows;
-        const int dyn = H.dyn;
-        float3 dvA = make_float3(0.f, 0.f, 0.f), dwA = dvA, dvB = dvA, dwB = dvA;
-        if (!first) {
-            if (GATHER4) {
-                // the copies four at a time (same sums as body_average)
-                if (dyn & 1) body_average_range(V, H.sA, H.eA, inBuf, dvA, dwA);
-                if (dyn & 2) body_average_range(V, H.sB, H.eB, inBuf, dvB, dwB);
-            } else {
-                if (dyn & 1) body_average_se(V, H.sA, H.eA, inBuf, dvA, dwA);
-                if (dyn & 2) body_average_se(V, H.sB, H.eB, inBuf, dvB, dwB);
+// Both bodies' averages as the pass over the bodies left them, in the first
+// record of each body's range.
+__device__ __forceinline__ void read_averages(const float4* __restrict__ copies, const Heads& H, float3& vA, float3& wA,
+                                              float3& vB, float3& wB) {
+    if (H.dyn & 1) {
+        vA = f3(__ldcg(&copies[2 * (size_t)H.sA]));
+        wA = f3(__ldcg(&copies[2 * (size_t)H.sA + 1]));
+    }
+    if (H.dyn & 2) {
+        vB = f3(__ldcg(&copies[2 * (size_t)H.sB]));
+        wB = f3(__ldcg(&copies[2 * (size_t)H.sB + 1]));
+    }
+}
+
+// The normal rows of one manifold in order, from the copies' velocities at
+// the phase's start; the impulses go back to their stream.
+template <bool TAPE, class Rows>
+__device__ __forceinline__ void normal_rows(const Rows& S, int nRows, float3& dvA, float3& dwA, float3& dvB,
+                                            float3& dwB, float4* tape) {
+    const float4 nn = S(kNorm), ia = S(kInA), ib = S(kInB), l4 = S(kLamN);
+    float4 a[4], b[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {  // past the last point: that one again
+        const int k = kPoint0 + 4 * min(j, nRows - 1);
+        a[j] = S(k);
+        b[j] = S(k + 1);
+    }
+    float lam[4] = {l4.x, l4.y, l4.z, l4.w};
+    const float3 n = f3(nn);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (j < nRows)
+            solve_row(n, arm(f3(a[j]), n), arm_neg(f3(b[j]), n), a[j].w, b[j].w, lam[j], 0.f, 1e10f, nn.w, ia.w, f3(ia),
+                      f3(ib), dvA, dwA, dvB, dwB);
+    const float4 r = make_float4(lam[0], lam[1], lam[2], lam[3]);
+    S(kLamN) = r;
+    if (TAPE) *tape = r;
+}
+
+// The friction rows, two per point that carries a normal impulse. Points are
+// fetched one ahead of the one being solved.
+template <bool TAPE, class Rows>
+__device__ __forceinline__ void friction_rows(const Rows& S, int nRows, float mu, float3& dvA, float3& dwA,
+                                              float3& dvB, float3& dwB, float4* tape, size_t cap) {
+    const float4 n4 = S(kLamN), ia = S(kInA), ib = S(kInB);
+    const float imA = S(kNorm).w;
+    const float ln[4] = {n4.x, n4.y, n4.z, n4.w};
+    float4 l4[2] = {S(kLamF), S(kLamF + 1)};
+    const float4 q4[2] = {S(kFJac), S(kFJac + 1)};
+    float4 a, b, d2, d1;
+    auto fetch = [&](int j) {
+        const int k = kPoint0 + 4 * j;
+        a = S(k);
+        b = S(k + 1);
+        d2 = S(k + 2);
+        d1 = S(k + 3);
+    };
+    fetch(0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (j < nRows) {
+            const float4 ca = a, cb = b, c2 = d2, c1 = d1;
+            if (j < 3) fetch(min(j + 1, nRows - 1));
+            if (ln[j] > 0.f) {
+                const float lim = mu * ln[j];
+                const float3 r1 = f3(ca), r2 = f3(cb);
+                float& m2 = (j & 1) ? l4[j >> 1].z : l4[j >> 1].x;
+                float& m1 = (j & 1) ? l4[j >> 1].w : l4[j >> 1].y;
+                const float j2 = (j & 1) ? q4[j >> 1].z : q4[j >> 1].x, j1 = (j & 1) ? q4[j >> 1].w : q4[j >> 1].y;
+                solve_row(f3(c2), arm(r1, f3(c2)), arm_rev(r2, f3(c2)), c2.w, j2, m2, -lim, lim, imA, ia.w, f3(ia), f3(ib),
+                          dvA, dwA, dvB, dwB);
+                solve_row(f3(c1), arm(r1, f3(c1)), arm_rev(r2, f3(c1)), c1.w, j1, m1, -lim, lim, imA, ia.w, f3(ia), f3(ib),
+                          dvA, dwA, dvB, dwB);
             }
         }
-        float lam[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (nRows > 0) {
-            const float4 h1 = R(V, 1, m);
-            const float4 h2 = R(V, 2, m);
-            const float4 h3 = R(V, 3, m);
-            const float imA = h1.x, imB = h1.y, mu = h1.z;
-            const float3 iiA = f3(h2), iiB = f3(h3);
-            if (!friction) {
-                for (int j = 0; j < nRows; ++j) {
-                    const int s = kNormal0 + 3 * j;
-                    const float4 r0 = R(V, s, m), r1 = R(V, s + 1, m);
-                    float4 r2 = R(V, s + 2, m);
-                    solve_row(r0, r1, r2, 0.f, 1e10f, imA, imB, iiA, iiB, dvA, dwA, dvB, dwB);
-                    R(V, s + 2, m).w = r2.w;
-                    if (TAPE) lam[j] = r2.w;
-                }
-            } else {
-                for (int j = 0; j < nRows; ++j) {
-                    const float total = R(V, kNormal0 + 3 * j + 2, m).w;
-                    if (TAPE) {
-                        lam[2 * j] = R(V, kFric0 + 3 * (2 * j) + 2, m).w;
-                        lam[2 * j + 1] = R(V, kFric0 + 3 * (2 * j + 1) + 2, m).w;
-                    }
-                    if (!(total > 0.f)) continue;
-                    const float lim = mu * total;
-                    for (int q = 0; q < 2; ++q) {
-                        const int s = kFric0 + 3 * (2 * j + q);
-                        const float4 r0 = R(V, s, m), r1 = R(V, s + 1, m);
-                        float4 r2 = R(V, s + 2, m);
-                        solve_row(r0, r1, r2, -lim, lim, imA, imB, iiA, iiB, dvA, dwA, dvB, dwB);
-                        R(V, s + 2, m).w = r2.w;
-                        if (TAPE) lam[2 * j + q] = r2.w;
-                    }
-                }
-            }
-        }
-        if (dyn & 1) {
-            const size_t at = (size_t)(outBuf * 2 + 0) * V.cap + m;
-            V.copyLin[at] = f4(dvA);
-            V.copyAng[at] = f4(dwA);
-        }
-        if (dyn & 2) {
-            const size_t at = (size_t)(outBuf * 2 + 1) * V.cap + m;
-            V.copyLin[at] = f4(dvB);
-            V.copyAng[at] = f4(dwB);
-        }
+    }
+    S(kLamF) = l4[0];
+    S(kLamF + 1) = l4[1];
+    if (TAPE) {
+        tape[0] = l4[0];
+        tape[cap] = l4[1];
+    }
+}
+
+// One phase for one manifold: start each copy from its body's average of the
+// previous phase (zero in the first phase), solve the manifold's normal or
+// friction rows in order, store both copies in `out`. A copy of a manifold
+// without rows keeps the average, as in the reference. PASS: the averages were
+// formed by a pass over the bodies; otherwise each side gathers its body's
+// copies here.
+template <bool TAPE, bool PASS, class Rows>
+__device__ __forceinline__ void solve_manifold(const Rows& S, bool friction, bool first, const float4* __restrict__ in,
+                                               float4* __restrict__ out, int m, size_t cap, const b3::JacobiTape& T,
+                                               int phase) {
+    const Heads H = load_heads(S);
+    float3 dvA = make_float3(0.f, 0.f, 0.f), dwA = dvA, dvB = dvA, dwB = dvA;
+    if (!first) {
+        if (PASS) read_averages(in, H, dvA, dwA, dvB, dwB);
+        else gather_averages<4>(in, H, dvA, dwA, dvB, dwB);
+    }
+    float4* tn = TAPE ? T.lamN + (size_t)(phase >> 1) * cap + m : nullptr;
+    float4* tf = TAPE ? T.lamF + (size_t)(phase & ~1) * cap + m : nullptr;
+    if (H.nRows > 0) {
+        if (!friction) normal_rows<TAPE>(S, H.nRows, dvA, dwA, dvB, dwB, tn);
+        else friction_rows<TAPE>(S, H.nRows, H.mu, dvA, dwA, dvB, dwB, tf, cap);
+    } else if (TAPE) {
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!friction) *tn = zero;
+        else tf[0] = tf[cap] = zero;
+    }
+    float4* const tape = TAPE ? T.copies + (size_t)phase * 4 * cap : nullptr;
+    if (H.dyn & 1) {
+        __stcg(&out[2 * (size_t)H.pA], f4(dvA));
+        __stcg(&out[2 * (size_t)H.pA + 1], f4(dwA));
         if (TAPE) {
-            // every phase's copies and the impulses after it, for the
-            // reverse sweep (both sides, zero for a static side)
-            const size_t a0 = (size_t)(phase * 2 + 0) * V.cap + m, a1 = (size_t)(phase * 2 + 1) * V.cap + m;
-            T.copyLin[a0] = f4(dvA);
-            T.copyAng[a0] = f4(dwA);
-            T.copyLin[a1] = f4(dvB);
-            T.copyAng[a1] = f4(dwB);
-            const int it = phase >> 1;
-            if (!friction) {
-                T.lamN[(size_t)it * V.cap + m] = make_float4(lam[0], lam[1], lam[2], lam[3]);
-            } else {
-                T.lamF[(size_t)(2 * it) * V.cap + m] = make_float4(lam[0], lam[1], lam[2], lam[3]);
-                T.lamF[(size_t)(2 * it + 1) * V.cap + m] = make_float4(lam[4], lam[5], lam[6], lam[7]);
-            }
+            tape[2 * (size_t)H.pA] = f4(dvA);
+            tape[2 * (size_t)H.pA + 1] = f4(dwA);
+        }
+    }
+    if (H.dyn & 2) {
+        __stcg(&out[2 * (size_t)H.pB], f4(dvB));
+        __stcg(&out[2 * (size_t)H.pB + 1], f4(dwB));
+        if (TAPE) {
+            tape[2 * (size_t)H.pB] = f4(dvB);
+            tape[2 * (size_t)H.pB + 1] = f4(dwB);
         }
     }
 }
 
-template <bool TAPE, bool GATHER4>
-__device__ __forceinline__ void solve_manifold(const SolverView& V, int m, bool friction, bool first, int inBuf,
-                                               int outBuf, const b3::JacobiTape& T, int phase) {
-    MHead H;
-    load_head(V, m, H);
-    solve_manifold_h<TAPE, GATHER4>(V, m, H, friction, first, inBuf, outBuf, T, phase);
+__device__ __forceinline__ float4* copy_buffer(const SolverView& V, int buf) {
+    return V.copies + (size_t)buf * 4 * V.cap;
 }
 
-template <bool TAPE, bool GATHER4>
-__device__ void manifold_phase(const SolverView& V, int M, bool friction, bool first, int inBuf, int outBuf,
-                               const b3::JacobiTape& T, int phase) {
-    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x)
-        solve_manifold<TAPE, GATHER4>(V, m, friction, first, inBuf, outBuf, T, phase);
+// test of the give-up path: block 0 arrives late (bounded sleep)
+__device__ __forceinline__ void hold_back(const SolverView& V) {
+    if (V.holdMicros > 0 && blockIdx.x == 0 && threadIdx.x == 0)
+        for (int i = 0; i < V.holdMicros; ++i) __nanosleep(1000);
 }
 
 // Phases p = 0 .. 2*iterations-1 alternate normal (even) and friction (odd)
@@ -340,38 +452,81 @@ __device__ void manifold_phase(const SolverView& V, int M, bool friction, bool f
 // phase from the double-buffered copies, so phases are separated by one
 // bounded grid barrier each.
 //
-// GATHER4 (a tuning choice): each copy's body averages are gathered with
-// their loads issued four at a time. Shorter dependent-load chains per
-// phase, more registers per thread: the autotuner weighs the two.
-template <bool TAPE, bool GATHER4>
-__global__ void __launch_bounds__(256)
-k_jacobi(SolverView V, int iterations, uint32_t* bar, int32_t* err, b3Counters* counters, b3::JacobiTape T) {
+// k_jacobi, small scenes: what counts is the chain of a phase (barrier, copies,
+// rows, copies out). Each thread keeps the streams of its first `resident`
+// manifolds in shared memory for all phases, so between two barriers one round
+// of L2 reads is left, the copies of its bodies, which lie side by side.
+// 4,096 stacked cubes (10,550 manifolds): 219 -> 109 us for 20 phases; before,
+// rows were streamed in every phase and each copy was found through its id.
+template <bool TAPE>
+__global__ void __launch_bounds__(256, 1)
+k_jacobi(SolverView V, int iterations, int resident, uint32_t* bar, int32_t* err, b3Counters* counters,
+         b3::JacobiTape T) {
+    extern __shared__ float4 kept[];  // [resident][kPhaseSlots][blockDim]
+    GridBarrier barrier(bar, err, counters, V.spinLimit);
     const int M = *V.numManifolds;
-    const uint32_t nb = gridDim.x;
     const int phases = 2 * iterations;
     const int m0 = blockIdx.x * blockDim.x + threadIdx.x;
     const int stride = gridDim.x * blockDim.x;
-    // the headers and incidence ranges of this thread's first kJacobiHeads
-    // manifolds stay in shared memory for every phase: after each barrier
-    // only the copy ids and the copies remain to be loaded from L2
-    __shared__ MHead heads[kJacobiHeads][kJacobiMaxThreads];
-    for (int k = 0; k < kJacobiHeads; ++k)
-        if (m0 + k * stride < M) load_head(V, m0 + k * stride, heads[k][threadIdx.x]);
+    const int tb = (int)blockDim.x;
+    for (int k = 0; k < resident; ++k) {
+        const int m = m0 + k * stride;
+        if (m < M) {
+            float4* at = kept + (size_t)k * kPhaseSlots * tb + threadIdx.x;
+#pragma unroll
+            for (int s = 0; s < kPhaseSlots; ++s) at[s * tb] = R(V, s, m);
+        }
+    }
     for (int p = 0; p < phases; ++p) {
-        if (p == 1 && V.holdMicros > 0 && blockIdx.x == 0 && threadIdx.x == 0) {
-            // test of the give-up path: block 0 arrives late (bounded sleep)
-            for (int i = 0; i < V.holdMicros; ++i) __nanosleep(1000);
-        }
-        if (p > 0 && !grid_barrier(bar, bar + 1, nb, err, counters, V.spinLimit)) return;
+        if (p == 1) hold_back(V);
+        if (p > 0 && !barrier.wait()) return;
         const bool friction = (p & 1) != 0, first = p == 0;
-        const int inBuf = (p - 1) & 1, outBuf = p & 1;
-        int k = 0;
-        for (int m = m0; m < M; m += stride, ++k) {
-            MHead H;
-            if (k < kJacobiHeads) H = heads[k][threadIdx.x];
-            else load_head(V, m, H);
-            solve_manifold_h<TAPE, GATHER4>(V, m, H, friction, first, inBuf, outBuf, T, p);
+        const float4* in = copy_buffer(V, (p - 1) & 1);
+        float4* out = copy_buffer(V, p & 1);
+        int m = m0;
+        for (int k = 0; k < resident && m < M; ++k, m += stride)
+            solve_manifold<TAPE, false>(SharedRows{kept + (size_t)k * kPhaseSlots * tb + threadIdx.x, tb},
+                                                 friction, first, in, out, m, V.cap, T, p);
+        for (; m < M; m += stride)
+            solve_manifold<TAPE, false>(GlobalRows{V.rows + m, (size_t)V.cap}, friction, first, in, out, m,
+                                                 V.cap, T, p);
+    }
+}
+
+// k_jacobi_pass, large scenes: what counts is the bytes of a phase. A body's
+// copies are read once, by a pass over the bodies between two barriers that
+// leaves the average in the first record of the body's range, instead of once
+// per manifold of the body (at 5.4 copies a body, 64 B instead of 350 B of L2
+// reads per manifold and phase); the extra barrier is a few microseconds.
+// 1,048,576 cubes (2.85 M manifolds): 7.22 -> 5.58 ms, of which the streams
+// take 2.5 ms at 6.65 TB/s; 131,072 mixed bodies (395 K): 1.26 -> 0.90 ms.
+template <bool TAPE>
+__global__ void __launch_bounds__(256, 2)
+k_jacobi_pass(SolverView V, int iterations, uint32_t* bar, int32_t* err, b3Counters* counters, b3::JacobiTape T) {
+    GridBarrier barrier(bar, err, counters, V.spinLimit);
+    const int M = *V.numManifolds;
+    const int phases = 2 * iterations;
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int stride = gridDim.x * blockDim.x;
+    for (int p = 0; p < phases; ++p) {
+        if (p == 1) hold_back(V);
+        const float4* in = copy_buffer(V, (p - 1) & 1);
+        if (p > 0) {
+            if (!barrier.wait()) return;
+            float4* mean = copy_buffer(V, (p - 1) & 1);
+            for (int b = t0; b < V.numBodies; b += stride) {
+                const uint32_t s = V.incStart[b], e = V.incEnd[b];
+                if (e <= s + 1) continue;  // no copies, or its own average
+                float3 l, a;
+                copy_average<4>(in, s, e, l, a);
+                __stcg(&mean[2 * (size_t)s], f4(l));
+                __stcg(&mean[2 * (size_t)s + 1], f4(a));
+            }
+            if (!barrier.wait()) return;
         }
+        for (int m = t0; m < M; m += stride)
+            solve_manifold<TAPE, true>(GlobalRows{V.rows + m, (size_t)V.cap}, (p & 1) != 0, p == 0, in,
+                                                 copy_buffer(V, p & 1), m, V.cap, T, p);
     }
 }
 
@@ -388,13 +543,13 @@ __global__ void k_world_ranges(SolverView V, const int* __restrict__ worldId, in
                                int* __restrict__ end) {
     const int M = *V.numManifolds;
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
-        const int w = worldId[__float_as_int(R(V, 0, m).x)];
-        if (m == 0 || worldId[__float_as_int(R(V, 0, m - 1).x)] != w) atomicMin(&start[w], m);
-        if (m == M - 1 || worldId[__float_as_int(R(V, 0, m + 1).x)] != w) atomicMax(&end[w], m + 1);
+        const int w = worldId[__float_as_int(R(V, kIds, m).x)];
+        if (m == 0 || worldId[__float_as_int(R(V, kIds, m - 1).x)] != w) atomicMin(&start[w], m);
+        if (m == M - 1 || worldId[__float_as_int(R(V, kIds, m + 1).x)] != w) atomicMax(&end[w], m + 1);
     }
 }
 
-template <bool TAPE, bool GATHER4>
+template <bool TAPE>
 __global__ void __launch_bounds__(256)
 k_jacobi_worlds(SolverView V, int iterations, const int* __restrict__ start, const int* __restrict__ end,
                 int numWorlds, const int* __restrict__ worldId, b3::JacobiTape T) {
@@ -405,8 +560,10 @@ k_jacobi_worlds(SolverView V, int iterations, const int* __restrict__ start, con
         for (int p = 0; p < phases; ++p) {
             if (p > 0) __syncthreads();
             for (int m = s + (int)threadIdx.x; m < e; m += blockDim.x)
-                if (worldId[__float_as_int(R(V, 0, m).x)] == w)
-                    solve_manifold<TAPE, GATHER4>(V, m, (p & 1) != 0, p == 0, (p - 1) & 1, p & 1, T, p);
+                if (worldId[__float_as_int(R(V, kIds, m).x)] == w)
+                    solve_manifold<TAPE, false>(GlobalRows{V.rows + m, (size_t)V.cap}, (p & 1) != 0, p == 0,
+                                                          copy_buffer(V, (p - 1) & 1), copy_buffer(V, p & 1), m, V.cap,
+                                                          T, p);
         }
         __syncthreads();
     }
@@ -432,7 +589,7 @@ __global__ void k_integrate(b3::BodiesDev Bd, SolverView V, int finalBuf, Integr
     if (applySolve && V.incEnd[i] > V.incStart[i]) {
         const uint32_t k = V.incEnd[i] - V.incStart[i];
         float3 sl, sa;
-        body_average(V, i, finalBuf, sl, sa);
+        copy_average<4>(copy_buffer(V, finalBuf), V.incStart[i], V.incEnd[i], sl, sa);
         for (uint32_t c = 0; c < k; ++c) {
             v.x += sl.x; v.y += sl.y; v.z += sl.z;
             w.x += sa.x; w.y += sa.y; w.z += sa.z;
@@ -477,11 +634,8 @@ SolverView b3solver::solver_view(b3World_t* w) {
     SolverView V;
     V.rows = w->d.rows;
     V.cap = w->cfg.maxPairs;
-    V.copyLin = w->d.incLin;
-    V.copyAng = w->d.incAng;
-    V.avgLin = w->d.avgLin;
-    V.avgAng = w->d.avgAng;
-    V.incVals = w->d.incVals;
+    V.copies = w->d.copies;
+    V.incPos = w->d.incPos;
     V.incStart = w->d.bodyIncStart;
     V.incEnd = w->d.bodyIncEnd;
     V.numManifolds = w->d.scalars + b3::S_NUM_MANIFOLDS;
@@ -515,14 +669,8 @@ int launch_manifolds(b3World_t* w, cudaStream_t st) {
     B3_TRY(radix_sort_pairs(w->d.incKeys, w->d.incVals, w->d.incKeysAlt, w->d.incValsAlt,
                             w->d.scalars + S_NUM_INC, 2LL * cap, w->bodyBits, w->d.incSortScratch,
                             w->d.incSortScratchBytes, w->d.scalars + S_ERR, st, &alt, w->ctx->numSMs));
-    if (alt) {
-        B3_CUDA(cudaMemcpyAsync(w->d.incKeys, w->d.incKeysAlt, sizeof(uint32_t) * 2 * (size_t)cap,
-                                cudaMemcpyDeviceToDevice, st));
-        B3_CUDA(cudaMemcpyAsync(w->d.incVals, w->d.incValsAlt, sizeof(uint32_t) * 2 * (size_t)cap,
-                                cudaMemcpyDeviceToDevice, st));
-    }
-    k_body_ranges<<<g, 256, 0, st>>>(w->d.incKeys, w->d.scalars + S_NUM_INC, w->d.bodyIncStart,
-                                    w->d.bodyIncEnd, N);
+    k_body_ranges<<<g, 256, 0, st>>>(alt ? w->d.incKeysAlt : w->d.incKeys, alt ? w->d.incValsAlt : w->d.incVals,
+                                    w->d.scalars + S_NUM_INC, w->d.bodyIncStart, w->d.bodyIncEnd, w->d.incPos, N);
     B3_CHECK_LAUNCH();
     return B3_OK;
 }
@@ -556,10 +704,7 @@ int launch_solver_taped(b3World_t* w, cudaStream_t st, const JacobiTape* tape) {
         k_world_ranges<<<w->ctx->numSMs * 4, 256, 0, st>>>(V, w->d.worldId, w->d.worldMStart, w->d.worldMEnd);
         B3_CHECK_LAUNCH();
         const int threads = w->solverThreads;
-        // the taped forward keeps the plain gather (same results either way)
-        const void* kw = tape ? (const void*)k_jacobi_worlds<true, false>
-                              : (w->solverGather ? (const void*)k_jacobi_worlds<false, true>
-                                                 : (const void*)k_jacobi_worlds<false, false>);
+        const void* kw = tape ? (const void*)k_jacobi_worlds<true> : (const void*)k_jacobi_worlds<false>;
         int occ = 1;
         B3_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kw, threads, 0));
         occ = occ < 1 ? 1 : occ;
@@ -577,27 +722,43 @@ int launch_solver_taped(b3World_t* w, cudaStream_t st, const JacobiTape* tape) {
     // persistent cooperative Jacobi
     B3_CUDA(cudaMemsetAsync(w->d.scalars + S_BAR_COUNT, 0, sizeof(int32_t) * 2, st));
     const int threads = w->solverThreads;
-    int occ = 1;
-    const void* kern = tape ? (const void*)k_jacobi<true, false>
-                            : (w->solverGather ? (const void*)k_jacobi<false, true> : (const void*)k_jacobi<false, false>);
-    B3_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, 0));
-    occ = occ < 1 ? 1 : occ;
-    occ = occ > w->solverOccCap ? w->solverOccCap : occ;
     // size the persistent grid to the expected manifold count (about 3 per
     // body): fewer blocks make each grid barrier cheaper on small scenes
     const long long est = std::min<long long>((long long)w->cfg.maxPairs, 3LL * (long long)w->bodies.size());
     const int want = (int)std::max<long long>(1, (est + threads - 1) / threads);
+    const bool pass = w->solverGather == 1;
+    const void* kern = pass ? (tape ? (const void*)k_jacobi_pass<true> : (const void*)k_jacobi_pass<false>)
+                            : (tape ? (const void*)k_jacobi<true> : (const void*)k_jacobi<false>);
+    int occ = 1, resident = 0;
+    size_t smem = 0;
+    if (!pass) {
+        // shared memory for as many of a thread's manifolds as the scene is
+        // expected to have, up to one block's share of an SM
+        const size_t one = (size_t)kPhaseSlots * threads * sizeof(float4);
+        const int blocks = std::min(w->ctx->numSMs * w->solverOccCap, want);
+        const int perSm = (blocks + w->ctx->numSMs - 1) / w->ctx->numSMs;
+        const int need = (int)((est + (long long)blocks * threads - 1) / ((long long)blocks * threads));
+        resident = std::min(need, (int)((size_t)w->ctx->maxSmemOptin / perSm / one));
+        smem = one * resident;
+        if (smem > 48 * 1024)
+            B3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    }
+    B3_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem));
+    occ = occ < 1 ? 1 : occ;
+    occ = occ > w->solverOccCap ? w->solverOccCap : occ;
     const int grid = std::min(w->ctx->numSMs * occ, want);
     int iters = w->sim.iterations;
     uint32_t* bar = (uint32_t*)(w->d.scalars + S_BAR_COUNT);
     int32_t* err = w->d.scalars + S_ERR;
     b3Counters* ctr = w->d.counters;
     JacobiTape T = tape ? *tape : JacobiTape{};
-    void* args[] = {&V, &iters, &bar, &err, &ctr, &T};
+    void* argsPass[] = {&V, &iters, &bar, &err, &ctr, &T};
+    void* argsGather[] = {&V, &iters, &resident, &bar, &err, &ctr, &T};
+    void** args = pass ? argsPass : argsGather;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;

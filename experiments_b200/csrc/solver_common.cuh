@@ -9,24 +9,40 @@ namespace b3solver {
 
 using namespace b3m;
 
-// Row storage: kRowSlots float4 streams of length maxManifolds.
-//  slot 0..3   header: (A,B,nRows,flags as int), (invMassA, invMassB, mu, -),
-//              (invInertiaA.xyz, countA), (invInertiaB.xyz, countB)
-//  normal row j (j<4):   4 + 3j + {0,1,2}
-//  friction row r (r<8): 16 + 3r + {0,1,2}; r = 2j + {0: dir2, 1: dir1}
-//  each row: (n.xyz, rhs), (r1xn.xyz, jacDiagABInv), (r2xn.xyz, applied)
-constexpr int kRowSlots = 40;
-constexpr int kNormal0 = 4;
-constexpr int kFric0 = 16;
+// Row storage: kRowSlots float4 streams of length cap (slot major), one
+// element per manifold.
+//   kHead0  sA, eA, pA, sB as ints: [s, e) is the body's range of the copy
+//           array, p this manifold's own copy in it (s = e for a static side)
+//   kHead1  eB, pB, nRows | dyn << 16 as ints, mu
+//   kNorm   n.xyz, invMassA
+//   kInA    invInertiaA.xyz, invMassB
+//   kInB    invInertiaB.xyz, -
+//   kIds    bodies A and B as ints, copy counts A and B (set-up and the
+//           adjoint only; no phase reads it)
+//   point j (j < 4), kPoint0 + 4j: (r1, rhs) and (r2, 1/diag) of its normal
+//           row, (d2, rhs) and (d1, rhs) of its two friction rows
+//   kFJac   1/diag of the friction rows, two streams of four (row 2j: d2,
+//           row 2j + 1: d1)
+//   kLamN   impulses of the four normal rows; kLamF, + 1: of the friction rows
+// A row's angular parts are r1 x axis and -(r2 x axis): recomputing them (12
+// FMAs) costs less than the 32 bytes a row they would take, since the large
+// scenes' solve is bound by these streams: 592 B per manifold and iteration
+// at three points, 752 B with every row's angular parts stored.
+constexpr int kHead0 = 0, kHead1 = 1, kNorm = 2, kInA = 3, kInB = 4;
+constexpr int kPoint0 = 5;
+constexpr int kFJac = 21;
+constexpr int kLamN = 23;
+constexpr int kLamF = 24;
+constexpr int kIds = 26;
+constexpr int kRowSlots = 27;
 
 struct SolverView {
     float4* rows;       // [kRowSlots][cap]
     int cap;            // manifold capacity (stride)
-    float4* copyLin;    // [2][cap]
-    float4* copyAng;    // [2][cap]
-    float4* avgLin;     // [N]
-    float4* avgAng;     // [N]
-    const uint32_t* incVals;   // sorted copy ids (2m + side)
+    // solver-body copies, (linear, angular) pairs sorted by body: the copies
+    // of body b are [incStart[b], incEnd[b]), in manifold order
+    float4* copies;     // [2 buffers][2 cap][2]
+    const uint32_t* incPos;    // manifold side 2m + side -> its copy
     const uint32_t* incStart;  // per body
     const uint32_t* incEnd;
     const int32_t* numManifolds;
@@ -62,120 +78,163 @@ __device__ __forceinline__ void plane_space(float3 n, float3& p, float3& q) {
 // ---------------------------------------------------------------------------
 // Persistent-kernel helpers
 // ---------------------------------------------------------------------------
-// Every block arrives, the last one releases the others. A waiter gives up
-// after spinLimit polls: it sets *err, counts a timeout and the kernel's
-// blocks leave at this or their next barrier (an error set by anyone makes
-// every barrier fail), so the launch always ends.
-__device__ __forceinline__ bool grid_barrier(uint32_t* count, uint32_t* gen, uint32_t nblocks,
-                                             int32_t* err, b3Counters* counters,
-                                             int spinLimit = b3dev::kSpinLimit) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        ok = 1;
-        const uint32_t g = b3dev::ld_acquire_u32(gen);
-        __threadfence();
-        const uint32_t arrived = atomicAdd(count, 1u);
-        if (arrived == nblocks - 1) {
-            atomicExch(count, 0u);
-            __threadfence();
-            b3dev::st_release_u32(gen, g + 1u);
-        } else {
-            int spins = 0;
-            while (b3dev::ld_acquire_u32(gen) == g) {
+// Grid barrier of a cooperative launch. Blocks add to one 64-bit word with a
+// release and poll it with an acquire until all of this round have arrived;
+// the count only grows within a launch (the host clears it before), so no
+// second word has to be released and a wait ends one L2 round trip after the
+// last arrival. A waiter gives up after spinLimit polls: it sets *err, counts
+// a timeout and sets the word's top bit, on which every block leaves at this
+// or its next barrier, so the launch always ends. An error that was set
+// before the launch ends it at the first barrier.
+struct GridBarrier {
+    unsigned long long* word;
+    unsigned long long target;
+    int32_t* err;
+    b3Counters* counters;
+    int spinLimit;
+    int before;  // thread 0: *err at the kernel's start
+
+    __device__ __forceinline__ GridBarrier(uint32_t* w, int32_t* e, b3Counters* c, int limit)
+        : word(reinterpret_cast<unsigned long long*>(w)), target(0), err(e), counters(c), spinLimit(limit), before(0) {
+        if (threadIdx.x == 0) before = *(volatile int32_t*)e;
+    }
+    __device__ __forceinline__ bool wait() {
+        constexpr unsigned long long kAbort = 1ull << 63;
+        int ok = 1;
+        target += gridDim.x;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(1ull) : "memory");
+            unsigned long long v = b3dev::ld_acquire_u64(word);
+            for (int spins = 0; !(v & kAbort) && v < target; v = b3dev::ld_acquire_u64(word)) {
                 if (++spins > spinLimit) {
                     atomicExch(err, 1);
                     atomicAdd(&counters->timeouts, 1);
-                    ok = 0;
+                    atomicOr(word, kAbort);
+                    v = kAbort;
                     break;
                 }
-                __nanosleep(64);
+                if (spins > 16) __nanosleep(64);
             }
+            ok = !(v & kAbort) && before == 0;
         }
-        if (*(volatile int32_t*)err) ok = 0;
+        return __syncthreads_and(ok) != 0;
     }
-    __syncthreads();
-    return ok != 0;
+};
+
+// Angular part of a row, r x axis, formed again in every phase: one multiply
+// and one fused multiply-add per component, by name.
+__device__ __forceinline__ float3 arm(float3 r, float3 axis) {
+    return make_float3(__fmaf_rn(r.y, axis.z, -__fmul_rn(r.z, axis.y)), __fmaf_rn(r.z, axis.x, -__fmul_rn(r.x, axis.z)),
+                       __fmaf_rn(r.x, axis.y, -__fmul_rn(r.y, axis.x)));
 }
 
-__device__ __forceinline__ void solve_row(const float4 r0, const float4 r1, float4& r2, float lo, float hi,
-                                          float imA, float imB, float3 iiA, float3 iiB,
-                                          float3& dvA, float3& dwA, float3& dvB, float3& dwB) {
-    const float3 n = f3(r0), t1 = f3(r1), t2 = f3(r2);
-    const float rhs = r0.w, jac = r1.w, applied = r2.w;
+// The other body's part, -(r x axis): of a normal row the negated product above,
+// of a friction row r x -axis, with the subtraction turned round.
+__device__ __forceinline__ float3 arm_neg(float3 r, float3 axis) {
+    return make_float3(__fmaf_rn(-r.y, axis.z, __fmul_rn(r.z, axis.y)), __fmaf_rn(-r.z, axis.x, __fmul_rn(r.x, axis.z)),
+                       __fmaf_rn(-r.x, axis.y, __fmul_rn(r.y, axis.x)));
+}
+__device__ __forceinline__ float3 arm_rev(float3 r, float3 axis) {
+    return make_float3(__fmaf_rn(r.z, axis.y, -__fmul_rn(r.y, axis.z)), __fmaf_rn(r.x, axis.z, -__fmul_rn(r.z, axis.x)),
+                       __fmaf_rn(r.y, axis.x, -__fmul_rn(r.x, axis.y)));
+}
+__device__ __forceinline__ float dot_fma(float3 a, float3 b) {
+    return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+__device__ __forceinline__ float3 fma3(float3 a, float s, float3 c) {
+    return make_float3(__fmaf_rn(a.x, s, c.x), __fmaf_rn(a.y, s, c.y), __fmaf_rn(a.z, s, c.z));
+}
+
+// One row: axis n, angular parts t1 and t2, applied impulse lam in and out.
+__device__ __forceinline__ void solve_row(float3 n, float3 t1, float3 t2, float rhs, float jac, float& lam, float lo,
+                                          float hi, float imA, float imB, float3 iiA, float3 iiB, float3& dvA,
+                                          float3& dwA, float3& dvB, float3& dwB) {
     float delta = rhs;  // - applied * cfm (cfm = 0)
-    const float dv1 = dot(n, dvA) + dot(t1, dwA);
-    const float dv2 = -dot(n, dvB) + dot(t2, dwB);
-    delta -= dv1 * jac;
-    delta -= dv2 * jac;
-    const float sum = applied + delta;
+    // every product and sum by name: the compiler contracts such expressions
+    // by their surroundings (unrolled or not, velocities known to be zero or
+    // not), and all forms of the solve have to give the same bits
+    const float dv1 = __fadd_rn(dot_fma(n, dvA), dot_fma(t1, dwA));
+    const float dv2 = __fsub_rn(dot_fma(t2, dwB), dot_fma(n, dvB));
+    delta = __fmaf_rn(-dv1, jac, delta);
+    delta = __fmaf_rn(-dv2, jac, delta);
+    const float sum = lam + delta;
     float na;
     if (sum < lo) {
-        delta = lo - applied;
+        delta = lo - lam;
         na = lo;
     } else if (sum > hi) {
-        delta = hi - applied;
+        delta = hi - lam;
         na = hi;
     } else {
         na = sum;
     }
-    r2.w = na;
-    dvA += n * (imA * delta);
-    dwA += mulv(iiA, t1) * delta;
-    dvB += (-n * imB) * delta;
-    dwB += mulv(iiB, t2) * delta;
+    lam = na;
+    dvA = fma3(n, imA * delta, dvA);
+    dwA = fma3(mulv(iiA, t1), delta, dwA);
+    dvB = fma3(-n * imB, delta, dvB);
+    dwB = fma3(mulv(iiB, t2), delta, dwB);
 }
 
-// Averaged delta velocity of body b over its copies in buffer buf
-// (averageVelocities, P2/btPgsJacobiSolver.cpp:1683-1720): copies in
-// manifold order, sum then multiply by 1/count.
-__device__ __forceinline__ void body_average_se(const SolverView& V, uint32_t s, uint32_t e, int buf, float3& lin,
-                                                float3& ang) {
-    float3 sl = make_float3(0.f, 0.f, 0.f), sa = sl;
-    for (uint32_t i = s; i < e; ++i) {
-        const uint32_t cid = V.incVals[i];
-        const size_t at = (size_t)(buf * 2 + (int)(cid & 1u)) * V.cap + (cid >> 1);
-        sl += f3(V.copyLin[at]);
-        sa += f3(V.copyAng[at]);
+// A row as the adjoint replays it: axis, angular parts, rhs and 1/diag of
+// normal row r, or of friction row r, of manifold m.
+struct RowData {
+    float3 n, t1, t2;
+    float rhs, jac;
+};
+__device__ __forceinline__ RowData load_row(const SolverView& V, int m, bool friction, int r) {
+    const int j = friction ? r >> 1 : r;
+    const float4 a = R(V, kPoint0 + 4 * j, m), b = R(V, kPoint0 + 4 * j + 1, m);
+    RowData D;
+    if (friction) {
+        const float4 d = R(V, kPoint0 + 4 * j + 2 + (r & 1), m);
+        const float4 q = R(V, kFJac + (r >> 2), m);
+        D.n = f3(d);
+        D.rhs = d.w;
+        D.jac = (r & 3) == 0 ? q.x : (r & 3) == 1 ? q.y : (r & 3) == 2 ? q.z : q.w;
+    } else {
+        D.n = f3(R(V, kNorm, m));
+        D.rhs = a.w;
+        D.jac = b.w;
     }
-    const float factor = 1.f / (float)(e - s);
-    lin = sl * factor;
-    ang = sa * factor;
-}
-__device__ __forceinline__ void body_average(const SolverView& V, int b, int buf, float3& lin, float3& ang) {
-    body_average_se(V, V.incStart[b], V.incEnd[b], buf, lin, ang);
+    D.t1 = arm(f3(a), D.n);
+    D.t2 = friction ? arm_rev(f3(b), D.n) : arm_neg(f3(b), D.n);
+    return D;
 }
 
-// One body's average given its incidence range, with the loads issued four
-// copies at a time (copy ids, then the copies): the same copies, order and
-// operations as body_average, hence the same result.
-__device__ __forceinline__ void body_average_range(const SolverView& V, uint32_t s, uint32_t e, int buf, float3& lin,
-                                                   float3& ang) {
+// a * s rounded by itself: fused into the row that adds to it, an average
+// would round differently where it is formed next to the rows and where it is
+// read back from memory.
+__device__ __forceinline__ float3 scaled(float3 a, float s) {
+    return make_float3(__fmul_rn(a.x, s), __fmul_rn(a.y, s), __fmul_rn(a.z, s));
+}
+
+// Average over the copies [s, e) of one body (averageVelocities,
+// P2/btPgsJacobiSolver.cpp:1683-1720): copies in manifold order, sum then
+// multiply by 1/count. K records are in flight at a time; the order of the
+// sum does not depend on K.
+template <int K>
+__device__ __forceinline__ void copy_average(const float4* __restrict__ copies, uint32_t s, uint32_t e, float3& lin,
+                                             float3& ang) {
     float3 sl = make_float3(0.f, 0.f, 0.f), sa = sl;
-    for (uint32_t i0 = s; i0 < e; i0 += 4) {
-        uint32_t cid[4];
+    for (uint32_t i0 = s; i0 < e; i0 += K) {
+        float4 l[K], a[K];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) cid[u] = i0 + u < e ? V.incVals[i0 + u] : 0u;
-        float4 cl[4], ca[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            if (i0 + u < e) {
-                const size_t at = (size_t)(buf * 2 + (int)(cid[u] & 1u)) * V.cap + (cid[u] >> 1);
-                cl[u] = V.copyLin[at];
-                ca[u] = V.copyAng[at];
-            }
+        for (int u = 0; u < K; ++u) {  // past the end: the last record again
+            const float4* r = copies + 2 * (size_t)min(i0 + u, e - 1u);
+            l[u] = __ldcg(r);
+            a[u] = __ldcg(r + 1);
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < K; ++u) {
             if (i0 + u < e) {
-                sl += f3(cl[u]);
-                sa += f3(ca[u]);
+                sl += f3(l[u]);
+                sa += f3(a[u]);
             }
         }
     }
-    const float factor = 1.f / (float)(e - s);
-    lin = sl * factor;
-    ang = sa * factor;
+    lin = scaled(sl, 1.f / (float)(e - s));
+    ang = scaled(sa, 1.f / (float)(e - s));
 }
 
 SolverView solver_view(b3World_t* w);

@@ -75,7 +75,7 @@ void free_all(b3::DevBuffers& d) {
                     d.pairs, d.contacts, d.manifoldFlag, d.pairSep, d.npFast, d.npSlow, d.npDefer, d.npDefer2, d.npDefer3, d.npCand, d.manifoldScan,
                     d.manifoldPair,
                     d.incKeys, d.incVals, d.incKeysAlt, d.incValsAlt, d.bodyIncStart,
-                    d.bodyIncEnd, d.rows, d.manifoldHdr, d.incLin, d.incAng, d.avgLin, d.avgAng,
+                    d.bodyIncEnd, d.rows, d.incPos, d.copies,
                     d.scalars, d.counters, d.sortScratch, d.incSortScratch, d.scanScratch,
                     d.worldStats, d.worldMStart, d.worldMEnd, d.gsCell, d.gsSlotBatch,
                     d.gsSlotOfManifold, d.gsMinRank, d.gsTaken, d.gsBatchCount, d.gsGroupCount, d.gsGroupFill,
@@ -150,6 +150,20 @@ b3::ShapesDev b3World_t::shapesDev() const {
     S.numIndices = (int)indices.size();
     S.numEdges = (int)edges4.size() / 4;
     return S;
+}
+
+// Jacobi launch shapes of a world that was not tuned, by the manifolds it is
+// expected to have (3 per body). Iterations of the solve, microseconds, mixed
+// heaps, gathered / pass over the bodies: 8,000 bodies 127 / 152, 16,000
+// 168 / 197, 24,000 246 / 217, 33,000 303 / 289, 65,000 592 / 432, 131,000
+// 1,198 / 904; the first form wins while most rows fit the shared memories.
+// CTAs of 64 threads (127 us at 8,000 bodies, 137 with 128) until there are
+// two per SM of 128.
+void b3World_t::defaultShapes() {
+    const long long est = 3LL * (long long)bodies.size();
+    solverGather = est > 64 * 1024 ? 1 : 0;
+    solverThreads = est <= 32 * 1024 ? 64 : 128;
+    solverOccCap = solverGather ? (est <= 128 * 1024 ? 2 : 4) : 8;
 }
 
 extern "C" void b3_world_config_default(b3WorldConfig* c) {
@@ -655,8 +669,6 @@ static int ensure_capacity(b3World w) {
         B3_TRY(dalloc(d.valsAlt, nb));
         B3_TRY(dalloc(d.bodyIncStart, nb));
         B3_TRY(dalloc(d.bodyIncEnd, nb));
-        B3_TRY(dalloc(d.avgLin, nb));
-        B3_TRY(dalloc(d.avgAng, nb));
         if (w->gs) {
             B3_TRY(dalloc(d.gsMinRank, 4 * (size_t)nb));
             B3_TRY(dalloc(d.gsTaken, 4 * (size_t)nb));
@@ -684,11 +696,11 @@ static int ensure_capacity(b3World w) {
         B3_TRY(dalloc(d.incVals, 2 * c));
         B3_TRY(dalloc(d.incKeysAlt, 2 * c));
         B3_TRY(dalloc(d.incValsAlt, 2 * c));
-        B3_TRY(dalloc(d.rows, 40 * c));
-        B3_TRY(dalloc(d.incLin, 4 * c));  // [2 phase buffers][2 sides][capacity]
-        B3_TRY(dalloc(d.incAng, 4 * c));
+        B3_TRY(dalloc(d.incPos, 2 * c));
+        B3_TRY(dalloc(d.rows, b3::kSolverRowSlots * c));
+        B3_TRY(dalloc(d.copies, 8 * c));  // [2 phase buffers][2 sides][capacity][2]
         if (w->gs) {
-            static_assert(sizeof(b3Constraint4) <= 40 * sizeof(float4), "Constraint4 fits a manifold's rows");
+            static_assert(sizeof(b3Constraint4) <= b3::kSolverRowSlots * sizeof(float4), "Constraint4 fits a manifold's rows");
             d.gsConstraints = reinterpret_cast<b3Constraint4*>(d.rows);
             B3_TRY(dalloc(d.gsCell, c));
             B3_TRY(dalloc(d.gsSlotBatch, c));
@@ -861,8 +873,6 @@ extern "C" int b3_write_bodies(b3World w, void* stream) {
     B3_CUDA(cudaMemcpyAsync(d.invInertia, ii.data(), sizeof(float4) * N, cudaMemcpyHostToDevice, st));
     B3_CUDA(cudaMemcpyAsync(d.collidable, col.data(), sizeof(int) * N, cudaMemcpyHostToDevice, st));
     B3_CUDA(cudaMemcpyAsync(d.worldId, w->worldIds.data(), sizeof(int) * N, cudaMemcpyHostToDevice, st));
-    B3_CUDA(cudaMemsetAsync(d.avgLin, 0, sizeof(float4) * N, st));
-    B3_CUDA(cudaMemsetAsync(d.avgAng, 0, sizeof(float4) * N, st));
     B3_CUDA(cudaMemsetAsync(d.bodyIncStart, 0, sizeof(uint32_t) * N, st));
     B3_CUDA(cudaMemsetAsync(d.bodyIncEnd, 0, sizeof(uint32_t) * N, st));
     const int32_t hs[1] = {ns};
@@ -874,6 +884,7 @@ extern "C" int b3_write_bodies(b3World w, void* stream) {
         w->graphExec = nullptr;
     }
     w->graphValid = false;
+    if (!w->tuned) w->defaultShapes();
     w->written = true;
     return B3_OK;
 }
@@ -1520,6 +1531,7 @@ extern "C" int b3_autotune(b3World w, int trialSteps, void* stream) {
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     cudaFree(save);
+    w->tuned = w->tuned || rc == B3_OK;
     w->graphValid = false;  // recapture with the chosen shapes
     return rc;
 }
@@ -1542,6 +1554,7 @@ extern "C" int b3_set_tuning(b3World w, const int* values, int count) {
     w->solverGather = gather;
     w->pairSearchMode = pairMode;
     w->clipGroups = clipG;
+    w->tuned = true;
     w->graphValid = false;
     return B3_OK;
 }

@@ -598,7 +598,7 @@ int b3_batch_world_offsets(b3World w, int* offsets, int maxWorlds, int* numWorld
  * (thread or warp per body), each timed on three searches over the same
  * sorted keys; then the Jacobi launch shapes
  * jointly, every combination of CTA size (64/128/256), persistent blocks
- * per SM (1/2/4/8), body-average gather (one-at-a-time / four-wide) and,
+ * per SM (1/2/4/8), body-average form (gathered / pass) and,
  * for batched worlds, mode (grid-barrier / block-per-world), each timed on
  * three solves of the same contacts (the knobs interact, so they are not
  * tuned one at a time). With the batched Gauss-Seidel solver its grid width
@@ -611,14 +611,16 @@ int b3_autotune(b3World w, int trialSteps, void* stream);
  * Jacobi blocks per SM cap, configurations timed by the autotuner, Jacobi
  * mode (0 = persistent grid with grid barriers, 1 = one block per world
  * with block barriers; batched worlds only, bit-identical results), Jacobi
- * body-average gather (0 = one copy at a time, 1 = four loads in flight;
- * bit-identical results), grid pair search form (0 = one thread per body
+ * body averages (0 = gathered by every manifold, rows kept in shared memory;
+ * 1 = formed by a pass over the bodies between two grid barriers, for large
+ * scenes; bit-identical results), grid pair search form (0 = one thread per body
  * over its 27 cells, 1 = one warp per body, a lane per cell; the same pair
  * list and overflow counts bit for bit), narrowphase lane groups (0 = one
  * warp per pair in the FP32 clip and the float-float stages, 1 = eight-lane
  * groups there, four pairs per warp, with the warp form for pairs that do
  * not fit a group's 16-vertex tables or 8 candidates; bit-identical
- * results). */
+ * results). A world that was neither tuned nor set has its Jacobi shapes
+ * chosen by its number of bodies in b3_write_bodies. */
 int b3_get_tuning(b3World w, int* values, int max, int* count);
 /* Set the tunables in b3_get_tuning's order (count >= 3; the pair-search
  * CTA size, the launch count and the trial count are read-only, indices 4,
