@@ -35,11 +35,19 @@ struct ShapesDev {
     const float* inradius;    // per polyhedron: lower bound of its support about localCenter
     const b3ChildShape* children;  // the compounds' children
     // the hulls' vertices two at a time for the packed FP32x2 projection:
-    // pair j of polyhedron p at polyPack[p] + j holds (x0, x1, y0, y1) in
-    // vpXY and (z0, z1) in vpZ (an odd count repeats the last vertex)
+    // (x0, x1, y0, y1) in vpXY and (z0, z1) in vpZ; an odd count repeats the
+    // last vertex, and a hull that is symmetric about its origin (every -v a
+    // vertex, bit for bit) holds one vertex of each v, -v
     const float4* vpXY;
     const float2* vpZ;
-    const int* polyPack;
+    // faces that are distinct axes: their indices within the polyhedron at
+    // axisFaces[faceOffset ..]; a face whose normal is an earlier one's
+    // negative, bit for bit, is left out
+    const int* axisFaces;
+    // per polyhedron: (localCenter, |mE|), ints (face offset, face axes, edge
+    // offset, edges), ints (first vertex pair, vertex pairs, < 0 when
+    // symmetric, faces, -)
+    const float4* info;
     int numPolys, numVerts, numFaces, numIndices, numEdges;
 };
 
@@ -74,7 +82,8 @@ struct DevBuffers {
     b3ChildShape* childShapes = nullptr;
     float4* vpXY = nullptr;  // vertex pairs (x0, x1, y0, y1)
     float2* vpZ = nullptr;   // vertex pairs (z0, z1)
-    int* polyPack = nullptr; // per polyhedron: its first vertex pair
+    int* axisFaces = nullptr; // faces that are distinct axes, at the polyhedron's face offset
+    float4* polyInfo = nullptr;  // three per polyhedron (ShapesDev.info)
     // compound and mesh pairs: sub-pair records (body A, body B, side A,
     // side B; a side is a child shape >= 0 or -(polytope + 1)), per pair
     // counts and their exclusive scan
@@ -101,7 +110,8 @@ struct DevBuffers {
     float4* pairSep = nullptr;        // per pair: FP32 separating axis of the sweep
     int* npFast = nullptr;            // queue: pairs whose axis the FP32 sweep decided
     int* npSlow = nullptr;            // queue: pairs for the float-float path
-    int* npDefer = nullptr;           // queue: clip pairs the lane groups pass to the warp clip
+    int* npDefer = nullptr;           // queue: pairs of the warp sweep, then
+                                      // clip pairs the lane groups pass to the warp clip
     int* npDefer2 = nullptr;          // queue: slow-queue positions for the warp float-float stage
     int* npDefer3 = nullptr;          // queue: slow-queue positions for the warp ranking
     int* npCand = nullptr;            // near-minimum axes of queued pairs (kNpCandSlots x 32)
@@ -166,7 +176,10 @@ enum ScalarSlot {
     S_NP_WORK6 = 21,
     S_NP_DEFER3 = 22,     // slow-queue positions the lane-group ranking passed to k_np_refine
     S_NP_WORK7 = 23,
-    S_NUM_SCALARS = 24
+    S_NP_BIG = 24,        // items of the warp sweep's queue
+    S_NP_WORK8 = 25,
+    S_NP_SMALL = 26,      // items of the group sweep's queue
+    S_NUM_SCALARS = 28
 };
 
 }  // namespace b3
@@ -185,7 +198,10 @@ struct b3World_t {
     std::vector<float> verts4, edges4, localAabb8;
     std::vector<float> polyInradius;
     std::vector<float> vpXY, vpZ;  // vertex pairs, built at upload
-    std::vector<int> polyPack;
+    std::vector<int> axisFaces;
+    std::vector<float> polyInfo;   // 12 per polyhedron
+    bool smallPairs = false, largePairs = false;  // hulls register pairs for the group sweep / the warp sweep
+    int maxFaces = 0;              // faces of the hull with the most
     std::vector<b3ChildShape> childShapes;  // children of the compounds
     int numSpheres = 0, numPlanes = 0, numCompounds = 0, numMeshes = 0;
     bool hasSpheresPlanes() const { return numSpheres > 0 && (numSpheres > 1 || numPlanes > 0); }

@@ -249,14 +249,16 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
     return d;
 }
 
-// FP32 projection of polyhedron h (index pi) onto world axis dir relative to
-// its own position, two vertices per packed FP32x2 instruction: x * d.x,
-// then + y * d.y, then + z * d.z, each rounded once.
-__device__ __forceinline__ void project_packed(const b3::ShapesDev& S, const b3ConvexPolyhedron& h, int pi,
-                                               const Mat3& R, float3 dir, float& mn, float& mx) {
+// FP32 projection of polyhedron pi onto world axis dir relative to its own
+// position, two vertices per packed FP32x2 instruction: x * d.x, then + y * d.y,
+// then + z * d.z, each rounded once. A symmetric hull keeps one vertex of each
+// v, -v: rounding is symmetric too, so its extent is +-max |v . d|.
+__device__ __forceinline__ void project_packed(const b3::ShapesDev& S, int pi, const Mat3& R, float3 dir, float& mn,
+                                               float& mx) {
     const float3 ld = mul_t(R, dir);
     const unsigned long long lx = pack2(ld.x, ld.x), ly = pack2(ld.y, ld.y), lz = pack2(ld.z, ld.z);
-    const int off = __ldg(&S.polyPack[pi]), np = (h.numVertices + 1) >> 1;
+    const int4 pk = __ldg(reinterpret_cast<const int4*>(&S.info[3 * pi + 2]));
+    const int off = pk.x, np = abs(pk.y);
     float lo = FLT_MAX, hi = -FLT_MAX;
 #pragma unroll 4
     for (int j = 0; j < np; ++j) {
@@ -270,18 +272,17 @@ __device__ __forceinline__ void project_packed(const b3::ShapesDev& S, const b3C
         lo = fminf(lo, fminf(d0, d1));
         hi = fmaxf(hi, fmaxf(d0, d1));
     }
-    mn = lo;
-    mx = hi;
+    const float ext = fmaxf(hi, -lo);
+    mn = pk.y < 0 ? -ext : lo;
+    mx = pk.y < 0 ? ext : hi;
 }
 
 // FP32 depth along the oriented axis n (P2/sat.cl:227-252, relative to
 // body A's position).
 __device__ __forceinline__ float axis_depth(const PairCtx& c, const b3::ShapesDev& S, float3 rel, float3 n) {
-    const b3ConvexPolyhedron& pa = *c.pa;
-    const b3ConvexPolyhedron& pb = *c.pb;
     float mn0, mx0, mn1, mx1;
-    project_packed(S, pa, (int)(c.pa - S.polys), c.RA, n, mn0, mx0);
-    project_packed(S, pb, (int)(c.pb - S.polys), c.RB, n, mn1, mx1);
+    project_packed(S, (int)(c.pa - S.polys), c.RA, n, mn0, mx0);
+    project_packed(S, (int)(c.pb - S.polys), c.RB, n, mn1, mx1);
     const float off = dot(rel, n);  // posB - posA along n
     mn1 += off;
     mx1 += off;
@@ -1499,6 +1500,7 @@ __device__ __forceinline__ void emit_contact(int p, const PairCtx& c, const FfVe
 }
 
 __device__ __forceinline__ int next_work(int32_t* counter, int limit, int chunk) {
+    if (limit <= 0) return -1;  // nothing queued: thousands of additions to one counter would take microseconds
     int w = 0;
     if ((threadIdx.x & 31) == 0) w = atomicAdd(counter, chunk);
     w = __shfl_sync(0xffffffffu, w, 0);
@@ -1514,41 +1516,40 @@ __device__ __forceinline__ int push(int* queue, int32_t* count, int p) {
     return __shfl_sync(0xffffffffu, slot, 0);
 }
 
-// Stage 1, every pair: the FP32 separating-axis sweep. Separated pairs are
-// finished here; pairs whose axis the sweep decides go to the FP32 clip
-// queue with that axis; pairs with near-minimum candidates go to the
-// float-float queue.
-// kSub: the items are the sub-pairs of compound and mesh pairs, in the
-// slots after the pairs' (slot = numPairs + sub-pair).
+// Stage 1, pairs of many axes (and those the lane groups pass on), a warp each.
+// Separated pairs are finished here; pairs whose axis the sweep decides go to
+// the FP32 clip queue with that axis; pairs with near-minimum candidates go to
+// the float-float queue. queue: their slots, or null when every item is one.
+// kSub: the items are the sub-pairs of compound and mesh pairs, in the slots
+// after the pairs' (slot = numPairs + sub-pair).
 // Six blocks per SM (80 registers): with the projection loop unrolled the
 // extra resident warps hide more of the vertex loads' latency than the
 // spills cost (settled 131,072-body step: sweep 4.01 -> 3.46 ms).
 template <bool kEarlyFaces, bool kSub>
 __global__ void __launch_bounds__(128, 6)
 k_np_sweep(const int2* __restrict__ pairs, const int4* __restrict__ subs, const int32_t* __restrict__ numPairsDev,
-           b3::BodiesDev Bd, b3::ShapesDev S, uint32_t* __restrict__ manifoldFlag, float4* __restrict__ pairSep,
-           int* __restrict__ fastQ, int* __restrict__ slowQ, int* __restrict__ cand, int candSlots,
-           int32_t* __restrict__ scalars, b3Counters* __restrict__ counters) {
+           b3::BodiesDev Bd, b3::ShapesDev S, const int* __restrict__ queue, uint32_t* __restrict__ manifoldFlag,
+           float4* __restrict__ pairSep, int* __restrict__ fastQ, int* __restrict__ slowQ, int* __restrict__ cand,
+           int candSlots, int32_t* __restrict__ scalars, b3Counters* __restrict__ counters) {
     extern __shared__ __align__(16) unsigned char np_smem[];
     const int lane = threadIdx.x & 31;
     unsigned char* wbase = np_smem + (size_t)(threadIdx.x >> 5) * kSweepWarpSmem;
     PairPre* pre = reinterpret_cast<PairPre*>(wbase);
     int* wcand = reinterpret_cast<int*>(wbase + sizeof(PairPre) * kPreChunk);
-    const int numItems = kSub ? scalars[b3::S_NUM_SUB] : *numPairsDev;
+    const int numItems = queue ? scalars[b3::S_NP_BIG] : kSub ? scalars[b3::S_NUM_SUB] : *numPairsDev;
     const int base = kSub ? *numPairsDev : 0;
     for (;;) {
-        const int chunk = next_work(scalars + b3::S_NP_WORK, numItems, kPreChunk);
+        const int chunk = next_work(scalars + b3::S_NP_WORK8, numItems, kPreChunk);
         if (chunk < 0) break;
         const int n = min(kPreChunk, numItems - chunk);
-        if (lane < n) item_prefetch<kSub>(pre[lane], base + chunk + lane, pairs, subs, base, Bd, S);
+        if (lane < n) item_prefetch<kSub>(pre[lane], queue ? queue[chunk + lane] : base + chunk + lane, pairs, subs, base, Bd, S);
         __syncwarp();
         for (int i = 0; i < n; ++i) {
-            const int p = base + chunk + i;
+            const int p = pre[i].p;
             PairCtx c;
             int r = 0, count = 0;
             float3 sepf = make_float3(0.f, 0.f, 0.f);
-            if (pair_from_pre(c, pre[i], S))
-                r = sweep_axes<kEarlyFaces>(c, S, wcand, sepf, count, &counters->clipOverflow);
+            if (pair_from_pre(c, pre[i], S)) r = sweep_axes<kEarlyFaces>(c, S, wcand, sepf, count, &counters->clipOverflow);
             if (r == 0) {
                 if (lane == 0) manifoldFlag[p] = 0u;
             } else if (r == 1) {
@@ -1680,6 +1681,8 @@ __device__ __forceinline__ void grp_argmin(float& v, int& idx, unsigned m) {
     idx = (int)__reduce_min_sync(m, k == km ? (unsigned)idx : 0xffffffffu);
     v = fkey_inv(km);
 }
+
+#include "sweep_groups.cuh"
 
 // select_face over the group's lanes; faces within the window of the FP32
 // extreme only set *tied (the pair then goes to the float-float stage,
@@ -2810,10 +2813,10 @@ namespace b3 {
 // The four narrowphase stages over the pairs (kSub false) or the sub-pairs
 // of compound and mesh pairs (kSub true).
 template <bool kSub>
-static int launch_np_stages(b3World_t* w, cudaStream_t st, const NpParams& P, bool early) {
-    // work counters and queue lengths S_NP_WORK .. S_NP_WORK4, S_NP_DEFER .. S_NP_WORK7
+static int launch_np_stages(b3World_t* w, cudaStream_t st, const NpParams& P) {
+    // work counters and queue lengths S_NP_WORK .. S_NP_WORK4, S_NP_DEFER onwards
     B3_CUDA(cudaMemsetAsync(w->d.scalars + S_NP_WORK, 0, sizeof(int32_t) * 6, st));
-    B3_CUDA(cudaMemsetAsync(w->d.scalars + S_NP_DEFER, 0, sizeof(int32_t) * 6, st));
+    B3_CUDA(cudaMemsetAsync(w->d.scalars + S_NP_DEFER, 0, sizeof(int32_t) * (S_NUM_SCALARS - S_NP_DEFER), st));
     const int threads = 32 * w->npWarpsPerBlock;
     const size_t smem = sizeof(WarpScratch) * w->npWarpsPerBlock;
     const size_t smemGroups = sizeof(GroupScratch) * (32 / kClipGroup) * w->npWarpsPerBlock;
@@ -2826,16 +2829,39 @@ static int launch_np_stages(b3World_t* w, cudaStream_t st, const NpParams& P, bo
     const b3::ShapesDev S = w->shapesDev();
     int32_t* sc = w->d.scalars;
     const size_t smemSweep = (size_t)kSweepWarpSmem * w->npWarpsPerBlock;
-    auto sweep = early ? k_np_sweep<true, kSub> : k_np_sweep<false, kSub>;
-    int occS = 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occS, sweep, threads, smemSweep) != cudaSuccess || occS < 1)
-        occS = 1;
+    const size_t smemSweepG = sizeof(SweepScratch) * w->npWarpsPerBlock;
     // per-kernel events only in eagerly timed steps of the pairs (never inside a capture)
     const bool tk = !kSub && w->timing && w->npEv[0] != nullptr;
     if (tk) B3_CUDA(cudaEventRecord(w->npEv[0], st));
+    // Sorted into the two sweeps' queues where the scene has pairs for both.
+    // The groups' queue lies in a buffer that the manifold list uses later. The
+    // warp sweep always runs: it takes what the groups cannot hold.
+    const bool small = w->smallPairs, both = small && w->largePairs;
+    int* smallQ = both ? reinterpret_cast<int*>(w->d.manifoldScan) : nullptr;
+    if (both) {
+        k_np_bin<kSub><<<w->ctx->numSMs * 4, 256, 0, st>>>(w->d.pairs, w->d.subPairs, sc + S_NUM_PAIRS, Bd, S, sc,
+                                                          w->d.manifoldFlag, smallQ, w->d.npDefer);
+        B3_CHECK_LAUNCH();
+    }
+    const int candSlots = std::min(w->cfg.maxPairs, kNpCandSlots);
+    int occS = 1;
+    if (small) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occS, k_np_sweep_groups<kSub>, threads, smemSweepG) !=
+                cudaSuccess || occS < 1)
+            occS = 1;
+        k_np_sweep_groups<kSub><<<w->ctx->numSMs * occS, threads, smemSweepG, st>>>(
+            w->d.pairs, w->d.subPairs, sc + S_NUM_PAIRS, Bd, S, smallQ, w->d.manifoldFlag, w->d.pairSep, w->d.npFast,
+            w->d.npSlow, w->d.npDefer, w->d.npCand, candSlots, sc);
+        B3_CHECK_LAUNCH();
+    }
+    // the early face test only where some pair can have more than 64 faces (a
+    // hull may pair with another instance of itself)
+    auto sweep = 2 * w->maxFaces > 64 ? k_np_sweep<true, kSub> : k_np_sweep<false, kSub>;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occS, sweep, threads, smemSweep) != cudaSuccess || occS < 1)
+        occS = 1;
     sweep<<<w->ctx->numSMs * occS, threads, smemSweep, st>>>(
-        w->d.pairs, w->d.subPairs, sc + S_NUM_PAIRS, Bd, S, w->d.manifoldFlag, w->d.pairSep, w->d.npFast,
-        w->d.npSlow, w->d.npCand, std::min(w->cfg.maxPairs, kNpCandSlots), sc, w->d.counters);
+        w->d.pairs, w->d.subPairs, sc + S_NUM_PAIRS, Bd, S, small ? w->d.npDefer : nullptr, w->d.manifoldFlag,
+        w->d.pairSep, w->d.npFast, w->d.npSlow, w->d.npCand, candSlots, sc, w->d.counters);
     B3_CHECK_LAUNCH();
     if (tk) B3_CUDA(cudaEventRecord(w->npEv[1], st));
     const size_t smemFF = sizeof(GroupScratchFF) * (32 / kClipGroup) * w->npWarpsPerBlock;
@@ -2911,14 +2937,6 @@ int launch_narrowphase(b3World_t* w, cudaStream_t st) {
     P.skipDist = (float)((double)w->sim.contactProcessing - (double)w->sim.slopOffset);
     P.frictionCombine = w->sim.frictionCombine;
     P.maxPairs = w->cfg.maxPairs;
-    // the early face test only where some pair can have more than 64 faces
-    // (a hull may pair with another instance of itself); mesh triangles are
-    // polytopes of 5 faces
-    int maxFaces = 0;
-    for (const b3Collidable& c : w->cols)
-        if (c.shapeType == B3_SHAPE_CONVEX_HULL) maxFaces = std::max(maxFaces, w->polys[c.shapeIndex].numFaces);
-    if (w->numMeshes) maxFaces = std::max(maxFaces, 5);
-    const bool early = 2 * maxFaces > 64;
     const size_t smem = sizeof(WarpScratch) * w->npWarpsPerBlock;
     if (smem > 48 * 1024 && (size_t)w->npSmemAttr < smem) {
         // more than the default dynamic shared memory per block (8 warps);
@@ -2947,7 +2965,7 @@ int launch_narrowphase(b3World_t* w, cudaStream_t st) {
             B3_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemFF));
     }
     {
-        B3_TRY(launch_np_stages<false>(w, st, P, early));
+        B3_TRY(launch_np_stages<false>(w, st, P));
         if (w->hasSubPairs()) {
             // expand compound and mesh pairs into sub-pairs, then their stages
             const b3::BodiesDev Bd = w->bodiesDev();
@@ -2964,7 +2982,7 @@ int launch_narrowphase(b3World_t* w, cudaStream_t st) {
             k_sub_write<<<g, 256, 0, st>>>(w->d.pairs, w->d.scalars + S_NUM_PAIRS, Bd, S, w->d.aabbMin, w->d.aabbMax,
                                           w->d.subOffset, w->d.scalars, w->d.subPairs);
             B3_CHECK_LAUNCH();
-            B3_TRY(launch_np_stages<true>(w, st, P, early));
+            B3_TRY(launch_np_stages<true>(w, st, P));
         }
     }
     if (w->hasSpheresPlanes()) {

@@ -70,7 +70,7 @@ int dalloc(T*& p, size_t count) {
 void free_all(b3::DevBuffers& d) {
     void* ptrs[] = {d.pos, d.quat, d.linVel, d.angVel, d.invMass, d.friction, d.restitution,
                     d.invInertia, d.collidable, d.worldId, d.cols, d.polys, d.verts, d.faces,
-                    d.indices, d.edges, d.localAabb, d.polyInradius, d.childShapes, d.vpXY, d.vpZ, d.polyPack, d.subPairs, d.subCount, d.subOffset, d.aabbMin, d.aabbMax, d.smallSlot,
+                    d.indices, d.edges, d.localAabb, d.polyInradius, d.childShapes, d.vpXY, d.vpZ, d.axisFaces, d.polyInfo, d.subPairs, d.subCount, d.subOffset, d.aabbMin, d.aabbMax, d.smallSlot,
                     d.largeStart, d.largeList, d.sapSmall, d.sapLarge, d.sapSorted, d.sapCount, d.sapOffset, d.keys, d.vals, d.keysAlt, d.valsAlt, d.cellTable,
                     d.pairs, d.contacts, d.manifoldFlag, d.pairSep, d.npFast, d.npSlow, d.npDefer, d.npDefer2, d.npDefer3, d.npCand, d.manifoldScan,
                     d.manifoldPair,
@@ -143,7 +143,8 @@ b3::ShapesDev b3World_t::shapesDev() const {
     S.children = d.childShapes;
     S.vpXY = d.vpXY;
     S.vpZ = d.vpZ;
-    S.polyPack = d.polyPack;
+    S.axisFaces = d.axisFaces;
+    S.info = d.polyInfo;
     S.numPolys = (int)polys.size();
     S.numVerts = (int)verts4.size() / 4;
     S.numFaces = (int)faces.size();
@@ -757,29 +758,96 @@ static int upload_shapes(b3World w, cudaStream_t st) {
     B3_CUDA(cudaMemcpyAsync(d.localAabb, w->localAabb8.data(), sizeof(float) * w->localAabb8.size(), cudaMemcpyHostToDevice, st));
     B3_CUDA(cudaMemcpyAsync(d.polyInradius, w->polyInradius.data(), sizeof(float) * w->polyInradius.size(),
                             cudaMemcpyHostToDevice, st));
-    // vertex pairs per polyhedron (the packed projection's layout)
+    // vertex pairs per polyhedron (the packed projection's layout) and the
+    // faces that are distinct axes
     w->vpXY.clear();
     w->vpZ.clear();
-    w->polyPack.assign(w->polys.size(), 0);
+    w->polyInfo.assign(12 * w->polys.size(), 0.f);
+    w->axisFaces.assign(w->faces.size(), 0);
     for (size_t p = 0; p < w->polys.size(); ++p) {
         const b3ConvexPolyhedron& h = w->polys[p];
-        w->polyPack[p] = (int)(w->vpZ.size() / 2);
-        for (int j = 0; j < h.numVertices; j += 2) {
-            const float* a = &w->verts4[4 * (size_t)(h.vertexOffset + j)];
-            const float* b = &w->verts4[4 * (size_t)(h.vertexOffset + std::min(j + 1, h.numVertices - 1))];
+        auto vertex = [&](int j) { return &w->verts4[4 * (size_t)(h.vertexOffset + j)]; };
+        // one vertex of each v, -v when every vertex has its opposite
+        std::vector<int> pick;
+        std::vector<char> used(std::max(h.numVertices, 0), 0);
+        bool sym = h.numVertices > 0 && h.numVertices <= 4096;
+        for (int j = 0; sym && j < h.numVertices; ++j) {
+            if (used[j]) continue;
+            const float* a = vertex(j);
+            int k = j + 1;
+            for (; k < h.numVertices; ++k) {
+                const float* b = vertex(k);
+                if (!used[k] && a[0] == -b[0] && a[1] == -b[1] && a[2] == -b[2]) break;
+            }
+            sym = k < h.numVertices;
+            if (sym) used[k] = 1;
+            pick.push_back(j);
+        }
+        if (!sym) {
+            pick.resize(std::max(h.numVertices, 0));
+            for (int j = 0; j < (int)pick.size(); ++j) pick[j] = j;
+        }
+        const int pairs = ((int)pick.size() + 1) / 2;
+        const int firstPair = (int)(w->vpZ.size() / 2);
+        for (size_t j = 0; j < pick.size(); j += 2) {
+            const float* a = vertex(pick[j]);
+            const float* b = vertex(pick[std::min(j + 1, pick.size() - 1)]);
             w->vpXY.insert(w->vpXY.end(), {a[0], b[0], a[1], b[1]});
             w->vpZ.insert(w->vpZ.end(), {a[2], b[2]});
         }
+        // (the polyhedron of a whole mesh is never swept: its triangles are)
+        int axes = 0;
+        for (int f = 0; f < h.numFaces; ++f) {
+            const float* n = w->faces[h.faceOffset + f].plane;
+            bool twin = false;
+            for (int k = 0; k < axes && !twin && h.numFaces <= 1024; ++k) {
+                const float* m = w->faces[h.faceOffset + w->axisFaces[h.faceOffset + k]].plane;
+                twin = n[0] == -m[0] && n[1] == -m[1] && n[2] == -m[2];
+            }
+            if (!twin) w->axisFaces[h.faceOffset + axes++] = f;
+        }
+        float* info = &w->polyInfo[12 * p];
+        for (int k = 0; k < 3; ++k) info[k] = h.localCenter[k];
+        info[3] = std::sqrt(std::fma(h.mE[2], h.mE[2], std::fma(h.mE[0], h.mE[0], h.mE[1] * h.mE[1])));
+        const int ints[8] = {h.faceOffset, axes, h.uniqueEdgesOffset, h.numUniqueEdges,
+                             firstPair, sym ? -pairs : pairs, h.numFaces, 0};
+        memcpy(info + 4, ints, sizeof(ints));
     }
+    // which sweeps the scene's pairs can need (the rule of sweep_small over the
+    // distinct (axes, edges) of the hulls and mesh triangles)
+    std::vector<std::pair<int, int>> kinds;
+    w->maxFaces = 0;
+    auto kind = [&](int p) {
+        int v[3];
+        memcpy(v, &w->polyInfo[12 * (size_t)p + 5], sizeof(v));
+        w->maxFaces = std::max(w->maxFaces, w->polys[p].numFaces);
+        const std::pair<int, int> k(v[0], v[2]);
+        if (std::find(kinds.begin(), kinds.end(), k) == kinds.end()) kinds.push_back(k);
+    };
+    for (const b3Collidable& c : w->cols) {
+        if (c.shapeType == B3_SHAPE_CONVEX_HULL) kind(c.shapeIndex);
+        else if (c.shapeType == B3_SHAPE_CONCAVE_TRIMESH)
+            for (int t = 0; t < c.numChildShapes; ++t) kind(w->polys[c.shapeIndex].unused + t);
+    }
+    w->smallPairs = w->largePairs = false;
+    for (const auto& a : kinds)
+        for (const auto& b : kinds) {
+            const int n = a.first + b.first;
+            (n <= 8 && a.second * b.second <= 16 - n && a.second > 0 && b.second > 0 ? w->smallPairs : w->largePairs) = true;
+        }
     B3_TRY(dalloc(d.vpXY, w->vpXY.size() / 4 + 1));
     B3_TRY(dalloc(d.vpZ, w->vpZ.size() / 2 + 1));
-    B3_TRY(dalloc(d.polyPack, w->polyPack.size() + 1));
+    B3_TRY(dalloc(d.polyInfo, w->polyInfo.size() / 4 + 1));
+    B3_TRY(dalloc(d.axisFaces, w->axisFaces.size() + 1));
     if (!w->vpXY.empty()) {
         B3_CUDA(cudaMemcpyAsync(d.vpXY, w->vpXY.data(), sizeof(float) * w->vpXY.size(), cudaMemcpyHostToDevice, st));
         B3_CUDA(cudaMemcpyAsync(d.vpZ, w->vpZ.data(), sizeof(float) * w->vpZ.size(), cudaMemcpyHostToDevice, st));
     }
-    if (!w->polyPack.empty())
-        B3_CUDA(cudaMemcpyAsync(d.polyPack, w->polyPack.data(), sizeof(int) * w->polyPack.size(),
+    if (!w->polyInfo.empty())
+        B3_CUDA(cudaMemcpyAsync(d.polyInfo, w->polyInfo.data(), sizeof(float) * w->polyInfo.size(),
+                                cudaMemcpyHostToDevice, st));
+    if (!w->axisFaces.empty())
+        B3_CUDA(cudaMemcpyAsync(d.axisFaces, w->axisFaces.data(), sizeof(int) * w->axisFaces.size(),
                                 cudaMemcpyHostToDevice, st));
     B3_TRY(dalloc(d.childShapes, w->childShapes.size()));
     if (!w->childShapes.empty())
