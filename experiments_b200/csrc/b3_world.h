@@ -141,9 +141,7 @@ struct DevBuffers {
     int* gsCell = nullptr;            // per manifold: cell x + 16 z
     int* gsSlotBatch = nullptr;       // per sorted slot: batch
     int* gsSlotOfManifold = nullptr;  // per manifold: index of its Constraint4
-    int* gsMinRank = nullptr;         // [4][bodies]
-    int* gsTaken = nullptr;           // [4][bodies]
-    int* gsBatchCount = nullptr;      // [4] batches per class, then 5 round counters
+    float4* gsVel = nullptr;          // [bodies][2] velocities with their versions
     uint32_t* gsGroupCount = nullptr; // [4 * kGsMaxBatch]
     uint32_t* gsGroupFill = nullptr;  // [4 * kGsMaxBatch]
     uint32_t* gsGroupOffset = nullptr;  // [4 * kGsMaxBatch + 1]
@@ -243,7 +241,7 @@ struct b3World_t {
     int solverThreads = 256;   // Jacobi CTA size
     int solverOccCap = 4;      // Jacobi persistent blocks per SM (at most)
     int solverMode = 0;        // Jacobi: 0 = grid barriers, 1 = one block per world (batched);
-                               // batched Gauss-Seidel: grid width 0 = manifolds / 8, 1 = manifolds / 64
+                               // batched Gauss-Seidel: resident blocks, 0 = 8 and 2 per SM, 1 = half of them
     int solverGather = 0;      // Jacobi body averages: 0 = gathered by every manifold, 1 = a pass over the bodies
     int pairSearchMode = 0;    // grid pair search: 0 = thread per body, 1 = warp per body
     int clipGroups = 1;        // clip and float-float stages: 0 = a warp per pair, 1 = 8-lane groups

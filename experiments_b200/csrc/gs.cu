@@ -10,24 +10,34 @@
 //                  mapping, ST/solveContact.cl:418-426); radix sort by
 //                  (class, cell), stable, so each class lists its manifolds
 //                  in (cell, manifold) order
-//   k_gs_colour    greedy colouring of every class at once, persistent and
-//                  cooperative: batch after batch, rounds of "a manifold
-//                  joins when it is the first undecided manifold of each of
-//                  its dynamic bodies; manifolds sharing a body with a
-//                  joined one wait for the next batch", which reproduces the
-//                  sequential greedy pass of sortConstraintByBatch
-//                  (P1/btGpuNarrowPhaseAndSolver.cpp:752-852) run over the
-//                  class in order, with exact body identities
+//   k_gs_sides     one entry per manifold and dynamic body; radix sort by
+//   k_gs_links     body: each body's manifolds in slot order, and for every
+//                  entry the one before it on the same body and class
+//   k_gs_colour    greedy colouring of every class at once: a manifold takes
+//                  the lowest batch that no earlier manifold on its bodies
+//                  has, which is what the sequential greedy pass of
+//                  sortConstraintByBatch (P1/btGpuNarrowPhaseAndSolver.cpp:
+//                  752-852) arrives at batch after batch, run over the class
+//                  in order, with exact body identities
+//   k_gs_rank      each entry's place in its body's solve order
 //   k_gs_inertia   world inverse inertia R diag(I^-1) R^T per body
 //                  (setupBodiesKernel, broadphaseKernel.cl:189-201)
 //   k_gs_setup     Constraint4 per manifold (setConstraint4,
 //                  ST/solverSetup.cl:520-609), stored grouped by
 //                  (class, batch) (counting sort)
 //   k_gs_solve     4 contact then 4 friction iterations; in each, the
-//                  classes in order and their batches in order, every batch
-//                  solved in parallel (no dynamic body twice), grid
-//                  barriers in between (ST/Solver.cpp:561-700;
-//                  solveContact.cl:272-365, solveFriction.cl:297-391)
+//                  classes in order and their batches in order
+//                  (ST/Solver.cpp:561-700; solveContact.cl:272-365,
+//                  solveFriction.cl:297-391)
+//
+// B200 mapping: both passes are sequential per body and independent elsewhere,
+// so a manifold waits for its own two bodies and not for the whole grid. In the
+// colouring it waits for the previous entry on each body, in the solve until
+// each body's velocity carries the version that its place in the body's order
+// calls for. A wait is about one L2 round trip after what it waits for, against
+// a grid barrier per batch (8 x some 50 batches) and three per colouring round
+// (some 290 rounds): 65,537 mixed bodies (196 K manifolds), colouring 2,619 and
+// solve 2,499 us with barriers. All waits are bounded.
 // Velocities are written to the bodies directly; integration then applies
 // no Jacobi averages.
 #include <algorithm>
@@ -38,7 +48,6 @@
 #include "solver_common.cuh"
 
 using namespace b3m;
-using b3solver::GridBarrier;
 
 namespace {
 
@@ -48,7 +57,6 @@ constexpr float kScale = 0.5f;    // 1 / (N_OBJ_PER_SPLIT * m_averageExtent) = 1
 constexpr float kFriction = 0.7f; // m_linear.w (ST/solverSetup.cl:541), ST/solveFriction.cl:319
 constexpr float kDrift = 0.005f;  // ConstraintCfg::m_positionDrift
 constexpr float kPosCoeff = 0.2f; // ConstraintCfg::m_positionConstraintCoeff
-constexpr int kNone = 0x7fffffff;
 
 __device__ __forceinline__ int class_of(int cell) { return (cell & 1) + 2 * ((cell / kSplit) & 1); }
 
@@ -73,115 +81,156 @@ __global__ void k_gs_keys(const b3Contact4* __restrict__ contacts, const int* __
     }
 }
 
+// Polls of a wait on another manifold before it gives up (about a microsecond
+// each).
+constexpr int kGsSpins = 1 << 20;
+
+// A wait gave up: the step's error flag, as a grid barrier sets it.
+__device__ __forceinline__ void gave_up(int32_t* err, b3Counters* counters) {
+    if (atomicExch(err, 1) == 0) atomicAdd(&counters->timeouts, 1);
+}
+
+// One entry per manifold side: key = its dynamic body (numBodies for a static
+// one, past every body), value = 2 slot + side.
+__global__ void k_gs_sides(const uint32_t* __restrict__ vals, const b3Contact4* __restrict__ contacts,
+                           const int* __restrict__ manifoldPair, const float* __restrict__ invMass,
+                           const int32_t* __restrict__ numManifolds, int numBodies, uint32_t* __restrict__ bodyKeys,
+                           uint32_t* __restrict__ bodyVals, int* __restrict__ slotBatch,
+                           unsigned long long* __restrict__ used, int32_t* __restrict__ numSides) {
+    const int M = *numManifolds;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *numSides = 2 * M;
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < M; s += gridDim.x * blockDim.x) {
+        const b3Contact4& c = contacts[manifoldPair[vals[s]]];
+        const int A = abs(c.bodyAPtrAndSignBit), B = abs(c.bodyBPtrAndSignBit);
+        bodyKeys[2 * s] = invMass[A] != 0.f ? (uint32_t)A : (uint32_t)numBodies;
+        bodyKeys[2 * s + 1] = invMass[B] != 0.f ? (uint32_t)B : (uint32_t)numBodies;
+        bodyVals[2 * s] = 2u * s;
+        bodyVals[2 * s + 1] = 2u * s + 1u;
+        slotBatch[s] = -1;
+        used[2 * s] = used[2 * s + 1] = 0ull;
+    }
+}
+
+// Per body its range of the sorted entries; per entry the previous one on the
+// same body in the same class (-1: none, -2: a static side).
+__global__ void k_gs_links(const uint32_t* __restrict__ bodyKeys, const uint32_t* __restrict__ bodyVals,
+                           const uint32_t* __restrict__ keys, const int32_t* __restrict__ numSides, int numBodies,
+                           uint32_t* __restrict__ start, uint32_t* __restrict__ end, int* __restrict__ prev) {
+    const int n = *numSides;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t k = bodyKeys[i], v = bodyVals[i];
+        if (k >= (uint32_t)numBodies) {
+            prev[v] = -2;
+            continue;
+        }
+        const bool first = i == 0 || bodyKeys[i - 1] != k;
+        if (first) start[k] = (uint32_t)i;
+        if (i == n - 1 || bodyKeys[i + 1] != k) end[k] = (uint32_t)(i + 1);
+        const uint32_t before = first ? 0u : bodyVals[i - 1];
+        prev[v] = !first && keys[before >> 1] >> 8 == keys[v >> 1] >> 8 ? (int)before : -1;
+    }
+}
+
 struct ColourView {
-    const uint32_t* keys;     // sorted (class << 8 | cell)
-    const uint32_t* vals;     // sorted manifold ids
-    const b3Contact4* contacts;
-    const int* manifoldPair;
-    const float* invMass;
+    const int* prev;           // per entry
     const int32_t* numManifolds;
-    int numBodies;
-    int* minRank;             // [4][numBodies]: first undecided slot per body this round
-    int* taken;               // [4][numBodies]: batch + 1 of the last batch that took the body
-    int* slotBatch;           // per slot: batch, -1 undecided, -2 waiting for the next batch
-    int* batchCount;          // [4]: batches per class
-    int* roundCount;          // [5]: undecided after a round (three in rotation: a block may
-                              // still read the last round's while block 0 clears the next),
-                              // then waiting after a batch (two)
-    uint32_t* bar;            // barrier count, generation
+    unsigned long long* used;  // per entry: batches taken on its body up to it, kDone when final
+    int* slotBatch;            // per slot
     int32_t* err;
     b3Counters* counters;
     int maxBatch;
 };
+constexpr unsigned long long kDone = 1ull << 63;  // the 63 bits below: batches 0 to 62
 
-__device__ __forceinline__ void slot_bodies(const ColourView& V, int s, int& cls, int& a, int& b) {
-    cls = (int)(V.keys[s] >> 8);
-    const b3Contact4& c = V.contacts[V.manifoldPair[V.vals[s]]];
-    const int A = abs(c.bodyAPtrAndSignBit), B = abs(c.bodyBPtrAndSignBit);
-    a = V.invMass[A] != 0.f ? A : -1;  // dynamic bodies only
-    b = V.invMass[B] != 0.f ? B : -1;
-}
-
-__global__ void __launch_bounds__(256) k_gs_colour(ColourView V) {
-    const int M = *V.numManifolds;
-    const int N = V.numBodies;
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int stride = gridDim.x * blockDim.x;
-    GridBarrier barrier(V.bar, V.err, V.counters, b3dev::kSpinLimit);
-    for (int s = tid; s < M; s += stride) V.slotBatch[s] = -1;
-    if (tid < 4) V.batchCount[tid] = 0;
-    if (tid < 5) V.roundCount[tid] = 0;
-    if (!barrier.wait()) return;
-    int round = 0;
-    for (int batch = 0;; ++batch) {
-        if (batch >= V.maxBatch) {
-            if (tid == 0) atomicExch(V.err, 2);
-            return;
-        }
-        for (;; ++round) {
-            // A: the first undecided slot of every dynamic body
-            if (tid == 0) V.roundCount[(round + 1) % 3] = 0;
-            for (int s = tid; s < M; s += stride) {
-                if (__ldcg(&V.slotBatch[s]) != -1) continue;
-                int cls, a, b;
-                slot_bodies(V, s, cls, a, b);
-                if (a >= 0) atomicMin(&V.minRank[cls * N + a], s);
-                if (b >= 0) atomicMin(&V.minRank[cls * N + b], s);
-            }
-            if (!barrier.wait()) return;
-            // B: join where first on every dynamic body
-            for (int s = tid; s < M; s += stride) {
-                if (__ldcg(&V.slotBatch[s]) != -1) continue;
-                int cls, a, b;
-                slot_bodies(V, s, cls, a, b);
-                if ((a < 0 || __ldcg(&V.minRank[cls * N + a]) == s) && (b < 0 || __ldcg(&V.minRank[cls * N + b]) == s)) {
-                    __stcg(&V.slotBatch[s], batch);
-                    if (a >= 0) __stcg(&V.taken[cls * N + a], batch + 1);
-                    if (b >= 0) __stcg(&V.taken[cls * N + b], batch + 1);
-                    atomicMax(&V.batchCount[cls], batch + 1);
-                }
-            }
-            if (!barrier.wait()) return;
-            // C: wait when a body was taken; clear the ranks; count the rest
-            int undecided = 0;
-            for (int s = tid; s < M; s += stride) {
-                const int sb = __ldcg(&V.slotBatch[s]);
-                if (sb != -1 && sb != -2 && sb != batch) continue;
-                int cls, a, b;
-                slot_bodies(V, s, cls, a, b);
-                if (a >= 0) __stcg(&V.minRank[cls * N + a], kNone);
-                if (b >= 0) __stcg(&V.minRank[cls * N + b], kNone);
-                if (sb != -1) continue;
-                if ((a >= 0 && __ldcg(&V.taken[cls * N + a]) == batch + 1) ||
-                    (b >= 0 && __ldcg(&V.taken[cls * N + b]) == batch + 1)) {
-                    __stcg(&V.slotBatch[s], -2);
-                } else {
-                    ++undecided;
-                }
-            }
-            if (undecided) atomicAdd(&V.roundCount[round % 3], undecided);
-            if (!barrier.wait()) return;
-            if (__ldcg(&V.roundCount[round % 3]) == 0) {
-                ++round;
-                break;
-            }
-        }
-        // the waiting slots are the next batch's undecided ones
-        if (tid == 0) V.roundCount[3 + ((batch + 1) & 1)] = 0;
-        int waiting = 0;
-        for (int s = tid; s < M; s += stride)
-            if (__ldcg(&V.slotBatch[s]) == -2) {
-                __stcg(&V.slotBatch[s], -1);
-                ++waiting;
-            }
-        if (waiting) atomicAdd(&V.roundCount[3 + (batch & 1)], waiting);
-        if (!barrier.wait()) return;
-        if (__ldcg(&V.roundCount[3 + (batch & 1)]) == 0) return;
+// The lowest batch from 63 on that no earlier entry of either chain has.
+__device__ int late_batch(const ColourView& V, int pa, int pb) {
+    __threadfence();
+    for (int b = 63;; ++b) {
+        bool taken = false;
+        for (int p = pa; p >= 0 && !taken; p = V.prev[p]) taken = __ldcg(&V.slotBatch[p >> 1]) == b;
+        for (int p = pb; p >= 0 && !taken; p = V.prev[p]) taken = __ldcg(&V.slotBatch[p >> 1]) == b;
+        if (!taken) return b;
     }
 }
 
-// world inverse inertia rows per body (zero for static bodies)
-__global__ void k_gs_inertia(b3::BodiesDev Bd, float4* __restrict__ Iw) {
+// One thread per slot, slots in order. A block hands batches on within its 256
+// slots through shared memory (most chains run through neighbouring slots: a
+// body's manifolds follow each other), other blocks read them from L2. The grid
+// is resident and its blocks go through the slots in order, so the first slot
+// without a batch always has all it waits for.
+constexpr int kColourThreads = 256;
+__global__ void __launch_bounds__(kColourThreads) k_gs_colour(ColourView V) {
+    __shared__ volatile unsigned long long local[2 * kColourThreads];
+    const int M = *V.numManifolds;
+    const int t = threadIdx.x;
+    for (int s0 = blockIdx.x * kColourThreads; s0 < M; s0 += gridDim.x * kColourThreads) {
+        const int s = s0 + t;
+        local[2 * t] = local[2 * t + 1] = 0ull;
+        __syncthreads();
+        bool done = s >= M;
+        const int pa = done ? -1 : V.prev[2 * s], pb = done ? -1 : V.prev[2 * s + 1];
+        unsigned long long ua = 0, ub = 0;
+        bool hasA = pa < 0, hasB = pb < 0;
+        auto look = [&](int p, unsigned long long& u) {
+            const int at = p - 2 * s0;
+            u = at >= 0 ? local[at] : b3dev::ld_acquire_u64(V.used + p);
+            return u != 0ull;
+        };
+        int spins = 0;
+        while (!__all_sync(0xffffffffu, done)) {
+            if (!done) {
+                if (!hasA) hasA = look(pa, ua);
+                if (!hasB) hasB = look(pb, ub);
+                if (hasA && hasB) {
+                    const unsigned long long free = ~(ua | ub) & (kDone - 1);
+                    int batch = free ? __ffsll((long long)free) - 1 : late_batch(V, pa, pb);
+                    if (batch >= V.maxBatch) {
+                        atomicExch(V.err, 2);
+                        batch = -1;
+                    }
+                    __stcg(&V.slotBatch[s], batch);
+                    if (batch >= 63) __threadfence();
+                    const unsigned long long mine = kDone | (batch >= 0 && batch < 63 ? 1ull << batch : 0ull);
+                    local[2 * t] = ua | mine;
+                    local[2 * t + 1] = ub | mine;
+                    b3dev::st_release_u64(V.used + 2 * s, ua | mine);
+                    b3dev::st_release_u64(V.used + 2 * s + 1, ub | mine);
+                    done = true;
+                } else if (++spins > kGsSpins || ((spins & 1023) == 0 && *(volatile int32_t*)V.err == 1)) {
+                    gave_up(V.err, V.counters);
+                    done = true;
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Place of each entry in its body's solve order: how many of the body's
+// entries have an earlier (class, batch), and how many there are. (No batch has
+// a body twice.)
+__global__ void k_gs_rank(const uint32_t* __restrict__ bodyKeys, const uint32_t* __restrict__ bodyVals,
+                          const uint32_t* __restrict__ keys, const int* __restrict__ slotBatch,
+                          const int32_t* __restrict__ numSides, int numBodies, const uint32_t* __restrict__ start,
+                          const uint32_t* __restrict__ end, int maxBatch, int2* __restrict__ place) {
+    const int n = *numSides;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t k = bodyKeys[i], v = bodyVals[i];
+        int2 r = make_int2(0, 0);
+        if (k < (uint32_t)numBodies) {
+            const uint32_t s = start[k], e = end[k];
+            auto order = [&](uint32_t at) { return (int)(keys[at >> 1] >> 8) * maxBatch + slotBatch[at >> 1]; };
+            const int mine = order(v);
+            for (uint32_t j = s; j < e; ++j) r.x += order(bodyVals[j]) < mine ? 1 : 0;
+            r.y = (int)(e - s);
+        }
+        place[v] = r;
+    }
+}
+
+// world inverse inertia rows per body (zero for static bodies), and the
+// velocities as the solve passes them on, (linear, angular) with version 0
+__global__ void k_gs_inertia(b3::BodiesDev Bd, float4* __restrict__ Iw, float4* __restrict__ vel) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= Bd.n) return;
     float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0, r2 = r0;
@@ -199,6 +248,8 @@ __global__ void k_gs_inertia(b3::BodiesDev Bd, float4* __restrict__ Iw) {
     Iw[3 * i + 0] = r0;
     Iw[3 * i + 1] = r1;
     Iw[3 * i + 2] = r2;
+    vel[2 * i] = f4(f3(Bd.linVel[i]));
+    vel[2 * i + 1] = f4(f3(Bd.angVel[i]));
 }
 
 struct M3 {
@@ -290,8 +341,9 @@ __global__ void k_gs_setup(const uint32_t* __restrict__ keys, const uint32_t* __
                            const int* __restrict__ slotBatch, const int32_t* __restrict__ numManifolds,
                            const uint32_t* __restrict__ groupOffset, uint32_t* __restrict__ groupFill,
                            const b3Contact4* __restrict__ contacts, const int* __restrict__ manifoldPair,
-                           b3::BodiesDev Bd, const float4* __restrict__ Iw, b3Constraint4* __restrict__ cs,
-                           int* __restrict__ slotOfManifold, SetupParams P) {
+                           b3::BodiesDev Bd, const float4* __restrict__ Iw, const int2* __restrict__ place,
+                           b3Constraint4* __restrict__ cs, int4* __restrict__ turn, int* __restrict__ slotOfManifold,
+                           SetupParams P) {
     const int M = *numManifolds;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < M; s += gridDim.x * blockDim.x) {
         const int cls = (int)(keys[s] >> 8);
@@ -304,6 +356,8 @@ __global__ void k_gs_setup(const uint32_t* __restrict__ keys, const uint32_t* __
         const int g = cls * P.maxBatch + batch;
         const int q = (int)(groupOffset[g] + atomicAdd(&groupFill[g], 1u));
         slotOfManifold[m] = q;
+        const int2 ta = place[2 * s], tb = place[2 * s + 1];
+        turn[q] = make_int4(ta.x, ta.y, tb.x, tb.y);
         const b3Contact4 c = contacts[manifoldPair[m]];
         const int A = abs(c.bodyAPtrAndSignBit), B = abs(c.bodyBPtrAndSignBit);
         const float imA = Bd.invMass[A], imB = Bd.invMass[B];
@@ -358,35 +412,48 @@ __global__ void k_gs_setup(const uint32_t* __restrict__ keys, const uint32_t* __
 }
 
 struct SolveView {
-    b3Constraint4* cs;
-    const uint32_t* groupOffset;  // [4 * maxBatch + 1]
-    const int* batchCount;        // [4]
-    int maxBatch;
+    b3Constraint4* cs;             // grouped by (class, batch)
+    const int4* turn;              // per constraint: place and count on A, on B
+    const int32_t* numManifolds;
+    float4* vel;                   // [bodies][2]: linear and angular velocity, w = version
     float4* pos;
     float4* linVel;
     float4* angVel;
     const float* invMass;
     const float4* Iw;
-    uint32_t* bar;
     int32_t* err;
     b3Counters* counters;
 };
 
-__device__ __forceinline__ float3 ldv(const float4* p) {
-    const float4 v = __ldcg(p);
-    return make_float3(v.x, v.y, v.z);
+// 16 bytes read or written as one: a velocity and its version.
+__device__ __forceinline__ float4 ld_whole(const float4* p) {
+    unsigned long long lo, hi;
+    asm volatile(
+        "{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+        : "=l"(lo), "=l"(hi)
+        : "l"(p)
+        : "memory");
+    return make_float4(__uint_as_float((uint32_t)lo), __uint_as_float((uint32_t)(lo >> 32)),
+                       __uint_as_float((uint32_t)hi), __uint_as_float((uint32_t)(hi >> 32)));
+}
+__device__ __forceinline__ void st_whole(float4* p, float4 v) {
+    const unsigned long long lo = __float_as_uint(v.x) | (unsigned long long)__float_as_uint(v.y) << 32;
+    const unsigned long long hi = __float_as_uint(v.z) | (unsigned long long)__float_as_uint(v.w) << 32;
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+                 "l"(lo), "l"(hi)
+                 : "memory");
 }
 
-// One constraint with the data that does not change during the solve:
-// its Constraint4 record and its bodies' positions, inverse masses and world
-// inverse inertias. The solve fetches the next batch's before each barrier,
-// so that after it only the velocities are still to be loaded.
+// One constraint with the data that does not change during the solve: its
+// Constraint4 record, its turn, and its bodies' inverse masses and world
+// inverse inertias (positions are read with the rest). All of it is fetched
+// before the wait, so that after it only the velocities are still to come.
 struct Pending {
-    int q;  // constraint index, -1 for none
     union {
         b3Constraint4 c;
         float4 raw[11];
     };
+    int4 turn;
     int A, B;
     float imA, imB;
     float3 posA, posB;
@@ -395,11 +462,10 @@ struct Pending {
 static_assert(sizeof(b3Constraint4) == 11 * sizeof(float4), "Constraint4 is 176 bytes");
 
 __device__ __forceinline__ void fetch(const SolveView& V, int q, Pending& P) {
-    P.q = q;
-    if (q < 0) return;
     const float4* src = reinterpret_cast<const float4*>(V.cs + q);
 #pragma unroll
     for (int k = 0; k < 11; ++k) P.raw[k] = src[k];
+    P.turn = __ldg(&V.turn[q]);
     P.A = (int)P.c.bodyA;
     P.B = (int)P.c.bodyB;
     P.imA = V.invMass[P.A];
@@ -410,23 +476,19 @@ __device__ __forceinline__ void fetch(const SolveView& V, int q, Pending& P) {
     P.IB = load_iw(V.Iw, P.B);
 }
 
-// the constraint, contact (phase 0) or friction (phase 1); a static
-// body's velocity is read and written as zero
-__device__ void solve_one(const SolveView& V, Pending& P, int phase) {
+// the constraint, contact (phase 0) or friction (phase 1), on its bodies'
+// velocities
+__device__ void solve_one(const SolveView& V, Pending& P, int q, int phase, float3& vA, float3& wA, float3& vB,
+                          float3& wB) {
     b3Constraint4& c = P.c;
-    const int A = P.A, B = P.B;
     const float imA = P.imA, imB = P.imB;
     const bool dA = imA != 0.f, dB = imB != 0.f;
-    float3 vA = dA ? ldv(&V.linVel[A]) : make_float3(0.f, 0.f, 0.f);
-    float3 wA = dA ? ldv(&V.angVel[A]) : make_float3(0.f, 0.f, 0.f);
-    float3 vB = dB ? ldv(&V.linVel[B]) : make_float3(0.f, 0.f, 0.f);
-    float3 wB = dB ? ldv(&V.angVel[B]) : make_float3(0.f, 0.f, 0.f);
     const float3 posA = P.posA, posB = P.posB;
     const M3& IA = P.IA;
     const M3& IB = P.IB;
     const float3 lin = make_float3(c.linear[0], c.linear[1], c.linear[2]);
     const float3 n = -lin;
-    float4* dst = reinterpret_cast<float4*>(V.cs + P.q);
+    float4* dst = reinterpret_cast<float4*>(V.cs + q);
     if (phase == 0) {
         // solveContact (ST/solveContact.cl:272-309): impulses clamped to [0, inf)
 #pragma unroll
@@ -478,60 +540,82 @@ __device__ void solve_one(const SolveView& V, Pending& P, int phase) {
         }
         dst[9] = P.raw[9];  // fJacCoeffInv, fAppliedRambdaDt
     }
-    __stcg(&V.linVel[A], dA ? make_float4(vA.x, vA.y, vA.z, 0.f) : make_float4(0.f, 0.f, 0.f, 0.f));
-    __stcg(&V.angVel[A], dA ? make_float4(wA.x, wA.y, wA.z, 0.f) : make_float4(0.f, 0.f, 0.f, 0.f));
-    __stcg(&V.linVel[B], dB ? make_float4(vB.x, vB.y, vB.z, 0.f) : make_float4(0.f, 0.f, 0.f, 0.f));
-    __stcg(&V.angVel[B], dB ? make_float4(wB.x, wB.y, wB.z, 0.f) : make_float4(0.f, 0.f, 0.f, 0.f));
 }
 
-// (class, batch) group of step j of an iteration (classes in order, their
-// batches in order)
-__device__ __forceinline__ int group_of(int j, const int nb[4], int maxBatch) {
-    int cls = 0;
-    while (cls < 3 && j >= nb[cls]) {
-        j -= nb[cls];
-        ++cls;
-    }
-    return cls * maxBatch + j;
-}
-
-__global__ void __launch_bounds__(256) k_gs_solve(SolveView V) {
-    GridBarrier barrier(V.bar, V.err, V.counters, b3dev::kSpinLimit);
+// Iterations in order, constraints in order; a thread has the same constraints
+// in every iteration, so their impulses are its own. Constraint q's turn on a
+// body comes when the body's velocity has version it * count + place; static
+// bodies take no turns: their velocity is read and written as zero. The warp's
+// lanes look in turn and solve as they can. The grid is resident and each
+// thread goes through its constraints in order, so the first one unsolved
+// always has its turn.
+__global__ void __launch_bounds__(128) k_gs_solve(SolveView V) {
+    const int M = *V.numManifolds;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int stride = gridDim.x * blockDim.x;
-    int nb[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) nb[c] = min(__ldcg(&V.batchCount[c]), V.maxBatch);
-    const int G = nb[0] + nb[1] + nb[2] + nb[3];  // batch steps per iteration
-    const int steps = 2 * kIterations * G;        // contact iterations, then friction
-    if (steps == 0) return;
-    int g = group_of(0, nb, V.maxBatch);
-    int q0 = (int)V.groupOffset[g], q1 = (int)V.groupOffset[g + 1];
-    Pending P;
-    fetch(V, q0 + tid < q1 ? q0 + tid : -1, P);
-    for (int k = 0; k < steps; ++k) {
-        const int phase = k / (kIterations * G);
-        if (P.q >= 0) solve_one(V, P, phase);
-        for (int q = q0 + tid + stride; q < q1; q += stride) {
-            Pending T;
-            fetch(V, q, T);
-            solve_one(V, T, phase);
+    if (*(volatile int32_t*)V.err) return;  // the colouring stopped: the records are not complete
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int it = 0; it < 2 * kIterations; ++it) {
+        const int phase = it / kIterations;
+        for (int q0 = tid & ~31; q0 < M; q0 += stride) {
+            const int q = q0 + (tid & 31);
+            bool done = q >= M;
+            Pending P;
+            if (!done) fetch(V, q, P);
+            const bool dA = !done && P.imA != 0.f, dB = !done && P.imB != 0.f;
+            const int turnA = done ? 0 : it * P.turn.y + P.turn.x, turnB = done ? 0 : it * P.turn.w + P.turn.z;
+            int spins = 0;
+            while (!__all_sync(0xffffffffu, done)) {
+                if (!done) {
+                    float4 lA = zero, aA = zero, lB = zero, aB = zero;
+                    if (dA) {
+                        lA = ld_whole(&V.vel[2 * P.A]);
+                        aA = ld_whole(&V.vel[2 * P.A + 1]);
+                    }
+                    if (dB) {
+                        lB = ld_whole(&V.vel[2 * P.B]);
+                        aB = ld_whole(&V.vel[2 * P.B + 1]);
+                    }
+                    const bool ready = (!dA || (__float_as_int(lA.w) == turnA && __float_as_int(aA.w) == turnA)) &&
+                                       (!dB || (__float_as_int(lB.w) == turnB && __float_as_int(aB.w) == turnB));
+                    if (ready) {
+                        float3 vA = f3(lA), wA = f3(aA), vB = f3(lB), wB = f3(aB);
+                        solve_one(V, P, q, phase, vA, wA, vB, wB);
+                        if (dA) {
+                            st_whole(&V.vel[2 * P.A], f4(vA, __int_as_float(turnA + 1)));
+                            st_whole(&V.vel[2 * P.A + 1], f4(wA, __int_as_float(turnA + 1)));
+                        }
+                        if (dB) {
+                            st_whole(&V.vel[2 * P.B], f4(vB, __int_as_float(turnB + 1)));
+                            st_whole(&V.vel[2 * P.B + 1], f4(wB, __int_as_float(turnB + 1)));
+                        }
+                        // the last turn of a body leaves its velocity
+                        if (!dA || turnA + 1 == 2 * kIterations * P.turn.y) {
+                            V.linVel[P.A] = dA ? f4(vA) : zero;
+                            V.angVel[P.A] = dA ? f4(wA) : zero;
+                        }
+                        if (!dB || turnB + 1 == 2 * kIterations * P.turn.w) {
+                            V.linVel[P.B] = dB ? f4(vB) : zero;
+                            V.angVel[P.B] = dB ? f4(wB) : zero;
+                        }
+                        done = true;
+                    } else if (++spins > kGsSpins || ((spins & 1023) == 0 && *(volatile int32_t*)V.err)) {
+                        gave_up(V.err, V.counters);
+                        done = true;
+                    } else if (spins > 4) {
+                        __nanosleep(50);
+                    }
+                }
+            }
         }
-        // the next batch's records and static body data: no thread of this
-        // batch writes them (a record belongs to its own thread)
-        if (k + 1 < steps) {
-            g = group_of((k + 1) % G, nb, V.maxBatch);
-            q0 = (int)V.groupOffset[g];
-            q1 = (int)V.groupOffset[g + 1];
-            fetch(V, q0 + tid < q1 ? q0 + tid : -1, P);
-        }
-        if (!barrier.wait()) return;
     }
 }
 
-int cooperative_grid(const void* kern, int threads, int numSMs, long long work) {
+// Blocks of a resident grid: at most perSm on each SM, and no more than the work.
+int cooperative_grid(const void* kern, int threads, int numSMs, int perSm, long long work) {
     int occ = 1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, 0) != cudaSuccess || occ < 1) occ = 1;
+    occ = std::min(occ, perSm);
     const long long want = std::max<long long>(1, (work + threads - 1) / threads);
     return (int)std::min<long long>((long long)numSMs * occ, want);
 }
@@ -571,38 +655,54 @@ int launch_gs_solver(b3World_t* w, cudaStream_t st) {
                             d.incSortScratchBytes, d.scalars + S_ERR, st, &alt, w->ctx->numSMs));
     const uint32_t* keys = alt ? d.incKeysAlt : d.incKeys;
     const uint32_t* vals = alt ? d.incValsAlt : d.incVals;
-    // 2. colouring
-    B3_CUDA(cudaMemsetAsync(d.gsMinRank, 0x7f, sizeof(int) * 4 * (size_t)N, st));  // 0x7f7f7f7f: no rank
-    B3_CUDA(cudaMemsetAsync(d.gsTaken, 0, sizeof(int) * 4 * (size_t)N, st));
-    B3_CUDA(cudaMemsetAsync(d.scalars + S_BAR_COUNT, 0, sizeof(int32_t) * 2, st));
+    // 2. colouring. The Constraint4 records take 11 of a manifold's row streams;
+    // the entries' buffers lie in the others.
+    static_assert(11 * sizeof(float4) + 2 * (5 * sizeof(uint32_t) + sizeof(unsigned long long) + sizeof(int2)) +
+                          sizeof(int4) <= kSolverRowSlots * sizeof(float4),
+                  "the solver's buffers fit a manifold's rows");
+    const size_t c = (size_t)cap;
+    int4* turn = reinterpret_cast<int4*>(d.rows + 11 * c);
+    unsigned long long* used = reinterpret_cast<unsigned long long*>(turn + c);
+    int2* place = reinterpret_cast<int2*>(used + 2 * c);
+    uint32_t* bodyKeys = reinterpret_cast<uint32_t*>(place + 2 * c);
+    uint32_t* bodyVals = bodyKeys + 2 * c;
+    uint32_t* bodyKeysAlt = bodyVals + 2 * c;
+    uint32_t* bodyValsAlt = bodyKeysAlt + 2 * c;
+    int* prev = reinterpret_cast<int*>(bodyValsAlt + 2 * c);
+    int32_t* numSides = d.scalars + S_NUM_INC;
+    k_gs_sides<<<g, 256, 0, st>>>(vals, d.contacts, d.manifoldPair, d.invMass, M, N, bodyKeys, bodyVals, d.gsSlotBatch,
+                                  used, numSides);
+    B3_CHECK_LAUNCH();
+    bool altB = false;
+    B3_TRY(radix_sort_pairs(bodyKeys, bodyVals, bodyKeysAlt, bodyValsAlt, numSides, 2LL * cap, w->bodyBits,
+                            d.incSortScratch, d.incSortScratchBytes, d.scalars + S_ERR, st, &altB, w->ctx->numSMs));
+    if (altB) {
+        std::swap(bodyKeys, bodyKeysAlt);
+        std::swap(bodyVals, bodyValsAlt);
+    }
+    k_gs_links<<<g, 256, 0, st>>>(bodyKeys, bodyVals, keys, numSides, N, d.bodyIncStart, d.bodyIncEnd, prev);
+    B3_CHECK_LAUNCH();
     ColourView CV;
-    CV.keys = keys;
-    CV.vals = vals;
-    CV.contacts = d.contacts;
-    CV.manifoldPair = d.manifoldPair;
-    CV.invMass = d.invMass;
+    CV.prev = prev;
     CV.numManifolds = M;
-    CV.numBodies = N;
-    CV.minRank = d.gsMinRank;
-    CV.taken = d.gsTaken;
+    CV.used = used;
     CV.slotBatch = d.gsSlotBatch;
-    CV.batchCount = d.gsBatchCount;
-    CV.roundCount = d.gsBatchCount + 4;  // 5 more ints
-    CV.bar = (uint32_t*)(d.scalars + S_BAR_COUNT);
     CV.err = d.scalars + S_ERR;
     CV.counters = d.counters;
     CV.maxBatch = maxBatch;
+    // Resident threads are the slots (constraints) looked ahead of the first one
+    // undone. Colouring, 196 K and 900 K manifolds: 1 block an SM 747 / 3,779
+    // us, 2 blocks 434 / 2,290, 4 blocks 334 / 1,411, 8 blocks 207 / 840. Solve:
+    // 1 block (of 128) 587 / 1,269 us, 2 blocks 505 / 1,052, 3 blocks 522 /
+    // 1,044. solverMode 1 (the narrow width) halves both.
+    const int narrow = w->solverMode == 1 ? 2 : 1;
     const long long estM = std::min<long long>((long long)cap, 3LL * N);
     {
-        // the narrow width of the solve (solverMode 1) also narrows the
-        // colouring: each round passes over every slot, but costs three
-        // barriers
-        const int grid = cooperative_grid((const void*)k_gs_colour, 256, w->ctx->numSMs,
-                                          w->solverMode == 1 ? estM / 8 : estM);
+        const int grid = cooperative_grid((const void*)k_gs_colour, kColourThreads, w->ctx->numSMs, 8 / narrow, estM);
         void* args[] = {&CV};
-        B3_TRY(launch_cooperative((const void*)k_gs_colour, grid, 256, args, st));
+        B3_TRY(launch_cooperative((const void*)k_gs_colour, grid, kColourThreads, args, st));
     }
-    // 3. groups (class, batch): counts, offsets, constraints
+    // 3. groups (class, batch): counts, offsets, turns, constraints
     const int groups = 4 * maxBatch;
     B3_CUDA(cudaMemsetAsync(d.gsGroupCount, 0, sizeof(uint32_t) * groups, st));
     B3_CUDA(cudaMemsetAsync(d.gsGroupFill, 0, sizeof(uint32_t) * groups, st));
@@ -610,38 +710,36 @@ int launch_gs_solver(b3World_t* w, cudaStream_t st) {
     B3_CHECK_LAUNCH();
     k_gs_offsets<<<1, 1024, 0, st>>>(d.gsGroupCount, d.gsGroupOffset, groups);
     B3_CHECK_LAUNCH();
-    k_gs_inertia<<<(N + 255) / 256, 256, 0, st>>>(w->bodiesDev(), d.gsInertia);
+    k_gs_rank<<<g, 256, 0, st>>>(bodyKeys, bodyVals, keys, d.gsSlotBatch, numSides, N, d.bodyIncStart, d.bodyIncEnd,
+                                 maxBatch, place);
+    B3_CHECK_LAUNCH();
+    k_gs_inertia<<<(N + 255) / 256, 256, 0, st>>>(w->bodiesDev(), d.gsInertia, d.gsVel);
     B3_CHECK_LAUNCH();
     SetupParams SP;
     SP.dtInv = 1.f / w->sim.dt;
     SP.maxBatch = maxBatch;
     k_gs_setup<<<g, 128, 0, st>>>(keys, vals, d.gsSlotBatch, M, d.gsGroupOffset, d.gsGroupFill, d.contacts,
-                                  d.manifoldPair, w->bodiesDev(), d.gsInertia, d.gsConstraints, d.gsSlotOfManifold,
-                                  SP);
+                                  d.manifoldPair, w->bodiesDev(), d.gsInertia, place, d.gsConstraints, turn,
+                                  d.gsSlotOfManifold, SP);
     B3_CHECK_LAUNCH();
     // 4. Gauss-Seidel iterations
-    B3_CUDA(cudaMemsetAsync(d.scalars + S_BAR_COUNT, 0, sizeof(int32_t) * 2, st));
     SolveView SV;
     SV.cs = d.gsConstraints;
-    SV.groupOffset = d.gsGroupOffset;
-    SV.batchCount = d.gsBatchCount;
-    SV.maxBatch = maxBatch;
+    SV.turn = turn;
+    SV.numManifolds = M;
+    SV.vel = d.gsVel;
     SV.pos = d.pos;
     SV.linVel = d.linVel;
     SV.angVel = d.angVel;
     SV.invMass = d.invMass;
     SV.Iw = d.gsInertia;
-    SV.bar = (uint32_t*)(d.scalars + S_BAR_COUNT);
     SV.err = d.scalars + S_ERR;
     SV.counters = d.counters;
     {
-        // a batch holds a fraction of the manifolds, and fewer blocks make
-        // each grid barrier cheaper: the autotuner picks the width
-        // (solverMode 0: manifolds / 8 threads, 1: manifolds / 64)
         const void* kg = (const void*)k_gs_solve;
-        const int grid = cooperative_grid(kg, 256, w->ctx->numSMs, estM / (w->solverMode == 1 ? 64 : 8));
+        const int grid = cooperative_grid(kg, 128, w->ctx->numSMs, 2 / narrow, estM);
         void* args[] = {&SV};
-        B3_TRY(launch_cooperative(kg, grid, 256, args, st));
+        B3_TRY(launch_cooperative(kg, grid, 128, args, st));
     }
     return B3_OK;
 }

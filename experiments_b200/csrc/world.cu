@@ -78,7 +78,7 @@ void free_all(b3::DevBuffers& d) {
                     d.bodyIncEnd, d.rows, d.incPos, d.copies,
                     d.scalars, d.counters, d.sortScratch, d.incSortScratch, d.scanScratch,
                     d.worldStats, d.worldMStart, d.worldMEnd, d.gsCell, d.gsSlotBatch,
-                    d.gsSlotOfManifold, d.gsMinRank, d.gsTaken, d.gsBatchCount, d.gsGroupCount, d.gsGroupFill,
+                    d.gsSlotOfManifold, d.gsVel, d.gsGroupCount, d.gsGroupFill,
                     d.gsGroupOffset, d.gsInertia};  // gsConstraints shares the row storage
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -671,8 +671,7 @@ static int ensure_capacity(b3World w) {
         B3_TRY(dalloc(d.bodyIncStart, nb));
         B3_TRY(dalloc(d.bodyIncEnd, nb));
         if (w->gs) {
-            B3_TRY(dalloc(d.gsMinRank, 4 * (size_t)nb));
-            B3_TRY(dalloc(d.gsTaken, 4 * (size_t)nb));
+            B3_TRY(dalloc(d.gsVel, 2 * (size_t)nb));
             B3_TRY(dalloc(d.gsInertia, 3 * (size_t)nb));
         }
         d.sortScratchBytes = b3::radix_scratch_bytes(nb, w->keyBits);
@@ -706,7 +705,6 @@ static int ensure_capacity(b3World w) {
             B3_TRY(dalloc(d.gsCell, c));
             B3_TRY(dalloc(d.gsSlotBatch, c));
             B3_TRY(dalloc(d.gsSlotOfManifold, c));
-            B3_TRY(dalloc(d.gsBatchCount, 16));
             B3_TRY(dalloc(d.gsGroupCount, 4 * (size_t)b3::kGsMaxBatch));
             B3_TRY(dalloc(d.gsGroupFill, 4 * (size_t)b3::kGsMaxBatch));
             B3_TRY(dalloc(d.gsGroupOffset, 4 * (size_t)b3::kGsMaxBatch + 1));

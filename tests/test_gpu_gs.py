@@ -165,3 +165,47 @@ def test_adjoint_form_refuses_the_batched_solver(ctx, scene_cache):
     w, _ = make_pair(ctx, scene_cache["column"], flags=GS)
     with pytest.raises(b3.B3Error):
         b3.Adjoint(w, 2, 1)
+
+
+@pytest.mark.parametrize("n,plate", [(1, False), (70, False), (600, True), (9000, False)])
+def test_colouring_over_block_edges_and_long_chains(ctx, n, plate):
+    """Lattices of touching cubes below, at and well past one block of slots;
+    with `plate`, a dynamic slab that hundreds of manifolds share, whose batches
+    go past the 63 that one word holds. The batches are the oracle's."""
+    side = max(1, int(round((2.0 * n) ** (1 / 3))))
+    if plate:
+        side = 25
+    i = np.arange(n)
+    pos = np.stack([(i % side) * 1.02, 0.49 + (i // (side * side)) * 0.99, (i // side % side) * 1.02], 1)
+    quat = scenes.yaw_quat(scenes.uniform(5, 2, n, 0.0, 0.3))
+    shapes = [scenes.box_vertices(100.0, 0.5, 100.0), scenes.box_vertices(0.5, 0.5, 0.5),
+              scenes.box_vertices(14.0, 0.25, 14.0)]
+    sid, mass = np.ones(n, np.int32), scenes.uniform(5, 3, n, 0.5, 2.0)
+    if plate:
+        pos[:, 1] += 0.49
+        pos = np.concatenate([pos, [[12.0, 0.24, 12.0]]])
+        quat = np.concatenate([quat, [[0, 0, 0, 1.0]]])
+        sid, mass = np.append(sid, 2), np.append(mass, 80.0)
+    b = scenes._concat([scenes.ground(), scenes._bodies(sid, mass, pos, quat, np.full(len(sid), 0.6),
+                                                        np.zeros(len(sid)))])
+    sc = scenes.Scene(name="lattice", shapes=shapes, num_worlds=1, config=dict(cellSize=1.0, gridDims=(64, 16, 64)), **b)
+    w, o = make_pair(ctx, sc, flags=GS)
+    for s in ("aabbs", "broadphase", "narrowphase", "solve"):
+        w.stage(s)
+    g, c = w.gs_batches(), w.contacts()
+    assert len(g) == len(c["bodyA"]) and w.counters()["timeouts"] == 0
+    # the sequential greedy pass in (class, cell, manifold) order: the lowest
+    # batch that no earlier manifold on the same dynamic bodies of the class has
+    dyn = np.asarray(sc.mass) > 0
+    cls = (g[:, 0] & 1) + 2 * ((g[:, 0] // 16) & 1)
+    seen = {}
+    for m in np.lexsort((np.arange(len(g)), g[:, 0], cls)):
+        bodies = [(int(cls[m]), x) for x in (abs(int(c["bodyA"][m])), abs(int(c["bodyB"][m]))) if dyn[x]]
+        taken = set().union(*[seen.get(x, set()) for x in bodies]) if bodies else set()
+        want = next(k for k in range(len(taken) + 1) if k not in taken)
+        assert int(g[m, 1]) == want, m
+        for x in bodies:
+            seen.setdefault(x, set()).add(want)
+    if plate:
+        assert g[:, 1].max() > 70
+    w.close()
