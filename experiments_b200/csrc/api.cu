@@ -115,27 +115,15 @@ extern "C" int b3_fill_int2(b3Context ctx, int32_t* d_dst_int2, int32_t x, int32
                          as_stream(stream));
 }
 
-// scratch layout for primitive calls: [n (int32) at 0][pad to 256][payload]
-static int prim_scratch(b3Context ctx, size_t payload, int64_t n, cudaStream_t st, int32_t** n_dev,
-                        int32_t** err, void** body) {
+// scratch layout for primitive calls: [error flag, total (one word each)]
+// [pad to 256][payload]; the flag is cleared on the stream. The element count
+// goes to the kernels by value.
+static int prim_scratch(b3Context ctx, size_t payload, cudaStream_t st, int32_t** err, void** body) {
     if (ctx->device < 0) return B3_ERR_NO_DEVICE;
     B3_TRY(ctx->ensureScratch(256 + payload));
-    *n_dev = (int32_t*)ctx->scratch;
-    *err = *n_dev + 1;
+    *err = (int32_t*)ctx->scratch;
     *body = (unsigned char*)ctx->scratch + 256;
-    const int32_t hv[2] = {(int32_t)n, 0};
-    B3_CUDA(cudaMemcpyAsync(ctx->scratch, hv, sizeof(hv), cudaMemcpyHostToDevice, st));
-    return B3_OK;
-}
-
-static int check_err_flag(int32_t* err, cudaStream_t st) {
-    int32_t e = 0;
-    B3_CUDA(cudaMemcpyAsync(&e, err, sizeof(e), cudaMemcpyDeviceToHost, st));
-    B3_CUDA(cudaStreamSynchronize(st));
-    if (e) {
-        b3_set_error("a bounded device wait gave up");
-        return B3_ERR_TIMEOUT;
-    }
+    B3_CUDA(cudaMemsetAsync(ctx->scratch, 0, 2 * sizeof(int32_t), st));
     return B3_OK;
 }
 
@@ -143,17 +131,23 @@ extern "C" int b3_prefix_scan_u32(b3Context ctx, const uint32_t* d_src, uint32_t
                                   uint32_t* d_sum, uint32_t* h_sum, void* stream) {
     if (!ctx || n < 0 || n > (int64_t)0x7fffffff || (n > 0 && (!d_src || !d_dst))) return B3_ERR_INVALID_ARG;
     cudaStream_t st = as_stream(stream);
-    int32_t *n_dev, *err;
+    int32_t* err;
     void* body;
     const size_t sb = b3::scan_scratch_bytes(n);
-    B3_TRY(prim_scratch(ctx, sb + 64, n, st, &n_dev, &err, &body));
-    uint32_t* tot = (uint32_t*)((unsigned char*)body + sb);
+    B3_TRY(prim_scratch(ctx, sb, st, &err, &body));
+    uint32_t* tot = (uint32_t*)(err + 1);
     // in-place scans are safe: each tile reads its input before it writes
-    B3_TRY(b3::exclusive_scan_u32(d_src, d_dst, n_dev, n, tot, body, sb, err, st, ctx->numSMs));
+    B3_TRY(b3::exclusive_scan_u32(d_src, d_dst, nullptr, n, tot, body, sb, err, st, ctx->numSMs));
     if (d_sum) B3_CUDA(cudaMemcpyAsync(d_sum, tot, 4, cudaMemcpyDeviceToDevice, st));
     if (h_sum) {
-        B3_CUDA(cudaMemcpyAsync(h_sum, tot, 4, cudaMemcpyDeviceToHost, st));
-        return check_err_flag(err, st);
+        int32_t hv[2] = {0, 0};  // the flag and the total, one copy
+        B3_CUDA(cudaMemcpyAsync(hv, err, sizeof(hv), cudaMemcpyDeviceToHost, st));
+        B3_CUDA(cudaStreamSynchronize(st));
+        *h_sum = (uint32_t)hv[1];
+        if (hv[0]) {
+            b3_set_error("a bounded device wait gave up");
+            return B3_ERR_TIMEOUT;
+        }
     }
     return B3_OK;
 }
@@ -166,13 +160,13 @@ static int sort_impl(b3Context ctx, uint32_t* d_keys, uint32_t* d_values, int64_
     cudaStream_t st = as_stream(stream);
     const size_t rb = b3::radix_scratch_bytes(n, key_bits);
     const size_t alt = ((size_t)n * 4 + 255) / 256 * 256;
-    int32_t *n_dev, *err;
+    int32_t* err;
     void* body;
-    B3_TRY(prim_scratch(ctx, rb + 2 * alt, n, st, &n_dev, &err, &body));
+    B3_TRY(prim_scratch(ctx, rb + 2 * alt, st, &err, &body));
     uint32_t* kalt = (uint32_t*)((unsigned char*)body + rb);
     uint32_t* valt = d_values ? (uint32_t*)((unsigned char*)body + rb + alt) : nullptr;
     bool in_alt = false;
-    B3_TRY(b3::radix_sort_pairs(d_keys, d_values, kalt, valt, n_dev, n, key_bits, body, rb, err, st,
+    B3_TRY(b3::radix_sort_pairs(d_keys, d_values, kalt, valt, nullptr, n, key_bits, body, rb, err, st,
                                 &in_alt, ctx->numSMs));
     if (in_alt) {
         B3_CUDA(cudaMemcpyAsync(d_keys, kalt, 4 * (size_t)n, cudaMemcpyDeviceToDevice, st));
@@ -211,12 +205,12 @@ extern "C" int b3_radix_sort32_kv_out(b3Context ctx, const uint32_t* d_keys_in, 
     }
     const size_t rb = b3::radix_scratch_bytes(n, key_bits);
     const size_t alt = ((size_t)n * 4 + 255) / 256 * 256;
-    int32_t *n_dev, *err;
+    int32_t* err;
     void* body;
-    B3_TRY(prim_scratch(ctx, rb + 2 * alt, n, st, &n_dev, &err, &body));
+    B3_TRY(prim_scratch(ctx, rb + 2 * alt, st, &err, &body));
     uint32_t* ktmp = (uint32_t*)((unsigned char*)body + rb);
     uint32_t* vtmp = d_values_in ? (uint32_t*)((unsigned char*)body + rb + alt) : nullptr;
-    return b3::radix_sort_kv_out(d_keys_in, d_values_in, d_keys_out, d_values_out, ktmp, vtmp, n_dev, n, key_bits,
+    return b3::radix_sort_kv_out(d_keys_in, d_values_in, d_keys_out, d_values_out, ktmp, vtmp, nullptr, n, key_bits,
                                  body, rb, err, st, ctx->numSMs);
 }
 
@@ -232,13 +226,13 @@ extern "C" int b3_radix_sort32_sortdata(b3Context ctx, int32_t* d_key_values, in
     if (n <= 1) return B3_OK;
     cudaStream_t st = as_stream(stream);
     const size_t rb = b3::radix_scratch_bytes(n, key_bits);
-    int32_t *n_dev, *err;
+    int32_t* err;
     void* body;
-    B3_TRY(prim_scratch(ctx, rb + 8 * (size_t)n, n, st, &n_dev, &err, &body));
+    B3_TRY(prim_scratch(ctx, rb + 8 * (size_t)n, st, &err, &body));
     uint2* kv = reinterpret_cast<uint2*>(d_key_values);
     uint2* alt = (uint2*)((unsigned char*)body + rb);  // rb is a multiple of 256
     bool in_alt = false;
-    B3_TRY(b3::radix_sort_interleaved(kv, alt, n_dev, n, key_bits, body, rb, err, st, &in_alt, ctx->numSMs));
+    B3_TRY(b3::radix_sort_interleaved(kv, alt, nullptr, n, key_bits, body, rb, err, st, &in_alt, ctx->numSMs));
     if (in_alt) B3_CUDA(cudaMemcpyAsync(kv, alt, 8 * (size_t)n, cudaMemcpyDeviceToDevice, st));
     return B3_OK;
 }
@@ -252,10 +246,7 @@ extern "C" int b3_bound_search(b3Context ctx, const uint32_t* d_sorted_keys, int
     cudaStream_t st = as_stream(stream);
     if (mode == 2) B3_TRY(b3::fill_u32(d_dst, 0u, n_dst, st));
     if (n_src == 0) return B3_OK;
-    int32_t *n_dev, *err;
-    void* body;
-    B3_TRY(prim_scratch(ctx, 0, n_src, st, &n_dev, &err, &body));
-    return b3::bound_search(d_sorted_keys, n_dev, n_src, d_dst, n_dst, mode, st);
+    return b3::bound_search(d_sorted_keys, nullptr, n_src, d_dst, n_dst, mode, st);
 }
 
 extern "C" int b3_bound_search_sortdata(b3Context ctx, const int32_t* d_sorted_key_values, int64_t n_src,
@@ -267,9 +258,6 @@ extern "C" int b3_bound_search_sortdata(b3Context ctx, const int32_t* d_sorted_k
     cudaStream_t st = as_stream(stream);
     if (mode == 2) B3_TRY(b3::fill_u32(d_dst, 0u, n_dst, st));
     if (n_src == 0) return B3_OK;
-    int32_t *n_dev, *err;
-    void* body;
-    B3_TRY(prim_scratch(ctx, 0, n_src, st, &n_dev, &err, &body));
-    return b3::bound_search_interleaved(reinterpret_cast<const uint2*>(d_sorted_key_values), n_dev, n_src, d_dst,
+    return b3::bound_search_interleaved(reinterpret_cast<const uint2*>(d_sorted_key_values), nullptr, n_src, d_dst,
                                         n_dst, mode, st);
 }

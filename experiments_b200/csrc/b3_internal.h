@@ -54,7 +54,8 @@ static inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStre
 // ---------------------------------------------------------------------------
 // Device-wide primitives (implemented in primitives.cu). All take a device
 // side element count (n_dev) so they can be captured in CUDA graphs without
-// host synchronisation; n_max bounds the grid and scratch sizes.
+// host synchronisation; n_max bounds the grid and scratch sizes, and is the
+// count itself where n_dev is null. n_expect (0: n_max) is the likely count.
 // ---------------------------------------------------------------------------
 namespace b3 {
 
@@ -65,12 +66,11 @@ constexpr int kDefaultSpinLimit = 1 << 22;
 // Onesweep radix sort scratch: returns bytes for n_max elements.
 size_t radix_scratch_bytes(int64_t n_max, int key_bits);
 // Sort (keys, vals) of device count *n_dev (<= n_max). The sorted result
-// ends in (keys_alt, vals_alt) when the number of passes is odd, else in
-// (keys, vals); *result_in_alt tells which. vals may be null (keys only).
+// ends in (keys_alt, vals_alt) or in (keys, vals); *result_in_alt tells which. vals may be null (keys only).
 int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt,
                      const int32_t* n_dev, int64_t n_max, int key_bits, void* scratch,
                      size_t scratch_bytes, int32_t* err_flag, cudaStream_t st, bool* result_in_alt,
-                     int numSMs);
+                     int numSMs, int64_t n_expect = 0);
 
 // Out-of-place sort: (keys_in, vals_in) are only read; the sorted result
 // lands in (keys_out, vals_out); (keys_tmp, vals_tmp) hold the passes in
@@ -125,6 +125,50 @@ __device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned l
 // short back-off (well under a second), after which the waiter records an
 // error and proceeds instead of hanging the GPU.
 constexpr int kSpinLimit = b3::kDefaultSpinLimit;
+
+// Grid barrier of a cooperative launch. Blocks add to one 64-bit word with a
+// release and poll it with an acquire until all of this round have arrived;
+// the count only grows within a launch (the host clears it before), so no
+// second word has to be released and a wait ends one L2 round trip after the
+// last arrival. A waiter gives up after spinLimit polls: it sets *err, counts
+// a timeout and sets the word's top bit, on which every block leaves at this
+// or its next barrier, so the launch always ends. An error that was set
+// before the launch ends it at the first barrier.
+struct GridBarrier {
+    unsigned long long* word;
+    unsigned long long target;
+    int32_t* err;
+    b3Counters* counters;
+    int spinLimit;
+    int before;  // thread 0: *err at the kernel's start
+
+    __device__ __forceinline__ GridBarrier(uint32_t* w, int32_t* e, b3Counters* c, int limit)
+        : word(reinterpret_cast<unsigned long long*>(w)), target(0), err(e), counters(c), spinLimit(limit), before(0) {
+        if (threadIdx.x == 0) before = *(volatile int32_t*)e;
+    }
+    __device__ __forceinline__ bool wait() {
+        constexpr unsigned long long kAbort = 1ull << 63;
+        int ok = 1;
+        target += gridDim.x;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(1ull) : "memory");
+            unsigned long long v = ld_acquire_u64(word);
+            for (int spins = 0; !(v & kAbort) && v < target; v = ld_acquire_u64(word)) {
+                if (++spins > spinLimit) {
+                    atomicExch(err, 1);
+                    if (counters) atomicAdd(&counters->timeouts, 1);
+                    atomicOr(word, kAbort);
+                    v = kAbort;
+                    break;
+                }
+                if (spins > 16) __nanosleep(64);
+            }
+            ok = !(v & kAbort) && before == 0;
+        }
+        return __syncthreads_and(ok) != 0;
+    }
+};
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;

@@ -652,7 +652,7 @@ int launch_gs_solver(b3World_t* w, cudaStream_t st) {
     B3_CHECK_LAUNCH();
     bool alt = false;
     B3_TRY(radix_sort_pairs(d.incKeys, d.incVals, d.incKeysAlt, d.incValsAlt, M, cap, 10, d.incSortScratch,
-                            d.incSortScratchBytes, d.scalars + S_ERR, st, &alt, w->ctx->numSMs));
+                            d.incSortScratchBytes, d.scalars + S_ERR, st, &alt, w->ctx->numSMs, 3LL * N));
     const uint32_t* keys = alt ? d.incKeysAlt : d.incKeys;
     const uint32_t* vals = alt ? d.incValsAlt : d.incVals;
     // 2. colouring. The Constraint4 records take 11 of a manifold's row streams;
@@ -675,7 +675,8 @@ int launch_gs_solver(b3World_t* w, cudaStream_t st) {
     B3_CHECK_LAUNCH();
     bool altB = false;
     B3_TRY(radix_sort_pairs(bodyKeys, bodyVals, bodyKeysAlt, bodyValsAlt, numSides, 2LL * cap, w->bodyBits,
-                            d.incSortScratch, d.incSortScratchBytes, d.scalars + S_ERR, st, &altB, w->ctx->numSMs));
+                            d.incSortScratch, d.incSortScratchBytes, d.scalars + S_ERR, st, &altB, w->ctx->numSMs,
+                            6LL * N));
     if (altB) {
         std::swap(bodyKeys, bodyKeysAlt);
         std::swap(bodyVals, bodyValsAlt);

@@ -668,7 +668,7 @@ int launch_manifolds(b3World_t* w, cudaStream_t st) {
     bool alt = false;
     B3_TRY(radix_sort_pairs(w->d.incKeys, w->d.incVals, w->d.incKeysAlt, w->d.incValsAlt,
                             w->d.scalars + S_NUM_INC, 2LL * cap, w->bodyBits, w->d.incSortScratch,
-                            w->d.incSortScratchBytes, w->d.scalars + S_ERR, st, &alt, w->ctx->numSMs));
+                            w->d.incSortScratchBytes, w->d.scalars + S_ERR, st, &alt, w->ctx->numSMs, 6LL * N));
     k_body_ranges<<<g, 256, 0, st>>>(alt ? w->d.incKeysAlt : w->d.incKeys, alt ? w->d.incValsAlt : w->d.incVals,
                                     w->d.scalars + S_NUM_INC, w->d.bodyIncStart, w->d.bodyIncEnd, w->d.incPos, N);
     B3_CHECK_LAUNCH();

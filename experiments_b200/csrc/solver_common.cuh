@@ -78,49 +78,7 @@ __device__ __forceinline__ void plane_space(float3 n, float3& p, float3& q) {
 // ---------------------------------------------------------------------------
 // Persistent-kernel helpers
 // ---------------------------------------------------------------------------
-// Grid barrier of a cooperative launch. Blocks add to one 64-bit word with a
-// release and poll it with an acquire until all of this round have arrived;
-// the count only grows within a launch (the host clears it before), so no
-// second word has to be released and a wait ends one L2 round trip after the
-// last arrival. A waiter gives up after spinLimit polls: it sets *err, counts
-// a timeout and sets the word's top bit, on which every block leaves at this
-// or its next barrier, so the launch always ends. An error that was set
-// before the launch ends it at the first barrier.
-struct GridBarrier {
-    unsigned long long* word;
-    unsigned long long target;
-    int32_t* err;
-    b3Counters* counters;
-    int spinLimit;
-    int before;  // thread 0: *err at the kernel's start
-
-    __device__ __forceinline__ GridBarrier(uint32_t* w, int32_t* e, b3Counters* c, int limit)
-        : word(reinterpret_cast<unsigned long long*>(w)), target(0), err(e), counters(c), spinLimit(limit), before(0) {
-        if (threadIdx.x == 0) before = *(volatile int32_t*)e;
-    }
-    __device__ __forceinline__ bool wait() {
-        constexpr unsigned long long kAbort = 1ull << 63;
-        int ok = 1;
-        target += gridDim.x;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(1ull) : "memory");
-            unsigned long long v = b3dev::ld_acquire_u64(word);
-            for (int spins = 0; !(v & kAbort) && v < target; v = b3dev::ld_acquire_u64(word)) {
-                if (++spins > spinLimit) {
-                    atomicExch(err, 1);
-                    atomicAdd(&counters->timeouts, 1);
-                    atomicOr(word, kAbort);
-                    v = kAbort;
-                    break;
-                }
-                if (spins > 16) __nanosleep(64);
-            }
-            ok = !(v & kAbort) && before == 0;
-        }
-        return __syncthreads_and(ok) != 0;
-    }
-};
+using b3dev::GridBarrier;
 
 // Angular part of a row, r x axis, formed again in every phase: one multiply
 // and one fused multiply-add per component, by name.
