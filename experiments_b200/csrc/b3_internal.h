@@ -67,6 +67,7 @@ constexpr int kDefaultSpinLimit = 1 << 22;
 size_t radix_scratch_bytes(int64_t n_max, int key_bits);
 // Sort (keys, vals) of device count *n_dev (<= n_max). The sorted result
 // ends in (keys_alt, vals_alt) or in (keys, vals); *result_in_alt tells which. vals may be null (keys only).
+bool radix_result_in_alt(int64_t n_max, int key_bits);  // what *result_in_alt will be
 int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt,
                      const int32_t* n_dev, int64_t n_max, int key_bits, void* scratch,
                      size_t scratch_bytes, int32_t* err_flag, cudaStream_t st, bool* result_in_alt,

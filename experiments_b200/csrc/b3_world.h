@@ -102,7 +102,8 @@ struct DevBuffers {
     uint32_t* sapCount = nullptr;     // pairs per sorted proxy, then their offsets
     uint32_t* sapOffset = nullptr;
     uint32_t *keys = nullptr, *vals = nullptr, *keysAlt = nullptr, *valsAlt = nullptr;
-    uint2* cellTable = nullptr;    // (stamp, first sorted index) per (world, cell)
+    uint4* cellTable = nullptr;    // (stamp, first sorted index, end, -) per (world, cell)
+    float4* sortedAabb = nullptr;  // small bodies' (min, max) in sorted order
     int2* pairs = nullptr;
     // narrowphase
     b3Contact4* contacts = nullptr;   // one slot per pair

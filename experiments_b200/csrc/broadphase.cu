@@ -14,9 +14,11 @@
 //     gravity update (BB/broadphaseKernel.cl:163-213) into one pass over the
 //     float4 body streams; the AABB arithmetic uses non-contracting
 //     intrinsics so keys are bit-reproducible.
-//   * Cell starts live in a (stamp, index) table indexed by the full key,
+//   * Cells live in a (stamp, first, end) table indexed by the full key,
 //     so no per-step clear of the 128^3 cell array is needed (the reference
-//     clears 2M cells per step).
+//     clears 2M cells per step). The AABBs are copied into sorted order with
+//     it, so that a cell's candidates lie side by side and the search reads
+//     them without going through the body ids.
 //   * k_find_pairs searches the 27 neighbour cells exactly like
 //     findPairsInCell (bucket cap, id(other) < id(self), inclusive AABB test),
 //     adds a pass over the world's large bodies (kFindPairsLarge precedent,
@@ -113,13 +115,20 @@ k_aabb_hash(b3::BodiesDev B, const float4* __restrict__ localAabb, GridParams g,
     }
 }
 
-// kFindCellStart (G3/bt3dGridBroadphaseOCL.cl:61-87) into a stamped table.
-__global__ void k_cell_start(const uint32_t* __restrict__ keys, int n, const int32_t* stamp_dev,
-                             uint2* __restrict__ table) {
+// kFindCellStart (G3/bt3dGridBroadphaseOCL.cl:61-87) into a stamped table, with
+// the cells' ends; the AABBs in sorted order (min.w holds the body id).
+__global__ void k_cells(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals, int n,
+                        const int32_t* stamp_dev, const float4* __restrict__ aabbMin,
+                        const float4* __restrict__ aabbMax, uint4* __restrict__ table, float4* __restrict__ sorted) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t k = keys[i];
-    if (i == 0 || keys[i - 1] != k) table[k] = make_uint2((uint32_t)*stamp_dev, (uint32_t)i);
+    const uint32_t b = vals[i];
+    sorted[2 * (size_t)i] = aabbMin[b];
+    sorted[2 * (size_t)i + 1] = aabbMax[b];
+    if (i == 0 || keys[i - 1] != k)
+        *reinterpret_cast<uint2*>(&table[k]) = make_uint2((uint32_t)*stamp_dev, (uint32_t)i);
+    if (i == n - 1 || keys[i + 1] != k) table[k].z = (uint32_t)(i + 1);
 }
 
 __device__ __forceinline__ bool aabb_overlap(float4 mn0, float4 mx0, float4 mn1, float4 mx1) {
@@ -194,15 +203,21 @@ __device__ uint32_t tile_lookback(int tile, int num_tiles, uint32_t agg, const G
     return excl;
 }
 
+// One thread per small body: its 27 cells in the reference's z, y, x order,
+// nine table entries and four candidates in flight at a time (one at a time, a
+// thread waited for some 27 + 2 x candidates L2 round trips in a row). Search,
+// us, before and now: 4,097 stacked cubes 44 -> 30, 20,012 spheres 111 -> 38,
+// 131,073 mixed 145 -> 89, 1,048,577 cubes 526 -> 360, 493,741 bodies of 4,096
+// worlds 371 -> 210; the sort and the cells with it 33 -> 17, 36 -> 25, 58 -> 37,
+// 105 -> 88, 85 -> 58 (the one-launch sort included).
 __global__ void __launch_bounds__(kPairTile)
-k_find_pairs(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
-             const float4* __restrict__ aabbMin, const float4* __restrict__ aabbMax,
-             const uint2* __restrict__ table, const int32_t* stamp_dev,
+k_find_pairs(const uint32_t* __restrict__ keys, const float4* __restrict__ sorted, const float4* __restrict__ aabbMin,
+             const float4* __restrict__ aabbMax, const uint4* __restrict__ table, const int32_t* stamp_dev,
              const int* __restrict__ largeStart, const int* __restrict__ largeList, GridParams g,
              int2* __restrict__ pairs, int32_t* __restrict__ numPairs,
              unsigned long long* __restrict__ status, int32_t* __restrict__ tile_counter,
              b3Counters* __restrict__ counters, int32_t* __restrict__ err_flag) {
-    extern __shared__ int pbuf[];  // [kPairTile][maxPairsPerBody]
+    extern __shared__ int pbuf[];  // [maxPairsPerBody][kPairTile]
     __shared__ uint32_t warp_tot[32];
     __shared__ uint32_t tile_total, tile_excl;
     __shared__ int tile_sh;
@@ -217,50 +232,54 @@ k_find_pairs(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ val
         if (tile >= num_tiles) break;
         const int i = tile * kPairTile + threadIdx.x;
         int cnt = 0;
-        int* buf = pbuf + threadIdx.x * g.maxPairsPerBody;
+        uint32_t self = 0;
+        int* buf = pbuf + threadIdx.x;
         int ovf = 0, covf = 0;
         if (i < n) {
-            const uint32_t key = keys[i];
-            const uint32_t self = vals[i];
-            const uint32_t world = key >> g.cellBits;
-            const float4 mn0 = aabbMin[self], mx0 = aabbMax[self];
+            const uint32_t world = keys[i] >> g.cellBits;
+            const float4 mn0 = sorted[2 * (size_t)i], mx0 = sorted[2 * (size_t)i + 1];
+            self = (uint32_t)__float_as_int(mn0.w);
             const float cx = mrn(arn(mn0.x, mx0.x), 0.5f);
             const float cy = mrn(arn(mn0.y, mx0.y), 0.5f);
             const float cz = mrn(arn(mn0.z, mx0.z), 0.5f);
             const int gx = grid_coord(cx, g.invCell, g.dimX);
             const int gy = grid_coord(cy, g.invCell, g.dimY);
             const int gz = grid_coord(cz, g.invCell, g.dimZ);
-            bool full = false;
             for (int dz = -1; dz <= 1; ++dz) {
                 const int zz = (gz + dz) & (g.dimZ - 1);
-                for (int dy = -1; dy <= 1; ++dy) {
-                    const int yy = (gy + dy) & (g.dimY - 1);
-                    for (int dx = -1; dx <= 1; ++dx) {
-                        const int xx = (gx + dx) & (g.dimX - 1);
-                        const uint32_t h = (world << g.cellBits) |
-                                           (uint32_t)(zz * g.dimY * g.dimX + yy * g.dimX + xx);
-                        const uint2 e = table[h];
-                        if (e.x != stamp) continue;
-                        const int start = (int)e.y;
-                        const int end = min(start + g.maxBodiesPerCell, n);
-                        int j = start;
-                        for (; j < end; ++j) {
-                            if (keys[j] != h) break;
-                            const uint32_t other = vals[j];
-                            if (other < self) {
-                                if (aabb_overlap(mn0, mx0, aabbMin[other], aabbMax[other])) {
-                                    if (cnt >= cap) {
-                                        ovf++;
-                                        full = true;
-                                        break;
-                                    }
-                                    buf[cnt++] = (int)other;
+                uint4 e[9];
+#pragma unroll
+                for (int c = 0; c < 9; ++c) {
+                    const int yy = (gy + c / 3 - 1) & (g.dimY - 1), xx = (gx + c % 3 - 1) & (g.dimX - 1);
+                    e[c] = __ldg(&table[(world << g.cellBits) | (uint32_t)(zz * g.dimY * g.dimX + yy * g.dimX + xx)]);
+                }
+#pragma unroll
+                for (int c = 0; c < 9; ++c) {
+                    if (e[c].x != stamp) continue;
+                    const int start = (int)e[c].y, end = min((int)e[c].z, start + g.maxBodiesPerCell);
+                    bool full = false;
+                    for (int j = start; j < end && !full; j += 4) {
+                        float4 mn[4], mx[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {  // past the end: the last candidate again
+                            const size_t at = 2 * (size_t)min(j + u, end - 1);
+                            mn[u] = sorted[at];
+                            mx[u] = sorted[at + 1];
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const uint32_t other = (uint32_t)__float_as_int(mn[u].w);
+                            if (j + u < end && !full && other < self && aabb_overlap(mn0, mx0, mn[u], mx[u])) {
+                                if (cnt >= cap) {
+                                    ovf++;
+                                    full = true;
+                                } else {
+                                    buf[kPairTile * cnt++] = (int)other;
                                 }
                             }
                         }
-                        if (!full && j == end && end < n && keys[end] == h) covf++;
-                        full = false;
                     }
+                    if (!full && (int)e[c].z > end) covf++;
                 }
             }
             // large bodies of this world
@@ -272,7 +291,7 @@ k_find_pairs(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ val
                         ovf++;
                         break;
                     }
-                    buf[cnt++] = L;
+                    buf[kPairTile * cnt++] = L;
                 }
             }
         }
@@ -284,11 +303,10 @@ k_find_pairs(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ val
         if (covf) atomicAdd(&counters->cellOverflow, covf);
         __syncthreads();
         if (i < n) {
-            const uint32_t self = vals[i];
             const uint32_t base = tile_excl + texcl;
             for (int c = 0; c < cnt; ++c) {
                 const uint32_t o = base + c;
-                if (o < (uint32_t)g.maxPairs) pairs[o] = make_int2((int)self, buf[c]);
+                if (o < (uint32_t)g.maxPairs) pairs[o] = make_int2((int)self, buf[kPairTile * c]);
             }
         }
         __syncthreads();
@@ -310,9 +328,9 @@ k_find_pairs(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ val
 // warp) are compacted like k_find_pairs' 128-body tiles, so the pair list,
 // pair count and overflow counters are identical to it bit for bit.
 __global__ void __launch_bounds__(kWarpPairThreads)
-k_find_pairs_warp(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
+k_find_pairs_warp(const uint32_t* __restrict__ keys, const float4* __restrict__ sorted,
                   const float4* __restrict__ aabbMin, const float4* __restrict__ aabbMax,
-                  const uint2* __restrict__ table, const int32_t* stamp_dev,
+                  const uint4* __restrict__ table, const int32_t* stamp_dev,
                   const int* __restrict__ largeStart, const int* __restrict__ largeList, GridParams g,
                   int2* __restrict__ pairs, int32_t* __restrict__ numPairs,
                   unsigned long long* __restrict__ status, int32_t* __restrict__ tile_counter,
@@ -343,60 +361,40 @@ k_find_pairs_warp(const uint32_t* __restrict__ keys, const uint32_t* __restrict_
             const int i = tile * kWarpPairTile + local;
             int cnt = 0;
             if (i < n) {  // warp-uniform
-                const uint32_t key = keys[i];
-                const uint32_t self = vals[i];
-                const uint32_t world = key >> g.cellBits;
-                const float4 mn0 = aabbMin[self], mx0 = aabbMax[self];
+                const uint32_t world = keys[i] >> g.cellBits;
+                const float4 mn0 = sorted[2 * (size_t)i], mx0 = sorted[2 * (size_t)i + 1];
+                const uint32_t self = (uint32_t)__float_as_int(mn0.w);
                 const float cx = mrn(arn(mn0.x, mx0.x), 0.5f);
                 const float cy = mrn(arn(mn0.y, mx0.y), 0.5f);
                 const float cz = mrn(arn(mn0.z, mx0.z), 0.5f);
-                int c = 0, start = 0, end = 0;
-                uint32_t h = 0;
-                bool active = false;
+                int c = 0, start = 0, end = 0, past = 0;
                 unsigned long long mask = 0;  // candidate positions 0..63 of the bucket
                 if (lane < 27) {
                     const int zz = (grid_coord(cz, g.invCell, g.dimZ) + dz) & (g.dimZ - 1);
                     const int yy = (grid_coord(cy, g.invCell, g.dimY) + dy) & (g.dimY - 1);
                     const int xx = (grid_coord(cx, g.invCell, g.dimX) + dx) & (g.dimX - 1);
-                    h = (world << g.cellBits) | (uint32_t)(zz * g.dimY * g.dimX + yy * g.dimX + xx);
-                    const uint2 e = table[h];
+                    const uint4 e = table[(world << g.cellBits) | (uint32_t)(zz * g.dimY * g.dimX + yy * g.dimX + xx)];
                     if (e.x == stamp) {
-                        active = true;
                         start = (int)e.y;
-                        end = min(start + g.maxBodiesPerCell, n);
+                        end = min((int)e.z, start + g.maxBodiesPerCell);
+                        past = (int)e.z - end;
                         for (int j = start; j < end; j += 4) {
-                            bool in[4], cand[4];
-                            uint32_t oo[4];
                             float4 amn[4], amx[4];
 #pragma unroll
                             for (int u = 0; u < 4; ++u) {
-                                const int jj = j + u;
-                                in[u] = false;
-                                oo[u] = 0;
-                                if (jj < end) {
-                                    in[u] = keys[jj] == h;
-                                    oo[u] = vals[jj];
-                                }
+                                const size_t at = 2 * (size_t)min(j + u, end - 1);
+                                amn[u] = sorted[at];
+                                amx[u] = sorted[at + 1];
                             }
 #pragma unroll
                             for (int u = 0; u < 4; ++u) {
-                                cand[u] = in[u] && oo[u] < self;
-                                amn[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                                amx[u] = amn[u];
-                                if (cand[u]) {
-                                    amn[u] = aabbMin[oo[u]];
-                                    amx[u] = aabbMax[oo[u]];
-                                }
-                            }
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) {
-                                if (cand[u] && aabb_overlap(mn0, mx0, amn[u], amx[u])) {
+                                if (j + u < end && (uint32_t)__float_as_int(amn[u].w) < self &&
+                                    aabb_overlap(mn0, mx0, amn[u], amx[u])) {
                                     const int pos = j + u - start;
                                     if (pos < 64) mask |= 1ull << pos;
                                     ++c;
                                 }
                             }
-                            if (!in[3]) break;  // keys are sorted: the bucket ended in this batch
                         }
                     }
                 }
@@ -412,7 +410,7 @@ k_find_pairs_warp(const uint32_t* __restrict__ keys, const uint32_t* __restrict_
                 const int keep = min(c, room);
                 const bool cell_ovf = c > room;
                 ovf += cell_ovf ? 1 : 0;
-                if (active && !cell_ovf && end < n && keys[end] == h) ++covf;
+                if (past > 0 && !cell_ovf) ++covf;
                 cnt = min(__shfl_sync(full, incl, 31), cap);
                 int* buf = pbuf + local * g.maxPairsPerBody;
                 if (keep > 0) {
@@ -421,13 +419,13 @@ k_find_pairs_warp(const uint32_t* __restrict__ keys, const uint32_t* __restrict_
                     while (m && w < keep) {
                         const int pos = __ffsll((long long)m) - 1;
                         m &= m - 1;
-                        buf[before + w++] = (int)vals[start + pos];
+                        buf[before + w++] = __float_as_int(sorted[2 * (size_t)(start + pos)].w);
                     }
                     for (int j = start + 64; j < end && w < keep; ++j) {
-                        if (keys[j] != h) break;
-                        const uint32_t other = vals[j];
-                        if (other < self && aabb_overlap(mn0, mx0, aabbMin[other], aabbMax[other]))
-                            buf[before + w++] = (int)other;
+                        const float4 mn = sorted[2 * (size_t)j];
+                        if ((uint32_t)__float_as_int(mn.w) < self &&
+                            aabb_overlap(mn0, mx0, mn, sorted[2 * (size_t)j + 1]))
+                            buf[before + w++] = __float_as_int(mn.w);
                     }
                 }
                 // large bodies of this world
@@ -470,7 +468,7 @@ k_find_pairs_warp(const uint32_t* __restrict__ keys, const uint32_t* __restrict_
             const int local = warp * kPerWarp + b;
             const int i = tile * kWarpPairTile + local;
             if (i >= n) break;
-            const int self = (int)vals[i];
+            const int self = __float_as_int(sorted[2 * (size_t)i].w);
             const uint32_t base = tile_excl + offs[local];
             const int c = cnts[local];
             for (int k = lane; k < c; k += 32) {
@@ -500,6 +498,12 @@ GridParams grid_params(const b3World_t* w) {
 
 namespace b3 {
 
+// Whether the cell sort's input goes to keysAlt / valsAlt, because its passes
+// end in the buffer they did not start from.
+static bool key_buffers_swapped(const b3World_t* w) {
+    return !w->sap && radix_result_in_alt(w->numSmall, w->keyBits);
+}
+
 int launch_aabb_hash(b3World_t* w, cudaStream_t st) {
     const int n = (int)w->bodies.size();
     if (n == 0) return B3_OK;
@@ -508,7 +512,7 @@ int launch_aabb_hash(b3World_t* w, cudaStream_t st) {
                                    w->sim.gravity.z * w->sim.dt);
     k_aabb_hash<<<(n + kAabbThreads - 1) / kAabbThreads, kAabbThreads, 0, st>>>(
         w->bodiesDev(), w->d.localAabb, g, gdt, w->d.smallSlot, w->d.aabbMin, w->d.aabbMax,
-        w->d.keys, w->d.vals, 1);
+        key_buffers_swapped(w) ? w->d.keysAlt : w->d.keys, key_buffers_swapped(w) ? w->d.valsAlt : w->d.vals, 1);
     B3_CHECK_LAUNCH();
     return B3_OK;
 }
@@ -517,19 +521,16 @@ int launch_sort_and_cells(b3World_t* w, cudaStream_t st) {
     if (w->sap) return launch_sap_sort(w, st);
     const int ns = w->numSmall;
     if (ns == 0) return B3_OK;
+    // (keys and values were written where the passes bring them to keys / vals)
+    const bool swap = key_buffers_swapped(w);
     bool alt = false;
-    B3_TRY(radix_sort_pairs(w->d.keys, w->d.vals, w->d.keysAlt, w->d.valsAlt,
+    B3_TRY(radix_sort_pairs(swap ? w->d.keysAlt : w->d.keys, swap ? w->d.valsAlt : w->d.vals,
+                            swap ? w->d.keys : w->d.keysAlt, swap ? w->d.vals : w->d.valsAlt,
                             w->d.scalars + S_NUM_SMALL, ns, w->keyBits, w->d.sortScratch,
                             w->d.sortScratchBytes, w->d.scalars + S_ERR, st, &alt,
                             w->ctx->numSMs));
-    if (alt) {
-        B3_CUDA(cudaMemcpyAsync(w->d.keys, w->d.keysAlt, sizeof(uint32_t) * ns,
-                                cudaMemcpyDeviceToDevice, st));
-        B3_CUDA(cudaMemcpyAsync(w->d.vals, w->d.valsAlt, sizeof(uint32_t) * ns,
-                                cudaMemcpyDeviceToDevice, st));
-    }
-    k_cell_start<<<(ns + 255) / 256, 256, 0, st>>>(w->d.keys, ns, w->d.scalars + S_STAMP,
-                                                  w->d.cellTable);
+    k_cells<<<(ns + 255) / 256, 256, 0, st>>>(w->d.keys, w->d.vals, ns, w->d.scalars + S_STAMP, w->d.aabbMin,
+                                             w->d.aabbMax, w->d.cellTable, w->d.sortedAabb);
     B3_CHECK_LAUNCH();
     return B3_OK;
 }
@@ -562,13 +563,13 @@ int launch_find_pairs(b3World_t* w, cudaStream_t st) {
     const int grid = std::min(tiles, w->ctx->numSMs * occ);
     if (warp)
         k_find_pairs_warp<<<grid, threads, smem, st>>>(
-            w->d.keys, w->d.vals, w->d.aabbMin, w->d.aabbMax, w->d.cellTable, w->d.scalars + S_STAMP,
+            w->d.keys, w->d.sortedAabb, w->d.aabbMin, w->d.aabbMax, w->d.cellTable, w->d.scalars + S_STAMP,
             w->d.largeStart, w->d.largeList, g, w->d.pairs, w->d.scalars + S_NUM_PAIRS,
             (unsigned long long*)w->d.scanScratch, w->d.scalars + S_TILE, w->d.counters,
             w->d.scalars + S_ERR);
     else
         k_find_pairs<<<grid, threads, smem, st>>>(
-            w->d.keys, w->d.vals, w->d.aabbMin, w->d.aabbMax, w->d.cellTable, w->d.scalars + S_STAMP,
+            w->d.keys, w->d.sortedAabb, w->d.aabbMin, w->d.aabbMax, w->d.cellTable, w->d.scalars + S_STAMP,
             w->d.largeStart, w->d.largeList, g, w->d.pairs, w->d.scalars + S_NUM_PAIRS,
             (unsigned long long*)w->d.scanScratch, w->d.scalars + S_TILE, w->d.counters,
             w->d.scalars + S_ERR);

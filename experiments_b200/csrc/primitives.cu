@@ -641,15 +641,14 @@ static int radix_sort_core(const uint32_t* kin, const uint32_t* vin, uint32_t* k
     return sort_grid<kPairs, kSortItems>(A, n_expect, st, numSMs);
 }
 
+bool radix_result_in_alt(int64_t n_max, int key_bits) { return !fits_block(n_max) && (sort_passes(key_bits) & 1) != 0; }
+
 int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt,
                      const int32_t* n_dev, int64_t n_max, int key_bits, void* scratch,
                      size_t scratch_bytes, int32_t* err_flag, cudaStream_t st, bool* result_in_alt,
                      int numSMs, int64_t n_expect) {
-    if (fits_block(n_max)) {
-        *result_in_alt = false;
-        return block_sort_any<false>(keys, vals, keys, vals, n_dev, n_max, key_bits, st);
-    }
-    *result_in_alt = (sort_passes(key_bits) & 1) != 0;
+    *result_in_alt = radix_result_in_alt(n_max, key_bits);
+    if (fits_block(n_max)) return block_sort_any<false>(keys, vals, keys, vals, n_dev, n_max, key_bits, st);
     return radix_sort_core<false>(keys, vals, keys_alt, vals ? vals_alt : nullptr, keys, vals, n_dev, n_max,
                                   n_expect > 0 ? n_expect : n_max, key_bits, scratch, scratch_bytes, err_flag, st,
                                   numSMs);
@@ -675,11 +674,8 @@ int radix_sort_interleaved(uint2* kv, uint2* kv_alt, const int32_t* n_dev, int64
                            bool* result_in_alt, int numSMs) {
     uint32_t* a = reinterpret_cast<uint32_t*>(kv_alt);
     uint32_t* b = reinterpret_cast<uint32_t*>(kv);
-    if (fits_block(n_max)) {
-        *result_in_alt = false;
-        return block_sort_any<true>(b, nullptr, b, nullptr, n_dev, n_max, key_bits, st);
-    }
-    *result_in_alt = (sort_passes(key_bits) & 1) != 0;
+    *result_in_alt = radix_result_in_alt(n_max, key_bits);
+    if (fits_block(n_max)) return block_sort_any<true>(b, nullptr, b, nullptr, n_dev, n_max, key_bits, st);
     return radix_sort_core<true>(b, nullptr, a, nullptr, b, nullptr, n_dev, n_max, n_max, key_bits, scratch,
                                  scratch_bytes, err_flag, st, numSMs);
 }

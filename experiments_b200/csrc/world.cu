@@ -71,7 +71,7 @@ void free_all(b3::DevBuffers& d) {
     void* ptrs[] = {d.pos, d.quat, d.linVel, d.angVel, d.invMass, d.friction, d.restitution,
                     d.invInertia, d.collidable, d.worldId, d.cols, d.polys, d.verts, d.faces,
                     d.indices, d.edges, d.localAabb, d.polyInradius, d.childShapes, d.vpXY, d.vpZ, d.axisFaces, d.polyInfo, d.subPairs, d.subCount, d.subOffset, d.aabbMin, d.aabbMax, d.smallSlot,
-                    d.largeStart, d.largeList, d.sapSmall, d.sapLarge, d.sapSorted, d.sapCount, d.sapOffset, d.keys, d.vals, d.keysAlt, d.valsAlt, d.cellTable,
+                    d.largeStart, d.largeList, d.sapSmall, d.sapLarge, d.sapSorted, d.sapCount, d.sapOffset, d.keys, d.vals, d.keysAlt, d.valsAlt, d.cellTable, d.sortedAabb,
                     d.pairs, d.contacts, d.manifoldFlag, d.pairSep, d.npFast, d.npSlow, d.npDefer, d.npDefer2, d.npDefer3, d.npCand, d.manifoldScan,
                     d.manifoldPair,
                     d.incKeys, d.incVals, d.incKeysAlt, d.incValsAlt, d.bodyIncStart,
@@ -638,7 +638,7 @@ static int ensure_capacity(b3World w) {
         B3_TRY(dalloc(d.cellTable, cells));
         B3_TRY(dalloc(d.scalars, b3::S_NUM_SCALARS));
         B3_TRY(dalloc(d.counters, 1));
-        B3_CUDA(cudaMemset(d.cellTable, 0, sizeof(uint2) * cells));
+        B3_CUDA(cudaMemset(d.cellTable, 0, sizeof(uint4) * cells));
         B3_CUDA(cudaMemset(d.scalars, 0, sizeof(int32_t) * b3::S_NUM_SCALARS));
         B3_CUDA(cudaMemset(d.counters, 0, sizeof(b3Counters)));
     }
@@ -657,6 +657,7 @@ static int ensure_capacity(b3World w) {
         B3_TRY(dalloc(d.aabbMin, nb));
         B3_TRY(dalloc(d.aabbMax, nb));
         B3_TRY(dalloc(d.smallSlot, nb));
+        if (!w->sap) B3_TRY(dalloc(d.sortedAabb, 2 * (size_t)nb));
         if (w->sap) {
             B3_TRY(dalloc(d.sapSmall, nb));
             B3_TRY(dalloc(d.sapLarge, nb));
