@@ -56,6 +56,8 @@ static inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStre
 // side element count (n_dev) so they can be captured in CUDA graphs without
 // host synchronisation; n_max bounds the grid and scratch sizes, and is the
 // count itself where n_dev is null. n_expect (0: n_max) is the likely count.
+// cleared: the scratch is cleared already (a sort's first 16 bytes, by a kernel
+// after the last sort; all of a scan's, with other buffers).
 // ---------------------------------------------------------------------------
 namespace b3 {
 
@@ -71,7 +73,7 @@ bool radix_result_in_alt(int64_t n_max, int key_bits);  // what *result_in_alt w
 int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt,
                      const int32_t* n_dev, int64_t n_max, int key_bits, void* scratch,
                      size_t scratch_bytes, int32_t* err_flag, cudaStream_t st, bool* result_in_alt,
-                     int numSMs, int64_t n_expect = 0);
+                     int numSMs, int64_t n_expect = 0, bool cleared = false);
 
 // Out-of-place sort: (keys_in, vals_in) are only read; the sorted result
 // lands in (keys_out, vals_out); (keys_tmp, vals_tmp) hold the passes in
@@ -89,7 +91,7 @@ size_t scan_scratch_bytes(int64_t n_max);
 // Exclusive scan of n_dev u32 values; total to d_total (may be null).
 int exclusive_scan_u32(const uint32_t* src, uint32_t* dst, const int32_t* n_dev, int64_t n_max,
                        uint32_t* d_total, void* scratch, size_t scratch_bytes, int32_t* err_flag,
-                       cudaStream_t st, int numSMs);
+                       cudaStream_t st, int numSMs, bool cleared = false);
 
 int fill_u32(uint32_t* dst, uint32_t v, int64_t n, cudaStream_t st);
 int bound_search(const uint32_t* keys, const int32_t* n_dev, int64_t n_max, uint32_t* dst,

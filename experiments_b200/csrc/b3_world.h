@@ -120,6 +120,10 @@ struct DevBuffers {
     int* manifoldPair = nullptr;      // manifold -> pair slot
     // solver
     uint32_t *incKeys = nullptr, *incVals = nullptr, *incKeysAlt = nullptr, *incValsAlt = nullptr;
+    // cleared together for every manifold list: its scan's words, then
+    // bodyIncStart and bodyIncEnd
+    unsigned char* manifoldZero = nullptr;
+    size_t manifoldScanBytes = 0;
     uint32_t *bodyIncStart = nullptr, *bodyIncEnd = nullptr;
     float4* rows = nullptr;           // constraint rows, see solver.cu
     uint32_t* incPos = nullptr;       // manifold side -> its copy in the body-sorted copy list
@@ -160,15 +164,16 @@ enum ScalarSlot {
     S_BAR_COUNT = 6,
     S_BAR_GEN = 7,
     S_TILE = 8,
-    S_NP_WORK = 9,
-    S_NP_FAST = 10,       // pairs queued for the FP32 clip
-    S_NP_SLOW = 11,       // pairs queued for the float-float path
-    S_NP_WORK2 = 12,
-    S_NP_WORK3 = 13,
-    S_NP_WORK4 = 14,
-    S_NUM_SUB = 15,       // sub-pairs of compound and mesh pairs this step (after the capacity cut)
-    S_NUM_SLOTS = 16,     // manifold slots: pairs, then sub-pairs
-    S_SUB_TOTAL = 17,     // sub-pairs before the capacity cut
+    S_NUM_SUB = 9,        // sub-pairs of compound and mesh pairs this step (after the capacity cut)
+    S_NUM_SLOTS = 10,     // manifold slots: pairs, then sub-pairs
+    S_SUB_TOTAL = 11,     // sub-pairs before the capacity cut
+    S_NP_FIRST = 12,      // from here on: the narrowphase's queues and work counters
+    S_NP_WORK = 12,
+    S_NP_FAST = 13,       // pairs queued for the FP32 clip
+    S_NP_SLOW = 14,       // pairs queued for the float-float path
+    S_NP_WORK2 = 15,
+    S_NP_WORK3 = 16,
+    S_NP_WORK4 = 17,
     S_NP_DEFER = 18,      // clip-queue pairs the lane-group clip passed to the warp clip
     S_NP_WORK5 = 19,
     S_NP_DEFER2 = 20,     // slow-queue positions the lane-group float-float clip passed to k_np_exact
@@ -265,6 +270,21 @@ struct b3World_t {
 };
 
 namespace b3 {
+#ifdef __CUDACC__
+// The beginning of a step, by one thread of its first kernel (k_aabb_hash).
+__device__ __forceinline__ void begin_step(int32_t* scalars, b3Counters* counters) {
+    scalars[S_STAMP] += 1;
+    counters->steps += 1;
+    counters->numContactPoints = 0;
+    counters->numManifolds = 0;
+    counters->numPairs = 0;
+    counters->refinedAxes = 0;
+    counters->refinedClips = 0;
+    counters->pairOverflow = 0;
+    counters->cellOverflow = 0;
+    counters->clipOverflow = 0;
+}
+#endif
 // slots of the narrowphase candidate store (pairs queued for float-float
 // axis ranking beyond this recompute their FP32 sweep)
 constexpr int kNpCandSlots = 1 << 20;
@@ -282,7 +302,8 @@ struct JacobiTape {
 // stage launchers (world.cu / broadphase.cu / narrowphase.cu / solver.cu)
 int launch_aabb_hash(b3World_t* w, cudaStream_t st);
 int launch_sort_and_cells(b3World_t* w, cudaStream_t st);
-int launch_find_pairs(b3World_t* w, cudaStream_t st);
+// cleared: launch_sort_and_cells ran before it and cleared its counters
+int launch_find_pairs(b3World_t* w, cudaStream_t st, bool cleared = true);
 // sweep-and-prune counterparts (sap.cu), called by the two above in SAP mode
 int launch_sap_sort(b3World_t* w, cudaStream_t st);
 int launch_sap_pairs(b3World_t* w, cudaStream_t st);

@@ -30,6 +30,8 @@
 #include "b3_math.cuh"
 #include "b3_world.h"
 
+#include <algorithm>
+
 using namespace b3m;
 
 namespace {
@@ -57,8 +59,9 @@ __global__ void __launch_bounds__(kAabbThreads)
 k_aabb_hash(b3::BodiesDev B, const float4* __restrict__ localAabb, GridParams g, float3 gdt,
             const int* __restrict__ smallSlot, float4* __restrict__ aabbMin,
             float4* __restrict__ aabbMax, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
-            int applyGravity) {
+            int applyGravity, int32_t* __restrict__ scalars, b3Counters* __restrict__ counters) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) b3::begin_step(scalars, counters);
     if (i >= B.n) return;
     const float4 p = B.pos[i];
     const float4 q = B.quat[i];
@@ -119,8 +122,18 @@ k_aabb_hash(b3::BodiesDev B, const float4* __restrict__ localAabb, GridParams g,
 // the cells' ends; the AABBs in sorted order (min.w holds the body id).
 __global__ void k_cells(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals, int n,
                         const int32_t* stamp_dev, const float4* __restrict__ aabbMin,
-                        const float4* __restrict__ aabbMax, uint4* __restrict__ table, float4* __restrict__ sorted) {
+                        const float4* __restrict__ aabbMax, uint4* __restrict__ table, float4* __restrict__ sorted,
+                        int32_t* __restrict__ scalars, unsigned long long* __restrict__ status, int tiles,
+                        unsigned long long* __restrict__ sortBarrier) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    // the pair search's counters and look-back words; the sort's barrier word
+    // for the next sort
+    if (i < tiles) status[i] = 0ull;
+    if (i == 0) {
+        *sortBarrier = 0ull;
+        scalars[b3::S_NUM_PAIRS] = 0;
+        scalars[b3::S_TILE] = 0;
+    }
     if (i >= n) return;
     const uint32_t k = keys[i];
     const uint32_t b = vals[i];
@@ -164,41 +177,43 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* warp_t
 }
 
 // Output offset of one pair tile by decoupled look-back over the tiles before
-// it (flag 1 = aggregate, 2 = inclusive prefix); the last tile publishes the
-// pair count, clamped to maxPairs with the excess counted as pair overflow.
-// Called by one thread of the tile.
+// it (flag 1 = aggregate, 2 = inclusive prefix), 32 of them at a time by the
+// tile's first warp; the last tile publishes the pair count, clamped to maxPairs
+// with the excess counted as pair overflow.
 __device__ uint32_t tile_lookback(int tile, int num_tiles, uint32_t agg, const GridParams& g,
                                   unsigned long long* __restrict__ status, int32_t* __restrict__ numPairs,
                                   b3Counters* __restrict__ counters, int32_t* __restrict__ err_flag) {
     const unsigned long long FA = 1ull << 32, FP = 2ull << 32;
+    const int lane = threadIdx.x;
     uint32_t excl = 0;
-    if (tile == 0) {
-        b3dev::st_release_u64(status, FP | agg);
-    } else {
-        b3dev::st_release_u64(status + tile, FA | agg);
-        int t = tile - 1;
-        while (t >= 0) {
-            unsigned long long s = 0;
-            int spins = 0;
-            while (((s = b3dev::ld_acquire_u64(status + t)) >> 32) == 0) {
-                if (++spins > b3dev::kSpinLimit) {
-                    atomicExch(err_flag, 1);
-                    atomicAdd(&counters->timeouts, 1);
-                    break;
-                }
-                __nanosleep(32);
+    if (lane == 0) b3dev::st_release_u64(status + tile, (tile == 0 ? FP : FA) | agg);
+    int t = tile - 1, spins = 0;
+    while (t >= 0) {
+        const unsigned long long s = t - lane >= 0 ? b3dev::ld_acquire_u64(status + t - lane) : FP;
+        const unsigned missing = __ballot_sync(0xffffffffu, (s >> 32) == 0);
+        const unsigned whole = __ballot_sync(0xffffffffu, (s >> 32) == 2);
+        // tiles up to the nearest inclusive prefix, and before a missing one
+        const int stop = whole ? __ffs(whole) - 1 : 31;
+        const int use = min(stop + 1, missing ? __ffs(missing) - 1 : 32);
+        excl += __reduce_add_sync(0xffffffffu, lane < use ? (uint32_t)s : 0u);
+        if (use == stop + 1 && whole) break;
+        t -= use;
+        if (use == 0 && ++spins > b3dev::kSpinLimit) {
+            if (lane == 0) {
+                atomicExch(err_flag, 1);
+                atomicAdd(&counters->timeouts, 1);
             }
-            excl += (uint32_t)s;
-            if ((s >> 32) != 1) break;
-            --t;
+            break;
         }
-        b3dev::st_release_u64(status + tile, FP | (unsigned long long)(excl + agg));
     }
-    if (tile == num_tiles - 1) {
-        const uint32_t total = excl + agg;
-        *numPairs = (int32_t)min(total, (uint32_t)g.maxPairs);
-        if (total > (uint32_t)g.maxPairs) atomicAdd(&counters->pairOverflow, (int)(total - (uint32_t)g.maxPairs));
-        counters->numPairs = (int32_t)min(total, (uint32_t)g.maxPairs);
+    if (lane == 0) {
+        if (tile > 0) b3dev::st_release_u64(status + tile, FP | (unsigned long long)(excl + agg));
+        if (tile == num_tiles - 1) {
+            const uint32_t total = excl + agg;
+            *numPairs = (int32_t)min(total, (uint32_t)g.maxPairs);
+            if (total > (uint32_t)g.maxPairs) atomicAdd(&counters->pairOverflow, (int)(total - (uint32_t)g.maxPairs));
+            counters->numPairs = (int32_t)min(total, (uint32_t)g.maxPairs);
+        }
     }
     return excl;
 }
@@ -297,8 +312,10 @@ k_find_pairs(const uint32_t* __restrict__ keys, const float4* __restrict__ sorte
         }
         // tile compaction with decoupled look-back
         const uint32_t texcl = block_excl_scan((uint32_t)cnt, warp_tot, &tile_total);
-        if (threadIdx.x == 0)
-            tile_excl = tile_lookback(tile, num_tiles, tile_total, g, status, numPairs, counters, err_flag);
+        if (threadIdx.x < 32) {
+            const uint32_t before = tile_lookback(tile, num_tiles, tile_total, g, status, numPairs, counters, err_flag);
+            if (threadIdx.x == 0) tile_excl = before;
+        }
         if (ovf) atomicAdd(&counters->pairOverflow, ovf);
         if (covf) atomicAdd(&counters->cellOverflow, covf);
         __syncthreads();
@@ -457,8 +474,10 @@ k_find_pairs_warp(const uint32_t* __restrict__ keys, const float4* __restrict__ 
         const uint32_t v = threadIdx.x < kWarpPairTile ? (uint32_t)cnts[threadIdx.x] : 0u;
         const uint32_t texcl = block_excl_scan(v, warp_tot, &tile_total);
         if (threadIdx.x < kWarpPairTile) offs[threadIdx.x] = texcl;
-        if (threadIdx.x == 0)
-            tile_excl = tile_lookback(tile, num_tiles, tile_total, g, status, numPairs, counters, err_flag);
+        if (threadIdx.x < 32) {
+            const uint32_t before = tile_lookback(tile, num_tiles, tile_total, g, status, numPairs, counters, err_flag);
+            if (threadIdx.x == 0) tile_excl = before;
+        }
         ovf = __reduce_add_sync(full, ovf);
         covf = __reduce_add_sync(full, covf);
         if (lane == 0 && ovf) atomicAdd(&counters->pairOverflow, ovf);
@@ -498,6 +517,11 @@ GridParams grid_params(const b3World_t* w) {
 
 namespace b3 {
 
+static int pair_tiles(const b3World_t* w) {
+    const int per = w->pairSearchMode == 1 ? kWarpPairTile : kPairTile;
+    return (w->numSmall + per - 1) / per;
+}
+
 // Whether the cell sort's input goes to keysAlt / valsAlt, because its passes
 // end in the buffer they did not start from.
 static bool key_buffers_swapped(const b3World_t* w) {
@@ -506,13 +530,14 @@ static bool key_buffers_swapped(const b3World_t* w) {
 
 int launch_aabb_hash(b3World_t* w, cudaStream_t st) {
     const int n = (int)w->bodies.size();
-    if (n == 0) return B3_OK;
     const GridParams g = grid_params(w);
     const float3 gdt = make_float3(w->sim.gravity.x * w->sim.dt, w->sim.gravity.y * w->sim.dt,
                                    w->sim.gravity.z * w->sim.dt);
-    k_aabb_hash<<<(n + kAabbThreads - 1) / kAabbThreads, kAabbThreads, 0, st>>>(
+    // (with no bodies, one block for the step's beginning)
+    k_aabb_hash<<<std::max(1, (n + kAabbThreads - 1) / kAabbThreads), kAabbThreads, 0, st>>>(
         w->bodiesDev(), w->d.localAabb, g, gdt, w->d.smallSlot, w->d.aabbMin, w->d.aabbMax,
-        key_buffers_swapped(w) ? w->d.keysAlt : w->d.keys, key_buffers_swapped(w) ? w->d.valsAlt : w->d.vals, 1);
+        key_buffers_swapped(w) ? w->d.keysAlt : w->d.keys, key_buffers_swapped(w) ? w->d.valsAlt : w->d.vals, 1,
+        w->d.scalars, w->d.counters);
     B3_CHECK_LAUNCH();
     return B3_OK;
 }
@@ -528,25 +553,31 @@ int launch_sort_and_cells(b3World_t* w, cudaStream_t st) {
                             swap ? w->d.keys : w->d.keysAlt, swap ? w->d.vals : w->d.valsAlt,
                             w->d.scalars + S_NUM_SMALL, ns, w->keyBits, w->d.sortScratch,
                             w->d.sortScratchBytes, w->d.scalars + S_ERR, st, &alt,
-                            w->ctx->numSMs));
+                            w->ctx->numSMs, 0, true));
     k_cells<<<(ns + 255) / 256, 256, 0, st>>>(w->d.keys, w->d.vals, ns, w->d.scalars + S_STAMP, w->d.aabbMin,
-                                             w->d.aabbMax, w->d.cellTable, w->d.sortedAabb);
+                                             w->d.aabbMax, w->d.cellTable, w->d.sortedAabb, w->d.scalars,
+                                             (unsigned long long*)w->d.scanScratch, pair_tiles(w),
+                                             (unsigned long long*)w->d.sortScratch);
     B3_CHECK_LAUNCH();
     return B3_OK;
 }
 
-int launch_find_pairs(b3World_t* w, cudaStream_t st) {
+int launch_find_pairs(b3World_t* w, cudaStream_t st, bool cleared) {
     if (w->sap) return launch_sap_pairs(w, st);
     const int ns = w->numSmall;
-    // numPairs = 0, tile counter = 0, status cleared
-    B3_CUDA(cudaMemsetAsync(w->d.scalars + S_NUM_PAIRS, 0, sizeof(int32_t), st));
-    B3_CUDA(cudaMemsetAsync(w->d.scalars + S_TILE, 0, sizeof(int32_t), st));
-    if (ns == 0) return B3_OK;
+    if (ns == 0) {
+        B3_CUDA(cudaMemsetAsync(w->d.scalars + S_NUM_PAIRS, 0, sizeof(int32_t), st));
+        return B3_OK;
+    }
     const bool warp = w->pairSearchMode == 1;
     const int tileBodies = warp ? kWarpPairTile : kPairTile;
     const int threads = warp ? kWarpPairThreads : kPairTile;
-    const int tiles = (ns + tileBodies - 1) / tileBodies;
-    B3_CUDA(cudaMemsetAsync(w->d.scanScratch, 0, sizeof(unsigned long long) * tiles, st));
+    const int tiles = pair_tiles(w);
+    if (!cleared) {
+        B3_CUDA(cudaMemsetAsync(w->d.scalars + S_NUM_PAIRS, 0, sizeof(int32_t), st));
+        B3_CUDA(cudaMemsetAsync(w->d.scalars + S_TILE, 0, sizeof(int32_t), st));
+        B3_CUDA(cudaMemsetAsync(w->d.scanScratch, 0, sizeof(unsigned long long) * tiles, st));
+    }
     const GridParams g = grid_params(w);
     const size_t smem = (size_t)tileBodies * w->cfg.maxPairsPerBody * sizeof(int);
     const void* fn = warp ? (const void*)k_find_pairs_warp : (const void*)k_find_pairs;

@@ -2627,10 +2627,11 @@ __device__ void write_point_contact(b3Contact4* __restrict__ out, int slot, int 
 }
 
 __global__ void k_np_special(const int2* __restrict__ pairs, const int32_t* __restrict__ numPairsDev, b3::BodiesDev Bd,
-                             b3::ShapesDev S, NpParams P, b3Contact4* __restrict__ contacts,
+                             b3::ShapesDev S, NpParams P, bool alone, b3Contact4* __restrict__ contacts,
                              uint32_t* __restrict__ manifoldFlag) {
     const int np = *numPairsDev;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
+        if (alone) manifoldFlag[p] = 0u;  // no hull stage ran
         const int2 pr = pairs[p];
         const int A = pr.x, B = pr.y;
         const b3Collidable cA = S.cols[Bd.collidable[A]], cB = S.cols[Bd.collidable[B]];
@@ -2814,9 +2815,7 @@ namespace b3 {
 // of compound and mesh pairs (kSub true).
 template <bool kSub>
 static int launch_np_stages(b3World_t* w, cudaStream_t st, const NpParams& P) {
-    // work counters and queue lengths S_NP_WORK .. S_NP_WORK4, S_NP_DEFER onwards
-    B3_CUDA(cudaMemsetAsync(w->d.scalars + S_NP_WORK, 0, sizeof(int32_t) * 6, st));
-    B3_CUDA(cudaMemsetAsync(w->d.scalars + S_NP_DEFER, 0, sizeof(int32_t) * (S_NUM_SCALARS - S_NP_DEFER), st));
+    B3_CUDA(cudaMemsetAsync(w->d.scalars + S_NP_FIRST, 0, sizeof(int32_t) * (S_NUM_SCALARS - S_NP_FIRST), st));
     const int threads = 32 * w->npWarpsPerBlock;
     const size_t smem = sizeof(WarpScratch) * w->npWarpsPerBlock;
     const size_t smemGroups = sizeof(GroupScratch) * (32 / kClipGroup) * w->npWarpsPerBlock;
@@ -2929,7 +2928,6 @@ static int launch_np_stages(b3World_t* w, cudaStream_t st, const NpParams& P) {
 }
 
 int launch_narrowphase(b3World_t* w, cudaStream_t st) {
-    B3_CUDA(cudaMemsetAsync(w->d.scalars + S_NP_WORK, 0, sizeof(int32_t) * 6, st));
     if (w->cfg.maxPairs == 0 || w->bodies.empty()) return B3_OK;
     NpParams P;
     P.minDist = -1e30f;
@@ -2964,7 +2962,15 @@ int launch_narrowphase(b3World_t* w, cudaStream_t st) {
                               (const void*)k_np_exact_groups<false>, (const void*)k_np_exact_groups<true>})
             B3_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemFF));
     }
-    {
+    // without hulls or mesh triangles there is nothing for the hull stages; the
+    // sphere and plane pass then writes every pair's flag
+    const bool hulls = w->smallPairs || w->largePairs;
+    if (!hulls && !w->hasSpheresPlanes())
+        B3_CUDA(cudaMemsetAsync(w->d.manifoldFlag, 0, sizeof(uint32_t) * (size_t)w->cfg.maxPairs, st));
+    if (!hulls && w->timing)
+        for (int k = 0; k < 5; ++k)
+            if (w->npEv[k]) B3_CUDA(cudaEventRecord(w->npEv[k], st));
+    if (hulls) {
         B3_TRY(launch_np_stages<false>(w, st, P));
         if (w->hasSubPairs()) {
             // expand compound and mesh pairs into sub-pairs, then their stages
@@ -2987,7 +2993,7 @@ int launch_narrowphase(b3World_t* w, cudaStream_t st) {
     }
     if (w->hasSpheresPlanes()) {
         k_np_special<<<w->ctx->numSMs * 4, 256, 0, st>>>(w->d.pairs, w->d.scalars + S_NUM_PAIRS, w->bodiesDev(),
-                                                          w->shapesDev(), P, w->d.contacts, w->d.manifoldFlag);
+                                                          w->shapesDev(), P, !hulls, w->d.contacts, w->d.manifoldFlag);
         B3_CHECK_LAUNCH();
     }
     return B3_OK;

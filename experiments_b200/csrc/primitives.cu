@@ -627,11 +627,12 @@ static int sort_grid(SortArgs& A, int64_t n_expect, cudaStream_t st, int numSMs)
 template <bool kPairs>
 static int radix_sort_core(const uint32_t* kin, const uint32_t* vin, uint32_t* kA, uint32_t* vA, uint32_t* kB,
                            uint32_t* vB, const int32_t* n_dev, int64_t n_max, int64_t n_expect, int key_bits,
-                           void* scratch, size_t scratch_bytes, int32_t* err_flag, cudaStream_t st, int numSMs) {
+                           void* scratch, size_t scratch_bytes, int32_t* err_flag, cudaStream_t st, int numSMs,
+                           bool cleared = false) {
     if (key_bits < 1 || key_bits > 32) return B3_ERR_INVALID_ARG;
     if (scratch_bytes < radix_scratch_bytes(n_max, key_bits)) return B3_ERR_CAPACITY;
     if (n_max <= 0) return B3_OK;
-    B3_CUDA(cudaMemsetAsync(scratch, 0, 16, st));
+    if (!cleared) B3_CUDA(cudaMemsetAsync(scratch, 0, 16, st));
     SortArgs A = {kin, vin, kA, vA, kB, vB, n_dev, (int)n_max, key_bits,
                   reinterpret_cast<uint32_t*>((unsigned char*)scratch + 256), (uint32_t*)scratch, err_flag};
     const int64_t each = n_expect / ((int64_t)numSMs * kSortThreads);
@@ -646,12 +647,12 @@ bool radix_result_in_alt(int64_t n_max, int key_bits) { return !fits_block(n_max
 int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt,
                      const int32_t* n_dev, int64_t n_max, int key_bits, void* scratch,
                      size_t scratch_bytes, int32_t* err_flag, cudaStream_t st, bool* result_in_alt,
-                     int numSMs, int64_t n_expect) {
+                     int numSMs, int64_t n_expect, bool cleared) {
     *result_in_alt = radix_result_in_alt(n_max, key_bits);
     if (fits_block(n_max)) return block_sort_any<false>(keys, vals, keys, vals, n_dev, n_max, key_bits, st);
     return radix_sort_core<false>(keys, vals, keys_alt, vals ? vals_alt : nullptr, keys, vals, n_dev, n_max,
                                   n_expect > 0 ? n_expect : n_max, key_bits, scratch, scratch_bytes, err_flag, st,
-                                  numSMs);
+                                  numSMs, cleared);
 }
 
 int radix_sort_kv_out(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out, uint32_t* vals_out,
@@ -687,10 +688,10 @@ size_t scan_scratch_bytes(int64_t n_max) {
 
 int exclusive_scan_u32(const uint32_t* src, uint32_t* dst, const int32_t* n_dev, int64_t n_max,
                        uint32_t* d_total, void* scratch, size_t scratch_bytes, int32_t* err_flag,
-                       cudaStream_t st, int numSMs) {
+                       cudaStream_t st, int numSMs, bool cleared) {
     const size_t need = scan_scratch_bytes(n_max);
     if (scratch_bytes < need) return B3_ERR_CAPACITY;
-    B3_CUDA(cudaMemsetAsync(scratch, 0, need, st));
+    if (!cleared) B3_CUDA(cudaMemsetAsync(scratch, 0, need, st));
     int32_t* counter = (int32_t*)scratch;
     unsigned long long* status = (unsigned long long*)((unsigned char*)scratch + 256);
     if (n_max <= 0) {

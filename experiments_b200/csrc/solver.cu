@@ -82,8 +82,10 @@ __global__ void k_manifold_emit(const uint32_t* __restrict__ flag, const uint32_
 // lie in it (a static side's place is past every body's range).
 __global__ void k_body_ranges(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
                               const int32_t* __restrict__ nDev, uint32_t* __restrict__ start,
-                              uint32_t* __restrict__ end, uint32_t* __restrict__ incPos, int numBodies) {
+                              uint32_t* __restrict__ end, uint32_t* __restrict__ incPos, int numBodies,
+                              unsigned long long* __restrict__ sortBarrier) {
     const int n = *nDev;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *sortBarrier = 0ull;  // for the next sort
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t k = keys[i];
         incPos[vals[i]] = (uint32_t)i;
@@ -122,8 +124,10 @@ __device__ __forceinline__ float setup_friction_row(const SolverView& V, int slo
 }
 
 __global__ void k_setup_rows(b3::BodiesDev Bd, SolverView V, const int* __restrict__ manifoldPair,
-                             const b3Contact4* __restrict__ contacts, SetupParams SP) {
+                             const b3Contact4* __restrict__ contacts, SetupParams SP,
+                             unsigned long long* __restrict__ barrier) {
     const int M = *V.numManifolds;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *barrier = 0ull;  // of the solve that follows
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
         const b3Contact4 c = contacts[manifoldPair[m]];
         const int A = abs(c.bodyAPtrAndSignBit), B = abs(c.bodyBPtrAndSignBit);
@@ -650,15 +654,19 @@ namespace b3 {
 int launch_manifolds(b3World_t* w, cudaStream_t st) {
     const int N = (int)w->bodies.size();
     const int cap = w->cfg.maxPairs;
-    B3_CUDA(cudaMemsetAsync(w->d.scalars + S_NUM_MANIFOLDS, 0, sizeof(int32_t) * 2, st));
-    B3_CUDA(cudaMemsetAsync(w->d.bodyIncStart, 0, sizeof(uint32_t) * N, st));
-    B3_CUDA(cudaMemsetAsync(w->d.bodyIncEnd, 0, sizeof(uint32_t) * N, st));
-    if (cap == 0 || N == 0) return B3_OK;
+    if (cap == 0 || N == 0) {
+        B3_CUDA(cudaMemsetAsync(w->d.scalars + S_NUM_MANIFOLDS, 0, sizeof(int32_t) * 2, st));
+        if (N > 0) B3_CUDA(cudaMemsetAsync(w->d.bodyIncStart, 0, 2 * sizeof(uint32_t) * (size_t)w->capBodies, st));
+        return B3_OK;
+    }
+    // the scan's words and the bodies' ranges in one
+    B3_CUDA(cudaMemsetAsync(w->d.manifoldZero, 0, w->d.manifoldScanBytes + 2 * sizeof(uint32_t) * (size_t)w->capBodies,
+                            st));
     // manifold slots: the pairs', then (compound and mesh worlds) the sub-pairs'
     const int32_t* slots = w->d.scalars + (w->hasSubPairs() ? S_NUM_SLOTS : S_NUM_PAIRS);
     B3_TRY(exclusive_scan_u32(w->d.manifoldFlag, w->d.manifoldScan, slots, cap,
-                              (uint32_t*)(w->d.scalars + S_NUM_MANIFOLDS), w->d.scanScratch,
-                              w->d.scanScratchBytes, w->d.scalars + S_ERR, st, w->ctx->numSMs));
+                              (uint32_t*)(w->d.scalars + S_NUM_MANIFOLDS), w->d.manifoldZero,
+                              w->d.manifoldScanBytes, w->d.scalars + S_ERR, st, w->ctx->numSMs, true));
     const int g = w->ctx->numSMs * 8;
     k_manifold_emit<<<g, 256, 0, st>>>(w->d.manifoldFlag, w->d.manifoldScan, slots,
                                       w->d.contacts, w->d.invMass, N, w->d.manifoldPair, w->d.incKeys,
@@ -668,9 +676,10 @@ int launch_manifolds(b3World_t* w, cudaStream_t st) {
     bool alt = false;
     B3_TRY(radix_sort_pairs(w->d.incKeys, w->d.incVals, w->d.incKeysAlt, w->d.incValsAlt,
                             w->d.scalars + S_NUM_INC, 2LL * cap, w->bodyBits, w->d.incSortScratch,
-                            w->d.incSortScratchBytes, w->d.scalars + S_ERR, st, &alt, w->ctx->numSMs, 6LL * N));
+                            w->d.incSortScratchBytes, w->d.scalars + S_ERR, st, &alt, w->ctx->numSMs, 6LL * N, true));
     k_body_ranges<<<g, 256, 0, st>>>(alt ? w->d.incKeysAlt : w->d.incKeys, alt ? w->d.incValsAlt : w->d.incVals,
-                                    w->d.scalars + S_NUM_INC, w->d.bodyIncStart, w->d.bodyIncEnd, w->d.incPos, N);
+                                    w->d.scalars + S_NUM_INC, w->d.bodyIncStart, w->d.bodyIncEnd, w->d.incPos, N,
+                                    (unsigned long long*)w->d.incSortScratch);
     B3_CHECK_LAUNCH();
     return B3_OK;
 }
@@ -693,7 +702,8 @@ int launch_solver_taped(b3World_t* w, cudaStream_t st, const JacobiTape* tape) {
     SP.contactProcessing = w->sim.contactProcessing;
     SP.slopOffset = w->sim.slopOffset;
     const int g = w->ctx->numSMs * 8;
-    k_setup_rows<<<g, 128, 0, st>>>(w->bodiesDev(), V, w->d.manifoldPair, w->d.contacts, SP);
+    k_setup_rows<<<g, 128, 0, st>>>(w->bodiesDev(), V, w->d.manifoldPair, w->d.contacts, SP,
+                                    (unsigned long long*)(w->d.scalars + S_BAR_COUNT));
     B3_CHECK_LAUNCH();
     if (w->timing && w->setupEv) B3_CUDA(cudaEventRecord(w->setupEv, st));
     if (w->solverMode == 1 && w->cfg.numWorlds > 1) {
@@ -720,7 +730,6 @@ int launch_solver_taped(b3World_t* w, cudaStream_t st, const JacobiTape* tape) {
         return B3_OK;
     }
     // persistent cooperative Jacobi
-    B3_CUDA(cudaMemsetAsync(w->d.scalars + S_BAR_COUNT, 0, sizeof(int32_t) * 2, st));
     const int threads = w->solverThreads;
     // size the persistent grid to the expected manifold count (about 3 per
     // body): fewer blocks make each grid barrier cheaper on small scenes

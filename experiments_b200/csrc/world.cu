@@ -5,7 +5,7 @@
 // btGpuNarrowphaseAndSolver (P1/btGpuNarrowPhaseAndSolver.h:63-123) behind
 // the C ABI in include/b3gpu.h. One step issues, on one stream and with no
 // host synchronisation (so it can be captured as a CUDA graph):
-//   k_step_begin -> k_aabb_hash -> radix sort -> k_cell_start -> k_find_pairs
+//   k_aabb_hash -> radix sort -> k_cells -> k_find_pairs
 //   -> k_narrowphase -> scan + k_manifold_emit -> radix sort -> k_body_ranges
 //   -> k_setup_rows -> k_jacobi (persistent) -> k_integrate
 // Every count that varies per step (pairs, manifolds, copies) stays on the
@@ -25,21 +25,6 @@ int ilog2(uint64_t v) {
     int b = 0;
     while ((1ull << b) < v) ++b;
     return b;
-}
-
-__global__ void k_step_begin(int32_t* scalars, b3Counters* counters) {
-    if (threadIdx.x == 0) {
-        scalars[b3::S_STAMP] += 1;
-        counters->steps += 1;
-        counters->numContactPoints = 0;
-        counters->numManifolds = 0;
-        counters->numPairs = 0;
-        counters->refinedAxes = 0;
-        counters->refinedClips = 0;
-        counters->pairOverflow = 0;
-        counters->cellOverflow = 0;
-        counters->clipOverflow = 0;
-    }
 }
 
 __global__ void k_world_stats(b3::BodiesDev Bd, float4* out, int numWorlds) {
@@ -74,8 +59,8 @@ void free_all(b3::DevBuffers& d) {
                     d.largeStart, d.largeList, d.sapSmall, d.sapLarge, d.sapSorted, d.sapCount, d.sapOffset, d.keys, d.vals, d.keysAlt, d.valsAlt, d.cellTable, d.sortedAabb,
                     d.pairs, d.contacts, d.manifoldFlag, d.pairSep, d.npFast, d.npSlow, d.npDefer, d.npDefer2, d.npDefer3, d.npCand, d.manifoldScan,
                     d.manifoldPair,
-                    d.incKeys, d.incVals, d.incKeysAlt, d.incValsAlt, d.bodyIncStart,
-                    d.bodyIncEnd, d.rows, d.incPos, d.copies,
+                    d.incKeys, d.incVals, d.incKeysAlt, d.incValsAlt,
+                    d.manifoldZero, d.rows, d.incPos, d.copies,
                     d.scalars, d.counters, d.sortScratch, d.incSortScratch, d.scanScratch,
                     d.worldStats, d.worldMStart, d.worldMEnd, d.gsCell, d.gsSlotBatch,
                     d.gsSlotOfManifold, d.gsVel, d.gsGroupCount, d.gsGroupFill,
@@ -669,14 +654,17 @@ static int ensure_capacity(b3World w) {
         B3_TRY(dalloc(d.vals, nb));
         B3_TRY(dalloc(d.keysAlt, nb));
         B3_TRY(dalloc(d.valsAlt, nb));
-        B3_TRY(dalloc(d.bodyIncStart, nb));
-        B3_TRY(dalloc(d.bodyIncEnd, nb));
+        d.manifoldScanBytes = (b3::scan_scratch_bytes(std::max<int64_t>(cap, 1)) + 255) / 256 * 256;
+        B3_TRY(dalloc(d.manifoldZero, d.manifoldScanBytes + 2 * sizeof(uint32_t) * (size_t)nb));
+        d.bodyIncStart = reinterpret_cast<uint32_t*>(d.manifoldZero + d.manifoldScanBytes);
+        d.bodyIncEnd = d.bodyIncStart + nb;
         if (w->gs) {
             B3_TRY(dalloc(d.gsVel, 2 * (size_t)nb));
             B3_TRY(dalloc(d.gsInertia, 3 * (size_t)nb));
         }
         d.sortScratchBytes = b3::radix_scratch_bytes(nb, w->keyBits);
         B3_TRY(dalloc((unsigned char*&)d.sortScratch, d.sortScratchBytes));
+        B3_CUDA(cudaMemset(d.sortScratch, 0, 16));  // the grid barrier's word; each step leaves it cleared
         w->capBodies = nb;
     }
     if (!d.pairs) {
@@ -722,6 +710,7 @@ static int ensure_capacity(b3World w) {
     if (incBytes > d.incSortScratchBytes) {
         d.incSortScratchBytes = incBytes;
         B3_TRY(dalloc((unsigned char*&)d.incSortScratch, incBytes));
+        B3_CUDA(cudaMemset(d.incSortScratch, 0, 16));
     }
     if (w->hasSubPairs() && !d.subPairs) {
         const size_t c = std::max(cap, 1);
@@ -977,15 +966,8 @@ extern "C" int b3_write_velocities(b3World w, const float* linVel3, const float*
 // ---------------------------------------------------------------------------
 // Step orchestration
 // ---------------------------------------------------------------------------
-static int step_begin(b3World w, cudaStream_t st) {
-    k_step_begin<<<1, 32, 0, st>>>(w->d.scalars, w->d.counters);
-    B3_CHECK_LAUNCH();
-    return B3_OK;
-}
-
 // One eager step; with a tape, the Jacobi solve records its phases.
 int b3::run_step(b3World_t* w, cudaStream_t st, const JacobiTape* tape) {
-    B3_TRY(step_begin(w, st));
     B3_TRY(b3::launch_aabb_hash(w, st));
     B3_TRY(b3::launch_sort_and_cells(w, st));
     B3_TRY(b3::launch_find_pairs(w, st));
@@ -1004,7 +986,6 @@ static int run_one_step_timed(b3World w, cudaStream_t st) {
     for (auto& e : w->npEv) B3_CUDA(cudaEventCreate(&e));
     B3_CUDA(cudaEventCreate(&w->setupEv));
     B3_CUDA(cudaEventRecord(ev[0], st));
-    B3_TRY(step_begin(w, st));
     B3_TRY(b3::launch_aabb_hash(w, st));
     B3_CUDA(cudaEventRecord(ev[1], st));
     B3_TRY(b3::launch_sort_and_cells(w, st));
@@ -1097,7 +1078,6 @@ extern "C" int b3_step(b3World w, int numSteps, void* stream) {
 extern "C" int b3_stage_aabbs(b3World w, void* stream) {
     if (!w || !w->written) return B3_ERR_STATE;
     cudaStream_t st = as_stream(stream);
-    B3_TRY(step_begin(w, st));
     return b3::launch_aabb_hash(w, st);
 }
 extern "C" int b3_stage_broadphase(b3World w, void* stream) {
@@ -1503,9 +1483,9 @@ extern "C" int b3_autotune(b3World w, int trialSteps, void* stream) {
     };
     // three pair searches over the same sorted keys, timed
     auto pair_trial = [&](float* ms) -> int {
-        B3_TRY(b3::launch_find_pairs(w, st));
+        B3_TRY(b3::launch_find_pairs(w, st, false));
         B3_CUDA(cudaEventRecord(e0, st));
-        for (int i = 0; i < 3; ++i) B3_TRY(b3::launch_find_pairs(w, st));
+        for (int i = 0; i < 3; ++i) B3_TRY(b3::launch_find_pairs(w, st, false));
         B3_CUDA(cudaEventRecord(e1, st));
         B3_CUDA(cudaEventSynchronize(e1));
         B3_CUDA(cudaEventElapsedTime(ms, e0, e1));
@@ -1545,7 +1525,6 @@ extern "C" int b3_autotune(b3World w, int trialSteps, void* stream) {
             // grid pair search: thread per body or warp per body, each timed
             // on three searches over the same sorted keys
             rc = restore();
-            if (rc == B3_OK) rc = step_begin(w, st);
             if (rc == B3_OK) rc = b3::launch_aabb_hash(w, st);
             if (rc == B3_OK) rc = b3::launch_sort_and_cells(w, st);
             int bp = w->pairSearchMode;
@@ -1565,7 +1544,6 @@ extern "C" int b3_autotune(b3World w, int trialSteps, void* stream) {
             // Jacobi: CTA size x blocks per SM x gather (x mode for batched
             // worlds), every combination timed on the same contacts
             rc = restore();
-            if (rc == B3_OK) rc = step_begin(w, st);
             if (rc == B3_OK) rc = b3::launch_aabb_hash(w, st);
             if (rc == B3_OK) rc = b3::launch_sort_and_cells(w, st);
             if (rc == B3_OK) rc = b3::launch_find_pairs(w, st);

@@ -106,3 +106,48 @@ def test_pair_search_forms_agree_on_the_full_mixed_hull_scene(ctx):
     assert np.array_equal(pairs[0], pairs[1])
     for a, b in zip(*states):
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+def test_stages_repeat_without_the_ones_before(ctx):
+    """Each stage entry point leaves what the next call of it needs: repeated
+    calls give the same lists (their counters and barrier words are cleared by
+    the kernels of the call itself)."""
+    sc = scenes.random_pile(15, n=9000, box=16.0, hull_frac=0.3)
+    w = scenes.build_world(ctx, sc)
+    w.stage("aabbs")
+    seen = []
+    for _ in range(3):
+        w.stage("broadphase")
+        w.stage("narrowphase")
+        w.stage("solve")
+        c = w.contacts()
+        seen.append((w.pairs(), c["pairIndex"], c["pos"], w.sorted_hash()))
+    w.close()
+    for p, i, x, h in seen[1:]:
+        assert np.array_equal(p, seen[0][0]) and np.array_equal(i, seen[0][1]) and np.array_equal(x, seen[0][2])
+        assert np.array_equal(h[0], seen[0][3][0]) and np.array_equal(h[1], seen[0][3][1])
+
+
+@pytest.mark.parametrize("spheres,plane", [(1, False), (1, True), (2, False)])
+def test_worlds_without_hulls(ctx, spheres, plane):
+    """No hull stage runs: the manifold flags are still those of the pairs."""
+    shapes = [{"kind": "sphere", "radius": 0.5}] * spheres + ([{"kind": "plane", "normal": [0.0, 1.0, 0.0],
+                                                                "constant": 0.0}] if plane else [])
+    n = 40
+    pos = np.stack([0.9 * (np.arange(n) % 5), 0.45 + 0.9 * (np.arange(n) // 25), 0.9 * (np.arange(n) // 5 % 5)], 1)
+    parts = [scenes._bodies(np.arange(n) % spheres, np.ones(n), pos, np.tile([0, 0, 0, 1.0], (n, 1)), np.full(n, 0.5),
+                            np.zeros(n))]
+    if plane:
+        parts.append(scenes._bodies([spheres], [0.0], [[0, 0, 0]], [[0, 0, 0, 1.0]], [0.6], [0]))
+    sc = scenes.Scene(name="s", shapes=shapes, num_worlds=1, config=dict(cellSize=1.0, gridDims=(16, 16, 16)),
+                      **scenes._concat(parts))
+    w, o = make_pair(ctx, sc)
+    for s in ("aabbs", "broadphase", "narrowphase"):
+        w.stage(s)
+    o.stage("aabbs")
+    o.set_pairs(w.pairs())
+    o.stage("narrowphase")
+    gc, oc = w.contacts(), o.contacts()
+    want = set(int(p) for p in oc["pairIndex"]) if spheres > 1 or plane else set()
+    assert len(w.pairs()) > 0 and set(int(p) for p in gc["pairIndex"]) == want
+    w.close()
