@@ -7,7 +7,7 @@
 //   integration   x' = x + v2 dt, q' = exp(phi(w2)) q (world-frame exp map
 //                 with the 0.25 pi / dt clamp), v2 = v1 + dv, w2 = d (w + dw)
 //   Jacobi solve  piecewise linear in the rows: the reverse sweep replays
-//                 each phase from its recorded inputs (averaged copies and
+//                 each phase from its recorded inputs (velocities and
 //                 impulses) to recover the clamp masks, then runs the rows
 //                 backwards; friction bounds carry mu and the normal impulse
 //   constraint    rows (n, rhs, r x n, 1/diag) as functions of the contact
@@ -29,9 +29,10 @@
 // differences agree with it on worlds whose active set does not change.
 //
 // Memory: body state is checkpointed every K steps; the reverse pass
-// recomputes each segment from its checkpoint, storing the K pre-step
-// states, then re-runs every step of the segment once more with the Jacobi
-// tape (every phase's solver-body copies and impulses) before reversing it.
+// recomputes each segment but the last from its checkpoint, storing the K
+// pre-step states (the forward run leaves the last segment's), then re-runs
+// every step of the segment once more with the Jacobi tape (every phase's
+// input velocities and impulses) before reversing it.
 // The inverse inertia is the inverse mass times a fixed shape factor (the
 // registration AABB rule), so its gradient folds into the mass gradient.
 #include "solver_common.cuh"
@@ -61,7 +62,13 @@ __device__ __forceinline__ Du du(float v, float d = 0.f) { return Du{v, d}; }
 __device__ __forceinline__ Du operator+(Du a, Du b) { return Du{a.v + b.v, a.d + b.d}; }
 __device__ __forceinline__ Du operator-(Du a, Du b) { return Du{a.v - b.v, a.d - b.d}; }
 __device__ __forceinline__ Du operator-(Du a) { return Du{-a.v, -a.d}; }
-__device__ __forceinline__ Du operator*(Du a, Du b) { return Du{a.v * b.v, a.d * b.v + a.v * b.d}; }
+// Products and sums of products by name: the compiler contracts them by their
+// surroundings, and where a contact hardly slides the direction of friction is a
+// quotient of two rounded sums (by other contractions the gradients of 16 steps
+// move by up to 3e-4 of their size).
+__device__ __forceinline__ Du operator*(Du a, Du b) {
+    return Du{a.v * b.v, __fmaf_rn(a.d, b.v, __fmul_rn(a.v, b.d))};
+}
 __device__ __forceinline__ Du operator*(Du a, float s) { return Du{a.v * s, a.d * s}; }
 __device__ __forceinline__ Du operator/(Du a, Du b) {
     const float r = 1.f / b.v;
@@ -85,9 +92,15 @@ __device__ __forceinline__ D3 operator+(D3 a, D3 b) { return D3{a.x + b.x, a.y +
 __device__ __forceinline__ D3 operator-(D3 a, D3 b) { return D3{a.x - b.x, a.y - b.y, a.z - b.z}; }
 __device__ __forceinline__ D3 operator-(D3 a) { return D3{-a.x, -a.y, -a.z}; }
 __device__ __forceinline__ D3 operator*(D3 a, Du s) { return D3{a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ Du ddot(D3 a, D3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__device__ __forceinline__ Du ddot(D3 a, D3 b) {
+    return Du{dot_fma(make_float3(a.x.v, a.y.v, a.z.v), make_float3(b.x.v, b.y.v, b.z.v)),
+              (a.x * b.x + a.y * b.y + a.z * b.z).d};
+}
+__device__ __forceinline__ Du dminor(Du a, Du b, Du c, Du d) {  // a b - c d
+    return Du{__fmaf_rn(a.v, b.v, -__fmul_rn(c.v, d.v)), (a * b - c * d).d};
+}
 __device__ __forceinline__ D3 dcross(D3 a, D3 b) {
-    return D3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+    return D3{dminor(a.y, b.z, a.z, b.y), dminor(a.z, b.x, a.x, b.z), dminor(a.x, b.y, a.y, b.x)};
 }
 __device__ __forceinline__ D3 dmulv(D3 a, D3 b) { return D3{a.x * b.x, a.y * b.y, a.z * b.z}; }
 __device__ __forceinline__ D3 dnormalize(D3 a) {
@@ -227,116 +240,126 @@ __device__ __forceinline__ void add4(float4& a, float3 v, float w = 0.f) {
     a.x += v.x; a.y += v.y; a.z += v.z; a.w += w;
 }
 
-__device__ void reverse_phase(const SolverView& V, const b3::JacobiTape& T, const AdjView& A, int m, int p,
-                              int phases) {
-    const float4 ids = R(V, kIds, m), hd0 = R(V, kHead0, m), hd1 = R(V, kHead1, m);
-    const int bA = __float_as_int(ids.x), bB = __float_as_int(ids.y);
-    const uint32_t sA = __float_as_uint(hd0.x), eA = __float_as_uint(hd0.y), pA = __float_as_uint(hd0.z);
-    const uint32_t sB = __float_as_uint(hd0.w), eB = __float_as_uint(hd1.x), pB = __float_as_uint(hd1.y);
-    const int nRows = __float_as_int(hd1.z) & 0xffff, dyn = __float_as_int(hd1.z) >> 16;
-    const float mu = hd1.w;
-    const bool friction = (p & 1) != 0;
-    const bool last = p == phases - 1;
-    // adjoint of this phase's copy outputs
-    float3 gvA = make_float3(0.f, 0.f, 0.f), gwA = gvA, gvB = gvA, gwB = gvA;
-    if (dyn & 1) {
-        if (last) { gvA = f3(A.gDv[bA]); gwA = f3(A.gDw[bA]); }
-        else copy_average<4>(A.gIn + (size_t)((p + 1) & 1) * 4 * V.cap, sA, eA, gvA, gwA);
+__device__ __forceinline__ float pick(const float4& v, int j) { return j < 2 ? (j ? v.y : v.x) : (j == 2 ? v.z : v.w); }
+__device__ __forceinline__ void put(float4& v, int j, float x) {
+    if (j == 0) v.x = x;
+    else if (j == 1) v.y = x;
+    else if (j == 2) v.z = x;
+    else v.w = x;
+}
+// Row adjoints are summed where they lie: the sum of one manifold's row is this
+// thread's alone, so the order is fixed, and nothing waits for the old value.
+__device__ __forceinline__ void red4(float4* p, float3 v, float w = 0.f) { atomicAdd(p, f4(v, w)); }
+
+// What the tape holds of one phase of one manifold.
+struct Taped {
+    float4 in[4];    // linear and angular velocity of A and B the phase started from
+    float4 lam[2];   // impulses of its rows before it
+    float4 normal;   // friction phase: impulses of the normal rows
+};
+__device__ __forceinline__ Taped load_tape(const b3::JacobiTape& T, int m, int p, size_t cap) {
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    Taped t;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) t.in[k] = T.in[((size_t)p * 4 + k) * cap + m];
+    const int it = p >> 1;
+    if (p & 1) {
+        const float4* f = T.lamF + ((size_t)2 * it * cap + m);
+        t.lam[0] = it > 0 ? f[-2 * (ptrdiff_t)cap] : zero;
+        t.lam[1] = it > 0 ? f[-(ptrdiff_t)cap] : zero;
+        t.normal = T.lamN[(size_t)it * cap + m];
+    } else {
+        t.lam[0] = it > 0 ? T.lamN[(size_t)(it - 1) * cap + m] : zero;
+        t.lam[1] = t.normal = zero;
     }
-    if (dyn & 2) {
-        if (last) { gvB = f3(A.gDv[bB]); gwB = f3(A.gDw[bB]); }
-        else copy_average<4>(A.gIn + (size_t)((p + 1) & 1) * 4 * V.cap, sB, eB, gvB, gwB);
-    }
-    const size_t cap = (size_t)V.cap;
-    float4 gLam0 = last ? make_float4(0.f, 0.f, 0.f, 0.f) : A.gLam[m];
-    float4 gLam1 = last ? make_float4(0.f, 0.f, 0.f, 0.f) : A.gLam[cap + m];
-    float4 gLam2 = last ? make_float4(0.f, 0.f, 0.f, 0.f) : A.gLam[2 * cap + m];
-    if (last) {
-        // first touch of this manifold in this step's reverse sweep
-        for (int s = 0; s < kAdjSlots; ++s) A.rowAdj[(size_t)s * cap + m] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    if (nRows > 0) {
-        const float4 ia = R(V, kInA, m), ib = R(V, kInB, m);
-        const float imA = R(V, kNorm, m).w, imB = ia.w;
-        const float3 iiA = f3(ia), iiB = f3(ib);
-        // inputs of the phase
-        float3 dvA = make_float3(0.f, 0.f, 0.f), dwA = dvA, dvB = dvA, dwB = dvA;
-        if (p > 0) {
-            const float4* tape = T.copies + (size_t)(p - 1) * 4 * cap;
-            if (dyn & 1) copy_average<4>(tape, sA, eA, dvA, dwA);
-            if (dyn & 2) copy_average<4>(tape, sB, eB, dvB, dwB);
+    return t;
+}
+
+// Row r of a phase: axis, angular parts, rhs and 1/diag (as normal_rows and
+// friction_rows form them).
+struct Row {
+    float3 n, t1, t2;
+    float rhs, jac;
+};
+template <bool kFriction>
+__device__ __forceinline__ Row form_row(const GlobalRows& S, const float4& norm, const float4& a, const float4& b, int j,
+                                        int q) {
+    Row w;
+    const float4 dir = kFriction ? S(kPoint0 + 4 * j + 2 + q) : norm;
+    w.n = f3(dir);
+    w.rhs = kFriction ? dir.w : a.w;
+    w.t1 = arm(f3(a), w.n);
+    w.t2 = kFriction ? arm_rev(f3(b), w.n) : arm_neg(f3(b), w.n);
+    w.jac = kFriction ? pick(S(kFJac + (j >> 1)), 2 * (j & 1) + q) : b.w;
+    return w;
+}
+
+// One phase of one manifold in reverse: the rows are solved again from the
+// tape, then run backwards. J dv of each row is kept in the impulses' streams,
+// which nothing reads after the solve.
+template <bool kFriction>
+__device__ __forceinline__ void reverse_rows(const GlobalRows& S, const AdjView& A, int m, int nRows, float mu,
+                                             const Taped& t, float4& g0, float4& g1, float4& g2, float3& gvA, float3& gwA,
+                                             float3& gvB, float3& gwB) {
+    constexpr int kPer = kFriction ? 2 : 1;
+    const size_t cap = (size_t)A.cap;
+    const float4 norm = S(kNorm), ia = S(kInA), ib = S(kInB);
+    const float imA = norm.w, imB = ia.w;
+    const float3 iiA = f3(ia), iiB = f3(ib);
+    float3 dvA = f3(t.in[0]), dwA = f3(t.in[1]), dvB = f3(t.in[2]), dwB = f3(t.in[3]);
+    float4 applied[2];
+    int clamped = 0;  // two bits a row: 1 at its lower limit, 2 at its upper one
+#pragma unroll 1
+    for (int j = 0; j < nRows; ++j) {
+        float lo = 0.f, hi = 1e10f;
+        if (kFriction) {
+            if (!(pick(t.normal, j) > 0.f)) continue;
+            hi = mu * pick(t.normal, j);
+            lo = -hi;
         }
-        const int it = p >> 1;
-        float lam[8], lamN[4] = {0.f, 0.f, 0.f, 0.f};
-        if (!friction) {
-            const float4 l = it > 0 ? T.lamN[(size_t)(it - 1) * cap + m] : make_float4(0.f, 0.f, 0.f, 0.f);
-            lam[0] = l.x; lam[1] = l.y; lam[2] = l.z; lam[3] = l.w;
-        } else {
-            const float4 l0 = it > 0 ? T.lamF[(size_t)(2 * it - 2) * cap + m] : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float4 l1 = it > 0 ? T.lamF[(size_t)(2 * it - 1) * cap + m] : make_float4(0.f, 0.f, 0.f, 0.f);
-            lam[0] = l0.x; lam[1] = l0.y; lam[2] = l0.z; lam[3] = l0.w;
-            lam[4] = l1.x; lam[5] = l1.y; lam[6] = l1.z; lam[7] = l1.w;
-            const float4 n4 = T.lamN[(size_t)it * cap + m];
-            lamN[0] = n4.x; lamN[1] = n4.y; lamN[2] = n4.z; lamN[3] = n4.w;
-        }
-        // replay: per row the applied change, the clamp state and J.dv
-        float dpr[8], jdv[8];
-        int st[8];
-        const int nr = friction ? 2 * nRows : nRows;
-        for (int r = 0; r < nr; ++r) {
-            st[r] = -1;  // skipped
-            const int j = friction ? (r >> 1) : r;
-            float lo = 0.f, hi = 1e10f;
-            if (friction) {
-                if (!(lamN[j] > 0.f)) continue;
-                hi = mu * lamN[j];
-                lo = -hi;
-            }
-            const RowData row = load_row(V, m, friction, r);
-            const float3 n = row.n, t1 = row.t1, t2 = row.t2;
-            const float rhs = row.rhs, jac = row.jac;
-            const float dv1 = dot(n, dvA) + dot(t1, dwA);
-            const float dv2 = -dot(n, dvB) + dot(t2, dwB);
-            jdv[r] = dv1 + dv2;
-            float delta = rhs;
-            delta -= dv1 * jac;
-            delta -= dv2 * jac;
-            const float sum = lam[r] + delta;
+        const float4 a = S(kPoint0 + 4 * j), b = S(kPoint0 + 4 * j + 1);
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const Row w = form_row<kFriction>(S, norm, a, b, j, q);
+            const int r = kPer * j + q;
+            // by name, as the solve forms them: the limits are decided by these
+            const float dv1 = __fadd_rn(dot_fma(w.n, dvA), dot_fma(w.t1, dwA));
+            const float dv2 = __fsub_rn(dot_fma(w.t2, dwB), dot_fma(w.n, dvB));
+            put(S(kLamF + (r >> 2)), r & 3, dv1 + dv2);
+            const float delta = __fmaf_rn(-dv2, w.jac, __fmaf_rn(-dv1, w.jac, w.rhs));
+            const float lam = pick(r < 4 ? t.lam[0] : t.lam[1], r & 3);
+            const float sum = lam + delta;
             float na;
-            if (sum < lo) { na = lo; st[r] = 1; }
-            else if (sum > hi) { na = hi; st[r] = 2; }
-            else { na = sum; st[r] = 0; }
-            const float d = na - lam[r];
-            dpr[r] = d;
-            lam[r] = na;
-            dvA += n * (imA * d);
-            dwA += mulv(iiA, t1) * d;
-            dvB += (-n * imB) * d;
-            dwB += mulv(iiB, t2) * d;
+            if (sum < lo) { na = lo; clamped |= 1 << 2 * r; }
+            else if (sum > hi) { na = hi; clamped |= 2 << 2 * r; }
+            else { na = sum; }
+            const float d = na - lam;
+            put(r < 4 ? applied[0] : applied[1], r & 3, d);
+            dvA = fma3(w.n, imA * d, dvA);
+            dwA = fma3(mulv(iiA, w.t1), d, dwA);
+            dvB = fma3(-w.n * imB, d, dvB);
+            dwB = fma3(mulv(iiB, w.t2), d, dwB);
         }
-        // reverse
-        float gl[8];
-        if (!friction) { gl[0] = gLam0.x; gl[1] = gLam0.y; gl[2] = gLam0.z; gl[3] = gLam0.w; }
-        else {
-            gl[0] = gLam1.x; gl[1] = gLam1.y; gl[2] = gLam1.z; gl[3] = gLam1.w;
-            gl[4] = gLam2.x; gl[5] = gLam2.y; gl[6] = gLam2.z; gl[7] = gLam2.w;
-        }
-        float glN[4] = {gLam0.x, gLam0.y, gLam0.z, gLam0.w};
-        float gimA = 0.f, gimB = 0.f, gmu = 0.f;
-        float3 giiA = make_float3(0.f, 0.f, 0.f), giiB = giiA;
-        for (int r = nr - 1; r >= 0; --r) {
-            if (st[r] < 0) continue;
-            const int j = friction ? (r >> 1) : r;
-            const int s = friction ? kFric0 + 3 * r : kNormal0 + 3 * r;
-            const RowData row = load_row(V, m, friction, r);
-            const float3 n = row.n, t1 = row.t1, t2 = row.t2;
-            const float jac = row.jac;
-            const float d = dpr[r];
+    }
+    float gimA = 0.f, gimB = 0.f, gmu = 0.f;
+    float3 giiA = make_float3(0.f, 0.f, 0.f), giiB = giiA;
+#pragma unroll 1
+    for (int j = nRows - 1; j >= 0; --j) {
+        const float ln = pick(t.normal, j);
+        if (kFriction && !(ln > 0.f)) continue;
+        const float4 a = S(kPoint0 + 4 * j), b = S(kPoint0 + 4 * j + 1);
+#pragma unroll
+        for (int q = kPer - 1; q >= 0; --q) {
+            const Row w = form_row<kFriction>(S, norm, a, b, j, q);
+            const int r = kPer * j + q;
+            const float3 n = w.n, t1 = w.t1, t2 = w.t2;
+            const float jac = w.jac, d = pick(r < 4 ? applied[0] : applied[1], r & 3);
+            const int st = clamped >> (2 * r) & 3;
             const float3 ktA = mulv(iiA, t1), ktB = mulv(iiB, t2);
             // inputs of this row (step back through its update)
             const float3 dvAi = dvA - n * (imA * d), dwAi = dwA - ktA * d;
             const float3 dvBi = dvB + n * (imB * d), dwBi = dwB - ktB * d;
-            const float S = imA * dot(n, gvA) + dot(ktA, gwA) - imB * dot(n, gvB) + dot(ktB, gwB);
+            const float S0 = imA * dot(n, gvA) + dot(ktA, gwA) - imB * dot(n, gvB) + dot(ktB, gwB);
             float3 gn = (gvA * imA - gvB * imB) * d;
             float3 gt1 = mulv(iiA, gwA) * d;
             float3 gt2 = mulv(iiB, gwB) * d;
@@ -344,14 +367,16 @@ __device__ void reverse_phase(const SolverView& V, const b3::JacobiTape& T, cons
             gimB -= d * dot(n, gvB);
             giiA += mulv(t1, gwA) * d;
             giiB += mulv(t2, gwB) * d;
-            const float gna = gl[r] + S;
-            float glIn = -S;
+            float4& gl = kFriction ? (j < 2 ? g1 : g2) : g0;
+            const int c = kFriction ? 2 * (j & 1) + q : j;
+            const float gna = pick(gl, c) + S0;
+            float glIn = -S0;
             float grhs = 0.f, gjac = 0.f;
-            if (st[r] == 0) {
+            if (st == 0) {
                 glIn += gna;
                 const float gdelta = gna;
                 grhs = gdelta;
-                gjac = -gdelta * jdv[r];
+                gjac = -gdelta * pick(S(kLamF + (r >> 2)), r & 3);
                 gn += (dvAi - dvBi) * (-gdelta * jac);
                 gt1 += dwAi * (-gdelta * jac);
                 gt2 += dwBi * (-gdelta * jac);
@@ -359,68 +384,125 @@ __device__ void reverse_phase(const SolverView& V, const b3::JacobiTape& T, cons
                 gwA += t1 * (-gdelta * jac);
                 gvB += n * (gdelta * jac);
                 gwB += t2 * (-gdelta * jac);
-            } else if (friction) {
+            } else if (kFriction) {
                 // bound +-mu * lambda_n
-                const float sg = st[r] == 2 ? 1.f : -1.f;
-                gmu += sg * lamN[j] * gna;
-                glN[j] += sg * mu * gna;
+                const float sg = st == 2 ? 1.f : -1.f;
+                gmu += sg * ln * gna;
+                put(g0, j, pick(g0, j) + sg * mu * gna);
             }
-            gl[r] = glIn;
-            float4& a0 = A.rowAdj[(size_t)s * cap + m];
-            float4& a1 = A.rowAdj[(size_t)(s + 1) * cap + m];
-            float4& a2 = A.rowAdj[(size_t)(s + 2) * cap + m];
-            add4(a0, gn, grhs);
-            add4(a1, gt1, gjac);
-            add4(a2, gt2, 0.f);
+            put(gl, c, glIn);
+            float4* at = A.rowAdj + (size_t)((kFriction ? kFric0 : kNormal0) + 3 * r) * cap + m;
+            red4(at, gn, grhs);
+            red4(at + cap, gt1, gjac);
+            red4(at + 2 * cap, gt2);
             dvA = dvAi; dwA = dwAi; dvB = dvBi; dwB = dwBi;
         }
-        float4& hA = A.rowAdj[cap + m];
-        hA.x += gimA; hA.y += gimB; hA.z += gmu;
-        add4(A.rowAdj[2 * cap + m], giiA, 0.f);
-        add4(A.rowAdj[3 * cap + m], giiB, 0.f);
-        if (!friction) {
-            gLam0 = make_float4(gl[0], gl[1], gl[2], gl[3]);
-        } else {
-            gLam1 = make_float4(gl[0], gl[1], gl[2], gl[3]);
-            gLam2 = make_float4(gl[4], gl[5], gl[6], gl[7]);
-            gLam0 = make_float4(glN[0], glN[1], glN[2], glN[3]);
-        }
     }
-    A.gLam[m] = gLam0;
-    A.gLam[cap + m] = gLam1;
-    A.gLam[2 * cap + m] = gLam2;
-    // adjoint of the phase inputs (the averages read at its start)
-    if (p > 0) {
-        float4* g = A.gIn + (size_t)(p & 1) * 4 * cap;
-        if (dyn & 1) { g[2 * (size_t)pA] = f4(gvA); g[2 * (size_t)pA + 1] = f4(gwA); }
-        if (dyn & 2) { g[2 * (size_t)pB] = f4(gvB); g[2 * (size_t)pB + 1] = f4(gwB); }
-    }
+    red4(A.rowAdj + cap + m, make_float3(gimA, gimB, gmu));
+    red4(A.rowAdj + 2 * cap + m, giiA);
+    red4(A.rowAdj + 3 * cap + m, giiB);
 }
 
-__global__ void __launch_bounds__(256)
-k_jacobi_adjoint(SolverView V, b3::JacobiTape T, AdjView A, int iterations, uint32_t* bar, int32_t* err,
+// The phases of the solve in reverse, one thread per manifold, a grid barrier
+// between phases. As in the solve the chain of a phase counts: a thread's first
+// `resident` manifolds keep their rows in shared memory, the tape's streams (read
+// in order, the phase's input velocities by manifold instead of every body's
+// copies again) are fetched before the barrier, and behind it one round of
+// L2 reads is left, the copies' adjoints. 32,308 manifolds, 20 phases: 521 -> 185
+// us; before, every phase read its rows and the row adjoints it adds to one after
+// another, with the rows' states in local memory.
+__global__ void __launch_bounds__(128, 2)
+k_jacobi_adjoint(SolverView V, b3::JacobiTape T, AdjView A, int iterations, int resident, uint32_t* bar, int32_t* err,
                  b3Counters* counters) {
+    extern __shared__ float4 kept[];  // [resident][kPhaseSlots][blockDim]
     GridBarrier barrier(bar, err, counters, b3dev::kSpinLimit);
     const int M = *V.numManifolds;
+    const size_t cap = (size_t)V.cap;
     const int phases = 2 * iterations;
+    const int m0 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int stride = gridDim.x * blockDim.x;
+    const int tb = (int)blockDim.x;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < resident; ++k) {
+        const int m = m0 + k * stride;
+        if (m < M) {
+            float4* at = kept + (size_t)k * kPhaseSlots * tb + threadIdx.x;
+#pragma unroll
+            for (int s = 0; s < kPhaseSlots; ++s) at[s * tb] = R(V, s, m);
+        }
+    }
+    for (int m = m0; m < M; m += stride)
+        for (int s = 1; s < kAdjSlots; ++s) A.rowAdj[(size_t)s * cap + m] = zero;
     for (int p = phases - 1; p >= 0; --p) {
-        if (p < phases - 1 && !barrier.wait()) return;
-        for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x)
-            reverse_phase(V, T, A, m, p, phases);
+        const bool last = p == phases - 1;
+        const float4* in = A.gIn + (size_t)((p + 1) & 1) * 4 * cap;
+        float4* out = A.gIn + (size_t)(p & 1) * 4 * cap;
+        int m = m0;
+        for (int k = 0; k == 0 || m < M; ++k, m += stride) {
+            const GlobalRows S = k < resident ? GlobalRows{kept + (size_t)k * kPhaseSlots * tb + threadIdx.x, (size_t)tb}
+                                              : GlobalRows{V.rows + m, cap};
+            Taped t;
+            float4 g0 = zero, g1 = zero, g2 = zero;
+            if (m < M) {
+                t = load_tape(T, m, p, cap);
+                if (!last) {
+                    g0 = A.gLam[m];
+                    g1 = A.gLam[cap + m];
+                    g2 = A.gLam[2 * cap + m];
+                }
+            }
+            if (k == 0 && !last && !barrier.wait()) return;
+            if (m >= M) continue;
+            const Heads H = load_heads(S);
+            // adjoint of this phase's copy outputs
+            float3 gvA = make_float3(0.f, 0.f, 0.f), gwA = gvA, gvB = gvA, gwB = gvA;
+            if (last) {
+                const float4 ids = R(V, kIds, m);
+                const int bA = __float_as_int(ids.x), bB = __float_as_int(ids.y);
+                if (H.dyn & 1) { gvA = f3(A.gDv[bA]); gwA = f3(A.gDw[bA]); }
+                if (H.dyn & 2) { gvB = f3(A.gDv[bB]); gwB = f3(A.gDw[bB]); }
+            } else {
+                gather_averages<4>(in, H, gvA, gwA, gvB, gwB);
+            }
+            if (H.nRows > 0) {
+                if (p & 1) reverse_rows<true>(S, A, m, H.nRows, H.mu, t, g0, g1, g2, gvA, gwA, gvB, gwB);
+                else reverse_rows<false>(S, A, m, H.nRows, H.mu, t, g0, g1, g2, gvA, gwA, gvB, gwB);
+            }
+            if (p > 0) {
+                A.gLam[m] = g0;
+                A.gLam[cap + m] = g1;
+                A.gLam[2 * cap + m] = g2;
+                // adjoint of the phase inputs (the averages read at its start)
+                if (H.dyn & 1) {
+                    __stcg(&out[2 * (size_t)H.pA], f4(gvA));
+                    __stcg(&out[2 * (size_t)H.pA + 1], f4(gwA));
+                }
+                if (H.dyn & 2) {
+                    __stcg(&out[2 * (size_t)H.pB], f4(gvB));
+                    __stcg(&out[2 * (size_t)H.pB + 1], f4(gwB));
+                }
+            }
+        }
     }
 }
 
 // ---------------------------------------------------------------------------
-// Constraint-setup and contact-geometry adjoint (one thread per manifold)
+// Constraint-setup and contact-geometry adjoint (kLanes lanes per manifold)
 // ---------------------------------------------------------------------------
 struct SetupIn {
     D3 xA, xB, vA, wA, vB, wB;
     Du imA, imB;
     D3 iiA, iiB;
     D3 n;
-    D3 p[4];
-    Du depth[4];
+    const float4* p;       // points and depths
+    int k;                 // the input whose tangent is one
 };
+// inputs: xA 0-2, xB 3-5, vA 6-8, wA 9-11, vB 12-14, wB 15-17, imA 18, imB 19,
+// iiA 20-22, iiB 23-25, n 26-28, p 29-40, depth 41-44
+constexpr int kInputs = 45, kInNormal = 26, kInPoint = 29, kInDepth = 41;
+__device__ __forceinline__ float3 unit_at(int k, int base) {
+    return make_float3(k == base ? 1.f : 0.f, k == base + 1 ? 1.f : 0.f, k == base + 2 ? 1.f : 0.f);
+}
 
 // k_setup_rows restated in dual numbers; returns the tangent of the rows
 // contracted with their adjoint.
@@ -430,10 +512,13 @@ __device__ float setup_tangent(const SetupIn& I, const SolverView& V, const AdjV
     float acc = 0.f;
     int nRows = 0;
     for (int j = 0; j < npts; ++j) {
-        const Du dist = I.depth[j] + du(P.slopOffset);
+        const float4 at = I.p[j];
+        const float3 tp = unit_at(I.k, kInPoint + 3 * j);
+        const float td = I.k == kInDepth + j ? 1.f : 0.f;
+        const Du dist = du(at.w, td) + du(P.slopOffset);
         if (!(dist.v <= P.contactProcessing)) continue;
         const D3 n = I.n;
-        const D3 posB = I.p[j];
+        const D3 posB = d3(f3(at), tp);
         const D3 posA = posB + n * dist;
         const D3 r1 = posA - I.xA;
         const D3 r2 = posB - I.xB;
@@ -547,9 +632,12 @@ __device__ D3 solve3(D3 a, D3 b, D3 c, Du ha, Du hb, Du hc) {
     return (bc * ha + ca * hb + ab * hc) * inv;
 }
 
-__device__ void geo_eval(const Geo& G, const b3::ShapesDev& S, const b3ConvexPolyhedron& hA,
-                         const b3ConvexPolyhedron& hB, const PoseD& PA, const PoseD& PB, int npts, D3& nOut,
-                         D3* pOut, Du* depthOut) {
+// Tangent of the contact geometry along the two poses' perturbation, contracted
+// with its adjoint gin (the axis at kInNormal, points, depths).
+__device__ float geo_tangent(const Geo& G, const b3::ShapesDev& S, const b3ConvexPolyhedron& hA,
+                             const b3ConvexPolyhedron& hB, const PoseD& PA, const PoseD& PB, int npts,
+                             const float* gin) {
+    D3 nOut;
     const b3Face fa = S.faces[hA.faceOffset + G.faceA];
     const b3Face fb = S.faces[hB.faceOffset + G.faceB];
     // separating axis
@@ -570,6 +658,8 @@ __device__ void geo_eval(const Geo& G, const b3::ShapesDev& S, const b3ConvexPol
     const float3 nAl = make_float3(fa.plane[0], fa.plane[1], fa.plane[2]);
     const D3 nAw = pose_dir(PA, nAl);
     const int nvA = fa.numIndices;
+    const float* gn = gin + kInNormal;
+    float acc = gn[0] * nOut.x.d + gn[1] * nOut.y.d + gn[2] * nOut.z.d;
     for (int j = 0; j < npts; ++j) {
         const GeoPoint& g = G.pt[j];
         D3 p;
@@ -599,9 +689,11 @@ __device__ void geo_eval(const Geo& G, const b3::ShapesDev& S, const b3ConvexPol
         } else {
             p = pose_point(PB, g.local);
         }
-        pOut[j] = p;
-        depthOut[j] = ddot(nAw, p - PA.x) + du(fa.plane[3]);
+        const Du depth = ddot(nAw, p - PA.x) + du(fa.plane[3]);
+        const float* gp = gin + kInPoint + 3 * j;
+        acc += gp[0] * p.x.d + gp[1] * p.y.d + gp[2] * p.z.d + gin[kInDepth + j] * depth.d;
     }
+    return acc;
 }
 
 // The corner of side planes k, l on the incident face plane is well defined
@@ -618,162 +710,200 @@ __device__ bool corner_ok(const b3::ShapesDev& S, const b3ConvexPolyhedron& hA, 
     return fabsf(dot(pk, cross(pl, nb))) > 1e-3f;
 }
 
-// Classify the manifold's points against reference face G.faceA and
-// incident face G.faceB (values only); returns how many points fit neither
-// an incident vertex, an incident edge cut by a side plane, nor a corner of
-// two side planes.
-__device__ int geo_points(Geo& G, const b3::ShapesDev& S, const b3ConvexPolyhedron& hA, const b3ConvexPolyhedron& hB,
-                          const Mat3& RA, const Mat3& RB, float3 xB, const float3* p, int npts) {
-    int miss = 0;
+// Classify a point of the manifold against reference face faceA and incident
+// face faceB (values only); true if it fits neither an incident vertex, an
+// incident edge cut by a side plane, nor a corner of two side planes.
+__device__ bool geo_point(GeoPoint& g, int faceA, int faceB, const b3::ShapesDev& S, const b3ConvexPolyhedron& hA,
+                          const b3ConvexPolyhedron& hB, const Mat3& RA, const Mat3& RB, float3 xB, float3 p) {
     // origin at body A's position (p and xB are given relative to it)
-    const b3Face fa = S.faces[hA.faceOffset + G.faceA];
-    const b3Face fb = S.faces[hB.faceOffset + G.faceB];
+    const b3Face fa = S.faces[hA.faceOffset + faceA];
+    const b3Face fb = S.faces[hB.faceOffset + faceB];
     const int nvA = fa.numIndices, nvB = fb.numIndices;
     const float3 nAw = mul(RA, make_float3(fa.plane[0], fa.plane[1], fa.plane[2]));
     const float tol = 5e-5f;
-    for (int j = 0; j < npts; ++j) {
-        GeoPoint& g = G.pt[j];
-        g.kind = PK_ATTACHED;
-        g.local = mul_t(RB, p[j] - xB);
-        float bestV = tol;
-        for (int i = 0; i < nvB; ++i) {
-            const float3 w = mul(RB, vtx(S, hB, face_vertex(S, fb, i))) + xB;
-            const float e = length(w - p[j]);
-            if (e < bestV) { bestV = e; g.kind = PK_VERTEX; g.i0 = i; }
-        }
-        if (g.kind == PK_VERTEX) continue;
-        // side planes containing the point
-        int on[2] = {-1, -1};
-        float onErr[2] = {tol, tol};
-        for (int k = 0; k < nvA; ++k) {
-            const float3 va = vtx(S, hA, face_vertex(S, fa, k));
-            const float3 vb = vtx(S, hA, face_vertex(S, fa, (k + 1) % nvA));
-            float3 pn = -cross(mul(RA, va - vb), nAw);
-            const float l = length(pn);
-            if (l <= 0.f) continue;
-            pn = pn * (1.f / l);
-            const float e = fabsf(dot(pn, p[j] - mul(RA, va)));
-            if (e < onErr[0]) { onErr[1] = onErr[0]; on[1] = on[0]; onErr[0] = e; on[0] = k; }
-            else if (e < onErr[1]) { onErr[1] = e; on[1] = k; }
-        }
-        if (on[0] < 0) { ++miss; continue; }
-        // an incident edge through the point, crossing the side plane
-        // (not lying in it: the intersection must be well defined)
-        const float3 vk = vtx(S, hA, face_vertex(S, fa, on[0]));
-        const float3 vk1 = vtx(S, hA, face_vertex(S, fa, (on[0] + 1) % nvA));
-        const float3 pnk = normalize(-cross(mul(RA, vk - vk1), nAw));
-        int edge = -1;
-        float bestE = tol;
-        for (int i = 0; i < nvB; ++i) {
-            const float3 a = mul(RB, vtx(S, hB, face_vertex(S, fb, i))) + xB;
-            const float3 b = mul(RB, vtx(S, hB, face_vertex(S, fb, (i + 1) % nvB))) + xB;
-            const float3 u = b - a;
-            const float uu = dot(u, u);
-            if (uu <= 0.f) continue;
-            if (fabsf(dot(pnk, u)) < 1e-3f * sqrtf(uu)) continue;
-            const float t = dot(p[j] - a, u) / uu;
-            if (t < -1e-4f || t > 1.f + 1e-4f) continue;
-            const float e = length(a + u * t - p[j]);
-            if (e < bestE) { bestE = e; edge = i; }
-        }
-        if (edge >= 0) {
-            g.kind = PK_EDGE;
-            g.i0 = edge;
-            g.i1 = (edge + 1) % nvB;
-            g.k = on[0];
-        } else if (on[1] >= 0 && corner_ok(S, hA, hB, fa, fb, RA, RB, nAw, on[0], on[1])) {
-            g.kind = PK_CORNER;
-            g.i0 = on[0];
-            g.i1 = on[1];
-        } else {
-            ++miss;
+    g.kind = PK_ATTACHED;
+    g.local = mul_t(RB, p - xB);
+    float bestV = tol;
+    for (int i = 0; i < nvB; ++i) {
+        const float3 w = mul(RB, vtx(S, hB, face_vertex(S, fb, i))) + xB;
+        const float e = length(w - p);
+        if (e < bestV) { bestV = e; g.kind = PK_VERTEX; g.i0 = i; }
+    }
+    if (g.kind == PK_VERTEX) return false;
+    // side planes containing the point
+    int on[2] = {-1, -1};
+    float onErr[2] = {tol, tol};
+    for (int k = 0; k < nvA; ++k) {
+        const float3 va = vtx(S, hA, face_vertex(S, fa, k));
+        const float3 vb = vtx(S, hA, face_vertex(S, fa, (k + 1) % nvA));
+        float3 pn = -cross(mul(RA, va - vb), nAw);
+        const float l = length(pn);
+        if (l <= 0.f) continue;
+        pn = pn * (1.f / l);
+        const float e = fabsf(dot(pn, p - mul(RA, va)));
+        if (e < onErr[0]) { onErr[1] = onErr[0]; on[1] = on[0]; onErr[0] = e; on[0] = k; }
+        else if (e < onErr[1]) { onErr[1] = e; on[1] = k; }
+    }
+    if (on[0] < 0) return true;
+    // an incident edge through the point, crossing the side plane
+    // (not lying in it: the intersection must be well defined)
+    const float3 vk = vtx(S, hA, face_vertex(S, fa, on[0]));
+    const float3 vk1 = vtx(S, hA, face_vertex(S, fa, (on[0] + 1) % nvA));
+    const float3 pnk = normalize(-cross(mul(RA, vk - vk1), nAw));
+    int edge = -1;
+    float bestE = tol;
+    for (int i = 0; i < nvB; ++i) {
+        const float3 a = mul(RB, vtx(S, hB, face_vertex(S, fb, i))) + xB;
+        const float3 b = mul(RB, vtx(S, hB, face_vertex(S, fb, (i + 1) % nvB))) + xB;
+        const float3 u = b - a;
+        const float uu = dot(u, u);
+        if (uu <= 0.f) continue;
+        if (fabsf(dot(pnk, u)) < 1e-3f * sqrtf(uu)) continue;
+        const float t = dot(p - a, u) / uu;
+        if (t < -1e-4f || t > 1.f + 1e-4f) continue;
+        const float e = length(a + u * t - p);
+        if (e < bestE) { bestE = e; edge = i; }
+    }
+    if (edge >= 0) {
+        g.kind = PK_EDGE;
+        g.i0 = edge;
+        g.i1 = (edge + 1) % nvB;
+        g.k = on[0];
+    } else if (on[1] >= 0 && corner_ok(S, hA, hB, fa, fb, RA, RB, nAw, on[0], on[1])) {
+        g.kind = PK_CORNER;
+        g.i0 = on[0];
+        g.i1 = on[1];
+    } else {
+        return true;
+    }
+    return false;
+}
+
+// The lanes of a manifold's group are half a warp; both halves go through the
+// same votes and shuffles, each with its own values.
+constexpr int kLanes = 16;
+__device__ __forceinline__ unsigned group_ballot(bool x) {
+    return __ballot_sync(0xffffffffu, x) >> (threadIdx.x & 16) & 0xffffu;
+}
+// Smallest value of the group and its index, the lowest index of equal ones.
+__device__ __forceinline__ void group_least(float& v, int& i) {
+#pragma unroll
+    for (int d = kLanes / 2; d > 0; d >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, v, d);
+        const int oi = __shfl_xor_sync(0xffffffffu, i, d);
+        if (ov < v || (ov == v && oi < i)) {
+            v = ov;
+            i = oi;
         }
     }
-    return miss;
 }
 
 // Faces of h whose sign * (n . sep) is within the forward's FP32 window
 // (4e-6) of the extreme, extreme first: clipHullAgainstHull's choice, or
 // its candidates where faces tie within FP32 (the forward decides those in
-// float-float, exact ties to the lowest index).
+// float-float, exact ties to the lowest index). By a group's lanes, to out.
 __device__ int face_candidates(const b3::ShapesDev& S, const b3ConvexPolyhedron& h, const Mat3& R, float3 sep,
                                float sign, int* out, int maxOut) {
+    const int lane = threadIdx.x & (kLanes - 1);
+    auto extent = [&](int f) {
+        const b3Face fc = S.faces[h.faceOffset + f];
+        return sign * dot(mul(R, make_float3(fc.plane[0], fc.plane[1], fc.plane[2])), sep);
+    };
     float best = FLT_MAX;
     int bi = 0;
-    for (int f = 0; f < h.numFaces; ++f) {
-        const b3Face fc = S.faces[h.faceOffset + f];
-        const float d = sign * dot(mul(R, make_float3(fc.plane[0], fc.plane[1], fc.plane[2])), sep);
+    for (int f = lane; f < h.numFaces; f += kLanes) {
+        const float d = extent(f);
         if (d < best) { best = d; bi = f; }
     }
-    int n = 0;
-    out[n++] = bi;
-    for (int f = 0; f < h.numFaces && n < maxOut; ++f) {
-        if (f == bi) continue;
-        const b3Face fc = S.faces[h.faceOffset + f];
-        const float d = sign * dot(mul(R, make_float3(fc.plane[0], fc.plane[1], fc.plane[2])), sep);
-        if (d <= best + 4e-6f) out[n++] = f;
+    group_least(best, bi);
+    if (lane == 0) out[0] = bi;
+    int n = 1;
+    const int faces = __reduce_max_sync(0xffffffffu, h.numFaces);
+    for (int f0 = 0; f0 < faces; f0 += kLanes) {
+        const int f = f0 + lane;
+        const bool near = f < h.numFaces && f != bi && extent(f) <= best + 4e-6f;
+        const unsigned all = group_ballot(near);
+        const int at = n + __popc(all & ((1u << lane) - 1u));
+        if (near && at < maxOut) out[at] = f;
+        n += __popc(all);
     }
-    return n;
+    return min(n, maxOut);
 }
 
-// Classify the stored manifold against the forward poses (values only).
-__device__ void geo_classify(Geo& G, const b3::ShapesDev& S, const b3ConvexPolyhedron& hA,
+// Classify the stored manifold against the forward poses (values only), by a
+// group's lanes; G and cand lie in shared memory.
+__device__ void geo_classify(Geo& G, int (*cand)[4], const b3::ShapesDev& S, const b3ConvexPolyhedron& hA,
                              const b3ConvexPolyhedron& hB, const Mat3& RA, const Mat3& RB, float3 xB, float3 sep,
-                             const float3* p, int npts, int* unclassified) {
-    // separating axis: the feature whose direction matches sep best
+                             float3 p, int npts, bool on, int* unclassified) {
+    const int lane = threadIdx.x & (kLanes - 1);
+    // separating axis: the feature whose direction matches sep best, in the
+    // order faces of A, faces of B, pairs of edges, each with both signs
+    const int nfA = hA.numFaces, nf = nfA + hB.numFaces;
+    const int total = nf + hA.numUniqueEdges * hB.numUniqueEdges;
     float best = 1e-4f;
-    G.axisKind = AX_ATTACHED;
-    G.ax0 = G.ax1 = 0;
-    G.axisSign = 1.f;
-    G.nLocalA = mul_t(RA, sep);
-    for (int side = 0; side < 2; ++side) {
-        const b3ConvexPolyhedron& h = side ? hB : hA;
-        const Mat3& R = side ? RB : RA;
-        for (int f = 0; f < h.numFaces; ++f) {
-            const b3Face fc = S.faces[h.faceOffset + f];
-            const float3 nw = mul(R, make_float3(fc.plane[0], fc.plane[1], fc.plane[2]));
-            for (int sg = 0; sg < 2; ++sg) {
-                const float s = sg ? -1.f : 1.f;
-                const float3 dlt = nw * s - sep;
-                const float e = fmaxf(fabsf(dlt.x), fmaxf(fabsf(dlt.y), fabsf(dlt.z)));
-                if (e < best) { best = e; G.axisKind = side ? AX_FACE_B : AX_FACE_A; G.ax0 = f; G.axisSign = s; }
-            }
-        }
-    }
-    for (int ea = 0; ea < hA.numUniqueEdges; ++ea) {
-        const float3 a = mul(RA, f3(S.edges[hA.uniqueEdgesOffset + ea]));
-        for (int eb = 0; eb < hB.numUniqueEdges; ++eb) {
+    int bi = 0x7fffffff;
+    for (int c = lane; c < total; c += kLanes) {
+        float3 dir;
+        if (c < nf) {
+            const b3Face fc = S.faces[c < nfA ? hA.faceOffset + c : hB.faceOffset + c - nfA];
+            dir = mul(c < nfA ? RA : RB, make_float3(fc.plane[0], fc.plane[1], fc.plane[2]));
+        } else {
+            const int ea = (c - nf) / hB.numUniqueEdges, eb = (c - nf) % hB.numUniqueEdges;
+            const float3 a = mul(RA, f3(S.edges[hA.uniqueEdgesOffset + ea]));
             const float3 b = mul(RB, f3(S.edges[hB.uniqueEdgesOffset + eb]));
-            const float3 c = cross(a, b);
-            const float l = length(c);
+            dir = cross(a, b);
+            const float l = length(dir);
             if (l < 1e-6f) continue;
-            const float3 cn = c * (1.f / l);
-            for (int sg = 0; sg < 2; ++sg) {
-                const float s = sg ? -1.f : 1.f;
-                const float3 dlt = cn * s - sep;
-                const float e = fmaxf(fabsf(dlt.x), fmaxf(fabsf(dlt.y), fabsf(dlt.z)));
-                if (e < best) { best = e; G.axisKind = AX_EDGES; G.ax0 = ea; G.ax1 = eb; G.axisSign = s; }
-            }
+            dir = dir * (1.f / l);
+        }
+        for (int sg = 0; sg < 2; ++sg) {
+            const float3 dlt = dir * (sg ? -1.f : 1.f) - sep;
+            const float e = fmaxf(fabsf(dlt.x), fmaxf(fabsf(dlt.y), fabsf(dlt.z)));
+            if (e < best) { best = e; bi = 2 * c + sg; }
         }
     }
-    if (G.axisKind == AX_ATTACHED) atomicAdd(unclassified, 1);
+    group_least(best, bi);
+    const bool attached = bi == 0x7fffffff;
+    if (lane == 0) {
+        const int c = bi >> 1;
+        G.axisKind = attached ? AX_ATTACHED : c < nfA ? AX_FACE_A : c < nf ? AX_FACE_B : AX_EDGES;
+        G.ax0 = G.ax1 = 0;
+        if (!attached) {
+            G.ax0 = c < nfA ? c : c < nf ? c - nfA : (c - nf) / hB.numUniqueEdges;
+            if (c >= nf) G.ax1 = (c - nf) % hB.numUniqueEdges;
+        }
+        G.axisSign = !attached && (bi & 1) ? -1.f : 1.f;
+        G.nLocalA = mul_t(RA, sep);
+    }
     // reference / incident faces: clipHullAgainstHull's choice, trying the
     // faces tied within FP32 until the points fit one pair of them
-    int candA[4], candB[4];
-    const int nA = face_candidates(S, hA, RA, sep, 1.f, candA, 4);
-    const int nB = face_candidates(S, hB, RB, sep, -1.f, candB, 4);
-    int bestMiss = 1 << 30, bestA = candA[0], bestB = candB[0];
-    for (int ia = 0; ia < nA && bestMiss > 0; ++ia)
-        for (int ib = 0; ib < nB && bestMiss > 0; ++ib) {
-            G.faceA = candA[ia];
-            G.faceB = candB[ib];
-            const int miss = geo_points(G, S, hA, hB, RA, RB, xB, p, npts);
-            if (miss < bestMiss) { bestMiss = miss; bestA = candA[ia]; bestB = candB[ib]; }
+    const int nA = face_candidates(S, hA, RA, sep, 1.f, cand[0], 4);
+    const int nB = face_candidates(S, hB, RB, sep, -1.f, cand[1], 4);
+    __syncwarp();
+    int least = 1 << 30, bestA = 0, bestB = 0;
+    GeoPoint g = {}, found = {};
+    for (int k = 0;; ++k) {
+        const bool run = k < nA * nB && least > 0;
+        if (!__any_sync(0xffffffffu, run)) break;
+        const int fA = run ? cand[0][k / nB] : 0, fB = run ? cand[1][k % nB] : 0;
+        bool miss = false;
+        if (run && lane < npts) miss = geo_point(g, fA, fB, S, hA, hB, RA, RB, xB, p);
+        const int misses = __popc(group_ballot(miss));
+        if (run && misses < least) {
+            least = misses;
+            bestA = fA;
+            bestB = fB;
+            found = g;
         }
-    G.faceA = bestA;
-    G.faceB = bestB;
-    const int miss = geo_points(G, S, hA, hB, RA, RB, xB, p, npts);
-    if (miss) atomicAdd(unclassified, miss);
+    }
+    if (lane < npts) G.pt[lane] = found;
+    if (lane == 0) {
+        G.faceA = bestA;
+        G.faceB = bestB;
+        if (on && attached) atomicAdd(unclassified, 1);
+        if (on && least) atomicAdd(unclassified, least);
+    }
+    __syncwarp();
 }
 
 struct ManifoldArgs {
@@ -788,146 +918,137 @@ struct ManifoldArgs {
     int* unclassified;
 };
 
+// A manifold's 45 set-up directions and 12 pose directions are passes of their
+// own over the same values, and the searches of the classification are minima:
+// a group of 16 lanes shares them. Bound by the instructions of the 45 passes;
+// 32,308 manifolds: 473 -> 268 us against a thread per manifold, whose arrays
+// went through local memory. One pass in reverse in place of the 45 takes 101
+// us, but rounds otherwise where a contact slides at 4e-4 m/s: the direction
+// of friction is a quotient of two such values there, and the gradients of 16
+// steps move by 1.5e-4 of their size.
 __global__ void __launch_bounds__(128)
 k_adj_manifold(SolverView V, AdjView A, ManifoldArgs MA, StepParams P) {
+    constexpr int kGroups = 128 / kLanes;
+    __shared__ struct {
+        Geo G;
+        int cand[2][4];
+        float4 p[4];     // points relative to body A, depths
+        float gin[kInputs];
+        float pose[12];
+    } shared[kGroups];
     const int M = *V.numManifolds;
     const size_t cap = (size_t)V.cap;
-    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & (kLanes - 1), group = threadIdx.x / kLanes;
+    auto& sh = shared[group];
+    const float3 z3 = make_float3(0.f, 0.f, 0.f);
+    for (int m0 = blockIdx.x * kGroups; m0 < M; m0 += gridDim.x * kGroups) {
+        const bool on = m0 + group < M;
+        const int m = min(m0 + group, M - 1);
         const float4 ids = R(V, kIds, m), nn = R(V, kNorm, m), ia = R(V, kInA, m), ib = R(V, kInB, m);
         const int bA = __float_as_int(ids.x), bB = __float_as_int(ids.y);
         const int dyn = __float_as_int(R(V, kHead1, m).z) >> 16;
         const float kA = ids.z, kB = ids.w;
-        const b3Contact4 c = MA.contacts[MA.manifoldPair[m]];
-        const int npts = (int)c.worldNormal[3];
+        const b3Contact4* const c = MA.contacts + MA.manifoldPair[m];
+        const int npts = (int)c->worldNormal[3];
         const bool dynA = dyn & 1, dynB = dyn & 2;
         // forward values; positions relative to body A's position
         const float3 oA = f3(MA.pos[bA]);
         const float3 xB = f3(MA.pos[bB]) - oA;
         const float3 g = P.gravity * P.dt;
-        const float3 vA = dynA ? f3(MA.linVel[bA]) + g : make_float3(0.f, 0.f, 0.f);
-        const float3 wA = dynA ? f3(MA.angVel[bA]) : make_float3(0.f, 0.f, 0.f);
-        const float3 vB = dynB ? f3(MA.linVel[bB]) + g : make_float3(0.f, 0.f, 0.f);
-        const float3 wB = dynB ? f3(MA.angVel[bB]) : make_float3(0.f, 0.f, 0.f);
+        const float3 vA = dynA ? f3(MA.linVel[bA]) + g : z3;
+        const float3 wA = dynA ? f3(MA.angVel[bA]) : z3;
+        const float3 vB = dynB ? f3(MA.linVel[bB]) + g : z3;
+        const float3 wB = dynB ? f3(MA.angVel[bB]) : z3;
         const float3 iiA = f3(ia), iiB = f3(ib);
         const float imA = nn.w, imB = ia.w;
-        const float3 n0 = normalize(make_float3(-c.worldNormal[0], -c.worldNormal[1], -c.worldNormal[2]));
-        float3 p0[4];
-        float dep0[4];
-        for (int j = 0; j < 4; ++j) {
-            p0[j] = make_float3(c.worldPos[j][0], c.worldPos[j][1], c.worldPos[j][2]) - oA;
-            dep0[j] = c.worldPos[j][3];
-        }
+        const float3 n0 = normalize(make_float3(-c->worldNormal[0], -c->worldNormal[1], -c->worldNormal[2]));
         const float restitution = MA.Bd.restitution[bA] * MA.Bd.restitution[bB];
+        const float* at = c->worldPos[lane & 3];
+        const float3 p = make_float3(at[0], at[1], at[2]) - oA;
+        if (lane < 4) sh.p[lane] = f4(p, at[3]);
+        __syncwarp();
         // --- setup: one forward-mode pass per input ---------------------
-        // inputs: xA 0-2, xB 3-5, vA 6-8, wA 9-11, vB 12-14, wB 15-17, imA 18,
-        // imB 19, iiA 20-22, iiB 23-25, n 26-28, p 29-40, depth 41-44
-        float gin[45];
-        const float3 z3 = make_float3(0.f, 0.f, 0.f);
-        for (int k = 0; k < 45; ++k) {
-            gin[k] = 0.f;
+        for (int k = lane; k < kInputs; k += kLanes) {
             const bool aSide = (k < 3) || (k >= 6 && k < 12) || k == 18 || (k >= 20 && k < 23);
             const bool bSide = (k >= 3 && k < 6) || (k >= 12 && k < 18) || k == 19 || (k >= 23 && k < 26);
-            if ((aSide && !dynA) || (bSide && !dynB)) continue;
-            if (k >= 29 && k < 41 && (k - 29) / 3 >= npts) continue;
-            if (k >= 41 && k - 41 >= npts) continue;
-            auto e = [&](int base) {
-                return make_float3(k == base ? 1.f : 0.f, k == base + 1 ? 1.f : 0.f, k == base + 2 ? 1.f : 0.f);
-            };
-            SetupIn I;
-            I.xA = d3(z3, e(0));
-            I.xB = d3(xB, e(3));
-            I.vA = d3(vA, e(6));
-            I.wA = d3(wA, e(9));
-            I.vB = d3(vB, e(12));
-            I.wB = d3(wB, e(15));
-            I.imA = du(imA, k == 18 ? 1.f : 0.f);
-            I.imB = du(imB, k == 19 ? 1.f : 0.f);
-            I.iiA = d3(iiA, e(20));
-            I.iiB = d3(iiB, e(23));
-            I.n = d3(n0, e(26));
-            for (int j = 0; j < 4; ++j) {
-                I.p[j] = d3(p0[j], e(29 + 3 * j));
-                I.depth[j] = du(dep0[j], k == 41 + j ? 1.f : 0.f);
+            const bool unused = (aSide && !dynA) || (bSide && !dynB) ||
+                                (k >= kInPoint && k < kInDepth && (k - kInPoint) / 3 >= npts) ||
+                                (k >= kInDepth && k - kInDepth >= npts);
+            float acc = 0.f;
+            if (!unused) {
+                SetupIn I;
+                I.xA = d3(z3, unit_at(k, 0));
+                I.xB = d3(xB, unit_at(k, 3));
+                I.vA = d3(vA, unit_at(k, 6));
+                I.wA = d3(wA, unit_at(k, 9));
+                I.vB = d3(vB, unit_at(k, 12));
+                I.wB = d3(wB, unit_at(k, 15));
+                I.imA = du(imA, k == 18 ? 1.f : 0.f);
+                I.imB = du(imB, k == 19 ? 1.f : 0.f);
+                I.iiA = d3(iiA, unit_at(k, 20));
+                I.iiB = d3(iiB, unit_at(k, 23));
+                I.n = d3(n0, unit_at(k, kInNormal));
+                I.p = sh.p;
+                I.k = k;
+                acc = setup_tangent(I, V, A, m, npts, kA, kB, restitution, P);
             }
-            gin[k] = setup_tangent(I, V, A, m, npts, kA, kB, restitution, P);
+            sh.gin[k] = acc;
         }
-        // header adjoints from the solve (inverse masses, inertias, mu)
-        const float4 ga1 = A.rowAdj[cap + m];
-        const float4 ga2 = A.rowAdj[2 * cap + m];
-        const float4 ga3 = A.rowAdj[3 * cap + m];
-        float gimA = ga1.x + gin[18], gimB = ga1.y + gin[19];
-        float3 giiA = f3(ga2) + make_float3(gin[20], gin[21], gin[22]);
-        float3 giiB = f3(ga3) + make_float3(gin[23], gin[24], gin[25]);
-        const float gmu = ga1.z;
         // --- geometry: 12 pose directions -------------------------------
-        float3 gxA = make_float3(gin[0], gin[1], gin[2]), gxB = make_float3(gin[3], gin[4], gin[5]);
-        float3 gthA = z3, gthB = z3;
         const int colA = MA.Bd.collidable[bA], colB = MA.Bd.collidable[bB];
         const b3ConvexPolyhedron hA = MA.S.polys[MA.S.cols[colA].shapeIndex];
         const b3ConvexPolyhedron hB = MA.S.polys[MA.S.cols[colB].shapeIndex];
         const Mat3 RA = quat_to_mat(MA.quat[bA]), RB = quat_to_mat(MA.quat[bB]);
-        Geo G;
-        geo_classify(G, MA.S, hA, hB, RA, RB, xB, n0, p0, npts, MA.unclassified);
-        const float3 gn = make_float3(gin[26], gin[27], gin[28]);
-        for (int k = 0; k < 12; ++k) {
-            const int body = k < 6 ? 0 : 1;
-            if ((body == 0 && !dynA) || (body == 1 && !dynB)) continue;
-            const int kk = k % 6;
-            const float3 ex = make_float3(kk == 0 ? 1.f : 0.f, kk == 1 ? 1.f : 0.f, kk == 2 ? 1.f : 0.f);
-            const float3 et = make_float3(kk == 3 ? 1.f : 0.f, kk == 4 ? 1.f : 0.f, kk == 5 ? 1.f : 0.f);
-            PoseD PA, PB;
-            PA.R = RA;
-            PB.R = RB;
-            PA.x = d3(z3, body == 0 ? ex : z3);
-            PA.th = body == 0 ? et : z3;
-            PB.x = d3(xB, body == 1 ? ex : z3);
-            PB.th = body == 1 ? et : z3;
-            D3 nD, pD[4];
-            Du dD[4];
-            geo_eval(G, MA.S, hA, hB, PA, PB, npts, nD, pD, dD);
-            float acc = dot(gn, tan3(nD));
-            for (int j = 0; j < npts; ++j)
-                acc += gin[29 + 3 * j] * pD[j].x.d + gin[30 + 3 * j] * pD[j].y.d + gin[31 + 3 * j] * pD[j].z.d +
-                       gin[41 + j] * dD[j].d;
-            if (!isfinite(acc)) {
-                // a degenerate feature slipped through the classification
-                atomicAdd(MA.unclassified, 1);
-                acc = 0.f;
+        geo_classify(sh.G, sh.cand, MA.S, hA, hB, RA, RB, xB, n0, p, npts, on, MA.unclassified);
+        if (lane < 12) {
+            const int body = lane < 6 ? 0 : 1, kk = lane - 6 * body;
+            float acc = 0.f;
+            if (body == 0 ? dynA : dynB) {
+                const float3 ex = unit_at(kk, 0), et = unit_at(kk, 3);
+                PoseD PA, PB;
+                PA.R = RA;
+                PB.R = RB;
+                PA.x = d3(z3, body == 0 ? ex : z3);
+                PA.th = body == 0 ? et : z3;
+                PB.x = d3(xB, body == 1 ? ex : z3);
+                PB.th = body == 1 ? et : z3;
+                acc = geo_tangent(sh.G, MA.S, hA, hB, PA, PB, npts, sh.gin);
+                if (!isfinite(acc)) {
+                    // a degenerate feature slipped through the classification
+                    if (on) atomicAdd(MA.unclassified, 1);
+                    acc = 0.f;
+                }
             }
-            float* dst = body == 0 ? (kk < 3 ? &gxA.x : &gthA.x) : (kk < 3 ? &gxB.x : &gthB.x);
-            dst[kk % 3] += acc;
+            sh.pose[lane] = acc;
         }
-        // --- friction of the pair -> the bodies' coefficients -----------
-        const float muA = MA.Bd.friction[bA], muB = MA.Bd.friction[bB];
-        float gmuA, gmuB;
-        if (P.frictionCombine == 1) {
-            gmuA = gmu * muB;
-            gmuB = gmu * muA;
-        } else {
-            const float mc = sqrtf(muA * muB);
-            gmuA = mc > 0.f ? gmu * 0.5f * mc / muA : 0.f;
-            gmuB = mc > 0.f ? gmu * 0.5f * mc / muB : 0.f;
-        }
-        // --- per-copy contributions --------------------------------------
-        for (int side = 0; side < 2; ++side) {
-            if (!(dyn & (1 << side))) continue;
-            const size_t slot = V.incPos[2 * m + side];
+        __syncwarp();
+        // --- one lane per dynamic side: the body's contribution ----------
+        if (on && lane < 2 && (dyn & (1 << lane))) {
+            // friction of the pair -> the bodies' coefficients
+            const float4 head = A.rowAdj[cap + m];
+            const float gmu = head.z;
+            const float muA = MA.Bd.friction[bA], muB = MA.Bd.friction[bB];
+            float gmuSide;
+            if (P.frictionCombine == 1) {
+                gmuSide = gmu * (lane ? muA : muB);
+            } else {
+                const float mc = sqrtf(muA * muB);
+                gmuSide = mc > 0.f ? gmu * 0.5f * mc / (lane ? muB : muA) : 0.f;
+            }
+            // header adjoints from the solve (inverse masses, inertias)
+            const float gim = (lane ? head.y : head.x) + sh.gin[18 + lane];
+            auto three = [&](int k) { return make_float3(sh.gin[k], sh.gin[k + 1], sh.gin[k + 2]); };
+            const float* ps = sh.pose + 6 * lane;
+            const size_t slot = V.incPos[2 * m + lane];
             const size_t stride = 2 * cap;
             float4* C = A.contrib;
-            if (side == 0) {
-                C[0 * stride + slot] = f4(gxA, gimA);
-                C[1 * stride + slot] = f4(gthA, gmuA);
-                C[2 * stride + slot] = make_float4(gin[6], gin[7], gin[8], 0.f);
-                C[3 * stride + slot] = make_float4(gin[9], gin[10], gin[11], 0.f);
-                C[4 * stride + slot] = f4(giiA, 0.f);
-            } else {
-                C[0 * stride + slot] = f4(gxB, gimB);
-                C[1 * stride + slot] = f4(gthB, gmuB);
-                C[2 * stride + slot] = make_float4(gin[12], gin[13], gin[14], 0.f);
-                C[3 * stride + slot] = make_float4(gin[15], gin[16], gin[17], 0.f);
-                C[4 * stride + slot] = f4(giiB, 0.f);
-            }
+            C[0 * stride + slot] = f4(three(3 * lane) + make_float3(ps[0], ps[1], ps[2]), gim);
+            C[1 * stride + slot] = f4(make_float3(ps[3], ps[4], ps[5]), gmuSide);
+            C[2 * stride + slot] = f4(three(6 + 6 * lane));
+            C[3 * stride + slot] = f4(three(9 + 6 * lane));
+            C[4 * stride + slot] = f4(f3(A.rowAdj[(size_t)(2 + lane) * cap + m]) + three(20 + 3 * lane));
         }
+        __syncwarp();  // before the next manifold's values
     }
 }
 
@@ -971,7 +1092,9 @@ struct b3Adjoint_t {
     int numSteps = 0, K = 1, N = 0, cap = 0, iterations = 0;
     int numCkpt = 0;
     float4* ckpt = nullptr;   // [numCkpt][4][N]
-    float4* seg = nullptr;    // [K][4][N]
+    float4* seg = nullptr;    // [K][4][N]: pre-step states of one segment
+    float4* lastPre = nullptr;  // [4][N]: state before the last step
+    int segHeld = -1;         // segment whose states seg holds
     b3::JacobiTape tape{};
     float4 *gX = nullptr, *gTh = nullptr, *gV = nullptr, *gW = nullptr, *gDv = nullptr, *gDw = nullptr;
     float *gInvMass = nullptr, *gMu = nullptr;
@@ -1042,22 +1165,31 @@ int reverse_step(b3Adjoint_t* a, const float4* pre, cudaStream_t st) {
     B3_CHECK_LAUNCH();
     if (a->iterations > 0) {
         B3_CUDA(cudaMemsetAsync(w->d.scalars + b3::S_BAR_COUNT, 0, sizeof(int32_t) * 2, st));
-        const int threads = 256;
-        int occ = 1;
-        B3_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_jacobi_adjoint, threads, 0));
-        occ = occ < 1 ? 1 : (occ > 4 ? 4 : occ);
+        // as in the solve: the grid from the expected manifolds (about 3 per
+        // body), up to two blocks an SM, shared memory for a thread's share
+        const int threads = 128, perSm = 2;
         const long long est = std::min<long long>((long long)w->cfg.maxPairs, 3LL * (long long)N);
         const int want = (int)std::max<long long>(1, (est + threads - 1) / threads);
-        const int grid = std::min(w->ctx->numSMs * occ, want);
+        const int blocks = std::min(w->ctx->numSMs * perSm, want);
+        const size_t one = (size_t)kPhaseSlots * threads * sizeof(float4);
+        const int need = (int)((est + (long long)blocks * threads - 1) / ((long long)blocks * threads));
+        int resident = std::min(need, (int)((size_t)w->ctx->maxSmemOptin / perSm / one));
+        const size_t smem = one * resident;
+        if (smem > 48 * 1024)
+            B3_CUDA(cudaFuncSetAttribute(k_jacobi_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        int occ = 1;
+        B3_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_jacobi_adjoint, threads, smem));
+        const int grid = std::min(w->ctx->numSMs * std::max(1, std::min(occ, perSm)), want);
         int iters = a->iterations;
         uint32_t* bar = (uint32_t*)(w->d.scalars + b3::S_BAR_COUNT);
         int32_t* err = w->d.scalars + b3::S_ERR;
         b3Counters* ctr = w->d.counters;
         b3::JacobiTape T = a->tape;
-        void* args[] = {&V, &T, &A, &iters, &bar, &err, &ctr};
+        void* args[] = {&V, &T, &A, &iters, &resident, &bar, &err, &ctr};
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(grid);
         cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeCooperative;
@@ -1077,7 +1209,7 @@ int reverse_step(b3Adjoint_t* a, const float4* pre, cudaStream_t st) {
     MA.contacts = w->d.contacts;
     MA.unclassified = a->unclassified;
     if (a->iterations > 0) {
-        const int g = w->ctx->numSMs * 4;
+        const int g = w->ctx->numSMs * 16;
         k_adj_manifold<<<g, 128, 0, st>>>(V, A, MA, P);
         B3_CHECK_LAUNCH();
         k_adj_gather<<<(N + 255) / 256, 256, 0, st>>>(N, w->d.invMass, w->d.invInertia, V, A);
@@ -1117,7 +1249,7 @@ extern "C" int b3_adjoint_create(b3World w, int numSteps, int checkpointEvery, b
     // one step and the adjoint buffers, checked against free device memory
     {
         const size_t f4 = sizeof(float4);
-        const size_t need = f4 * ((size_t)a->numCkpt * 4 * N + (size_t)a->K * 4 * N + phases * 4 * cap +
+        const size_t need = f4 * ((size_t)a->numCkpt * 4 * N + (size_t)a->K * 4 * N + 4 * N + phases * 4 * cap +
                                   (size_t)a->iterations * 3 * cap + 7 * N + (size_t)kAdjSlots * cap + 8 * cap +
                                   3 * cap + (size_t)kContrib * 2 * cap) +
                             2 * sizeof(float) * N;
@@ -1135,8 +1267,9 @@ extern "C" int b3_adjoint_create(b3World w, int numSteps, int checkpointEvery, b
     };
     if ((rc = aalloc(a, a->ckpt, (size_t)a->numCkpt * 4 * N)) != B3_OK) return fail(rc);
     if ((rc = aalloc(a, a->seg, (size_t)a->K * 4 * N)) != B3_OK) return fail(rc);
+    if ((rc = aalloc(a, a->lastPre, 4 * N)) != B3_OK) return fail(rc);
     if (phases > 0) {
-        if ((rc = aalloc(a, a->tape.copies, phases * 4 * cap)) != B3_OK) return fail(rc);
+        if ((rc = aalloc(a, a->tape.in, phases * 4 * cap)) != B3_OK) return fail(rc);
         if ((rc = aalloc(a, a->tape.lamN, (size_t)a->iterations * cap)) != B3_OK) return fail(rc);
         if ((rc = aalloc(a, a->tape.lamF, (size_t)a->iterations * 2 * cap)) != B3_OK) return fail(rc);
     }
@@ -1167,10 +1300,17 @@ extern "C" int b3_adjoint_forward(b3Adjoint a, void* stream) {
     B3_CUDA(cudaSetDevice(w->ctx->device));
     cudaStream_t st = as_stream(stream);
     const size_t N = (size_t)a->N;
+    // the last segment's pre-step states are kept as they come by, so that the
+    // reverse sweep starts without running that segment again
+    const int lastStart = (a->numCkpt - 1) * a->K;
+    a->segHeld = -1;
     for (int t = 0; t < a->numSteps; ++t) {
         if (t % a->K == 0) B3_TRY(copy_state(w, a->ckpt + (size_t)(t / a->K) * 4 * N, st, false));
+        if (t >= lastStart) B3_TRY(copy_state(w, a->seg + (size_t)(t - lastStart) * 4 * N, st, false));
+        if (t == a->numSteps - 1) B3_TRY(copy_state(w, a->lastPre, st, false));
         B3_TRY(b3_step(w, 1, stream));
     }
+    a->segHeld = a->numCkpt - 1;
     a->forwardDone = true;
     a->backwardDone = false;
     return B3_OK;
@@ -1201,10 +1341,14 @@ extern "C" int b3_adjoint_backward(b3Adjoint a, const float* dPos4, const float*
         const int t0 = sgi * a->K;
         const int t1 = std::min(t0 + a->K, a->numSteps);
         // recompute the segment's pre-step states from its checkpoint
-        B3_TRY(copy_state(w, a->ckpt + (size_t)sgi * 4 * N, st, true));
-        for (int t = t0; t < t1; ++t) {
-            B3_TRY(copy_state(w, a->seg + (size_t)(t - t0) * 4 * N, st, false));
-            if (t + 1 < t1) B3_TRY(b3::run_step(w, st, nullptr));
+        if (a->segHeld != sgi) {
+            a->segHeld = -1;
+            B3_TRY(copy_state(w, a->ckpt + (size_t)sgi * 4 * N, st, true));
+            for (int t = t0; t < t1; ++t) {
+                B3_TRY(copy_state(w, a->seg + (size_t)(t - t0) * 4 * N, st, false));
+                if (t + 1 < t1) B3_TRY(b3::run_step(w, st, nullptr));
+            }
+            a->segHeld = sgi;
         }
         for (int t = t1 - 1; t >= t0; --t) {
             const float4* pre = a->seg + (size_t)(t - t0) * 4 * N;
@@ -1214,8 +1358,8 @@ extern "C" int b3_adjoint_backward(b3Adjoint a, const float* dPos4, const float*
         }
     }
     // leave the world at the final state of the forward run
-    B3_TRY(copy_state(w, a->ckpt + (size_t)(a->numCkpt - 1) * 4 * N, st, true));
-    for (int t = (a->numCkpt - 1) * a->K; t < a->numSteps; ++t) B3_TRY(b3::run_step(w, st, nullptr));
+    B3_TRY(copy_state(w, a->lastPre, st, true));
+    B3_TRY(b3::run_step(w, st, nullptr));
     a->backwardDone = true;
     return B3_OK;
 }

@@ -291,10 +291,12 @@ constexpr int kNpCandSlots = 1 << 20;
 constexpr int kSolverRowSlots = 27;  // float4 streams of a manifold's constraint rows (solver_common.cuh)
 constexpr int kGsMaxBatch = 1024;  // batches per parity class (batched Gauss-Seidel)
 
-// Record of one Jacobi solve for the reverse sweep: every phase's solver-body
-// copies (dynamic sides) and the row impulses after it.
+// Record of one Jacobi solve for the reverse sweep: the velocities every phase
+// starts from, by manifold, and the row impulses after it.
 struct JacobiTape {
-    float4* copies;    // [2 * iterations][2 maxPairs][linear, angular], sorted by body
+    // [2 * iterations][4][maxPairs]: the velocities each phase started a manifold's
+    // copies from, linear and angular of A, then of B
+    float4* in;
     float4* lamN;      // [iterations][maxPairs]: normal rows 0..3 after each normal phase
     float4* lamF;      // [iterations][2][maxPairs]: friction rows 0..7 after each friction phase
 };

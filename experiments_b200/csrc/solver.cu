@@ -230,88 +230,6 @@ __global__ void k_setup_rows(b3::BodiesDev Bd, SolverView V, const int* __restri
 // ---------------------------------------------------------------------------
 // Persistent Jacobi kernels
 // ---------------------------------------------------------------------------
-// Streams of one manifold: in global memory (slot major, stride cap) or in
-// the block's shared memory (slot major, stride blockDim), where a thread
-// keeps the manifolds that it solves in every phase.
-struct GlobalRows {
-    float4* at;
-    size_t stride;
-    __device__ __forceinline__ float4& operator()(int slot) const { return at[(size_t)slot * stride]; }
-};
-struct SharedRows {
-    float4* at;
-    int stride;
-    __device__ __forceinline__ float4& operator()(int slot) const { return at[slot * stride]; }
-};
-// streams a phase reads or writes (all but kIds)
-constexpr int kPhaseSlots = kIds;
-static_assert(kIds == kRowSlots - 1, "the ids are the last stream");
-
-struct Heads {
-    uint32_t sA, eA, pA, sB, eB, pB;
-    int nRows, dyn;
-    float mu;
-};
-template <class Rows>
-__device__ __forceinline__ Heads load_heads(const Rows& S) {
-    const float4 a = S(kHead0), b = S(kHead1);
-    const int f = __float_as_int(b.z);
-    return Heads{__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z), __float_as_uint(a.w),
-                 __float_as_uint(b.x), __float_as_uint(b.y), f & 0xffff, f >> 16, b.w};
-}
-
-// Both bodies' averages, the first K copies of each side in flight at once
-// (past a range's end the last record again, which the sum leaves out).
-template <int K>
-__device__ __forceinline__ void gather_averages(const float4* __restrict__ copies, const Heads& H, float3& vA,
-                                                float3& wA, float3& vB, float3& wB) {
-    float4 l[2][K], a[2][K];
-    const uint32_t s[2] = {H.sA, H.sB}, e[2] = {H.eA, H.eB};
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int u = 0; u < K; ++u) {
-            const float4* r = copies + 2 * (size_t)min(s[h] + u, max(e[h], 1u) - 1u);
-            l[h][u] = __ldcg(r);
-            a[h][u] = __ldcg(r + 1);
-        }
-    float3 sl[2], sa[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        sl[h] = sa[h] = make_float3(0.f, 0.f, 0.f);
-#pragma unroll
-        for (int u = 0; u < K; ++u)
-            if (s[h] + u < e[h]) {
-                sl[h] += f3(l[h][u]);
-                sa[h] += f3(a[h][u]);
-            }
-        for (uint32_t i0 = s[h] + K; i0 < e[h]; i0 += K) {
-#pragma unroll
-            for (int u = 0; u < K; ++u) {
-                const float4* r = copies + 2 * (size_t)min(i0 + u, e[h] - 1u);
-                l[h][u] = __ldcg(r);
-                a[h][u] = __ldcg(r + 1);
-            }
-#pragma unroll
-            for (int u = 0; u < K; ++u)
-                if (i0 + u < e[h]) {
-                    sl[h] += f3(l[h][u]);
-                    sa[h] += f3(a[h][u]);
-                }
-        }
-    }
-    if (H.dyn & 1) {
-        const float f = 1.f / (float)(H.eA - H.sA);
-        vA = scaled(sl[0], f);
-        wA = scaled(sa[0], f);
-    }
-    if (H.dyn & 2) {
-        const float f = 1.f / (float)(H.eB - H.sB);
-        vB = scaled(sl[1], f);
-        wB = scaled(sa[1], f);
-    }
-}
-
 // Both bodies' averages as the pass over the bodies left them, in the first
 // record of each body's range.
 __device__ __forceinline__ void read_averages(const float4* __restrict__ copies, const Heads& H, float3& vA, float3& wA,
@@ -414,6 +332,13 @@ __device__ __forceinline__ void solve_manifold(const Rows& S, bool friction, boo
     }
     float4* tn = TAPE ? T.lamN + (size_t)(phase >> 1) * cap + m : nullptr;
     float4* tf = TAPE ? T.lamF + (size_t)(phase & ~1) * cap + m : nullptr;
+    float4* const tape = TAPE ? T.in + (size_t)phase * 4 * cap + m : nullptr;
+    if (TAPE) {
+        tape[0] = f4(dvA);
+        tape[cap] = f4(dwA);
+        tape[2 * cap] = f4(dvB);
+        tape[3 * cap] = f4(dwB);
+    }
     if (H.nRows > 0) {
         if (!friction) normal_rows<TAPE>(S, H.nRows, dvA, dwA, dvB, dwB, tn);
         else friction_rows<TAPE>(S, H.nRows, H.mu, dvA, dwA, dvB, dwB, tf, cap);
@@ -422,22 +347,13 @@ __device__ __forceinline__ void solve_manifold(const Rows& S, bool friction, boo
         if (!friction) *tn = zero;
         else tf[0] = tf[cap] = zero;
     }
-    float4* const tape = TAPE ? T.copies + (size_t)phase * 4 * cap : nullptr;
     if (H.dyn & 1) {
         __stcg(&out[2 * (size_t)H.pA], f4(dvA));
         __stcg(&out[2 * (size_t)H.pA + 1], f4(dwA));
-        if (TAPE) {
-            tape[2 * (size_t)H.pA] = f4(dvA);
-            tape[2 * (size_t)H.pA + 1] = f4(dwA);
-        }
     }
     if (H.dyn & 2) {
         __stcg(&out[2 * (size_t)H.pB], f4(dvB));
         __stcg(&out[2 * (size_t)H.pB + 1], f4(dwB));
-        if (TAPE) {
-            tape[2 * (size_t)H.pB] = f4(dvB);
-            tape[2 * (size_t)H.pB + 1] = f4(dwB);
-        }
     }
 }
 

@@ -134,32 +134,6 @@ __device__ __forceinline__ void solve_row(float3 n, float3 t1, float3 t2, float 
     dwB = fma3(mulv(iiB, t2), delta, dwB);
 }
 
-// A row as the adjoint replays it: axis, angular parts, rhs and 1/diag of
-// normal row r, or of friction row r, of manifold m.
-struct RowData {
-    float3 n, t1, t2;
-    float rhs, jac;
-};
-__device__ __forceinline__ RowData load_row(const SolverView& V, int m, bool friction, int r) {
-    const int j = friction ? r >> 1 : r;
-    const float4 a = R(V, kPoint0 + 4 * j, m), b = R(V, kPoint0 + 4 * j + 1, m);
-    RowData D;
-    if (friction) {
-        const float4 d = R(V, kPoint0 + 4 * j + 2 + (r & 1), m);
-        const float4 q = R(V, kFJac + (r >> 2), m);
-        D.n = f3(d);
-        D.rhs = d.w;
-        D.jac = (r & 3) == 0 ? q.x : (r & 3) == 1 ? q.y : (r & 3) == 2 ? q.z : q.w;
-    } else {
-        D.n = f3(R(V, kNorm, m));
-        D.rhs = a.w;
-        D.jac = b.w;
-    }
-    D.t1 = arm(f3(a), D.n);
-    D.t2 = friction ? arm_rev(f3(b), D.n) : arm_neg(f3(b), D.n);
-    return D;
-}
-
 // a * s rounded by itself: fused into the row that adds to it, an average
 // would round differently where it is formed next to the rows and where it is
 // read back from memory.
@@ -193,6 +167,88 @@ __device__ __forceinline__ void copy_average(const float4* __restrict__ copies, 
     }
     lin = scaled(sl, 1.f / (float)(e - s));
     ang = scaled(sa, 1.f / (float)(e - s));
+}
+
+// Streams of one manifold: in global memory (slot major, stride cap) or in
+// the block's shared memory (slot major, stride blockDim), where a thread
+// keeps the manifolds that it solves in every phase.
+struct GlobalRows {
+    float4* at;
+    size_t stride;
+    __device__ __forceinline__ float4& operator()(int slot) const { return at[(size_t)slot * stride]; }
+};
+struct SharedRows {
+    float4* at;
+    int stride;
+    __device__ __forceinline__ float4& operator()(int slot) const { return at[slot * stride]; }
+};
+// streams a phase reads or writes (all but kIds)
+constexpr int kPhaseSlots = kIds;
+static_assert(kIds == kRowSlots - 1, "the ids are the last stream");
+
+struct Heads {
+    uint32_t sA, eA, pA, sB, eB, pB;
+    int nRows, dyn;
+    float mu;
+};
+template <class Rows>
+__device__ __forceinline__ Heads load_heads(const Rows& S) {
+    const float4 a = S(kHead0), b = S(kHead1);
+    const int f = __float_as_int(b.z);
+    return Heads{__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z), __float_as_uint(a.w),
+                 __float_as_uint(b.x), __float_as_uint(b.y), f & 0xffff, f >> 16, b.w};
+}
+
+// Both bodies' averages, the first K copies of each side in flight at once
+// (past a range's end the last record again, which the sum leaves out).
+template <int K>
+__device__ __forceinline__ void gather_averages(const float4* __restrict__ copies, const Heads& H, float3& vA,
+                                                float3& wA, float3& vB, float3& wB) {
+    float4 l[2][K], a[2][K];
+    const uint32_t s[2] = {H.sA, H.sB}, e[2] = {H.eA, H.eB};
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int u = 0; u < K; ++u) {
+            const float4* r = copies + 2 * (size_t)min(s[h] + u, max(e[h], 1u) - 1u);
+            l[h][u] = __ldcg(r);
+            a[h][u] = __ldcg(r + 1);
+        }
+    float3 sl[2], sa[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        sl[h] = sa[h] = make_float3(0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < K; ++u)
+            if (s[h] + u < e[h]) {
+                sl[h] += f3(l[h][u]);
+                sa[h] += f3(a[h][u]);
+            }
+        for (uint32_t i0 = s[h] + K; i0 < e[h]; i0 += K) {
+#pragma unroll
+            for (int u = 0; u < K; ++u) {
+                const float4* r = copies + 2 * (size_t)min(i0 + u, e[h] - 1u);
+                l[h][u] = __ldcg(r);
+                a[h][u] = __ldcg(r + 1);
+            }
+#pragma unroll
+            for (int u = 0; u < K; ++u)
+                if (i0 + u < e[h]) {
+                    sl[h] += f3(l[h][u]);
+                    sa[h] += f3(a[h][u]);
+                }
+        }
+    }
+    if (H.dyn & 1) {
+        const float f = 1.f / (float)(H.eA - H.sA);
+        vA = scaled(sl[0], f);
+        wA = scaled(sa[0], f);
+    }
+    if (H.dyn & 2) {
+        const float f = 1.f / (float)(H.eB - H.sB);
+        vB = scaled(sl[1], f);
+        wB = scaled(sa[1], f);
+    }
 }
 
 SolverView solver_view(b3World_t* w);
