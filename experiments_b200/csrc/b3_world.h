@@ -101,6 +101,7 @@ struct DevBuffers {
     float4* sapSorted = nullptr;      // small AABBs sorted by min x: (min, max) per proxy
     uint32_t* sapCount = nullptr;     // pairs per sorted proxy, then their offsets
     uint32_t* sapOffset = nullptr;
+    int* sapKept = nullptr;           // kSapKeep partners per sorted proxy
     uint32_t *keys = nullptr, *vals = nullptr, *keysAlt = nullptr, *valsAlt = nullptr;
     uint4* cellTable = nullptr;    // (stamp, first sorted index, end, -) per (world, cell)
     float4* sortedAabb = nullptr;  // small bodies' (min, max) in sorted order
@@ -289,6 +290,7 @@ __device__ __forceinline__ void begin_step(int32_t* scalars, b3Counters* counter
 // axis ranking beyond this recompute their FP32 sweep)
 constexpr int kNpCandSlots = 1 << 20;
 constexpr int kSolverRowSlots = 27;  // float4 streams of a manifold's constraint rows (solver_common.cuh)
+constexpr int kSapKeep = 16;      // partners a proxy's counting pass leaves to the writing pass
 constexpr int kGsMaxBatch = 1024;  // batches per parity class (batched Gauss-Seidel)
 
 // Record of one Jacobi solve for the reverse sweep: the velocities every phase

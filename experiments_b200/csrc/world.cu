@@ -56,7 +56,7 @@ void free_all(b3::DevBuffers& d) {
     void* ptrs[] = {d.pos, d.quat, d.linVel, d.angVel, d.invMass, d.friction, d.restitution,
                     d.invInertia, d.collidable, d.worldId, d.cols, d.polys, d.verts, d.faces,
                     d.indices, d.edges, d.localAabb, d.polyInradius, d.childShapes, d.vpXY, d.vpZ, d.axisFaces, d.polyInfo, d.subPairs, d.subCount, d.subOffset, d.aabbMin, d.aabbMax, d.smallSlot,
-                    d.largeStart, d.largeList, d.sapSmall, d.sapLarge, d.sapSorted, d.sapCount, d.sapOffset, d.keys, d.vals, d.keysAlt, d.valsAlt, d.cellTable, d.sortedAabb,
+                    d.largeStart, d.largeList, d.sapSmall, d.sapLarge, d.sapSorted, d.sapCount, d.sapOffset, d.sapKept, d.keys, d.vals, d.keysAlt, d.valsAlt, d.cellTable, d.sortedAabb,
                     d.pairs, d.contacts, d.manifoldFlag, d.pairSep, d.npFast, d.npSlow, d.npDefer, d.npDefer2, d.npDefer3, d.npCand, d.manifoldScan,
                     d.manifoldPair,
                     d.incKeys, d.incVals, d.incKeysAlt, d.incValsAlt,
@@ -649,6 +649,7 @@ static int ensure_capacity(b3World w) {
             B3_TRY(dalloc(d.sapSorted, 2 * (size_t)nb));
             B3_TRY(dalloc(d.sapCount, (size_t)nb + 1));
             B3_TRY(dalloc(d.sapOffset, (size_t)nb + 1));
+            B3_TRY(dalloc(d.sapKept, (size_t)nb * b3::kSapKeep));
         }
         B3_TRY(dalloc(d.keys, nb));
         B3_TRY(dalloc(d.vals, nb));
