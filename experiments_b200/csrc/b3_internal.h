@@ -144,15 +144,18 @@ struct GridBarrier {
     b3Counters* counters;
     int spinLimit;
     int before;  // thread 0: *err at the kernel's start
+    unsigned blocks;  // that take part, block 0 on
 
-    __device__ __forceinline__ GridBarrier(uint32_t* w, int32_t* e, b3Counters* c, int limit)
-        : word(reinterpret_cast<unsigned long long*>(w)), target(0), err(e), counters(c), spinLimit(limit), before(0) {
+    __device__ __forceinline__ GridBarrier(uint32_t* w, int32_t* e, b3Counters* c, int limit,
+                                           unsigned taking = gridDim.x)
+        : word(reinterpret_cast<unsigned long long*>(w)), target(0), err(e), counters(c), spinLimit(limit), before(0),
+          blocks(taking) {
         if (threadIdx.x == 0) before = *(volatile int32_t*)e;
     }
     __device__ __forceinline__ bool wait() {
         constexpr unsigned long long kAbort = 1ull << 63;
         int ok = 1;
-        target += gridDim.x;
+        target += blocks;
         __syncthreads();
         if (threadIdx.x == 0) {
             asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(1ull) : "memory");
@@ -172,6 +175,26 @@ struct GridBarrier {
         return __syncthreads_and(ok) != 0;
     }
 };
+
+// 16 bytes read or written as one: a reader sees a record whole, of one version
+// or another, so a version number in it says that the rest is of that version.
+__device__ __forceinline__ float4 ld_whole(const float4* p) {
+    unsigned long long lo, hi;
+    asm volatile(
+        "{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+        : "=l"(lo), "=l"(hi)
+        : "l"(p)
+        : "memory");
+    return make_float4(__uint_as_float((uint32_t)lo), __uint_as_float((uint32_t)(lo >> 32)),
+                       __uint_as_float((uint32_t)hi), __uint_as_float((uint32_t)(hi >> 32)));
+}
+__device__ __forceinline__ void st_whole(float4* p, float4 v) {
+    const unsigned long long lo = __float_as_uint(v.x) | (unsigned long long)__float_as_uint(v.y) << 32;
+    const unsigned long long hi = __float_as_uint(v.z) | (unsigned long long)__float_as_uint(v.w) << 32;
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+                 "l"(lo), "l"(hi)
+                 : "memory");
+}
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;

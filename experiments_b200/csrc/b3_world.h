@@ -250,6 +250,7 @@ struct b3World_t {
     int solverMode = 0;        // Jacobi: 0 = grid barriers, 1 = one block per world (batched);
                                // batched Gauss-Seidel: resident blocks, 0 = 8 and 2 per SM, 1 = half of them
     int solverGather = 0;      // Jacobi body averages: 0 = gathered by every manifold, 1 = a pass over the bodies
+                               // where the rows do not fit the shared memories
     int pairSearchMode = 0;    // grid pair search: 0 = thread per body, 1 = warp per body
     int clipGroups = 1;        // clip and float-float stages: 0 = a warp per pair, 1 = 8-lane groups
                                // (a warp per pair for what does not fit)
@@ -265,6 +266,11 @@ struct b3World_t {
     int waitSpinLimit = b3::kDefaultSpinLimit;
     int waitHoldMicros = 0;
 
+    // manifolds per body that launches are sized for: about three where hulls
+    // touch, one between spheres and planes alone
+    long long expectedManifolds() const {
+        return (smallPairs || largePairs ? 3LL : 1LL) * (long long)bodies.size();
+    }
     void defaultShapes();      // launch shapes by the number of bodies, until they are tuned
     b3::BodiesDev bodiesDev() const;
     b3::ShapesDev shapesDev() const;

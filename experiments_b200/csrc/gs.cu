@@ -425,25 +425,6 @@ struct SolveView {
     b3Counters* counters;
 };
 
-// 16 bytes read or written as one: a velocity and its version.
-__device__ __forceinline__ float4 ld_whole(const float4* p) {
-    unsigned long long lo, hi;
-    asm volatile(
-        "{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
-        : "=l"(lo), "=l"(hi)
-        : "l"(p)
-        : "memory");
-    return make_float4(__uint_as_float((uint32_t)lo), __uint_as_float((uint32_t)(lo >> 32)),
-                       __uint_as_float((uint32_t)hi), __uint_as_float((uint32_t)(hi >> 32)));
-}
-__device__ __forceinline__ void st_whole(float4* p, float4 v) {
-    const unsigned long long lo = __float_as_uint(v.x) | (unsigned long long)__float_as_uint(v.y) << 32;
-    const unsigned long long hi = __float_as_uint(v.z) | (unsigned long long)__float_as_uint(v.w) << 32;
-    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
-                 "l"(lo), "l"(hi)
-                 : "memory");
-}
-
 // One constraint with the data that does not change during the solve: its
 // Constraint4 record, its turn, and its bodies' inverse masses and world
 // inverse inertias (positions are read with the rest). All of it is fetched
@@ -569,12 +550,12 @@ __global__ void __launch_bounds__(128) k_gs_solve(SolveView V) {
                 if (!done) {
                     float4 lA = zero, aA = zero, lB = zero, aB = zero;
                     if (dA) {
-                        lA = ld_whole(&V.vel[2 * P.A]);
-                        aA = ld_whole(&V.vel[2 * P.A + 1]);
+                        lA = b3dev::ld_whole(&V.vel[2 * P.A]);
+                        aA = b3dev::ld_whole(&V.vel[2 * P.A + 1]);
                     }
                     if (dB) {
-                        lB = ld_whole(&V.vel[2 * P.B]);
-                        aB = ld_whole(&V.vel[2 * P.B + 1]);
+                        lB = b3dev::ld_whole(&V.vel[2 * P.B]);
+                        aB = b3dev::ld_whole(&V.vel[2 * P.B + 1]);
                     }
                     const bool ready = (!dA || (__float_as_int(lA.w) == turnA && __float_as_int(aA.w) == turnA)) &&
                                        (!dB || (__float_as_int(lB.w) == turnB && __float_as_int(aB.w) == turnB));
@@ -582,12 +563,12 @@ __global__ void __launch_bounds__(128) k_gs_solve(SolveView V) {
                         float3 vA = f3(lA), wA = f3(aA), vB = f3(lB), wB = f3(aB);
                         solve_one(V, P, q, phase, vA, wA, vB, wB);
                         if (dA) {
-                            st_whole(&V.vel[2 * P.A], f4(vA, __int_as_float(turnA + 1)));
-                            st_whole(&V.vel[2 * P.A + 1], f4(wA, __int_as_float(turnA + 1)));
+                            b3dev::st_whole(&V.vel[2 * P.A], f4(vA, __int_as_float(turnA + 1)));
+                            b3dev::st_whole(&V.vel[2 * P.A + 1], f4(wA, __int_as_float(turnA + 1)));
                         }
                         if (dB) {
-                            st_whole(&V.vel[2 * P.B], f4(vB, __int_as_float(turnB + 1)));
-                            st_whole(&V.vel[2 * P.B + 1], f4(wB, __int_as_float(turnB + 1)));
+                            b3dev::st_whole(&V.vel[2 * P.B], f4(vB, __int_as_float(turnB + 1)));
+                            b3dev::st_whole(&V.vel[2 * P.B + 1], f4(wB, __int_as_float(turnB + 1)));
                         }
                         // the last turn of a body leaves its velocity
                         if (!dA || turnA + 1 == 2 * kIterations * P.turn.y) {

@@ -362,8 +362,8 @@ __device__ __forceinline__ float4* copy_buffer(const SolverView& V, int buf) {
 }
 
 // test of the give-up path: block 0 arrives late (bounded sleep)
-__device__ __forceinline__ void hold_back(const SolverView& V) {
-    if (V.holdMicros > 0 && blockIdx.x == 0 && threadIdx.x == 0)
+__device__ __forceinline__ void hold_back(const SolverView& V, unsigned block) {
+    if (V.holdMicros > 0 && block == 0 && threadIdx.x == 0)
         for (int i = 0; i < V.holdMicros; ++i) __nanosleep(1000);
 }
 
@@ -372,44 +372,284 @@ __device__ __forceinline__ void hold_back(const SolverView& V) {
 // phase from the double-buffered copies, so phases are separated by one
 // bounded grid barrier each.
 //
-// k_jacobi, small scenes: what counts is the chain of a phase (barrier, copies,
-// rows, copies out). Each thread keeps the streams of its first `resident`
-// manifolds in shared memory for all phases, so between two barriers one round
-// of L2 reads is left, the copies of its bodies, which lie side by side.
-// 4,096 stacked cubes (10,550 manifolds): 219 -> 109 us for 20 phases; before,
-// rows were streamed in every phase and each copy was found through its id.
-template <bool TAPE>
-__global__ void __launch_bounds__(256, 1)
-k_jacobi(SolverView V, int iterations, int resident, uint32_t* bar, int32_t* err, b3Counters* counters,
-         b3::JacobiTape T) {
-    extern __shared__ float4 kept[];  // [resident][kPhaseSlots][blockDim]
-    GridBarrier barrier(bar, err, counters, V.spinLimit);
-    const int M = *V.numManifolds;
-    const int phases = 2 * iterations;
-    const int m0 = blockIdx.x * blockDim.x + threadIdx.x;
-    const int stride = gridDim.x * blockDim.x;
-    const int tb = (int)blockDim.x;
-    for (int k = 0; k < resident; ++k) {
-        const int m = m0 + k * stride;
-        if (m < M) {
-            float4* at = kept + (size_t)k * kPhaseSlots * tb + threadIdx.x;
+// k_jacobi, small scenes: what counts is the chain of a phase (barrier, copies
+// in, rows, copies out). Two lanes share a manifold, one per body: each gathers
+// its body's copies, forms its half of a row's J dv and takes the other's by a
+// shuffle, so that a row is half the instructions in one warp. The first
+// `resident` manifolds of a pair of lanes stay in shared memory for all phases,
+// their rows with the angular parts formed. Of a phase's 3.5 us on 1,000 cubes a
+// third each is the barrier, the way of the copies through L2 and the rows. 20
+// phases, a lane per manifold -> two: 4,096 cubes (10,550 manifolds) 106 -> 90 us,
+// 20,011 spheres (12,361) 113 -> 74, 33,000 falling bodies (9,400) 123 -> 71; with
+// every row streamed in every phase 219, 162 and 211.
+//
+// Lane slots (float4 per lane): angular part and 1/diag of normal row j at j, of
+// friction row r at 4 + r, then (inverse mass, inverse inertia) and (s, e, p,
+// rows | dynamic << 16). Pair slots (float4 per manifold): (n, mu), rhs of the
+// normal rows, (axis, rhs) of each friction row, impulses.
+constexpr int kLaneBody = 12, kLaneHead = 13, kLaneSlots = 14;
+constexpr int kPairNorm = 0, kPairRhs = 1, kPairFric = 2, kPairLam = 10, kPairSlots = 13;
+
+struct LaneSide {
+    uint32_t s, e, p;
+    int nRows;
+    bool dyn;
+    float im;
+    float3 ii;
+};
+
+// One manifold's rows as a lane sees them: in shared memory, or formed from the
+// streams (manifolds beyond the resident ones).
+struct KeptRows {
+    static constexpr bool kKept = true;
+    float4 *lane, *pair;  // strides tb and tb / 2
+    int tb;
+    __device__ __forceinline__ float4& at(int k) const { return pair[k * (tb / 2)]; }
+    __device__ __forceinline__ float4 normal(int j, float3, bool) const { return lane[j * tb]; }
+    __device__ __forceinline__ void point(int, bool, float4&) const {}
+    __device__ __forceinline__ float4 friction(int r, const float4&, float3, bool, const float4*) const {
+        return lane[(4 + r) * tb];
+    }
+    __device__ __forceinline__ LaneSide side(bool) const {
+        const float4 b = lane[kLaneBody * tb], h = lane[kLaneHead * tb];
+        const int f = __float_as_int(h.w);
+        return LaneSide{__float_as_uint(h.x), __float_as_uint(h.y), __float_as_uint(h.z), f & 0xffff, (f >> 16) != 0,
+                        b.x, make_float3(b.y, b.z, b.w)};
+    }
+    __device__ __forceinline__ float4 jac(int) const { return make_float4(0.f, 0.f, 0.f, 0.f); }
+    __device__ __forceinline__ float4 norm() const { return at(kPairNorm); }
+    __device__ __forceinline__ float4 rhs() const { return at(kPairRhs); }
+    __device__ __forceinline__ float4 axis(int r) const { return at(kPairFric + r); }
+    __device__ __forceinline__ float4& lam(int k) const { return at(kPairLam + k); }
+};
+struct StreamRows {
+    static constexpr bool kKept = false;
+    SolverView V;
+    int m;
+    __device__ __forceinline__ float4 normal(int j, float3 n, bool isB) const {
+        const float4 a = R(V, kPoint0 + 4 * j, m), b = R(V, kPoint0 + 4 * j + 1, m);
+        return f4(isB ? arm_neg(f3(b), n) : arm(f3(a), n), b.w);
+    }
+    __device__ __forceinline__ void point(int j, bool isB, float4& r) const { r = R(V, kPoint0 + 4 * j + (isB ? 1 : 0), m); }
+    __device__ __forceinline__ float4 friction(int r, const float4& arm0, float3 d, bool isB, const float4* jac) const {
+        const float4 q = jac[r >> 2];
+        const float j = (r & 3) == 0 ? q.x : (r & 3) == 1 ? q.y : (r & 3) == 2 ? q.z : q.w;
+        return f4(isB ? arm_rev(f3(arm0), d) : arm(f3(arm0), d), j);
+    }
+    __device__ __forceinline__ LaneSide side(bool isB) const {
+        const Heads H = load_heads(GlobalRows{V.rows + m, (size_t)V.cap});
+        const float4 nn = R(V, kNorm, m), ia = R(V, kInA, m), ib = R(V, kInB, m);
+        return isB ? LaneSide{H.sB, H.eB, H.pB, H.nRows, (H.dyn & 2) != 0, ia.w, f3(ib)}
+                   : LaneSide{H.sA, H.eA, H.pA, H.nRows, (H.dyn & 1) != 0, nn.w, f3(ia)};
+    }
+    __device__ __forceinline__ float4 jac(int k) const { return R(V, kFJac + k, m); }
+    __device__ __forceinline__ float4 norm() const {
+        const float4 n = R(V, kNorm, m);
+        return make_float4(n.x, n.y, n.z, R(V, kHead1, m).w);
+    }
+    __device__ __forceinline__ float4 rhs() const {
+        return make_float4(R(V, kPoint0, m).w, R(V, kPoint0 + 4, m).w, R(V, kPoint0 + 8, m).w, R(V, kPoint0 + 12, m).w);
+    }
+    __device__ __forceinline__ float4 axis(int r) const { return R(V, kPoint0 + 4 * (r >> 1) + 2 + (r & 1), m); }
+    __device__ __forceinline__ float4& lam(int k) const { return R(V, k == 0 ? kLamN : kLamF + k - 1, m); }
+};
+
+// A row by its two lanes: solve_row with each side's products in its own lane.
+__device__ __forceinline__ void half_row(float3 n, const float4& t, float rhs, float& lam, float lo, float hi, bool on,
+                                         bool isB, const LaneSide& L, float3& v, float3& w) {
+    const float x = dot_fma(n, v), y = dot_fma(f3(t), w);
+    const float own = __fadd_rn(y, isB ? -x : x);
+    const float other = __shfl_xor_sync(0xffffffffu, own, 1);
+    float delta = __fmaf_rn(-(isB ? other : own), t.w, rhs);
+    delta = __fmaf_rn(-(isB ? own : other), t.w, delta);
+    const float sum = lam + delta;
+    const float na = sum < lo ? lo : sum > hi ? hi : sum;
+    delta = sum < lo || sum > hi ? na - lam : delta;
+    delta = on ? delta : 0.f;  // a row that is not solved changes nothing
+    lam = on ? na : lam;
+    // A: v + n (im delta); B: v + (-n im) delta
+    v = fma3(n * (isB ? -L.im : 1.f), (isB ? 1.f : L.im) * delta, v);
+    w = fma3(mulv(L.ii, f3(t)), delta, w);
+}
+
+// The lane's body's average over its copies, the first K in flight at once.
+template <int K>
+__device__ __forceinline__ void gather_side(const float4* copies, const LaneSide& L, float3& v, float3& w) {
+    float3 sl = make_float3(0.f, 0.f, 0.f), sa = sl;
+    for (uint32_t i0 = L.s; i0 < L.e; i0 += K) {
+        float4 l[K], a[K];
 #pragma unroll
-            for (int s = 0; s < kPhaseSlots; ++s) at[s * tb] = R(V, s, m);
+        for (int u = 0; u < K; ++u) {
+            const float4* r = copies + 2 * (size_t)min(i0 + u, L.e - 1u);
+            l[u] = __ldcg(r);
+            a[u] = __ldcg(r + 1);
+        }
+#pragma unroll
+        for (int u = 0; u < K; ++u)
+            if (i0 + u < L.e) {
+                sl += f3(l[u]);
+                sa += f3(a[u]);
+            }
+    }
+    if (L.dyn) {
+        const float f = 1.f / (float)(L.e - L.s);
+        v = scaled(sl, f);
+        w = scaled(sa, f);
+    }
+}
+
+// A phase of one manifold by two lanes (a warp's lanes go through it together;
+// on: the manifold exists).
+template <bool TAPE, class Rows>
+__device__ __forceinline__ void pair_phase(const Rows& S, bool isB, bool on, bool friction, bool first, const float4* in,
+                                           float4* out, int m, size_t cap, const b3::JacobiTape& T, int phase) {
+    LaneSide L = Rows::kKept || on ? S.side(isB) : LaneSide{0u, 0u, 0u, 0, false, 0.f, make_float3(0.f, 0.f, 0.f)};
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float3 v = make_float3(0.f, 0.f, 0.f), w = v;
+    if (!first) gather_side<4>(in, L, v, w);
+    if (TAPE && on) {
+        float4* tape = T.in + ((size_t)phase * 4 + (isB ? 2 : 0)) * cap + m;
+        tape[0] = f4(v);
+        tape[cap] = f4(w);
+    }
+    const int most = __reduce_max_sync(0xffffffffu, L.nRows);
+    const float4 l4 = Rows::kKept || on ? S.lam(0) : zero;
+    float ln[4] = {l4.x, l4.y, l4.z, l4.w};
+    if (!friction) {
+        const float4 n4 = Rows::kKept || on ? S.norm() : zero, r4 = Rows::kKept || on ? S.rhs() : zero;
+        const float rhs[4] = {r4.x, r4.y, r4.z, r4.w};
+        const float3 n = f3(n4);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (j < most) {
+                const bool row = j < L.nRows;
+                half_row(n, Rows::kKept || row ? S.normal(j, n, isB) : zero, rhs[j], ln[j], 0.f, 1e10f, row, isB, L, v, w);
+            }
+        const float4 r = make_float4(ln[0], ln[1], ln[2], ln[3]);
+        if ((Rows::kKept || on) && !isB) {
+            S.lam(0) = r;
+            if (TAPE && on) T.lamN[(size_t)(phase >> 1) * cap + m] = r;
+        }
+    } else {
+        const float mu = Rows::kKept || on ? S.norm().w : 0.f;
+        float4 f0 = Rows::kKept || on ? S.lam(1) : zero, f1 = Rows::kKept || on ? S.lam(2) : zero;
+        float lam[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+        float4 jac[2] = {zero, zero}, arm0 = zero;
+        if (!Rows::kKept && on) {
+            jac[0] = S.jac(0);
+            jac[1] = S.jac(1);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (j < most) {
+                const bool row = j < L.nRows, solve = row && ln[j] > 0.f;
+                const float lim = mu * ln[j];
+                if (row) S.point(j, isB, arm0);
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const int r = 2 * j + q;
+                    const float4 d = Rows::kKept || row ? S.axis(r) : zero;
+                    half_row(f3(d), Rows::kKept || row ? S.friction(r, arm0, f3(d), isB, jac) : zero, d.w, lam[r], -lim, lim, solve, isB,
+                             L, v, w);
+                }
+            }
+        f0 = make_float4(lam[0], lam[1], lam[2], lam[3]);
+        f1 = make_float4(lam[4], lam[5], lam[6], lam[7]);
+        if ((Rows::kKept || on) && !isB) {
+            S.lam(1) = f0;
+            S.lam(2) = f1;
+            if (TAPE && on) {
+                float4* tf = T.lamF + (size_t)(phase & ~1) * cap + m;
+                tf[0] = f0;
+                tf[cap] = f1;
+            }
         }
     }
+    if (L.dyn) {
+        __stcg(&out[2 * (size_t)L.p], f4(v));
+        __stcg(&out[2 * (size_t)L.p + 1], f4(w));
+    }
+    __syncwarp();  // the impulses one lane writes, both read
+}
+
+// Blocks without a manifold leave: the barriers are among the others.
+template <bool TAPE>
+__global__ void __launch_bounds__(256, 1)
+k_jacobi(SolverView V, int iterations, int resident, int most, uint32_t* bar, int32_t* err, b3Counters* counters,
+         b3::JacobiTape T) {
+    extern __shared__ float4 kept[];  // [resident]([kLaneSlots][blockDim], [kPairSlots][blockDim / 2])
+    const int M = *V.numManifolds;
+    if (M > most) return;  // the pass over the bodies takes them
+    const int phases = 2 * iterations;
+    const int tb = (int)blockDim.x, tid = (int)threadIdx.x;
+    const unsigned busy = min(gridDim.x, (unsigned)(M + tb / 2 - 1) / (unsigned)(tb / 2));
+    // from the last block of the grid on: the first ones of a cooperative grid come
+    // several to an SM
+    const unsigned block = gridDim.x - 1 - blockIdx.x;
+    if (block >= busy) return;
+    GridBarrier barrier(bar, err, counters, V.spinLimit, busy);
+    const bool isB = tid & 1;
+    const int m0 = (block * tb + tid) >> 1, warp0 = (block * tb + (tid & ~31)) >> 1;
+    const int stride = (gridDim.x * tb) >> 1;
+    const int each = kLaneSlots * tb + kPairSlots * (tb / 2);
+    auto rows = [&](int k) {
+        float4* at = kept + (size_t)k * each;
+        return KeptRows{at + tid, at + kLaneSlots * tb + (tid >> 1), tb};
+    };
+    for (int k = 0; k < resident; ++k) {
+        const int m = m0 + k * stride;
+        const KeptRows K = rows(k);
+        if (m >= M) {  // no manifold: nothing to solve, no copies
+            for (int q = 0; q < kLaneSlots; ++q) K.lane[q * tb] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int q = 0; q < kPairSlots && !isB; ++q) K.at(q) = make_float4(0.f, 0.f, 0.f, 0.f);
+            continue;
+        }
+        const StreamRows S{V, m};
+        const LaneSide L = S.side(isB);
+        const float4 n = S.norm();
+        const float4 jac[2] = {S.jac(0), S.jac(1)};
+        K.lane[kLaneBody * tb] = make_float4(L.im, L.ii.x, L.ii.y, L.ii.z);
+        K.lane[kLaneHead * tb] = make_float4(__uint_as_float(L.s), __uint_as_float(L.e), __uint_as_float(L.p),
+                                             __int_as_float(L.nRows | (L.dyn ? 1 << 16 : 0)));
+        if (!isB) {
+            K.at(kPairNorm) = n;
+            K.at(kPairRhs) = S.rhs();
+#pragma unroll
+            for (int q = 0; q < 3; ++q) K.lam(q) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        // rows past the last one stay zero: a warp goes through as many as any of
+        // its manifolds has
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = L.nRows; j < 4; ++j) {
+            K.lane[j * tb] = K.lane[(4 + 2 * j) * tb] = K.lane[(5 + 2 * j) * tb] = zero;
+            if (!isB) K.at(kPairFric + 2 * j) = K.at(kPairFric + 2 * j + 1) = zero;
+        }
+        for (int j = 0; j < L.nRows; ++j) {
+            float4 arm0;
+            S.point(j, isB, arm0);
+            K.lane[j * tb] = S.normal(j, f3(n), isB);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const float4 d = S.axis(2 * j + q);
+                K.lane[(4 + 2 * j + q) * tb] = S.friction(2 * j + q, arm0, f3(d), isB, jac);
+                if (!isB) K.at(kPairFric + 2 * j + q) = d;
+            }
+        }
+    }
+    __syncwarp();
     for (int p = 0; p < phases; ++p) {
-        if (p == 1) hold_back(V);
+        if (p == 1) hold_back(V, block);
         if (p > 0 && !barrier.wait()) return;
         const bool friction = (p & 1) != 0, first = p == 0;
         const float4* in = copy_buffer(V, (p - 1) & 1);
         float4* out = copy_buffer(V, p & 1);
-        int m = m0;
-        for (int k = 0; k < resident && m < M; ++k, m += stride)
-            solve_manifold<TAPE, false>(SharedRows{kept + (size_t)k * kPhaseSlots * tb + threadIdx.x, tb},
-                                                 friction, first, in, out, m, V.cap, T, p);
-        for (; m < M; m += stride)
-            solve_manifold<TAPE, false>(GlobalRows{V.rows + m, (size_t)V.cap}, friction, first, in, out, m,
-                                                 V.cap, T, p);
+        int m = m0, k = 0;
+        for (int base = warp0; base < M; base += stride, m += stride, ++k) {
+            if (k < resident)
+                pair_phase<TAPE>(rows(k), isB, m < M, friction, first, in, out, m, V.cap, T, p);
+            else
+                pair_phase<TAPE>(StreamRows{V, min(m, M - 1)}, isB, m < M, friction, first, in, out, m, V.cap, T, p);
+        }
     }
 }
 
@@ -422,14 +662,16 @@ k_jacobi(SolverView V, int iterations, int resident, uint32_t* bar, int32_t* err
 // take 2.5 ms at 6.65 TB/s; 131,072 mixed bodies (395 K): 1.26 -> 0.90 ms.
 template <bool TAPE>
 __global__ void __launch_bounds__(256, 2)
-k_jacobi_pass(SolverView V, int iterations, uint32_t* bar, int32_t* err, b3Counters* counters, b3::JacobiTape T) {
-    GridBarrier barrier(bar, err, counters, V.spinLimit);
+k_jacobi_pass(SolverView V, int iterations, int above, uint32_t* bar, int32_t* err, b3Counters* counters,
+              b3::JacobiTape T) {
     const int M = *V.numManifolds;
+    if (M <= above) return;  // k_jacobi took them
+    GridBarrier barrier(bar, err, counters, V.spinLimit);
     const int phases = 2 * iterations;
     const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
     const int stride = gridDim.x * blockDim.x;
     for (int p = 0; p < phases; ++p) {
-        if (p == 1) hold_back(V);
+        if (p == 1) hold_back(V, blockIdx.x);
         const float4* in = copy_buffer(V, (p - 1) & 1);
         if (p > 0) {
             if (!barrier.wait()) return;
@@ -618,11 +860,12 @@ int launch_solver_taped(b3World_t* w, cudaStream_t st, const JacobiTape* tape) {
     SP.contactProcessing = w->sim.contactProcessing;
     SP.slopOffset = w->sim.slopOffset;
     const int g = w->ctx->numSMs * 8;
+    const bool worlds = w->solverMode == 1 && w->cfg.numWorlds > 1, pass = w->solverGather == 1;
     k_setup_rows<<<g, 128, 0, st>>>(w->bodiesDev(), V, w->d.manifoldPair, w->d.contacts, SP,
                                     (unsigned long long*)(w->d.scalars + S_BAR_COUNT));
     B3_CHECK_LAUNCH();
     if (w->timing && w->setupEv) B3_CUDA(cudaEventRecord(w->setupEv, st));
-    if (w->solverMode == 1 && w->cfg.numWorlds > 1) {
+    if (worlds) {
         // one block per world at a time, block barriers between phases
         const int nw = w->cfg.numWorlds;
         B3_CUDA(cudaMemsetAsync(w->d.worldMStart, 0x7f, sizeof(int) * nw, st));  // 0x7f7f7f7f: above any index
@@ -645,52 +888,60 @@ int launch_solver_taped(b3World_t* w, cudaStream_t st, const JacobiTape* tape) {
         B3_CUDA(cudaLaunchKernel(kw, dim3(grid), dim3(threads), args, 0, st));
         return B3_OK;
     }
-    // persistent cooperative Jacobi
-    const int threads = w->solverThreads;
-    // size the persistent grid to the expected manifold count (about 3 per
-    // body): fewer blocks make each grid barrier cheaper on small scenes
-    const long long est = std::min<long long>((long long)w->cfg.maxPairs, 3LL * (long long)w->bodies.size());
-    const int want = (int)std::max<long long>(1, (est + threads - 1) / threads);
-    const bool pass = w->solverGather == 1;
-    const void* kern = pass ? (tape ? (const void*)k_jacobi_pass<true> : (const void*)k_jacobi_pass<false>)
-                            : (tape ? (const void*)k_jacobi<true> : (const void*)k_jacobi<false>);
-    int occ = 1, resident = 0;
-    size_t smem = 0;
-    if (!pass) {
-        // shared memory for as many of a thread's manifolds as the scene is
-        // expected to have, up to one block's share of an SM
-        const size_t one = (size_t)kPhaseSlots * threads * sizeof(float4);
-        const int blocks = std::min(w->ctx->numSMs * w->solverOccCap, want);
-        const int perSm = (blocks + w->ctx->numSMs - 1) / w->ctx->numSMs;
-        const int need = (int)((est + (long long)blocks * threads - 1) / ((long long)blocks * threads));
-        resident = std::min(need, (int)((size_t)w->ctx->maxSmemOptin / perSm / one));
-        smem = one * resident;
-        if (smem > 48 * 1024)
-            B3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    }
-    B3_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem));
-    occ = occ < 1 ? 1 : occ;
-    occ = occ > w->solverOccCap ? w->solverOccCap : occ;
-    const int grid = std::min(w->ctx->numSMs * occ, want);
+    // persistent cooperative Jacobi: k_jacobi where the rows fit the shared
+    // memories, the pass over the bodies beyond; where the body count leaves it
+    // open both are launched and the one that the manifolds call for runs
     int iters = w->sim.iterations;
     uint32_t* bar = (uint32_t*)(w->d.scalars + S_BAR_COUNT);
     int32_t* err = w->d.scalars + S_ERR;
     b3Counters* ctr = w->d.counters;
     JacobiTape T = tape ? *tape : JacobiTape{};
-    void* argsPass[] = {&V, &iters, &bar, &err, &ctr, &T};
-    void* argsGather[] = {&V, &iters, &resident, &bar, &err, &ctr, &T};
-    void** args = pass ? argsPass : argsGather;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    B3_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
+    auto launch = [&](const void* kern, int threads, int occCap, int want, size_t smem, void** args) -> int {
+        if (smem > 48 * 1024)
+            B3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        int occ = 1;
+        B3_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem));
+        occ = std::max(1, std::min(occ, occCap));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(std::min(w->ctx->numSMs * occ, want));
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        B3_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
+        return B3_OK;
+    };
+    const long long est = std::min<long long>((long long)w->cfg.maxPairs, w->expectedManifolds());
+    const bool open = pass && est <= 512 * 1024;
+    int above = -1;
+    if (!pass || open) {
+        // shared memory for as many of a thread's manifolds as the scene is
+        // expected to have, up to one block's share of an SM
+        const int threads = open ? 128 : w->solverThreads, share = threads / 2;
+        const int occCap = open ? 4 : w->solverOccCap;
+        const int want = (int)std::max<long long>(1, (est + share - 1) / share);
+        const size_t one = (size_t)(kLaneSlots * threads + kPairSlots * share) * sizeof(float4);
+        const int blocks = std::min(w->ctx->numSMs * occCap, want);
+        const int perSm = (blocks + w->ctx->numSMs - 1) / w->ctx->numSMs;
+        const int need = open ? 1 : (int)((est + (long long)blocks * share - 1) / ((long long)blocks * share));
+        int resident = std::min(need, (int)(((size_t)w->ctx->maxSmemOptin - 1024 * (perSm - 1)) / perSm / one));
+        int most = 0x7fffffff;
+        if (open) above = most = blocks * share * resident;
+        void* args[] = {&V, &iters, &resident, &most, &bar, &err, &ctr, &T};
+        B3_TRY(launch(tape ? (const void*)k_jacobi<true> : (const void*)k_jacobi<false>, threads, occCap, want,
+                      one * resident, args));
+    }
+    if (pass) {
+        const int threads = w->solverThreads;
+        const int want = (int)std::max<long long>(1, (est + threads - 1) / threads);
+        void* args[] = {&V, &iters, &above, &bar, &err, &ctr, &T};
+        B3_TRY(launch(tape ? (const void*)k_jacobi_pass<true> : (const void*)k_jacobi_pass<false>, threads,
+                      w->solverOccCap, want, 0, args));
+    }
     return B3_OK;
 }
 

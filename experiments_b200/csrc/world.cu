@@ -139,17 +139,19 @@ b3::ShapesDev b3World_t::shapesDev() const {
 }
 
 // Jacobi launch shapes of a world that was not tuned, by the manifolds it is
-// expected to have (3 per body). Iterations of the solve, microseconds, mixed
-// heaps, gathered / pass over the bodies: 8,000 bodies 127 / 152, 16,000
-// 168 / 197, 24,000 246 / 217, 33,000 303 / 289, 65,000 592 / 432, 131,000
-// 1,198 / 904; the first form wins while most rows fit the shared memories.
-// CTAs of 64 threads (127 us at 8,000 bodies, 137 with 128) until there are
-// two per SM of 128.
+// expected to have. Iterations of the solve, microseconds, rows in shared memory /
+// pass over the bodies: cubes with 10,550 manifolds 90 / 131, 21,057 111 / 154,
+// 42,971 (a fifth of the rows streamed) 230 / 194, mixed heaps with 395,028 1,723 /
+// 905: the shared memories hold 37,888 manifolds with four CTAs of 128 an SM. A
+// world that may have more launches both, and the device takes the one for the
+// manifolds it has (3 us for the other: falling bodies have a tenth of a heap's).
+// CTAs of 64 up to 2,500 bodies: 1,000 cubes 70 us, 74 with 128; four an SM where
+// two would take two rounds: 26,000 manifolds 111 / 146.
 void b3World_t::defaultShapes() {
-    const long long est = 3LL * (long long)bodies.size();
-    solverGather = est > 64 * 1024 ? 1 : 0;
-    solverThreads = est <= 32 * 1024 ? 64 : 128;
-    solverOccCap = solverGather ? (est <= 128 * 1024 ? 2 : 4) : 8;
+    const long long est = expectedManifolds();
+    solverGather = est > 36 * 1024 ? 1 : 0;
+    solverThreads = est <= 8 * 1024 ? 64 : 128;
+    solverOccCap = solverGather ? (est <= 128 * 1024 ? 2 : 4) : est <= 20 * 1024 ? 2 : 4;
 }
 
 extern "C" void b3_world_config_default(b3WorldConfig* c) {

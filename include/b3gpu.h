@@ -612,8 +612,9 @@ int b3_autotune(b3World w, int trialSteps, void* stream);
  * mode (0 = persistent grid with grid barriers, 1 = one block per world
  * with block barriers; batched worlds only, bit-identical results), Jacobi
  * body averages (0 = gathered by every manifold, rows kept in shared memory;
- * 1 = formed by a pass over the bodies between two grid barriers, for large
- * scenes; bit-identical results), grid pair search form (0 = one thread per body
+ * 1 = formed by a pass over the bodies between two grid barriers wherever the
+ * rows do not fit the shared memories, which the device decides in worlds of
+ * up to 170,000 bodies; bit-identical results), grid pair search form (0 = one thread per body
  * over its 27 cells, 1 = one warp per body, a lane per cell; the same pair
  * list and overflow counts bit for bit), narrowphase lane groups (0 = one
  * warp per pair in the FP32 clip and the float-float stages, 1 = eight-lane

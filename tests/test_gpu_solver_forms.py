@@ -51,7 +51,7 @@ def _run(ctx, sc, threads, cap, mode, form, steps=4):
 
 # one manifold; under and over one CTA; a body with hundreds of copies; more
 # manifolds than 64-thread CTAs keep in shared memory, the rest streamed
-@pytest.mark.parametrize("n,plate", [(1, False), (20, False), (300, True), (24000, False)])
+@pytest.mark.parametrize("n,plate", [(1, False), (20, False), (300, True), (9000, False), (24000, False), (24000, True)])
 def test_forms_give_the_same_bits(ctx, n, plate):
     sc = _heap(n, plate)
     ref, c = _run(ctx, sc, 256, 4, 0, 1)
