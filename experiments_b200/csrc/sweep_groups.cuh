@@ -12,15 +12,16 @@
 //     and orientation are the other's bit for bit (ShapesDev.axisFaces).
 // 406,661 pairs of cubes: 1.30 -> 0.46 ns a pair; the sweep of 1,048,576 cubes
 // (7.32 M pairs) 7.44 -> 2.21 ms, of 131,072 mixed bodies (a quarter of the
-// 1.60 M pairs boxes) 2.74 -> 2.14 ms.
+// 1.60 M pairs boxes) 2.74 -> 2.14 ms, before pairs that are apart were
+// left out.
 // All 32 lanes go through one control flow, with whole-warp masks throughout:
 // a vote or reduction with a group's own mask splits the warp, and the four
 // groups then run one after another.
 //
 // Pairs with more axes stay with the warp sweep, whose lanes they fill (eight
 // lanes measured: hull-hull 3.9 ns a pair against 1.7, icosphere-icosphere 14
-// against 7). k_np_bin sorts the pairs into the two queues; a scene of small
-// shapes only needs no sorting.
+// against 7). k_np_bin sorts the pairs into the two queues and leaves out
+// most of those that are apart.
 // Each axis is computed with the warp sweep's arithmetic, the candidates are
 // the same set, and the winner and its tests are the same. What a group cannot
 // hold (more than kGroupCand near-minimum axes) goes to the warp sweep, which
@@ -311,63 +312,93 @@ __device__ __forceinline__ bool sweep_small(const b3::ShapesDev& S, int pa, int 
     return nAx <= kClipGroup && a.w * b.w <= 2 * kClipGroup - nAx && a.w > 0 && b.w > 0;
 }
 
-// Sorts the items into the groups' queue and the warps', 2,048 to a round so
-// that the counters see one addition each per round; items the narrowphase
-// skips get their flag cleared here.
-constexpr int kBinItems = 8;
+// A pair is apart if the face of A that B's centre is farthest outside of, or the
+// face of B for A's centre, separates them by four times the bound on the FP32
+// depth's error: the sweep would then find that axis' depth below its own limit
+// (one such bound) and end there, so nothing but the work is different.
+__device__ __noinline__ bool pair_apart(const PairPre& pre, const b3::ShapesDev& S) {
+    SweepPair q;
+    sweep_pair(q, pre, S);
+    for (int side = 0; side < 2; ++side) {
+        const int pi = side ? q.pb : q.pa;
+        const Mat3& R = side ? q.RB : q.RA;
+        const float3 lc = f3(__ldg(&S.info[3 * pi])), ld = xmul_t(R, q.D);
+        const float3 x = side ? lc + ld : lc - ld;  // the other's centre in this one's frame
+        const b3ConvexPolyhedron& h = S.polys[pi];
+        const int f0 = h.faceOffset, nf = h.numFaces;
+        float best = -FLT_MAX;
+        float3 pn = make_float3(0.f, 0.f, 0.f);
+        for (int f = 0; f < nf; ++f) {
+            const float4 pl = __ldg((const float4*)&S.faces[f0 + f].plane[0]);
+            const float out = pl.x * x.x + pl.y * x.y + pl.z * x.z + pl.w;
+            if (out > best) {
+                best = out;
+                pn = f3(pl);
+            }
+        }
+        const float3 n = xmul(R, pn);
+        float mn0, mx0, mn1, mx1;
+        project_packed(S, q.pa, q.RA, n, mn0, mx0);
+        project_packed(S, q.pb, q.RB, n, mn1, mx1);
+        const float off = xdot(q.rel, n);
+        if (fminf(mx0 - (mn1 + off), (mx1 + off) - mn0) < -4.f * q.delta) return true;
+    }
+    return false;
+}
+
+// The queue of an item: 0 the groups', 1 the warps', -1 none (the narrowphase
+// skips it, or it is apart).
 template <bool kSub>
-__global__ void __launch_bounds__(256)
+__device__ __forceinline__ int bin_of(int slot, const int2* __restrict__ pairs, const int4* __restrict__ subs, int base,
+                                      const b3::BodiesDev& Bd, const b3::ShapesDev& S) {
+    PairPre q;
+    item_prefetch<kSub>(q, slot, pairs, subs, base, Bd, S);
+    if (q.shapeA < 0) return -1;
+    const int bin = sweep_small(S, q.shapeA, q.shapeB) ? 0 : 1;
+    return pair_apart(q, S) ? -1 : bin;
+}
+
+// Sorts the items into the groups' queue and the warps', up to 2,048 to a round so
+// that the counters see one addition each per round; items the narrowphase
+// skips, and pairs that are apart, get their flag cleared here. Three quarters of
+// the pairs in a settled heap are apart, and a thread finds most of them with two
+// faces in place of a warp's or a group's search. Bin and sweeps, the bin without
+// -> with the test: 4,096 piles (3.95 M pairs) 4.03 -> 2.07 ms, 131,072 mixed
+// bodies (1.60 M) 2.16 -> 1.67, 1,048,576 cubes (7.32 M, no bin before) 2.21 -> 1.54.
+constexpr int kBinThreads = 128, kBinItems = 16;
+template <bool kSub>
+__global__ void __launch_bounds__(kBinThreads, 6)
 k_np_bin(const int2* __restrict__ pairs, const int4* __restrict__ subs, const int32_t* __restrict__ numPairsDev,
          b3::BodiesDev Bd, b3::ShapesDev S, int32_t* __restrict__ scalars, uint32_t* __restrict__ manifoldFlag,
          int* __restrict__ smallQ, int* __restrict__ warpQ) {
     __shared__ int cnt[2], at[2];
+    __shared__ int list[kBinThreads * kBinItems];  // the groups' from the front, the warps' from the back
+    constexpr int kLast = kBinThreads * kBinItems - 1;
+    const int tid = (int)threadIdx.x;
     const int numItems = kSub ? scalars[b3::S_NUM_SUB] : *numPairsDev;
     const int base = kSub ? *numPairsDev : 0;
-    for (int start = blockIdx.x * 256 * kBinItems; start < numItems; start += gridDim.x * 256 * kBinItems) {
-        if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
+    const int all = (int)gridDim.x * kBinThreads;
+    const int items = min(kBinItems, (numItems + all - 1) / all);  // per thread and round
+    for (int start = blockIdx.x * kBinThreads * items; start < numItems; start += all * items) {
+        if (tid < 2) cnt[tid] = 0;
         __syncthreads();
-        int bin[kBinItems], rank[kBinItems];
-#pragma unroll
-        for (int u = 0; u < kBinItems; ++u) {
-            const int i = start + u * 256 + (int)threadIdx.x;
-            bin[u] = -1;
-            if (i < numItems) {
-                int pa = -1, pb = -1;
-                if (kSub) {
-                    const int4 sp = subs[i];
-                    pa = sp.z >= 0 ? S.cols[S.children[sp.z].shapeIndex].shapeIndex : -sp.z - 1;
-                    pb = sp.w >= 0 ? S.cols[S.children[sp.w].shapeIndex].shapeIndex : -sp.w - 1;
-                } else {
-                    const int2 pr = pairs[i];
-                    const b3Collidable cA = S.cols[Bd.collidable[pr.x]], cB = S.cols[Bd.collidable[pr.y]];
-                    if (cA.shapeType == B3_SHAPE_CONVEX_HULL && cB.shapeType == B3_SHAPE_CONVEX_HULL &&
-                        (Bd.invMass[pr.x] != 0.f || Bd.invMass[pr.y] != 0.f)) {
-                        pa = cA.shapeIndex;
-                        pb = cB.shapeIndex;
-                    }
-                }
-                if (pa >= 0) bin[u] = sweep_small(S, pa, pb) ? 0 : 1;
-                else manifoldFlag[base + i] = 0u;
-            }
-        }
-        // ranks within the round: by warp votes, one shared addition per warp
-#pragma unroll
-        for (int u = 0; u < kBinItems; ++u) {
-            const unsigned m0 = __ballot_sync(kAll, bin[u] == 0), m1 = __ballot_sync(kAll, bin[u] == 1);
+        for (int u = 0; u < items; ++u) {
+            const int i = start + u * kBinThreads + tid;
+            const int bin = i < numItems ? bin_of<kSub>(base + i, pairs, subs, base, Bd, S) : -1;
+            if (bin < 0 && i < numItems) manifoldFlag[base + i] = 0u;
+            const unsigned m0 = __ballot_sync(kAll, bin == 0), m1 = __ballot_sync(kAll, bin == 1);
             int r = 0;
-            if ((threadIdx.x & 31) == 0 && m0) r = atomicAdd(&cnt[0], __popc(m0));
-            if ((threadIdx.x & 31) == 1 && m1) r = atomicAdd(&cnt[1], __popc(m1));
+            if ((tid & 31) == 0 && m0) r = atomicAdd(&cnt[0], __popc(m0));
+            if ((tid & 31) == 1 && m1) r = atomicAdd(&cnt[1], __popc(m1));
             const int r0 = __shfl_sync(kAll, r, 0), r1 = __shfl_sync(kAll, r, 1);
-            rank[u] = bin[u] == 0 ? r0 + __popc(m0 & b3dev::lanemask_lt()) : r1 + __popc(m1 & b3dev::lanemask_lt());
+            if (bin == 0) list[r0 + __popc(m0 & b3dev::lanemask_lt())] = base + i;
+            if (bin == 1) list[kLast - (r1 + __popc(m1 & b3dev::lanemask_lt()))] = base + i;
         }
         __syncthreads();
-        if (threadIdx.x < 2 && cnt[threadIdx.x])
-            at[threadIdx.x] = atomicAdd(scalars + (threadIdx.x ? b3::S_NP_BIG : b3::S_NP_SMALL), cnt[threadIdx.x]);
+        if (tid < 2 && cnt[tid]) at[tid] = atomicAdd(scalars + (tid ? b3::S_NP_BIG : b3::S_NP_SMALL), cnt[tid]);
         __syncthreads();
-#pragma unroll
-        for (int u = 0; u < kBinItems; ++u)
-            if (bin[u] >= 0)
-                (bin[u] ? warpQ : smallQ)[at[bin[u]] + rank[u]] = base + start + u * 256 + (int)threadIdx.x;
+        for (int k = tid; k < cnt[0]; k += kBinThreads) smallQ[at[0] + k] = list[k];
+        for (int k = tid; k < cnt[1]; k += kBinThreads) warpQ[at[1] + k] = list[kLast - k];
         __syncthreads();
     }
 }

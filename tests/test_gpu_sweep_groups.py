@@ -93,3 +93,35 @@ def test_many_pairs_per_grab(ctx):
         v.close()
     for f in ("numPairs", "numManifolds", "numContactPoints"):
         assert c[f] == sum(p[f] for p in per), f
+
+
+@pytest.mark.parametrize("gap", [-0.01, 0.0, 2e-6, 0.05])
+def test_pairs_left_out_before_the_sweep(ctx, gap):
+    """Pairs that the sorting finds to be apart: the same cubes with so many far
+    ones beside them that the pairs are sorted give the same bits as alone."""
+    n, far = 2000, 7000
+    i = np.arange(n)
+    side = 13
+    pos = np.stack([i % side, i // (side * side), i // side % side], 1) * (1.0 + gap) + [3.0, 0.5 + gap, 3.0]
+    turned = (i % 3 > 0)[:, None]
+    pos = pos + np.where(turned, scenes.uniform(3, 1, 3 * n, -0.02, 0.02).reshape(n, 3), 0.0)
+    quat = np.where(turned, scenes.yaw_quat(scenes.uniform(3, 2, n, 0.0, 0.8)), [0.0, 0.0, 0.0, 1.0])
+    k = np.arange(far)
+    away = np.stack([20.0 + 2.0 * (k % 20), 10.0 + 2.0 * (k // 400), 20.0 + 2.0 * (k // 20 % 20)], 1)
+    shapes = [scenes.box_vertices(100.0, 0.5, 100.0), scenes.box_vertices(0.5, 0.5, 0.5)]
+    states = []
+    for extra in (0, far):
+        m = n + extra
+        p = np.concatenate([pos, away])[:m]
+        q = np.concatenate([quat, np.tile([0.0, 0.0, 0.0, 1.0], (far, 1))])[:m]
+        b = scenes._concat([scenes.ground(), scenes._bodies(np.ones(m, np.int32), np.ones(m), p, q, np.full(m, 0.6),
+                                                            np.zeros(m))])
+        w = scenes.build_world(ctx, scenes.Scene(name="beside", shapes=shapes, num_worlds=1,
+                                                 config=dict(cellSize=1.0, gridDims=(64, 64, 64)), **b))
+        w.stepSimulation(3)
+        c = w.counters()
+        states.append(([a[:n + 1].copy() for a in w.read_state()], c["numManifolds"], c["refinedAxes"]))
+        w.close()
+    assert states[0][1:] == states[1][1:]
+    for x, y in zip(states[0][0], states[1][0]):
+        assert np.array_equal(x, y)
