@@ -1672,39 +1672,27 @@ struct ClipWarp {
 };
 
 __device__ __forceinline__ int grp_lane() { return threadIdx.x & (kClipGroup - 1); }
-__device__ __forceinline__ unsigned grp_mask() {
-    return ((1u << kClipGroup) - 1u) << ((threadIdx.x & 31) & ~(kClipGroup - 1));
-}
-__device__ __forceinline__ float grp_max(float v, unsigned m) {
-    return fkey_inv(__reduce_max_sync(m, fkey(v, kNanMax)));
-}
-// (value, index) minimum over the group, as warp_argmin
-__device__ __forceinline__ void grp_argmin(float& v, int& idx, unsigned m) {
-    const int k = fkey(v, kNanMin);
-    const int km = __reduce_min_sync(m, k);
-    idx = (int)__reduce_min_sync(m, k == km ? (unsigned)idx : 0xffffffffu);
-    v = fkey_inv(km);
-}
-
-// The group's primitives in two forms: kWhole, every lane of the warp is in the
-// call and the masks are the warp's (a group's own mask splits the warp, and the
-// four groups run one after another); otherwise by the calling group alone.
-template <bool kWhole>
+// The groups' votes and reductions, taken by all lanes of the warp together: a
+// group's own mask would split the warp, and the four groups would run one after
+// another. A group without work goes along and leaves no trace.
 struct Grp {
     __device__ static __forceinline__ unsigned ballot(bool x) {  // bit i: lane i of the group
-        const unsigned b = __ballot_sync(kWhole ? 0xffffffffu : grp_mask(), x);
-        return b >> ((threadIdx.x & 31) & ~(kClipGroup - 1)) & ((1u << kClipGroup) - 1u);
+        return __ballot_sync(0xffffffffu, x) >> ((threadIdx.x & 31) & ~(kClipGroup - 1)) & ((1u << kClipGroup) - 1u);
     }
-    __device__ static __forceinline__ void sync() { __syncwarp(kWhole ? 0xffffffffu : grp_mask()); }
+    __device__ static __forceinline__ bool any(bool x) { return ballot(x) != 0u; }
     __device__ static __forceinline__ float max(float v) {
-        if (!kWhole) return grp_max(v, grp_mask());
         int k = fkey(v, kNanMax);
 #pragma unroll
         for (int q = kClipGroup / 2; q > 0; q >>= 1) k = ::max(k, __shfl_xor_sync(0xffffffffu, k, q));
         return fkey_inv(k);
     }
+    __device__ static __forceinline__ int min(int k) {
+#pragma unroll
+        for (int q = kClipGroup / 2; q > 0; q >>= 1) k = ::min(k, __shfl_xor_sync(0xffffffffu, k, q));
+        return k;
+    }
+    // (value, index) minimum over the group, as warp_argmin
     __device__ static __forceinline__ void argmin(float& v, int& idx) {
-        if (!kWhole) return grp_argmin(v, idx, grp_mask());
         int k = fkey(v, kNanMin);
         unsigned i = (unsigned)idx;
 #pragma unroll
@@ -1717,12 +1705,27 @@ struct Grp {
         idx = (int)i;
         v = fkey_inv(k);
     }
-    __device__ static __forceinline__ float xor_add(float v, int q) {
-        return v + __shfl_xor_sync(kWhole ? 0xffffffffu : grp_mask(), v, q);
+    // (hi, lo, index) minimum over the group, as warp_argmin_ff
+    __device__ static __forceinline__ void argmin(ff& v, int& idx) {
+        int h = fkey(v.hi, kNanMin), l = fkey(v.lo, kNanMin);
+        unsigned i = (unsigned)idx;
+#pragma unroll
+        for (int q = kClipGroup / 2; q > 0; q >>= 1) {
+            const int oh = __shfl_xor_sync(0xffffffffu, h, q), ol = __shfl_xor_sync(0xffffffffu, l, q);
+            const unsigned oi = __shfl_xor_sync(0xffffffffu, i, q);
+            const bool less = oh < h || (oh == h && (ol < l || (ol == l && oi < i)));
+            h = less ? oh : h;
+            l = less ? ol : l;
+            i = less ? oi : i;
+        }
+        idx = (int)i;
+        v.hi = fkey_inv(h);
+        v.lo = fkey_inv(l);
     }
-    // the largest of the groups' counts that a loop with votes has to cover
-    __device__ static __forceinline__ int most(int n) { return kWhole ? __reduce_max_sync(0xffffffffu, n) : n; }
-    __device__ static __forceinline__ bool run(bool x) { return kWhole ? __any_sync(0xffffffffu, x) != 0 : x; }
+    __device__ static __forceinline__ float xor_add(float v, int q) { return v + __shfl_xor_sync(0xffffffffu, v, q); }
+    // the largest of the groups' counts, which a loop with votes has to cover
+    __device__ static __forceinline__ int most(int n) { return __reduce_max_sync(0xffffffffu, n); }
+    __device__ static __forceinline__ bool run(bool x) { return __any_sync(0xffffffffu, x) != 0; }
 };
 __device__ __forceinline__ unsigned grp_below() { return (1u << grp_lane()) - 1u; }
 
@@ -1731,7 +1734,6 @@ __device__ __forceinline__ unsigned grp_below() { return (1u << grp_lane()) - 1u
 // select_face over the group's lanes; faces within the window of the FP32
 // extreme only set *tied (the pair then goes to the float-float stage,
 // which decides them).
-template <bool kWhole>
 __device__ __forceinline__ int select_face_g(const b3::ShapesDev& S, const PairCtx& c, bool sideA, float3 sepf,
                                           float sign, bool* tied) {
     const b3ConvexPolyhedron& h = sideA ? *c.pa : *c.pb;
@@ -1748,18 +1750,17 @@ __device__ __forceinline__ int select_face_g(const b3::ShapesDev& S, const PairC
     }
     float wv = bv;
     int wi = bi;
-    Grp<kWhole>::argmin(wv, wi);
-    if (!kWhole && wi == kNone) return kNone;
+    Grp::argmin(wv, wi);
     const float lim = wv + 4e-6f;
-    int inWin = __popc(Grp<kWhole>::ballot(d0 <= lim));
+    int inWin = __popc(Grp::ballot(d0 <= lim));
     // the faces past the lanes' first ones
-    for (int f = gl + kClipGroup; Grp<kWhole>::run(f - gl < h.numFaces); f += kClipGroup) {
+    for (int f = gl + kClipGroup; Grp::run(f - gl < h.numFaces); f += kClipGroup) {
         bool in = false;
         if (f < h.numFaces) {
             const float4 pl = __ldg((const float4*)&S.faces[h.faceOffset + f].plane[0]);
             in = sign * dot(mul(R, make_float3(pl.x, pl.y, pl.z)), sepf) <= lim;
         }
-        inWin += __popc(Grp<kWhole>::ballot(in));
+        inWin += __popc(Grp::ballot(in));
     }
     if (wi != kNone && inWin > 1) *tied = true;
     return wi;
@@ -1776,7 +1777,7 @@ __device__ __forceinline__ int clip_poly_f32_g(const ClipGeom& G, const FfVert* 
     const float apl = len_ub(ap);
     const unsigned newTag = (unsigned)(kPlaneTag + k);
     int total = 0;
-    const int most = Grp<true>::most(nin);
+    const int most = Grp::most(nin);
     for (int base = 0; base < most; base += kClipGroup) {
         const int ve = base + gl;
         int cnt = 0;
@@ -1813,7 +1814,7 @@ __device__ __forceinline__ int clip_poly_f32_g(const ClipGeom& G, const FfVert* 
                 }
             }
         }
-        const unsigned b1 = Grp<true>::ballot(cnt >= 1), b2 = Grp<true>::ballot(cnt == 2);
+        const unsigned b1 = Grp::ballot(cnt >= 1), b2 = Grp::ballot(cnt == 2);
         const unsigned below = grp_below();
         const int pos = total + __popc(b1 & below) + __popc(b2 & below);
         if (cnt >= 1 && pos < kGroupPoly) put_tagged(out[pos], o0, t0, r0);
@@ -1877,7 +1878,7 @@ __device__ __forceinline__ int clip_f32_g(const PairCtx& c, const b3::ShapesDev&
     __syncwarp();
     bool bad = false, over = false;
     int cur = 0;
-    for (int e0 = 0; Grp<true>::run(e0 < nvA && !over); ++e0) {
+    for (int e0 = 0; Grp::run(e0 < nvA && !over); ++e0) {
         const bool cut = e0 < nvA && !over;
         const int n = clip_poly_f32_g(G, W.poly[cur], cut ? nIn : 0, cut ? e0 : 0, W.poly[cur ^ 1], &bad, &over);
         if (cut) {
@@ -1892,7 +1893,7 @@ __device__ __forceinline__ int clip_f32_g(const PairCtx& c, const b3::ShapesDev&
     const float3 nAw = G.nAw;
     const b3Face& fA = G.fA;
     int total = 0;
-    const int most = Grp<true>::most(nIn);
+    const int most = Grp::most(nIn);
     for (int base = 0; base < most; base += kClipGroup) {
         const int k = base + gl;
         bool keep = false;
@@ -1908,19 +1909,18 @@ __device__ __forceinline__ int clip_f32_g(const PairCtx& c, const b3::ShapesDev&
             if (depth <= P.minDist) depth = P.minDist;
             keep = depth <= P.maxDist;
         }
-        const unsigned m = Grp<true>::ballot(keep);
+        const unsigned m = Grp::ballot(keep);
         const int pos = total + __popc(m & grp_below());
         if (keep) put_f32(W.poly[cur ^ 1][pos], p + c.posA, depth);
         total += __popc(m);
     }
     __syncwarp();
-    *doubt = Grp<true>::ballot(bad) != 0u;
+    *doubt = Grp::ballot(bad) != 0u;
     *outBuf = cur ^ 1;
     return total;
 }
 
 // reduce_f32 over the group, for n <= kGroupPoly points (two per lane).
-template <bool kWhole>
 __device__ __forceinline__ int4 reduce_f32_g(const FfVert* p, int n, float3 nearNormal, bool* tie) {
     const int gl = grp_lane();
     const float3 o = get_f32(p[0]);
@@ -1928,9 +1928,9 @@ __device__ __forceinline__ int4 reduce_f32_g(const FfVert* p, int n, float3 near
     for (int k = gl; k < n; k += kClipGroup) s += get_f32(p[k]) - o;
 #pragma unroll
     for (int q = kClipGroup / 2; q > 0; q >>= 1) {
-        s.x = Grp<kWhole>::xor_add(s.x, q);
-        s.y = Grp<kWhole>::xor_add(s.y, q);
-        s.z = Grp<kWhole>::xor_add(s.z, q);
+        s.x = Grp::xor_add(s.x, q);
+        s.y = Grp::xor_add(s.y, q);
+        s.z = Grp::xor_add(s.z, q);
     }
     const float3 cr = s * (1.f / (float)n);
     const float3 aV = -cr;
@@ -1945,14 +1945,14 @@ __device__ __forceinline__ int4 reduce_f32_g(const FfVert* p, int n, float3 near
         pm = fmaxf(pm, len_ub(q));
         rm = fmaxf(rm, len_ub((q - o) - cr));
     }
-    pm = Grp<kWhole>::max(pm);
-    rm = Grp<kWhole>::max(rm);
+    pm = Grp::max(pm);
+    rm = Grp::max(rm);
     const float eP = 4e-6f + 1.2e-7f * pm;
     const float du = 2.f * eP / fmaxf(ul, 1e-30f) + 4e-7f;
     float fw[2], fu[2], fv[2];
     float mw = FLT_MAX, f0 = FLT_MIN, f1 = FLT_MIN, f2 = FLT_MIN, f3v = FLT_MIN;
     int iw = kNone, i0 = kNone, i1 = kNone, i2 = kNone, i3 = kNone;
-    const int nj = Grp<kWhole>::run(n > kClipGroup) ? 2 : 1;
+    const int nj = Grp::run(n > kClipGroup) ? 2 : 1;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
         const int k = gl + kClipGroup * j;
@@ -1969,22 +1969,22 @@ __device__ __forceinline__ int4 reduce_f32_g(const FfVert* p, int n, float3 near
             if (-fv[j] < f3v) { f3v = -fv[j]; i3 = k; }
         }
     }
-    Grp<kWhole>::argmin(mw, iw);
-    Grp<kWhole>::argmin(f0, i0);
-    Grp<kWhole>::argmin(f1, i1);
-    Grp<kWhole>::argmin(f2, i2);
-    Grp<kWhole>::argmin(f3v, i3);
+    Grp::argmin(mw, iw);
+    Grp::argmin(f0, i0);
+    Grp::argmin(f1, i1);
+    Grp::argmin(f2, i2);
+    Grp::argmin(f3v, i3);
     const float gap = 2.f * (2.f * eP + rm * du) + 1e-6f, gapw = 2.f * eP + 1e-6f;
     int cw = 0, c0 = 0, c1 = 0, c2 = 0, c3 = 0;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
         if (j >= nj) break;
         const bool ok = gl + kClipGroup * j < n;
-        cw += __popc(Grp<kWhole>::ballot(ok && fw[j] <= mw + gapw));
-        c0 += __popc(Grp<kWhole>::ballot(ok && fu[j] <= f0 + gap));
-        c1 += __popc(Grp<kWhole>::ballot(ok && -fu[j] <= f1 + gap));
-        c2 += __popc(Grp<kWhole>::ballot(ok && fv[j] <= f2 + gap));
-        c3 += __popc(Grp<kWhole>::ballot(ok && -fv[j] <= f3v + gap));
+        cw += __popc(Grp::ballot(ok && fw[j] <= mw + gapw));
+        c0 += __popc(Grp::ballot(ok && fu[j] <= f0 + gap));
+        c1 += __popc(Grp::ballot(ok && -fu[j] <= f1 + gap));
+        c2 += __popc(Grp::ballot(ok && fv[j] <= f2 + gap));
+        c3 += __popc(Grp::ballot(ok && -fv[j] <= f3v + gap));
     }
     const int worst = max(max(cw, c0), max(max(c1, c2), c3));
     *tie = worst > 1 || fabsf(f0) <= gap || fabsf(f1) <= gap || fabsf(f2) <= gap || fabsf(f3v) <= gap;
@@ -2066,8 +2066,8 @@ k_np_clip_groups(const int2* __restrict__ pairs, const int4* __restrict__ subs, 
             const float4 s4 = pre.aux;
             const float3 sepf = make_float3(s4.x, s4.y, s4.z);
             bool faceTie = false;
-            const int bi = select_face_g<true>(S, c, false, sepf, -1.f, &faceTie);
-            const int ai = select_face_g<true>(S, c, true, sepf, 1.f, &faceTie);
+            const int bi = select_face_g(S, c, false, sepf, -1.f, &faceTie);
+            const int ai = select_face_g(S, c, true, sepf, 1.f, &faceTie);
             int buf = 0;
             bool slow = false, defer = false;
             const bool clips = !faceTie && ai != kNone && ref_face_clips(S, c, ai);
@@ -2077,7 +2077,7 @@ k_np_clip_groups(const int2* __restrict__ pairs, const int4* __restrict__ subs, 
             bool tie = false;
             const bool reduces = !defer && !faceTie && !slow && nOut > 4;
             if (__any_sync(0xffffffffu, reduces)) {
-                const int4 r = reduce_f32_g<true>(W.poly[buf], reduces ? nOut : 1, -sepf, &tie);
+                const int4 r = reduce_f32_g(W.poly[buf], reduces ? nOut : 1, -sepf, &tie);
                 if (reduces) {
                     idx = r;
                     nRed = 4;
@@ -2113,7 +2113,11 @@ k_np_clip_groups(const int2* __restrict__ pairs, const int4* __restrict__ subs, 
 // per-point arithmetic; order-independent reductions; compactions in the
 // sequential order). Pairs outside the group tables (more candidates, faces
 // or clipped points than they hold, or clip faces tied along the FP32 axis,
-// whose axis the full search must redo) are passed to the warp kernels.
+// whose axis the full search must redo) are passed to the warp kernels. A warp
+// gathers the entries that are its own out of up to 32, then the groups go
+// through them together. Bound by the float-float instructions. 1,048,576 cubes:
+// 489,000 rankings 0.96 -> 0.82 ms, 482,000 clips 1.88 -> 1.42; 4,096 cubes (1,700
+// of each) 30 -> 23 and 38 -> 30 us.
 // ---------------------------------------------------------------------------
 struct __align__(16) GroupScratchFF {
     FfVert poly[2][kGroupPoly];   // clip polygons; the ranking's staged vertices
@@ -2122,43 +2126,20 @@ struct __align__(16) GroupScratchFF {
     int cand[kClipGroup];
 };
 
-__device__ __forceinline__ void ensure_ff_g(PairCtx& c, unsigned gm) {
-    const bool have = c.haveFF;
-    __syncwarp(gm);
-    if (!have) {
-        const ffmat a = quat_mat(c.qA), b = quat_mat(c.qB);
-        if (grp_lane() == 0) {
-            c.FA = a;
-            c.FB = b;
-            c.haveFF = true;
-        }
-        __syncwarp(gm);
-    }
-}
+constexpr int kExactChunk = 32;  // queue entries per work grab at most
+struct FFWarp {
+    PairPre pre[kExactChunk];
+    GroupScratchFF group[32 / kClipGroup];
+};
 
-// (hi, lo, index) minimum over the group, as warp_argmin_ff
-__device__ __forceinline__ void grp_argmin_ff(ff& v, int& idx, unsigned m) {
-    const int kh = fkey(v.hi, kNanMin);
-    const int mh = __reduce_min_sync(m, kh);
-    const int kl = kh == mh ? fkey(v.lo, kNanMin) : kNanMin;
-    const int ml = __reduce_min_sync(m, kl);
-    idx = (int)__reduce_min_sync(m, kh == mh && kl == ml ? (unsigned)idx : 0xffffffffu);
-    v.hi = fkey_inv(mh);
-    v.lo = fkey_inv(ml);
-}
-
-// PairCtx of item p into the group's shared context (every lane computes,
-// the group leader stores)
-template <bool kSub>
-__device__ __forceinline__ void item_setup_group(PairCtx& c, int p, const int2* __restrict__ pairs,
-                                                 const int4* __restrict__ subs, int base, const b3::BodiesDev& Bd,
-                                                 const b3::ShapesDev& S, unsigned gm) {
-    PairPre q;
-    item_prefetch<kSub>(q, p, pairs, subs, base, Bd, S);
+// PairCtx of a prefetched pair into its group's shared context, with the
+// float-float rotations: half of the group's lanes form A's, half B's.
+__device__ __forceinline__ void ctx_ff_g(PairCtx& c, const PairPre& pre, const b3::ShapesDev& S) {
+    const int gl = grp_lane();
     PairCtx t;
-    pair_from_pre(t, q, S);
-    __syncwarp(gm);
-    if (grp_lane() == 0) {
+    pair_from_pre(t, pre, S);
+    const ffmat m = quat_mat(gl & 1 ? t.qB : t.qA);
+    if (gl == 0) {
         c.A = t.A;
         c.B = t.B;
         c.invMassA = t.invMassA;
@@ -2169,23 +2150,24 @@ __device__ __forceinline__ void item_setup_group(PairCtx& c, int p, const int2* 
         c.qB = t.qB;
         c.RA = t.RA;
         c.RB = t.RB;
-        c.haveFF = false;
+        c.FA = m;
+        c.haveFF = true;
         c.posA = t.posA;
         c.posB = t.posB;
+    } else if (gl == 1) {
+        c.FB = m;
     }
-    __syncwarp(gm);
+    __syncwarp();
 }
 
 // refine_axes over the group, count <= kClipGroup candidates in W.cand
-__device__ __noinline__ bool refine_axes_g(PairCtx& c, const b3::ShapesDev& S, GroupScratchFF& W, int count,
+__device__ __forceinline__ bool refine_axes_g(PairCtx& c, const b3::ShapesDev& S, GroupScratchFF& W, int count,
                                            ff3& sep) {
     const int gl = grp_lane();
-    const unsigned gm = grp_mask();
     const b3ConvexPolyhedron& pa = *c.pa;
     const b3ConvexPolyhedron& pb = *c.pb;
     const float3 lcA = make_float3(pa.localCenter[0], pa.localCenter[1], pa.localCenter[2]);
     const float3 lcB = make_float3(pb.localCenter[0], pb.localCenter[1], pb.localCenter[2]);
-    ensure_ff_g(c, gm);
     const ff3 lcAw = mrot(c.FA, make_float3(lcA.x, lcA.y, lcA.z));
     const ff3 lcBw = mrot(c.FB, make_float3(lcB.x, lcB.y, lcB.z));
     const ff3 Dff = sub3(add3(lcAw, mk3(c.posA.x, c.posA.y, c.posA.z)), add3(lcBw, mk3(c.posB.x, c.posB.y, c.posB.z)));
@@ -2196,10 +2178,10 @@ __device__ __noinline__ bool refine_axes_g(PairCtx& c, const b3::ShapesDev& S, G
         float4* st = reinterpret_cast<float4*>(&W.poly[0][0]);
         for (int k = gl; k < pa.numVertices; k += kClipGroup) st[k] = __ldg(&vA[k]);
         for (int k = gl; k < pb.numVertices; k += kClipGroup) st[pa.numVertices + k] = __ldg(&vB[k]);
-        __syncwarp(gm);
         vA = st;
         vB = st + pa.numVertices;
     }
+    __syncwarp();
     ff bd = mk(FLT_MAX);
     int bidx = kNone;
     ff3 bn = mk3(0.f, 0.f, 0.f);
@@ -2216,32 +2198,33 @@ __device__ __noinline__ bool refine_axes_g(PairCtx& c, const b3::ShapesDev& S, G
             bn = n;
         }
     }
-    if (__any_sync(gm, fsep)) return false;
+    const bool apart = Grp::any(fsep);
     ff wd = bd;
     int widx = bidx;
-    grp_argmin_ff(wd, widx, gm);
-    if (widx == kNone) return false;
-    widx = (int)__reduce_min_sync(gm, bidx != kNone && sub(bd, wd).hi <= kAxisTieTol ? (unsigned)bidx : 0xffffffffu);
-    const unsigned who = __ballot_sync(gm, bidx == widx);
-    const int src = __ffs(who) - 1;
-    sep.x.hi = __shfl_sync(gm, bn.x.hi, src);
-    sep.x.lo = __shfl_sync(gm, bn.x.lo, src);
-    sep.y.hi = __shfl_sync(gm, bn.y.hi, src);
-    sep.y.lo = __shfl_sync(gm, bn.y.lo, src);
-    sep.z.hi = __shfl_sync(gm, bn.z.hi, src);
-    sep.z.lo = __shfl_sync(gm, bn.z.lo, src);
+    Grp::argmin(wd, widx);
+    const bool none = widx == kNone;
+    const bool tied = bidx != kNone && !none && sub(bd, wd).hi <= kAxisTieTol;
+    widx = Grp::min(tied ? bidx : kNone);
+    const unsigned who = Grp::ballot(bidx == widx);
+    const int src = ((threadIdx.x & 31) & ~(kClipGroup - 1)) + __ffs((int)who) - 1;
+    sep.x.hi = __shfl_sync(0xffffffffu, bn.x.hi, src & 31);
+    sep.x.lo = __shfl_sync(0xffffffffu, bn.x.lo, src & 31);
+    sep.y.hi = __shfl_sync(0xffffffffu, bn.y.hi, src & 31);
+    sep.y.lo = __shfl_sync(0xffffffffu, bn.y.lo, src & 31);
+    sep.z.hi = __shfl_sync(0xffffffffu, bn.z.hi, src & 31);
+    sep.z.lo = __shfl_sync(0xffffffffu, bn.z.lo, src & 31);
     if (dot3(neg3(Dff), sep).hi > 0.f) sep = neg3(sep);
-    return true;
+    return !apart && !none;
 }
 
 // clip_poly_ff over the group; *over when the output exceeds kGroupPoly
-__device__ __noinline__ int clip_poly_ff_g(const FfVert* in, int nin, const FfVert& plane, FfVert* out, bool* over) {
+__device__ __forceinline__ int clip_poly_ff_g(const FfVert* in, int nin, const FfVert& plane, FfVert* out, bool* over) {
     const int gl = grp_lane();
-    const unsigned gm = grp_mask();
     const ff3 pn = vget(plane);
     const ff eq = wget(plane);
     int total = 0;
-    for (int base = 0; base < nin; base += kClipGroup) {
+    const int most = Grp::most(nin);
+    for (int base = 0; base < most; base += kClipGroup) {
         const int ve = base + gl;
         const int sv = ve == 0 ? nin - 1 : ve - 1;
         ff3 e = mk3(0.f, 0.f, 0.f), s = e;
@@ -2252,8 +2235,8 @@ __device__ __noinline__ int clip_poly_ff_g(const FfVert* in, int nin, const FfVe
             de = add(dot3(pn, e), eq);
         }
         ff ds;
-        ds.hi = __shfl_up_sync(gm, de.hi, 1, kClipGroup);
-        ds.lo = __shfl_up_sync(gm, de.lo, 1, kClipGroup);
+        ds.hi = __shfl_up_sync(0xffffffffu, de.hi, 1, kClipGroup);
+        ds.lo = __shfl_up_sync(0xffffffffu, de.lo, 1, kClipGroup);
         if (ve < nin && gl == 0) ds = add(dot3(pn, s), eq);
         int cnt = 0;
         ff3 o0 = mk3(0.f, 0.f, 0.f), o1 = o0;
@@ -2274,43 +2257,43 @@ __device__ __noinline__ int clip_poly_ff_g(const FfVert* in, int nin, const FfVe
                 }
             }
         }
-        const unsigned b1 = __ballot_sync(gm, cnt >= 1), b2 = __ballot_sync(gm, cnt == 2);
-        const unsigned below = b3dev::lanemask_lt();
+        const unsigned b1 = Grp::ballot(cnt >= 1), b2 = Grp::ballot(cnt == 2);
+        const unsigned below = grp_below();
         const int pos = total + __popc(b1 & below) + __popc(b2 & below);
         if (cnt >= 1 && pos < kGroupPoly) out[pos] = vput(o0, mk(0.f));
         if (cnt == 2 && pos + 1 < kGroupPoly) out[pos + 1] = vput(o1, mk(0.f));
         total += __popc(b1) + __popc(b2);
     }
-    __syncwarp(gm);
+    __syncwarp();
     if (total > kGroupPoly) *over = true;
     return min(total, kGroupPoly);
 }
 
 // clip_hull_hull over the group; *over: a face or the clipped polygon
 // exceeds the group's tables (nothing decided)
-__device__ __noinline__ int clip_hull_hull_g(PairCtx& c, const b3::ShapesDev& S, const NpParams& P, ff3 sep, int ai,
-                                             int bi, GroupScratchFF& W, int* outBuf, bool* over) {
-    const unsigned gm = grp_mask();
-    ensure_ff_g(c, gm);
+__device__ __forceinline__ int clip_hull_hull_g(PairCtx& c, const b3::ShapesDev& S, const NpParams& P, ff3 sep, int ai,
+                                             int bi, bool run, GroupScratchFF& W, int* outBuf, bool* over) {
     const int gl = grp_lane();
     const b3ConvexPolyhedron& pa = *c.pa;
     const b3ConvexPolyhedron& pb = *c.pb;
-    if (ai == kNone || bi == kNone) return 0;
+    // a group without a clip goes along with an empty polygon
+    run = run && ai != kNone && bi != kNone;
+    if (!run) ai = bi = 0;
     const b3Face fB = S.faces[pb.faceOffset + bi];
     const b3Face fA = S.faces[pa.faceOffset + ai];
     const ff3 posA = mk3(c.posA.x, c.posA.y, c.posA.z);
     const ff3 posB = mk3(c.posB.x, c.posB.y, c.posB.z);
     int nIn = min(fB.numIndices, kMaxPoly);
-    const int nvA = min(fA.numIndices, kMaxPoly);
-    if (nIn > kGroupPoly || nvA > kGroupPoly) {
+    int nvA = min(fA.numIndices, kMaxPoly);
+    if (run && (nIn > kGroupPoly || nvA > kGroupPoly)) {
         *over = true;
-        return 0;
+        run = false;
     }
+    if (!run) nIn = nvA = 0;
     for (int k = gl; k < nIn; k += kClipGroup) {
         const float4 v = __ldg(&S.verts[pb.vertexOffset + S.indices[fB.indexOffset + k]]);
         W.poly[0][k] = vput(add3(mrot(c.FB, make_float3(v.x, v.y, v.z)), posB), mk(0.f));
     }
-    __syncwarp(gm);
     int cur = 0;
     const ff3 nAw = mrot(c.FA, make_float3(fA.plane[0], fA.plane[1], fA.plane[2]));
     for (int e0 = gl; e0 < nvA; e0 += kClipGroup) {
@@ -2324,16 +2307,21 @@ __device__ __noinline__ int clip_hull_hull_g(PairCtx& c, const b3::ShapesDev& S,
         const ff3 wa = add3(mrot(c.FA, make_float3(a.x, a.y, a.z)), posA);
         W.planes[e0] = vput(pn, neg(dot3(wa, pn)));
     }
-    __syncwarp(gm);
-    for (int e0 = 0; e0 < nvA && !*over; ++e0) {
-        nIn = clip_poly_ff_g(W.poly[cur], nIn, W.planes[e0], W.poly[cur ^ 1], over);
-        cur ^= 1;
+    __syncwarp();
+    for (int e0 = 0; Grp::run(e0 < nvA && !*over); ++e0) {
+        const bool cut = e0 < nvA && !*over;
+        const int n = clip_poly_ff_g(W.poly[cur], cut ? nIn : 0, W.planes[cut ? e0 : 0], W.poly[cur ^ 1], over);
+        if (cut) {
+            nIn = n;
+            cur ^= 1;
+        }
     }
-    if (*over) return 0;
+    if (*over) nIn = 0;
     const ff eqA = sub(mk(fA.plane[3]), dot3(nAw, posA));
     const ff minD = mk(P.minDist), maxD = mk(P.maxDist);
     int total = 0;
-    for (int base = 0; base < nIn; base += kClipGroup) {
+    const int most = Grp::most(nIn);
+    for (int base = 0; base < most; base += kClipGroup) {
         const int k = base + gl;
         bool keep = false;
         ff3 p = mk3(0.f, 0.f, 0.f);
@@ -2344,12 +2332,12 @@ __device__ __noinline__ int clip_hull_hull_g(PairCtx& c, const b3::ShapesDev& S,
             if (le(depth, minD)) depth = minD;
             keep = le(depth, maxD);
         }
-        const unsigned m = __ballot_sync(gm, keep);
-        const int pos = total + __popc(m & b3dev::lanemask_lt());
+        const unsigned m = Grp::ballot(keep);
+        const int pos = total + __popc(m & grp_below());
         if (keep) W.poly[cur ^ 1][pos] = vput(p, depth);
         total += __popc(m);
     }
-    __syncwarp(gm);
+    __syncwarp();
     *outBuf = cur ^ 1;
     return total;
 }
@@ -2357,7 +2345,6 @@ __device__ __noinline__ int clip_hull_hull_g(PairCtx& c, const b3::ShapesDev& S,
 // reduce_manifold over the group
 __device__ __noinline__ int4 reduce_manifold_g(const FfVert* p, int n, ff3 nearNormal) {
     const int gl = grp_lane();
-    const unsigned gm = grp_mask();
     ff3 s = mk3(0.f, 0.f, 0.f);
     for (int k = 0; k < n; ++k) s = add3(s, vget(p[k]));
     const ff invn = div(mk(1.f), mk((float)n));
@@ -2379,11 +2366,11 @@ __device__ __noinline__ int4 reduce_manifold_g(const FfVert* p, int n, ff3 nearN
         if (lt(dv, f2)) { f2 = dv; i2 = k; }
         if (lt(neg(dv), f3v)) { f3v = neg(dv); i3 = k; }
     }
-    grp_argmin_ff(mw, iw, gm);
-    grp_argmin_ff(f0, i0, gm);
-    grp_argmin_ff(f1, i1, gm);
-    grp_argmin_ff(f2, i2, gm);
-    grp_argmin_ff(f3v, i3, gm);
+    Grp::argmin(mw, iw);
+    Grp::argmin(f0, i0);
+    Grp::argmin(f1, i1);
+    Grp::argmin(f2, i2);
+    Grp::argmin(f3v, i3);
     int4 idx = make_int4(i0 == kNone ? 0 : i0, i1 == kNone ? 1 : i1, i2 == kNone ? 2 : i2, i3 == kNone ? 3 : i3);
     const int minIndex = iw == kNone ? -1 : iw;
     if (idx.x != minIndex && idx.y != minIndex && idx.z != minIndex && idx.w != minIndex) idx.x = minIndex;
@@ -2401,46 +2388,61 @@ k_np_refine_groups(const int2* __restrict__ pairs, const int4* __restrict__ subs
                    int32_t* __restrict__ scalars, b3Counters* __restrict__ counters) {
     extern __shared__ __align__(16) unsigned char np_smem[];
     constexpr int kPerWarp = 32 / kClipGroup;
-    const int lane = threadIdx.x & 31;
-    const int g = lane / kClipGroup;
-    const int gl = grp_lane();
-    const unsigned gm = grp_mask();
-    GroupScratchFF& W = reinterpret_cast<GroupScratchFF*>(np_smem)[(threadIdx.x >> 5) * kPerWarp + g];
+    const int lane = threadIdx.x & 31, g = lane / kClipGroup, gl = grp_lane();
+    FFWarp& FW = reinterpret_cast<FFWarp*>(np_smem)[threadIdx.x >> 5];
+    GroupScratchFF& W = FW.group[g];
     const int nSlow = scalars[b3::S_NP_SLOW];  // the sweep's entries: the clip has not run
-    int refined = 0;
-    for (;;) {
-        const int chunk = next_work(scalars + b3::S_NP_WORK4, nSlow, kPerWarp);
-        if (chunk < 0) break;
-        const int q = chunk + g;
-        if (q < nSlow) {
-            const int p = slowQ[q];
-            const float4 s4 = pairSep[p];
+    const int warps = gridDim.x * (blockDim.x >> 5);
+    int per = kPerWarp, refined = 0;
+    while (per < kExactChunk && nSlow > 2 * per * warps) per *= 2;
+    int i0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per;
+    while (i0 < nSlow) {
+        const int q = i0 + lane;
+        bool mine = false;
+        int p = 0;
+        float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (lane < per && q < nSlow) {
+            p = slowQ[q];
+            s4 = pairSep[p];
             const int count = __float_as_int(s4.x);
             if ((int)s4.w == kSepRefine && count > 0) {
-                if (count > kClipGroup) {
-                    if (gl == 0) deferQ[atomicAdd(scalars + b3::S_NP_DEFER3, 1)] = q;
-                } else {
-                    PairCtx& c = W.ctx;
-                    item_setup_group<kSub>(c, p, pairs, subs, scalars[b3::S_NUM_PAIRS], Bd, S, gm);
-                    if (gl < count) W.cand[gl] = cand[(size_t)q * kMaxCand + gl];
-                    __syncwarp(gm);
-                    ff3 sep = mk3(0.f, 0.f, 0.f);
-                    const bool haveAxis = refine_axes_g(c, S, W, count, sep);
-                    ++refined;
-                    if (gl == 0) {
-                        slowQ[q] = -1;
-                        if (haveAxis) {
-                            const float3 sf = to_f3(sep);
-                            pairSep[p] = make_float4(sf.x, sf.y, sf.z, (float)kSepDecided);
-                            fastQ[atomicAdd(scalars + b3::S_NP_FAST, 1)] = p;
-                        } else {
-                            manifoldFlag[p] = 0u;
-                        }
-                    }
-                }
+                mine = count <= kClipGroup;
+                if (!mine) deferQ[atomicAdd(scalars + b3::S_NP_DEFER3, 1)] = q;
             }
         }
+        const unsigned who = __ballot_sync(0xffffffffu, mine);
+        const int n = __popc(who);
+        if (mine) {
+            PairPre& pre = FW.pre[__popc(who & b3dev::lanemask_lt())];
+            item_prefetch<kSub>(pre, p, pairs, subs, scalars[b3::S_NUM_PAIRS], Bd, S);
+            pre.aux = s4;
+            pre.pad[0] = q;
+        }
         __syncwarp();
+        for (int r0 = 0; r0 < n; r0 += kPerWarp) {
+            const bool on = r0 + g < n;
+            const PairPre& pre = FW.pre[min(r0 + g, n - 1)];
+            PairCtx& c = W.ctx;
+            ctx_ff_g(c, pre, S);
+            const int count = __float_as_int(pre.aux.x), at = pre.pad[0];
+            if (gl < count) W.cand[gl] = cand[(size_t)at * kMaxCand + gl];
+            ff3 sep = mk3(0.f, 0.f, 0.f);
+            const bool haveAxis = refine_axes_g(c, S, W, count, sep);
+            if (on && gl == 0) {
+                ++refined;
+                slowQ[at] = -1;
+                if (haveAxis) {
+                    const float3 sf = to_f3(sep);
+                    pairSep[pre.p] = make_float4(sf.x, sf.y, sf.z, (float)kSepDecided);
+                    fastQ[atomicAdd(scalars + b3::S_NP_FAST, 1)] = pre.p;
+                } else {
+                    manifoldFlag[pre.p] = 0u;
+                }
+            }
+            __syncwarp();
+        }
+        if (lane == 0) i0 = (warps + atomicAdd(scalars + b3::S_NP_WORK4, 1)) * per;
+        i0 = __shfl_sync(0xffffffffu, i0, 0);
     }
     if (gl == 0 && refined) atomicAdd(&counters->refinedAxes, refined);
 }
@@ -2457,64 +2459,74 @@ k_np_exact_groups(const int2* __restrict__ pairs, const int4* __restrict__ subs,
                   int32_t* __restrict__ scalars, b3Counters* __restrict__ counters) {
     extern __shared__ __align__(16) unsigned char np_smem[];
     constexpr int kPerWarp = 32 / kClipGroup;
-    const int lane = threadIdx.x & 31;
-    const int g = lane / kClipGroup;
-    const int gl = grp_lane();
-    const unsigned gm = grp_mask();
-    GroupScratchFF& W = reinterpret_cast<GroupScratchFF*>(np_smem)[(threadIdx.x >> 5) * kPerWarp + g];
+    const int lane = threadIdx.x & 31, g = lane / kClipGroup, gl = grp_lane();
+    FFWarp& FW = reinterpret_cast<FFWarp*>(np_smem)[threadIdx.x >> 5];
+    GroupScratchFF& W = FW.group[g];
     const int nSlow = scalars[b3::S_NP_SLOW];
-    int clips = 0;
-    for (;;) {
-        const int chunk = next_work(scalars + b3::S_NP_WORK3, nSlow, kPerWarp);
-        if (chunk < 0) break;
-        const int q = chunk + g;
-        if (q < nSlow) {
-            const int p = slowQ[q];
-            if (p >= 0) {
-                const float4 s4 = pairSep[p];
-                bool defer = (int)s4.w != kSepClipDoubt;
-                if (!defer) {
-                    PairCtx& c = W.ctx;
-                    item_setup_group<kSub>(c, p, pairs, subs, scalars[b3::S_NUM_PAIRS], Bd, S, gm);
-                    const ff3 sep = mk3(s4.x, s4.y, s4.z);
-                    const float3 sepf = to_f3(sep);
-                    bool faceTie = false;
-                    const int bi = select_face_g<false>(S, c, false, sepf, -1.f, &faceTie);
-                    const int ai = select_face_g<false>(S, c, true, sepf, 1.f, &faceTie);
-                    defer = faceTie;
-                    if (!defer) {
-                        int nOut = 0, buf = 0;
-                        bool over = false, clipped = false;
-                        if (ref_face_clips(S, c, ai)) {
-                            nOut = clip_hull_hull_g(c, S, P, sep, ai, bi, W, &buf, &over);
-                            clipped = true;
-                        }
-                        if (over) {
-                            defer = true;
-                        } else {
-                            if (clipped) ++clips;
-                            if (nOut > 0) {
-                                const FfVert* pts = W.poly[buf];
-                                const ff3 nrm = neg3(sep);
-                                int4 idx = make_int4(0, 1, 2, 3);
-                                int nRed = nOut;
-                                if (nOut > 4) {
-                                    bool tie = false;
-                                    idx = reduce_f32_g<false>(pts, nOut, to_f3(nrm), &tie);
-                                    if (tie) idx = reduce_manifold_g(pts, nOut, nrm);
-                                    nRed = 4;
-                                }
-                                emit_contact_g(p, c, pts, nRed, idx, to_f3(nrm), Bd, P, contacts, manifoldFlag);
-                            } else if (gl == 0) {
-                                manifoldFlag[p] = 0u;
-                            }
-                        }
-                    }
-                }
-                if (defer && gl == 0) deferQ[atomicAdd(scalars + b3::S_NP_DEFER2, 1)] = q;
-            }
+    const int warps = gridDim.x * (blockDim.x >> 5);
+    int per = kPerWarp, clips = 0;
+    while (per < kExactChunk && nSlow > 2 * per * warps) per *= 2;
+    int i0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per;
+    while (i0 < nSlow) {
+        const int q = i0 + lane;
+        const int p = lane < per && q < nSlow ? slowQ[q] : -1;
+        float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p >= 0) s4 = pairSep[p];
+        const bool mine = p >= 0 && (int)s4.w == kSepClipDoubt;
+        if (p >= 0 && !mine) deferQ[atomicAdd(scalars + b3::S_NP_DEFER2, 1)] = q;
+        const unsigned who = __ballot_sync(0xffffffffu, mine);
+        const int n = __popc(who);
+        if (mine) {
+            PairPre& pre = FW.pre[__popc(who & b3dev::lanemask_lt())];
+            item_prefetch<kSub>(pre, p, pairs, subs, scalars[b3::S_NUM_PAIRS], Bd, S);
+            pre.aux = s4;
+            pre.pad[0] = q;
         }
         __syncwarp();
+        for (int r0 = 0; r0 < n; r0 += kPerWarp) {
+            const bool on = r0 + g < n;
+            const PairPre& pre = FW.pre[min(r0 + g, n - 1)];
+            PairCtx& c = W.ctx;
+            ctx_ff_g(c, pre, S);
+            const ff3 sep = mk3(pre.aux.x, pre.aux.y, pre.aux.z);
+            const float3 sepf = to_f3(sep);
+            bool faceTie = false;
+            const int bi = select_face_g(S, c, false, sepf, -1.f, &faceTie);
+            const int ai = select_face_g(S, c, true, sepf, 1.f, &faceTie);
+            int buf = 0;
+            bool over = false;
+            const bool clipped = !faceTie && ai != kNone && ref_face_clips(S, c, ai);
+            const int nOut = clip_hull_hull_g(c, S, P, sep, ai, bi, clipped, W, &buf, &over);
+            const FfVert* pts = W.poly[buf];
+            const ff3 nrm = neg3(sep);
+            int4 idx = make_int4(0, 1, 2, 3);
+            int nRed = nOut;
+            const bool reduces = !faceTie && !over && nOut > 4;
+            if (Grp::run(reduces)) {
+                bool tie = false;
+                int4 r = reduce_f32_g(pts, reduces ? nOut : 1, to_f3(nrm), &tie);
+                tie = tie && reduces;
+                if (Grp::run(tie)) {
+                    const int4 e = reduce_manifold_g(pts, tie ? nOut : 1, nrm);
+                    if (tie) r = e;
+                }
+                if (reduces) {
+                    idx = r;
+                    nRed = 4;
+                }
+            }
+            if (!on) {
+            } else if (faceTie || over) {
+                if (gl == 0) deferQ[atomicAdd(scalars + b3::S_NP_DEFER2, 1)] = pre.pad[0];
+            } else {
+                if (clipped && gl == 0) ++clips;
+                if (nOut > 0) emit_contact_g(pre.p, c, pts, nRed, idx, to_f3(nrm), Bd, P, contacts, manifoldFlag);
+                else if (gl == 0) manifoldFlag[pre.p] = 0u;
+            }
+            __syncwarp();
+        }
+        if (lane == 0) i0 = (warps + atomicAdd(scalars + b3::S_NP_WORK3, 1)) * per;
+        i0 = __shfl_sync(0xffffffffu, i0, 0);
     }
     if (gl == 0 && clips) atomicAdd(&counters->refinedClips, clips);
 }
@@ -2932,7 +2944,7 @@ static int launch_np_stages(b3World_t* w, cudaStream_t st, const NpParams& P) {
         w->d.pairSep, w->d.npFast, w->d.npSlow, w->d.npCand, candSlots, sc, w->d.counters);
     B3_CHECK_LAUNCH();
     if (tk) B3_CUDA(cudaEventRecord(w->npEv[1], st));
-    const size_t smemFF = sizeof(GroupScratchFF) * (32 / kClipGroup) * w->npWarpsPerBlock;
+    const size_t smemFF = sizeof(FFWarp) * w->npWarpsPerBlock;
     auto grid_ff = [&](const void* k) -> int {
         int occ = 1;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, threads, smemFF) != cudaSuccess || occ < 1) occ = 1;
@@ -3024,7 +3036,7 @@ int launch_narrowphase(b3World_t* w, cudaStream_t st) {
         B3_CUDA(cudaFuncSetAttribute(k_np_clip_groups<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smemGroups));
     }
-    const size_t smemFF = sizeof(GroupScratchFF) * (32 / kClipGroup) * w->npWarpsPerBlock;
+    const size_t smemFF = sizeof(FFWarp) * w->npWarpsPerBlock;
     if (smemFF > 48 * 1024 && (size_t)w->npFFSmemAttr < smemFF) {
         w->npFFSmemAttr = (int)smemFF;
         for (const void* k : {(const void*)k_np_refine_groups<false>, (const void*)k_np_refine_groups<true>,
