@@ -92,10 +92,10 @@ def fp32_peak_tflops(sm_mhz):
 # and DRAM bytes (read + write), per pair or per manifold.
 NCU_SOURCE = "ncu capture of the settled 16,384-body mixed-hull step (profiles/)"
 NCU_PER_UNIT = {
-    "k_np_sweep": {"fp32_ops_per_pair": 26729.0, "dram_bytes_per_pair": 13.2, "source": NCU_SOURCE},
-    "k_np_clip": {"fp32_ops_per_manifold": 4740.0, "dram_bytes_per_manifold": 106.8, "source": NCU_SOURCE},
-    "k_setup_rows": {"dram_bytes_per_manifold": 301.3, "source": NCU_SOURCE},
-    "k_jacobi": {"dram_bytes_per_manifold": 618.5, "source": NCU_SOURCE},
+    "k_np_sweep": {"fp32_ops_per_pair": 17941.0, "dram_bytes_per_pair": 38.9, "source": NCU_SOURCE},
+    "k_np_clip": {"fp32_ops_per_manifold": 4685.0, "dram_bytes_per_manifold": 89.2, "source": NCU_SOURCE},
+    "k_setup_rows": {"dram_bytes_per_manifold": 214.3, "source": NCU_SOURCE},
+    "k_jacobi": {"dram_bytes_per_manifold": 409.8, "source": NCU_SOURCE},
 }
 
 

@@ -1509,7 +1509,7 @@ __device__ __forceinline__ int next_work(int32_t* counter, int limit, int chunk)
 
 // Pairs per grab of a kernel with a pair per warp: one while the pairs are few,
 // since a warp does those of a grab one after another (16 us each of the largest
-// hulls) and others would have none. The warp sweep of 2,000 bodies on terrain 64 ->
+// hulls) and others would have none. The warp sweep of 2,048 bodies on terrain 64 ->
 // 44 us, of 33,000 falling bodies 71 -> 24.
 __device__ __forceinline__ int per_grab(int limit) {
     const int warps = (int)(gridDim.x * (blockDim.x >> 5));
