@@ -116,14 +116,16 @@ extern "C" int b3_fill_int2(b3Context ctx, int32_t* d_dst_int2, int32_t x, int32
 }
 
 // scratch layout for primitive calls: [error flag, total (one word each)]
-// [pad to 256][payload]; the flag is cleared on the stream. The element count
-// goes to the kernels by value.
-static int prim_scratch(b3Context ctx, size_t payload, cudaStream_t st, int32_t** err, void** body) {
+// [pad to 256][payload]; the flag and the payload's first `clear` bytes (a sort's
+// barrier word, a scan's tiles) are cleared on the stream by one memset. The
+// element count goes to the kernels by value.
+constexpr size_t kSortClear = 16;
+static int prim_scratch(b3Context ctx, size_t payload, size_t clear, cudaStream_t st, int32_t** err, void** body) {
     if (ctx->device < 0) return B3_ERR_NO_DEVICE;
     B3_TRY(ctx->ensureScratch(256 + payload));
     *err = (int32_t*)ctx->scratch;
     *body = (unsigned char*)ctx->scratch + 256;
-    B3_CUDA(cudaMemsetAsync(ctx->scratch, 0, 2 * sizeof(int32_t), st));
+    B3_CUDA(cudaMemsetAsync(ctx->scratch, 0, 256 + clear, st));
     return B3_OK;
 }
 
@@ -134,10 +136,10 @@ extern "C" int b3_prefix_scan_u32(b3Context ctx, const uint32_t* d_src, uint32_t
     int32_t* err;
     void* body;
     const size_t sb = b3::scan_scratch_bytes(n);
-    B3_TRY(prim_scratch(ctx, sb, st, &err, &body));
+    B3_TRY(prim_scratch(ctx, sb, sb, st, &err, &body));
     uint32_t* tot = (uint32_t*)(err + 1);
     // in-place scans are safe: each tile reads its input before it writes
-    B3_TRY(b3::exclusive_scan_u32(d_src, d_dst, nullptr, n, tot, body, sb, err, st, ctx->numSMs));
+    B3_TRY(b3::exclusive_scan_u32(d_src, d_dst, nullptr, n, tot, body, sb, err, st, ctx->numSMs, true));
     if (d_sum) B3_CUDA(cudaMemcpyAsync(d_sum, tot, 4, cudaMemcpyDeviceToDevice, st));
     if (h_sum) {
         int32_t hv[2] = {0, 0};  // the flag and the total, one copy
@@ -162,12 +164,12 @@ static int sort_impl(b3Context ctx, uint32_t* d_keys, uint32_t* d_values, int64_
     const size_t alt = ((size_t)n * 4 + 255) / 256 * 256;
     int32_t* err;
     void* body;
-    B3_TRY(prim_scratch(ctx, rb + 2 * alt, st, &err, &body));
+    B3_TRY(prim_scratch(ctx, rb + 2 * alt, kSortClear, st, &err, &body));
     uint32_t* kalt = (uint32_t*)((unsigned char*)body + rb);
     uint32_t* valt = d_values ? (uint32_t*)((unsigned char*)body + rb + alt) : nullptr;
     bool in_alt = false;
     B3_TRY(b3::radix_sort_pairs(d_keys, d_values, kalt, valt, nullptr, n, key_bits, body, rb, err, st,
-                                &in_alt, ctx->numSMs));
+                                &in_alt, ctx->numSMs, 0, true));
     if (in_alt) {
         B3_CUDA(cudaMemcpyAsync(d_keys, kalt, 4 * (size_t)n, cudaMemcpyDeviceToDevice, st));
         if (d_values) B3_CUDA(cudaMemcpyAsync(d_values, valt, 4 * (size_t)n, cudaMemcpyDeviceToDevice, st));
@@ -207,11 +209,11 @@ extern "C" int b3_radix_sort32_kv_out(b3Context ctx, const uint32_t* d_keys_in, 
     const size_t alt = ((size_t)n * 4 + 255) / 256 * 256;
     int32_t* err;
     void* body;
-    B3_TRY(prim_scratch(ctx, rb + 2 * alt, st, &err, &body));
+    B3_TRY(prim_scratch(ctx, rb + 2 * alt, kSortClear, st, &err, &body));
     uint32_t* ktmp = (uint32_t*)((unsigned char*)body + rb);
     uint32_t* vtmp = d_values_in ? (uint32_t*)((unsigned char*)body + rb + alt) : nullptr;
     return b3::radix_sort_kv_out(d_keys_in, d_values_in, d_keys_out, d_values_out, ktmp, vtmp, nullptr, n, key_bits,
-                                 body, rb, err, st, ctx->numSMs);
+                                 body, rb, err, st, ctx->numSMs, true);
 }
 
 extern "C" int b3_radix_sort32_sortdata(b3Context ctx, int32_t* d_key_values, int64_t n, int key_bits,
@@ -228,11 +230,11 @@ extern "C" int b3_radix_sort32_sortdata(b3Context ctx, int32_t* d_key_values, in
     const size_t rb = b3::radix_scratch_bytes(n, key_bits);
     int32_t* err;
     void* body;
-    B3_TRY(prim_scratch(ctx, rb + 8 * (size_t)n, st, &err, &body));
+    B3_TRY(prim_scratch(ctx, rb + 8 * (size_t)n, kSortClear, st, &err, &body));
     uint2* kv = reinterpret_cast<uint2*>(d_key_values);
     uint2* alt = (uint2*)((unsigned char*)body + rb);  // rb is a multiple of 256
     bool in_alt = false;
-    B3_TRY(b3::radix_sort_interleaved(kv, alt, nullptr, n, key_bits, body, rb, err, st, &in_alt, ctx->numSMs));
+    B3_TRY(b3::radix_sort_interleaved(kv, alt, nullptr, n, key_bits, body, rb, err, st, &in_alt, ctx->numSMs, true));
     if (in_alt) B3_CUDA(cudaMemcpyAsync(kv, alt, 8 * (size_t)n, cudaMemcpyDeviceToDevice, st));
     return B3_OK;
 }

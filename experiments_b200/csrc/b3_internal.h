@@ -80,12 +80,13 @@ int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_
 // between (unused for one pass). vals_in may be null (keys only).
 int radix_sort_kv_out(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out, uint32_t* vals_out,
                       uint32_t* keys_tmp, uint32_t* vals_tmp, const int32_t* n_dev, int64_t n_max, int key_bits,
-                      void* scratch, size_t scratch_bytes, int32_t* err_flag, cudaStream_t st, int numSMs);
+                      void* scratch, size_t scratch_bytes, int32_t* err_flag, cudaStream_t st, int numSMs,
+                      bool cleared = false);
 // Interleaved (key, value) pairs (btSortData): result in kv_alt when
 // *result_in_alt, else in kv.
 int radix_sort_interleaved(uint2* kv, uint2* kv_alt, const int32_t* n_dev, int64_t n_max, int key_bits,
                            void* scratch, size_t scratch_bytes, int32_t* err_flag, cudaStream_t st,
-                           bool* result_in_alt, int numSMs);
+                           bool* result_in_alt, int numSMs, bool cleared = false);
 
 size_t scan_scratch_bytes(int64_t n_max);
 // Exclusive scan of n_dev u32 values; total to d_total (may be null).

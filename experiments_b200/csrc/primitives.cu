@@ -657,7 +657,8 @@ int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_
 
 int radix_sort_kv_out(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out, uint32_t* vals_out,
                       uint32_t* keys_tmp, uint32_t* vals_tmp, const int32_t* n_dev, int64_t n_max, int key_bits,
-                      void* scratch, size_t scratch_bytes, int32_t* err_flag, cudaStream_t st, int numSMs) {
+                      void* scratch, size_t scratch_bytes, int32_t* err_flag, cudaStream_t st, int numSMs,
+                      bool cleared) {
     if (fits_block(n_max))
         return block_sort_any<false>(keys_in, vals_in, keys_out, vals_out, n_dev, n_max, key_bits, st);
     // the first pass writes the buffer that makes the last pass land in out
@@ -667,18 +668,19 @@ int radix_sort_kv_out(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t
     uint32_t* kB = odd ? keys_tmp : keys_out;
     uint32_t* vB = odd ? vals_tmp : vals_out;
     return radix_sort_core<false>(keys_in, vals_in, kA, vals_in ? vA : nullptr, kB, vals_in ? vB : nullptr,
-                                  n_dev, n_max, n_max, key_bits, scratch, scratch_bytes, err_flag, st, numSMs);
+                                  n_dev, n_max, n_max, key_bits, scratch, scratch_bytes, err_flag, st, numSMs,
+                                  cleared);
 }
 
 int radix_sort_interleaved(uint2* kv, uint2* kv_alt, const int32_t* n_dev, int64_t n_max, int key_bits,
                            void* scratch, size_t scratch_bytes, int32_t* err_flag, cudaStream_t st,
-                           bool* result_in_alt, int numSMs) {
+                           bool* result_in_alt, int numSMs, bool cleared) {
     uint32_t* a = reinterpret_cast<uint32_t*>(kv_alt);
     uint32_t* b = reinterpret_cast<uint32_t*>(kv);
     *result_in_alt = radix_result_in_alt(n_max, key_bits);
     if (fits_block(n_max)) return block_sort_any<true>(b, nullptr, b, nullptr, n_dev, n_max, key_bits, st);
     return radix_sort_core<true>(b, nullptr, a, nullptr, b, nullptr, n_dev, n_max, n_max, key_bits, scratch,
-                                 scratch_bytes, err_flag, st, numSMs);
+                                 scratch_bytes, err_flag, st, numSMs, cleared);
 }
 
 size_t scan_scratch_bytes(int64_t n_max) {
