@@ -1539,15 +1539,17 @@ __device__ __forceinline__ int push(int* queue, int32_t* count, int p) {
 template <bool kEarlyFaces, bool kSub>
 __global__ void __launch_bounds__(128, 6)
 k_np_sweep(const int2* __restrict__ pairs, const int4* __restrict__ subs, const int32_t* __restrict__ numPairsDev,
-           b3::BodiesDev Bd, b3::ShapesDev S, const int* __restrict__ queue, uint32_t* __restrict__ manifoldFlag,
-           float4* __restrict__ pairSep, int* __restrict__ fastQ, int* __restrict__ slowQ, int* __restrict__ cand,
+           b3::BodiesDev Bd, b3::ShapesDev S, const int* __restrict__ queue, int unsortedUpTo,
+           uint32_t* __restrict__ manifoldFlag, float4* __restrict__ pairSep, int* __restrict__ fastQ, int* __restrict__ slowQ, int* __restrict__ cand,
            int candSlots, int32_t* __restrict__ scalars, b3Counters* __restrict__ counters) {
     extern __shared__ __align__(16) unsigned char np_smem[];
     const int lane = threadIdx.x & 31;
     unsigned char* wbase = np_smem + (size_t)(threadIdx.x >> 5) * kSweepWarpSmem;
     PairPre* pre = reinterpret_cast<PairPre*>(wbase);
     int* wcand = reinterpret_cast<int*>(wbase + sizeof(PairPre) * kPreChunk);
-    const int numItems = queue ? scalars[b3::S_NP_BIG] : kSub ? scalars[b3::S_NUM_SUB] : *numPairsDev;
+    const int items = kSub ? scalars[b3::S_NUM_SUB] : *numPairsDev;
+    if (items <= unsortedUpTo) queue = nullptr;
+    const int numItems = queue ? scalars[b3::S_NP_BIG] : items;
     const int base = kSub ? *numPairsDev : 0;
     const int per = per_grab(numItems);
     for (;;) {
@@ -2923,18 +2925,21 @@ static int launch_np_stages(b3World_t* w, cudaStream_t st, const NpParams& P) {
     const bool tk = !kSub && w->timing && w->npEv[0] != nullptr;
     if (tk) B3_CUDA(cudaEventRecord(w->npEv[0], st));
     // Sorted into the two sweeps' queues, without the pairs that are apart, where
-    // the scene has pairs for both or bodies enough for it to pay (sweeps of
-    // cubes without / with it: 4,000 bodies 25 / 30 us, 8,000 38 / 38, 33,000
-    // 97 / 74). The groups' queue lies in a buffer that the manifold list uses
-    // later. The warp sweep always runs: it takes what the groups cannot hold.
-    const bool small = w->smallPairs, sorted = (small && w->largePairs) || w->bodies.size() > 8192;
+    // the scene has pairs for both or bodies enough that they may be many. Pairs
+    // of one kind are not sorted while they are few, which the device sees (bin
+    // and sweep of cubes, without / with it: 25,662 pairs 25 / 30 us, 52,757 38 /
+    // 38, 227,239 97 / 74). The groups' queue lies in a buffer that the manifold
+    // list uses later. The warp sweep always runs: it takes what the groups cannot
+    // hold.
+    const bool small = w->smallPairs, both = small && w->largePairs, sorted = both || w->bodies.size() > 8192;
+    const int unsortedUpTo = both ? -1 : 50 * 1024;
     int occS = 1;
     int* smallQ = sorted ? reinterpret_cast<int*>(w->d.manifoldScan) : nullptr;
     if (sorted) {
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occS, k_np_bin<kSub>, kBinThreads, 0) != cudaSuccess || occS < 1)
             occS = 1;
         k_np_bin<kSub><<<w->ctx->numSMs * occS, kBinThreads, 0, st>>>(w->d.pairs, w->d.subPairs, sc + S_NUM_PAIRS, Bd, S, sc,
-                                                          w->d.manifoldFlag, smallQ, w->d.npDefer);
+                                                          w->d.manifoldFlag, smallQ, w->d.npDefer, unsortedUpTo);
         B3_CHECK_LAUNCH();
     }
     const int candSlots = std::min(w->cfg.maxPairs, kNpCandSlots);
@@ -2943,7 +2948,7 @@ static int launch_np_stages(b3World_t* w, cudaStream_t st, const NpParams& P) {
                 cudaSuccess || occS < 1)
             occS = 1;
         k_np_sweep_groups<kSub><<<w->ctx->numSMs * occS, threads, smemSweepG, st>>>(
-            w->d.pairs, w->d.subPairs, sc + S_NUM_PAIRS, Bd, S, smallQ, w->d.manifoldFlag, w->d.pairSep, w->d.npFast,
+            w->d.pairs, w->d.subPairs, sc + S_NUM_PAIRS, Bd, S, smallQ, unsortedUpTo, w->d.manifoldFlag, w->d.pairSep, w->d.npFast,
             w->d.npSlow, w->d.npDefer, w->d.npCand, candSlots, sc);
         B3_CHECK_LAUNCH();
     }
@@ -2953,7 +2958,7 @@ static int launch_np_stages(b3World_t* w, cudaStream_t st, const NpParams& P) {
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occS, sweep, threads, smemSweep) != cudaSuccess || occS < 1)
         occS = 1;
     sweep<<<w->ctx->numSMs * occS, threads, smemSweep, st>>>(
-        w->d.pairs, w->d.subPairs, sc + S_NUM_PAIRS, Bd, S, small || sorted ? w->d.npDefer : nullptr, w->d.manifoldFlag,
+        w->d.pairs, w->d.subPairs, sc + S_NUM_PAIRS, Bd, S, small || sorted ? w->d.npDefer : nullptr, small ? -1 : unsortedUpTo, w->d.manifoldFlag,
         w->d.pairSep, w->d.npFast, w->d.npSlow, w->d.npCand, candSlots, sc, w->d.counters);
     B3_CHECK_LAUNCH();
     if (tk) B3_CUDA(cudaEventRecord(w->npEv[1], st));

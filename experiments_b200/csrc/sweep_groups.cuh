@@ -370,13 +370,14 @@ template <bool kSub>
 __global__ void __launch_bounds__(kBinThreads, 6)
 k_np_bin(const int2* __restrict__ pairs, const int4* __restrict__ subs, const int32_t* __restrict__ numPairsDev,
          b3::BodiesDev Bd, b3::ShapesDev S, int32_t* __restrict__ scalars, uint32_t* __restrict__ manifoldFlag,
-         int* __restrict__ smallQ, int* __restrict__ warpQ) {
+         int* __restrict__ smallQ, int* __restrict__ warpQ, int unsortedUpTo) {
     __shared__ int cnt[2], at[2];
     __shared__ int list[kBinThreads * kBinItems];  // the groups' from the front, the warps' from the back
     constexpr int kLast = kBinThreads * kBinItems - 1;
     const int tid = (int)threadIdx.x;
     const int numItems = kSub ? scalars[b3::S_NUM_SUB] : *numPairsDev;
     const int base = kSub ? *numPairsDev : 0;
+    if (numItems <= unsortedUpTo) return;
     const int all = (int)gridDim.x * kBinThreads;
     const int items = min(kBinItems, (numItems + all - 1) / all);  // per thread and round
     for (int start = blockIdx.x * kBinThreads * items; start < numItems; start += all * items) {
@@ -407,19 +408,22 @@ k_np_bin(const int2* __restrict__ pairs, const int4* __restrict__ subs, const in
 // whose axis the sweep decides go to the FP32 clip queue with that axis, pairs
 // with near-minimum candidates to the float-float queue. kSub: the items are
 // the sub-pairs of compound and mesh pairs, in the slots after the pairs'.
-// queue: their slots, or null when every item is one.
+// queue: their slots, or null when every item is one (as they are up to
+// unsortedUpTo items).
 template <bool kSub>
 __global__ void __launch_bounds__(128, 5)
 k_np_sweep_groups(const int2* __restrict__ pairs, const int4* __restrict__ subs,
                   const int32_t* __restrict__ numPairsDev, b3::BodiesDev Bd, b3::ShapesDev S,
-                  const int* __restrict__ queue, uint32_t* __restrict__ manifoldFlag, float4* __restrict__ pairSep,
-                  int* __restrict__ fastQ, int* __restrict__ slowQ, int* __restrict__ warpQ, int* __restrict__ cand,
-                  int candSlots, int32_t* __restrict__ scalars) {
+                  const int* __restrict__ queue, int unsortedUpTo, uint32_t* __restrict__ manifoldFlag,
+                  float4* __restrict__ pairSep, int* __restrict__ fastQ, int* __restrict__ slowQ,
+                  int* __restrict__ warpQ, int* __restrict__ cand, int candSlots, int32_t* __restrict__ scalars) {
     extern __shared__ __align__(16) unsigned char np_smem[];
     const int lane = threadIdx.x & 31, grp = lane / kClipGroup, gl = grp_lane();
     SweepScratch& W = reinterpret_cast<SweepScratch*>(np_smem)[threadIdx.x >> 5];
     const int base = kSub ? *numPairsDev : 0;
-    const int total = queue ? scalars[b3::S_NP_SMALL] : kSub ? scalars[b3::S_NUM_SUB] : *numPairsDev;
+    const int items = kSub ? scalars[b3::S_NUM_SUB] : *numPairsDev;
+    if (items <= unsortedUpTo) queue = nullptr;
+    const int total = queue ? scalars[b3::S_NP_SMALL] : items;
     // pairs per grab: one round of the groups while the pairs are few, so that
     // all warps have some; 32 once there are enough
     const int warps = gridDim.x * (blockDim.x >> 5);

@@ -97,31 +97,59 @@ def test_many_pairs_per_grab(ctx):
 
 @pytest.mark.parametrize("gap", [-0.01, 0.0, 2e-6, 0.05])
 def test_pairs_left_out_before_the_sweep(ctx, gap):
-    """Pairs that the sorting finds to be apart: the same cubes with so many far
-    ones beside them that the pairs are sorted give the same bits as alone."""
-    n, far = 2000, 7000
+    """Pairs that the sorting finds to be apart: the same cubes give the same bits
+    alone, where their pairs are not sorted, and with a far icosphere beside them,
+    with which they are."""
+    n = 2000
     i = np.arange(n)
     side = 13
     pos = np.stack([i % side, i // (side * side), i // side % side], 1) * (1.0 + gap) + [3.0, 0.5 + gap, 3.0]
     turned = (i % 3 > 0)[:, None]
     pos = pos + np.where(turned, scenes.uniform(3, 1, 3 * n, -0.02, 0.02).reshape(n, 3), 0.0)
     quat = np.where(turned, scenes.yaw_quat(scenes.uniform(3, 2, n, 0.0, 0.8)), [0.0, 0.0, 0.0, 1.0])
-    k = np.arange(far)
-    away = np.stack([20.0 + 2.0 * (k % 20), 10.0 + 2.0 * (k // 400), 20.0 + 2.0 * (k // 20 % 20)], 1)
-    shapes = [scenes.box_vertices(100.0, 0.5, 100.0), scenes.box_vertices(0.5, 0.5, 0.5)]
+    boxes = [scenes.box_vertices(100.0, 0.5, 100.0), scenes.box_vertices(0.5, 0.5, 0.5)]
     states = []
-    for extra in (0, far):
+    for extra in (0, 1):
         m = n + extra
-        p = np.concatenate([pos, away])[:m]
-        q = np.concatenate([quat, np.tile([0.0, 0.0, 0.0, 1.0], (far, 1))])[:m]
-        b = scenes._concat([scenes.ground(), scenes._bodies(np.ones(m, np.int32), np.ones(m), p, q, np.full(m, 0.6),
-                                                            np.zeros(m))])
-        w = scenes.build_world(ctx, scenes.Scene(name="beside", shapes=shapes, num_worlds=1,
-                                                 config=dict(cellSize=1.0, gridDims=(64, 64, 64)), **b))
+        p = np.concatenate([pos, [[50.0, 30.0, 50.0]]])[:m]
+        q = np.concatenate([quat, [[0.0, 0.0, 0.0, 1.0]]])[:m]
+        sid = np.append(np.ones(n, np.int32), 2)[:m]
+        b = scenes._concat([scenes.ground(), scenes._bodies(sid, np.ones(m), p, q, np.full(m, 0.6), np.zeros(m))])
+        w = scenes.build_world(ctx, scenes.Scene(name="beside", shapes=boxes + [scenes.icosphere_vertices(0.5)] * extra,
+                                                 num_worlds=1, config=dict(cellSize=1.0, gridDims=(64, 64, 64)), **b))
         w.stepSimulation(3)
         c = w.counters()
         states.append(([a[:n + 1].copy() for a in w.read_state()], c["numManifolds"], c["refinedAxes"]))
         w.close()
     assert states[0][1:] == states[1][1:]
+    for x, y in zip(states[0][0], states[1][0]):
+        assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n", [8192, 16500])
+def test_sorted_by_size(ctx, n):
+    """One kind of pairs, where the bodies are just not enough for the sorting and
+    where the pairs are: the same bits as with an icosphere beside them."""
+    side = 26
+    i = np.arange(n)
+    pos = np.stack([i % side, i // (side * side), i // side % side], 1) * [1.01, 0.995, 1.01] + [3.0, 0.5, 3.0]
+    pos += scenes.uniform(4, 1, 3 * n, -0.01, 0.01).reshape(n, 3)
+    quat = scenes.yaw_quat(scenes.uniform(4, 2, n, 0.0, 0.3))
+    boxes = [scenes.box_vertices(100.0, 0.5, 100.0), scenes.box_vertices(0.5, 0.5, 0.5)]
+    states = []
+    for extra in (0, 1):
+        m = n + extra
+        p = np.concatenate([pos, [[50.0, 50.0, 50.0]]])[:m]
+        q = np.concatenate([quat, [[0.0, 0.0, 0.0, 1.0]]])[:m]
+        sid = np.append(np.ones(n, np.int32), 2)[:m]
+        b = scenes._concat([scenes.ground(), scenes._bodies(sid, np.ones(m), p, q, np.full(m, 0.6), np.zeros(m))])
+        w = scenes.build_world(ctx, scenes.Scene(name="sorted", shapes=boxes + [scenes.icosphere_vertices(0.5)] * extra,
+                                                 num_worlds=1, config=dict(cellSize=1.0, gridDims=(64, 64, 64)), **b))
+        w.stepSimulation(2)
+        c = w.counters()
+        states.append(([a[:n + 1].copy() for a in w.read_state()], c["numPairs"], c["numManifolds"]))
+        w.close()
+    assert states[0][1:] == states[1][1:]
+    assert states[0][1] > (51200 if n > 8192 else 0)
     for x, y in zip(states[0][0], states[1][0]):
         assert np.array_equal(x, y)
