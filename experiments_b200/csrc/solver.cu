@@ -96,7 +96,10 @@ __global__ void k_body_ranges(const uint32_t* __restrict__ keys, const uint32_t*
 }
 
 // ---------------------------------------------------------------------------
-// Constraint setup (one thread per manifold)
+// Constraint setup (one thread per manifold). The contact is read where it lies:
+// a copy of its 96 bytes, indexed by the point, went through local memory
+// (1,048,576 cubes, 2.85 M manifolds: 602 -> 541 us; the 96 bytes read and 432
+// written of each take 226 at 6.65 TB/s).
 // ---------------------------------------------------------------------------
 struct SetupParams {
     float dt;
@@ -129,7 +132,7 @@ __global__ void k_setup_rows(b3::BodiesDev Bd, SolverView V, const int* __restri
     const int M = *V.numManifolds;
     if (blockIdx.x == 0 && threadIdx.x == 0) *barrier = 0ull;  // of the solve that follows
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
-        const b3Contact4 c = contacts[manifoldPair[m]];
+        const b3Contact4& c = contacts[manifoldPair[m]];
         const int A = abs(c.bodyAPtrAndSignBit), B = abs(c.bodyBPtrAndSignBit);
         const float imA = Bd.invMass[A], imB = Bd.invMass[B];
         const bool dynA = imA != 0.f, dynB = imB != 0.f;
@@ -153,10 +156,11 @@ __global__ void k_setup_rows(b3::BodiesDev Bd, SolverView V, const int* __restri
         const bool solve = dynA || dynB;
         float3 n = normalize(make_float3(-c.worldNormal[0], -c.worldNormal[1], -c.worldNormal[2]));
         for (int j = 0; j < npts && solve; ++j) {
-            const float depth = c.worldPos[j][3];
+            const float4 wp = *reinterpret_cast<const float4*>(&c.worldPos[j][0]);
+            const float depth = wp.w;
             const float dist = depth + SP.slopOffset;
             if (!(dist <= SP.contactProcessing)) continue;
-            const float3 posB = make_float3(c.worldPos[j][0], c.worldPos[j][1], c.worldPos[j][2]);
+            const float3 posB = f3(wp);
             const float3 posA = posB + n * dist;
             const float3 r1 = posA - pA;
             const float3 r2 = posB - pB;
