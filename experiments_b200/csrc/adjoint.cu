@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(128, 2)
 k_jacobi_adjoint(SolverView V, b3::JacobiTape T, AdjView A, int iterations, int resident, uint32_t* bar, int32_t* err,
                  b3Counters* counters) {
     extern __shared__ float4 kept[];  // [resident][kPhaseSlots][blockDim]
-    GridBarrier barrier(bar, err, counters, b3dev::kSpinLimit);
+    GridBarrier barrier(bar, err, counters, b3dev::kSpinLimit, true);
     const int M = *V.numManifolds;
     const size_t cap = (size_t)V.cap;
     const int phases = 2 * iterations;

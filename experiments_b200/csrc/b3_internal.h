@@ -136,22 +136,24 @@ constexpr int kSpinLimit = b3::kDefaultSpinLimit;
 // second word has to be released and a wait ends one L2 round trip after the
 // last arrival. A waiter gives up after spinLimit polls: it sets *err, counts
 // a timeout and sets the word's top bit, on which every block leaves at this
-// or its next barrier, so the launch always ends. An error that was set
-// before the launch ends it at the first barrier.
+// or its next barrier, so the launch always ends. heed: an error that was set
+// before the launch ends it at the first barrier too (the solves, whose results
+// are void by then). A sort pays no heed to it: it is the host that clears an
+// error, steps go on until then, and what they index with is a sort's output.
 struct GridBarrier {
     unsigned long long* word;
     unsigned long long target;
     int32_t* err;
     b3Counters* counters;
     int spinLimit;
-    int before;  // thread 0: *err at the kernel's start
+    int before;  // thread 0: *err at the kernel's start, where that is heeded
     unsigned blocks;  // that take part, block 0 on
 
-    __device__ __forceinline__ GridBarrier(uint32_t* w, int32_t* e, b3Counters* c, int limit,
+    __device__ __forceinline__ GridBarrier(uint32_t* w, int32_t* e, b3Counters* c, int limit, bool heed,
                                            unsigned taking = gridDim.x)
         : word(reinterpret_cast<unsigned long long*>(w)), target(0), err(e), counters(c), spinLimit(limit), before(0),
           blocks(taking) {
-        if (threadIdx.x == 0) before = *(volatile int32_t*)e;
+        if (heed && threadIdx.x == 0) before = *(volatile int32_t*)e;
     }
     __device__ __forceinline__ bool wait() {
         constexpr unsigned long long kAbort = 1ull << 63;

@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kSortThreads, 1) k_sort(SortArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SortSmem<kItems>& S = *reinterpret_cast<SortSmem<kItems>*>(smem_raw);
     constexpr int kTile = kSortThreads * kItems;
-    b3dev::GridBarrier barrier(A.bar, A.err, nullptr, b3dev::kSpinLimit);
+    b3dev::GridBarrier barrier(A.bar, A.err, nullptr, b3dev::kSpinLimit, false);
     const int n = dev_n(A.n_dev, A.n_host);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const bool has_vals = kPairs || A.vin != nullptr;

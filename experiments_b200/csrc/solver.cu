@@ -593,7 +593,7 @@ k_jacobi(SolverView V, int iterations, int resident, int most, uint32_t* bar, in
     // several to an SM
     const unsigned block = gridDim.x - 1 - blockIdx.x;
     if (block >= busy) return;
-    GridBarrier barrier(bar, err, counters, V.spinLimit, busy);
+    GridBarrier barrier(bar, err, counters, V.spinLimit, true, busy);
     const bool isB = tid & 1;
     const int m0 = (block * tb + tid) >> 1, warp0 = (block * tb + (tid & ~31)) >> 1;
     const int stride = (gridDim.x * tb) >> 1;
@@ -672,7 +672,7 @@ k_jacobi_pass(SolverView V, int iterations, int above, uint32_t* bar, int32_t* e
               b3::JacobiTape T) {
     const int M = *V.numManifolds;
     if (M <= above) return;  // k_jacobi took them
-    GridBarrier barrier(bar, err, counters, V.spinLimit);
+    GridBarrier barrier(bar, err, counters, V.spinLimit, true);
     const int phases = 2 * iterations;
     const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
     const int stride = gridDim.x * blockDim.x;
