@@ -184,6 +184,7 @@ enum ScalarSlot {
     S_NP_BIG = 24,        // items of the warp sweep's queue
     S_NP_WORK8 = 25,
     S_NP_SMALL = 26,      // items of the group sweep's queue
+    S_GS_STOP = 27,       // batched Gauss-Seidel: the error flag before the colouring
     S_NUM_SCALARS = 28
 };
 

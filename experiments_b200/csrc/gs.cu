@@ -91,7 +91,8 @@ __device__ __forceinline__ void gave_up(int32_t* err, b3Counters* counters) {
 }
 
 // One entry per manifold side: key = its dynamic body (numBodies for a static
-// one, past every body), value = 2 slot + side.
+// one, past every body), value = 2 slot + side. (A sort that gave up may leave
+// other values than manifolds.)
 __global__ void k_gs_sides(const uint32_t* __restrict__ vals, const b3Contact4* __restrict__ contacts,
                            const int* __restrict__ manifoldPair, const float* __restrict__ invMass,
                            const int32_t* __restrict__ numManifolds, int numBodies, uint32_t* __restrict__ bodyKeys,
@@ -100,7 +101,7 @@ __global__ void k_gs_sides(const uint32_t* __restrict__ vals, const b3Contact4* 
     const int M = *numManifolds;
     if (blockIdx.x == 0 && threadIdx.x == 0) *numSides = 2 * M;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < M; s += gridDim.x * blockDim.x) {
-        const b3Contact4& c = contacts[manifoldPair[vals[s]]];
+        const b3Contact4& c = contacts[manifoldPair[min(vals[s], (uint32_t)(M - 1))]];
         const int A = abs(c.bodyAPtrAndSignBit), B = abs(c.bodyBPtrAndSignBit);
         bodyKeys[2 * s] = invMass[A] != 0.f ? (uint32_t)A : (uint32_t)numBodies;
         bodyKeys[2 * s + 1] = invMass[B] != 0.f ? (uint32_t)B : (uint32_t)numBodies;
@@ -112,11 +113,16 @@ __global__ void k_gs_sides(const uint32_t* __restrict__ vals, const b3Contact4* 
 }
 
 // Per body its range of the sorted entries; per entry the previous one on the
-// same body in the same class (-1: none, -2: a static side).
+// same body in the same class (-1: none, -2: a static side). With an error of
+// this step's sorts or an earlier step the solve is void: no links, no colouring
+// and no places then (the sorts may not have ended, and the entries are indexes).
 __global__ void k_gs_links(const uint32_t* __restrict__ bodyKeys, const uint32_t* __restrict__ bodyVals,
                            const uint32_t* __restrict__ keys, const int32_t* __restrict__ numSides, int numBodies,
-                           uint32_t* __restrict__ start, uint32_t* __restrict__ end, int* __restrict__ prev) {
-    const int n = *numSides;
+                           uint32_t* __restrict__ start, uint32_t* __restrict__ end, int* __restrict__ prev,
+                           const int32_t* __restrict__ err, int32_t* __restrict__ stop) {
+    const int n = *numSides, e = *err;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *stop = e;
+    if (e) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t k = bodyKeys[i], v = bodyVals[i];
         if (k >= (uint32_t)numBodies) {
@@ -136,6 +142,7 @@ struct ColourView {
     const int32_t* numManifolds;
     unsigned long long* used;  // per entry: batches taken on its body up to it, kDone when final
     int* slotBatch;            // per slot
+    const int32_t* stop;
     int32_t* err;
     b3Counters* counters;
     int maxBatch;
@@ -163,6 +170,7 @@ __global__ void __launch_bounds__(kColourThreads) k_gs_colour(ColourView V) {
     __shared__ volatile unsigned long long local[2 * kColourThreads];
     const int M = *V.numManifolds;
     const int t = threadIdx.x;
+    if (*V.stop) return;
     for (int s0 = blockIdx.x * kColourThreads; s0 < M; s0 += gridDim.x * kColourThreads) {
         const int s = s0 + t;
         local[2 * t] = local[2 * t + 1] = 0ull;
@@ -212,8 +220,10 @@ __global__ void __launch_bounds__(kColourThreads) k_gs_colour(ColourView V) {
 __global__ void k_gs_rank(const uint32_t* __restrict__ bodyKeys, const uint32_t* __restrict__ bodyVals,
                           const uint32_t* __restrict__ keys, const int* __restrict__ slotBatch,
                           const int32_t* __restrict__ numSides, int numBodies, const uint32_t* __restrict__ start,
-                          const uint32_t* __restrict__ end, int maxBatch, int2* __restrict__ place) {
+                          const uint32_t* __restrict__ end, int maxBatch, int2* __restrict__ place,
+                          const int32_t* __restrict__ stop) {
     const int n = *numSides;
+    if (*stop) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t k = bodyKeys[i], v = bodyVals[i];
         int2 r = make_int2(0, 0);
@@ -348,7 +358,7 @@ __global__ void k_gs_setup(const uint32_t* __restrict__ keys, const uint32_t* __
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < M; s += gridDim.x * blockDim.x) {
         const int cls = (int)(keys[s] >> 8);
         const int batch = slotBatch[s];
-        const int m = (int)vals[s];
+        const int m = (int)min(vals[s], (uint32_t)(M - 1));
         if (batch < 0 || batch >= P.maxBatch) {  // colouring stopped (error flag set)
             slotOfManifold[m] = -1;
             continue;
@@ -662,13 +672,15 @@ int launch_gs_solver(b3World_t* w, cudaStream_t st) {
         std::swap(bodyKeys, bodyKeysAlt);
         std::swap(bodyVals, bodyValsAlt);
     }
-    k_gs_links<<<g, 256, 0, st>>>(bodyKeys, bodyVals, keys, numSides, N, d.bodyIncStart, d.bodyIncEnd, prev);
+    k_gs_links<<<g, 256, 0, st>>>(bodyKeys, bodyVals, keys, numSides, N, d.bodyIncStart, d.bodyIncEnd, prev,
+                                  d.scalars + S_ERR, d.scalars + S_GS_STOP);
     B3_CHECK_LAUNCH();
     ColourView CV;
     CV.prev = prev;
     CV.numManifolds = M;
     CV.used = used;
     CV.slotBatch = d.gsSlotBatch;
+    CV.stop = d.scalars + S_GS_STOP;
     CV.err = d.scalars + S_ERR;
     CV.counters = d.counters;
     CV.maxBatch = maxBatch;
@@ -693,7 +705,7 @@ int launch_gs_solver(b3World_t* w, cudaStream_t st) {
     k_gs_offsets<<<1, 1024, 0, st>>>(d.gsGroupCount, d.gsGroupOffset, groups);
     B3_CHECK_LAUNCH();
     k_gs_rank<<<g, 256, 0, st>>>(bodyKeys, bodyVals, keys, d.gsSlotBatch, numSides, N, d.bodyIncStart, d.bodyIncEnd,
-                                 maxBatch, place);
+                                 maxBatch, place, d.scalars + S_GS_STOP);
     B3_CHECK_LAUNCH();
     k_gs_inertia<<<(N + 255) / 256, 256, 0, st>>>(w->bodiesDev(), d.gsInertia, d.gsVel);
     B3_CHECK_LAUNCH();

@@ -52,6 +52,16 @@ int dalloc(T*& p, size_t count) {
     return B3_OK;
 }
 
+// Entries of a sort's buffers: zero at first, so that what a sort leaves that gave
+// up (its input, parts of its output, what an earlier sort left) is a valid index
+// at every place.
+template <class T>
+int dalloc_zero(T*& p, size_t count) {
+    B3_TRY(dalloc(p, count));
+    if (p) B3_CUDA(cudaMemset(p, 0, sizeof(T) * count));
+    return B3_OK;
+}
+
 void free_all(b3::DevBuffers& d) {
     void* ptrs[] = {d.pos, d.quat, d.linVel, d.angVel, d.invMass, d.friction, d.restitution,
                     d.invInertia, d.collidable, d.worldId, d.cols, d.polys, d.verts, d.faces,
@@ -653,10 +663,10 @@ static int ensure_capacity(b3World w) {
             B3_TRY(dalloc(d.sapOffset, (size_t)nb + 1));
             B3_TRY(dalloc(d.sapKept, (size_t)nb * b3::kSapKeep));
         }
-        B3_TRY(dalloc(d.keys, nb));
-        B3_TRY(dalloc(d.vals, nb));
-        B3_TRY(dalloc(d.keysAlt, nb));
-        B3_TRY(dalloc(d.valsAlt, nb));
+        B3_TRY(dalloc_zero(d.keys, nb));
+        B3_TRY(dalloc_zero(d.vals, nb));
+        B3_TRY(dalloc_zero(d.keysAlt, nb));
+        B3_TRY(dalloc_zero(d.valsAlt, nb));
         d.manifoldScanBytes = (b3::scan_scratch_bytes(std::max<int64_t>(cap, 1)) + 255) / 256 * 256;
         B3_TRY(dalloc(d.manifoldZero, d.manifoldScanBytes + 2 * sizeof(uint32_t) * (size_t)nb));
         d.bodyIncStart = reinterpret_cast<uint32_t*>(d.manifoldZero + d.manifoldScanBytes);
@@ -684,11 +694,11 @@ static int ensure_capacity(b3World w) {
         B3_TRY(dalloc(d.npCand, (size_t)std::min<size_t>(c, b3::kNpCandSlots) * 32));
         B3_TRY(dalloc(d.manifoldScan, c));
         B3_TRY(dalloc(d.manifoldPair, c));
-        B3_TRY(dalloc(d.incKeys, 2 * c));
-        B3_TRY(dalloc(d.incVals, 2 * c));
-        B3_TRY(dalloc(d.incKeysAlt, 2 * c));
-        B3_TRY(dalloc(d.incValsAlt, 2 * c));
-        B3_TRY(dalloc(d.incPos, 2 * c));
+        B3_TRY(dalloc_zero(d.incKeys, 2 * c));
+        B3_TRY(dalloc_zero(d.incVals, 2 * c));
+        B3_TRY(dalloc_zero(d.incKeysAlt, 2 * c));
+        B3_TRY(dalloc_zero(d.incValsAlt, 2 * c));
+        B3_TRY(dalloc_zero(d.incPos, 2 * c));
         B3_TRY(dalloc(d.rows, b3::kSolverRowSlots * c));
         B3_TRY(dalloc(d.copies, 8 * c));  // [2 phase buffers][2 sides][capacity][2]
         if (w->gs) {
