@@ -630,7 +630,9 @@ static int ensure_capacity(b3World w) {
     const int N = (int)w->bodies.size();
     const int cap = w->cfg.maxPairs;
     auto& d = w->d;
+    bool cleared = false;
     if (!d.cellTable) {
+        cleared = true;
         const size_t cells = (size_t)w->cfg.numWorlds << w->cellBits;
         B3_TRY(dalloc(d.cellTable, cells));
         B3_TRY(dalloc(d.scalars, b3::S_NUM_SCALARS));
@@ -640,6 +642,7 @@ static int ensure_capacity(b3World w) {
         B3_CUDA(cudaMemset(d.counters, 0, sizeof(b3Counters)));
     }
     if (w->capBodies < N || !d.pos) {
+        cleared = true;
         const int nb = std::max(N, 1);
         B3_TRY(dalloc(d.pos, nb));
         B3_TRY(dalloc(d.quat, nb));
@@ -681,6 +684,7 @@ static int ensure_capacity(b3World w) {
         w->capBodies = nb;
     }
     if (!d.pairs) {
+        cleared = true;
         const size_t c = std::max(cap, 1);
         B3_TRY(dalloc(d.pairs, c));
         B3_TRY(dalloc(d.contacts, c));
@@ -721,6 +725,7 @@ static int ensure_capacity(b3World w) {
     const size_t incBytes = std::max(b3::radix_scratch_bytes(2LL * cap, w->bodyBits),
                                      w->gs ? b3::radix_scratch_bytes(cap, 10) : (size_t)0);
     if (incBytes > d.incSortScratchBytes) {
+        cleared = true;
         d.incSortScratchBytes = incBytes;
         B3_TRY(dalloc((unsigned char*&)d.incSortScratch, incBytes));
         B3_CUDA(cudaMemset(d.incSortScratch, 0, 16));
@@ -736,6 +741,8 @@ static int ensure_capacity(b3World w) {
         B3_TRY(dalloc(d.worldMStart, (size_t)w->cfg.numWorlds));
         B3_TRY(dalloc(d.worldMEnd, (size_t)w->cfg.numWorlds));
     }
+    // the clears are on the default stream, which the caller's need not wait for
+    if (cleared) B3_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     return B3_OK;
 }
 
