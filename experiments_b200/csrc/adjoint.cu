@@ -1175,8 +1175,7 @@ int reverse_step(b3Adjoint_t* a, const float4* pre, cudaStream_t st) {
         const int need = (int)((est + (long long)blocks * threads - 1) / ((long long)blocks * threads));
         int resident = std::min(need, (int)((size_t)w->ctx->maxSmemOptin / perSm / one));
         const size_t smem = one * resident;
-        if (smem > 48 * 1024)
-            B3_CUDA(cudaFuncSetAttribute(k_jacobi_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (smem > 48 * 1024) B3_TRY(allow_dynamic_smem(w->ctx, (const void*)k_jacobi_adjoint));
         int occ = 1;
         B3_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_jacobi_adjoint, threads, smem));
         const int grid = std::min(w->ctx->numSMs * std::max(1, std::min(occ, perSm)), want);

@@ -51,6 +51,17 @@ struct b3Context_t {
 
 static inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// Lets a kernel take all the dynamic shared memory that a block can have. The
+// attribute is the function's, on its device, and not a world's: every caller sets
+// the same value, so that none lowers it between another thread's set and launch.
+static inline int allow_dynamic_smem(b3Context ctx, const void* kern) {
+    cudaFuncAttributes a;
+    B3_CUDA(cudaFuncGetAttributes(&a, kern));
+    B3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 ctx->maxSmemOptin - (int)a.sharedSizeBytes));
+    return B3_OK;
+}
+
 // ---------------------------------------------------------------------------
 // Device-wide primitives (implemented in primitives.cu). All take a device
 // side element count (n_dev) so they can be captured in CUDA graphs without

@@ -903,8 +903,7 @@ int launch_solver_taped(b3World_t* w, cudaStream_t st, const JacobiTape* tape) {
     b3Counters* ctr = w->d.counters;
     JacobiTape T = tape ? *tape : JacobiTape{};
     auto launch = [&](const void* kern, int threads, int occCap, int want, size_t smem, void** args) -> int {
-        if (smem > 48 * 1024)
-            B3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (smem > 48 * 1024) B3_TRY(allow_dynamic_smem(w->ctx, kern));
         int occ = 1;
         B3_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem));
         occ = std::max(1, std::min(occ, occCap));
