@@ -252,6 +252,7 @@ struct b3World_t {
                                // batched Gauss-Seidel: resident blocks, 0 = 8 and 2 per SM, 1 = half of them
     int solverGather = 0;      // Jacobi body averages: 0 = gathered by every manifold, 1 = a pass over the bodies
                                // where the rows do not fit the shared memories
+    bool keysInAlt = false;    // this step's cell keys await their sort in keysAlt / valsAlt
     int pairSearchMode = 0;    // grid pair search: 0 = thread per body, 1 = warp per body
     int clipGroups = 1;        // clip and float-float stages: 0 = a warp per pair, 1 = 8-lane groups
                                // (a warp per pair for what does not fit)

@@ -539,6 +539,7 @@ int launch_aabb_hash(b3World_t* w, cudaStream_t st) {
         key_buffers_swapped(w) ? w->d.keysAlt : w->d.keys, key_buffers_swapped(w) ? w->d.valsAlt : w->d.vals, 1,
         w->d.scalars, w->d.counters);
     B3_CHECK_LAUNCH();
+    w->keysInAlt = key_buffers_swapped(w);
     return B3_OK;
 }
 
@@ -548,6 +549,7 @@ int launch_sort_and_cells(b3World_t* w, cudaStream_t st) {
     if (ns == 0) return B3_OK;
     // (keys and values were written where the passes bring them to keys / vals)
     const bool swap = key_buffers_swapped(w);
+    w->keysInAlt = false;
     bool alt = false;
     B3_TRY(radix_sort_pairs(swap ? w->d.keysAlt : w->d.keys, swap ? w->d.valsAlt : w->d.vals,
                             swap ? w->d.keys : w->d.keysAlt, swap ? w->d.vals : w->d.valsAlt,

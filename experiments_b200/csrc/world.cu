@@ -1296,8 +1296,10 @@ extern "C" int b3_get_sorted_hash(b3World w, uint32_t* keys, uint32_t* values, i
     if (!w->written) return B3_ERR_STATE;
     const int n = std::min(w->numSmall, max);
     cudaStream_t st = as_stream(stream);
-    if (keys && n) B3_CUDA(cudaMemcpyAsync(keys, w->d.keys, 4 * (size_t)n, cudaMemcpyDeviceToHost, st));
-    if (values && n) B3_CUDA(cudaMemcpyAsync(values, w->d.vals, 4 * (size_t)n, cudaMemcpyDeviceToHost, st));
+    const uint32_t* k = w->keysInAlt ? w->d.keysAlt : w->d.keys;
+    const uint32_t* v = w->keysInAlt ? w->d.valsAlt : w->d.vals;
+    if (keys && n) B3_CUDA(cudaMemcpyAsync(keys, k, 4 * (size_t)n, cudaMemcpyDeviceToHost, st));
+    if (values && n) B3_CUDA(cudaMemcpyAsync(values, v, 4 * (size_t)n, cudaMemcpyDeviceToHost, st));
     B3_CUDA(cudaStreamSynchronize(st));
     *count = w->numSmall;
     return B3_OK;
