@@ -76,7 +76,7 @@ namespace b3 {
 // limit can be changed per world, b3_set_wait_limits).
 constexpr int kDefaultSpinLimit = 1 << 22;
 
-// Onesweep radix sort scratch: returns bytes for n_max elements.
+// Radix sort scratch: bytes for n_max elements.
 size_t radix_scratch_bytes(int64_t n_max, int key_bits);
 // Sort (keys, vals) of device count *n_dev (<= n_max). The sorted result
 // ends in (keys_alt, vals_alt) or in (keys, vals); *result_in_alt tells which. vals may be null (keys only).

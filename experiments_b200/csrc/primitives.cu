@@ -1,4 +1,4 @@
-// GPU primitives for sm_100a: fill, single-pass exclusive scan, onesweep LSD
+// GPU primitives for sm_100a: fill, single-pass exclusive scan, one-launch LSD
 // radix sort (8-bit digits) and bound search.
 //
 // Replaces the reference's OpenCL primitive objects:
@@ -79,7 +79,7 @@ __global__ void k_fill_int2(int2* __restrict__ dst, int2 v, int64_t n) {
 }
 
 // ---------------------------------------------------------------------------
-// Radix sort: one-read histogram for all passes
+// Radix sort: keys and digits
 // ---------------------------------------------------------------------------
 // Key i of a sort input: split arrays hold the keys contiguously; the
 // interleaved form (btSortData, BB/btRadixSort32CL.h:7-11) holds (key, value)

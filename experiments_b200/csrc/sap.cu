@@ -16,7 +16,7 @@
 // (P2/CLPhysicsDemo.cpp:558-568).
 //
 // B200 layout: the keys and the stable sort reuse the grid's key buffers
-// and the onesweep sort; the sorted small proxies are copied into one
+// and the radix sort; the sorted small proxies are copied into one
 // contiguous (min, max) float4 array so a warp's sweep over later proxies
 // reads consecutive 32-byte records. The reference appends pairs
 // with atomics in an unspecified order; here every sorted proxy counts its

@@ -27,14 +27,16 @@
 // Impulses reach every solver body (the SIMD row solvers used by this
 // solver mode have no per-body guard).
 //
-// B200 mapping: rows within a copy are Gauss-Seidel, copies are independent,
-// so one thread owns one manifold and solves its rows in order, keeping the
-// two copies' delta velocities in registers. The per-body average is a
-// deterministic segmented sum over the body's copies in manifold order (the
-// copy list is a stable radix sort of (body, copy) entries). All 4 phases x
-// iterations run in one persistent cooperative kernel separated by a grid
-// barrier whose wait is bounded. Rows are stored structure-of-arrays
-// (row slot major) so each phase streams them with coalesced float4 loads.
+// B200 mapping: rows within a copy are Gauss-Seidel, copies are independent, so a
+// manifold is solved by one thread (k_jacobi_pass, k_jacobi_worlds) or by two
+// lanes, one per body (k_jacobi), its rows in order, the copies' delta velocities
+// in registers. The per-body average is a deterministic segmented sum over the
+// body's copies in manifold order (the copy list is a stable radix sort of (body,
+// copy) entries). All phases of all iterations run in one persistent cooperative
+// kernel, separated by a grid barrier whose wait is bounded. Rows are stored
+// structure-of-arrays (row slot major): k_jacobi keeps those of a lane pair's first
+// manifolds in shared memory, otherwise each phase streams them with coalesced
+// float4 loads.
 #include "solver_common.cuh"
 
 #include <algorithm>

@@ -35,6 +35,7 @@ constexpr int kLamN = 23;
 constexpr int kLamF = 24;
 constexpr int kIds = 26;
 constexpr int kRowSlots = 27;
+static_assert(kRowSlots == b3::kSolverRowSlots, "the allocation holds every stream");
 
 struct SolverView {
     float4* rows;       // [kRowSlots][cap]
@@ -169,18 +170,13 @@ __device__ __forceinline__ void copy_average(const float4* __restrict__ copies, 
     ang = scaled(sa, 1.f / (float)(e - s));
 }
 
-// Streams of one manifold: in global memory (slot major, stride cap) or in
-// the block's shared memory (slot major, stride blockDim), where a thread
-// keeps the manifolds that it solves in every phase.
+// Streams of one manifold: in global memory (slot major, stride cap), or in the
+// adjoint in the block's shared memory (slot major, stride blockDim), where a
+// thread keeps the manifolds that it takes in every phase.
 struct GlobalRows {
     float4* at;
     size_t stride;
     __device__ __forceinline__ float4& operator()(int slot) const { return at[(size_t)slot * stride]; }
-};
-struct SharedRows {
-    float4* at;
-    int stride;
-    __device__ __forceinline__ float4& operator()(int slot) const { return at[slot * stride]; }
 };
 // streams a phase reads or writes (all but kIds)
 constexpr int kPhaseSlots = kIds;

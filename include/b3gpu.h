@@ -232,7 +232,10 @@ int b3_prefix_scan_u32_static(const uint32_t* d_src, uint32_t* d_dst, int64_t n,
 /* btRadixSort32CL::execute (BB/btRadixSort32CL.cpp:161-535): stable LSD
  * key-value sort of n (key, value) pairs, in place. Only the low key_bits
  * bits of the keys are sorted (1..32); keys must not use higher bits unless
- * key_bits = 32. Onesweep with 8-bit digits: ceil(key_bits/8) passes. */
+ * key_bits = 32. 8-bit digits, ceil(key_bits/8) passes: up to 8,192 pairs in one
+ * block; more in one cooperative launch of at most one block of 1,024 threads and
+ * some 60 KB of shared memory per SM, which begins when all of its blocks fit
+ * beside what else runs on the device (the same holds for the forms below). */
 int b3_radix_sort32_kv(b3Context ctx, uint32_t* d_keys, uint32_t* d_values, int64_t n,
                        int key_bits, void* stream);
 /* Keys-only variant (RadixSort32 keys-only benchmark,
@@ -614,7 +617,8 @@ int b3_autotune(b3World w, int trialSteps, void* stream);
  * body averages (0 = gathered by every manifold, rows kept in shared memory;
  * 1 = formed by a pass over the bodies between two grid barriers wherever the
  * rows do not fit the shared memories, which the device decides in worlds of
- * up to 170,000 bodies; bit-identical results), grid pair search form (0 = one thread per body
+ * at most 524,288 expected manifolds: three per body with hulls or meshes, one
+ * without, and no more than maxPairs; bit-identical results), grid pair search form (0 = one thread per body
  * over its 27 cells, 1 = one warp per body, a lane per cell; the same pair
  * list and overflow counts bit for bit), narrowphase lane groups (0 = one
  * warp per pair in the FP32 clip and the float-float stages, 1 = eight-lane
