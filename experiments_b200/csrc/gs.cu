@@ -118,7 +118,7 @@ __global__ void k_gs_sides(const uint32_t* __restrict__ vals, const b3Contact4* 
 // of 64 and more start 64 places apart at least, so that the place of a run's 64th
 // entry, by 64, numbers its set.
 constexpr int kLateWords = b3::kGsMaxBatch / 64;
-static_assert(b3::kGsMaxBatch % 128 == 0, "a set is read two words at a time");
+static_assert(b3::kGsMaxBatch % 64 == 0, "a set is whole words");
 
 // Per body its range of the sorted entries; per entry its links. With an error of
 // this step's sorts or an earlier step the solve is void: no links, no colouring
@@ -180,41 +180,31 @@ constexpr unsigned long long kDone = 1ull << 63;  // the 63 bits below: batches 
 // taken; maxBatch if there is none. A run's batches from 63 on are in its set,
 // which is the slot's own by then: the run's entries are coloured one after
 // another. A side without a set has 62 entries before this one at most, and they
-// are looked at one by one. A step of 500 cubes on a dynamic plate: 4.1 ms, of
-// 1,500 11.9; walking a run of k entries for every candidate batch, k^3 / 6 reads,
-// took 18.5 ms and more than the waits last.
-__device__ __noinline__ int late_batch(const ColourView& V, int2 a, int2 b) {
+// are looked at one by one, for the words that the sets leave open. A step of 500
+// cubes on a dynamic plate: 4.1 ms, of 1,500 11.9; walking a run of k entries for
+// every candidate batch, k^3 / 6 reads, took 18.5 ms and more than the waits last.
+// Word by word and in line: the colouring counts on its eight blocks an SM (out of
+// line with the words in an array it took 48 registers, five blocks, and 65,537
+// mixed bodies 0.13 ms more).
+__device__ __forceinline__ int late_batch(const int2* link, unsigned long long* late, const int* slotBatch, int4 sides) {
     __threadfence();
-    unsigned long long taken[kLateWords];
-#pragma unroll
-    for (int w = 0; w < kLateWords; ++w) taken[w] = w ? 0ull : kDone - 1;
-    for (int h = 0; h < 2; ++h) {
-        const int2 side = h ? b : a;
-        if (side.y >= 0) {
-            const ulonglong2* set = reinterpret_cast<const ulonglong2*>(V.late + (size_t)side.y * kLateWords);
-#pragma unroll
-            for (int w = 0; w < kLateWords / 2; ++w) {
-                const ulonglong2 x = __ldcg(set + w);
-                taken[2 * w] |= x.x;
-                taken[2 * w + 1] |= x.y;
-            }
-        } else {
-            for (int p = side.x; p >= 0; p = V.link[p].x) {
-                const int t = __ldcg(&V.slotBatch[p >> 1]);
-                if (t >= 63) taken[t >> 6] |= 1ull << (t & 63);
-            }
-        }
+    for (int w = 0; w < kLateWords; ++w) {
+        unsigned long long taken = w ? 0ull : kDone - 1;
+        if (sides.y >= 0) taken |= __ldcg(&late[(size_t)sides.y * kLateWords + w]);
+        if (sides.w >= 0) taken |= __ldcg(&late[(size_t)sides.w * kLateWords + w]);
+        for (int h = 0; h < 2 && ~taken; ++h)
+            if ((h ? sides.w : sides.y) < 0)
+                for (int p = h ? sides.z : sides.x; p >= 0; p = link[p].x) {
+                    const int t = __ldcg(&slotBatch[p >> 1]);
+                    if (t >> 6 == w) taken |= 1ull << (t & 63);
+                }
+        if (!~taken) continue;
+        const unsigned long long bit = ~taken & (taken + 1);
+        if (sides.y >= 0) __stcg(&late[(size_t)sides.y * kLateWords + w], __ldcg(&late[(size_t)sides.y * kLateWords + w]) | bit);
+        if (sides.w >= 0) __stcg(&late[(size_t)sides.w * kLateWords + w], __ldcg(&late[(size_t)sides.w * kLateWords + w]) | bit);
+        return 64 * w + __ffsll((long long)bit) - 1;
     }
-    int batch = V.maxBatch;
-    for (int w = 0; w < kLateWords && batch == V.maxBatch; ++w)
-        if (~taken[w]) batch = 64 * w + __ffsll((long long)~taken[w]) - 1;
-    if (batch < V.maxBatch)
-        for (int h = 0; h < 2; ++h) {
-            const int set = h ? b.y : a.y;
-            unsigned long long* word = V.late + (size_t)max(set, 0) * kLateWords + (batch >> 6);
-            if (set >= 0) __stcg(word, __ldcg(word) | 1ull << (batch & 63));
-        }
-    return batch;
+    return b3::kGsMaxBatch;
 }
 
 // One thread per slot, slots in order. A block hands batches on within its 256
@@ -223,7 +213,7 @@ __device__ __noinline__ int late_batch(const ColourView& V, int2 a, int2 b) {
 // is resident and its blocks go through the slots in order, so the first slot
 // without a batch always has all it waits for.
 constexpr int kColourThreads = 256;
-__global__ void __launch_bounds__(kColourThreads) k_gs_colour(ColourView V) {
+__global__ void __launch_bounds__(kColourThreads, 8) k_gs_colour(ColourView V) {
     __shared__ volatile unsigned long long local[2 * kColourThreads];
     const int M = *V.numManifolds;
     const int t = threadIdx.x;
@@ -250,7 +240,7 @@ __global__ void __launch_bounds__(kColourThreads) k_gs_colour(ColourView V) {
                 if (hasA && hasB) {
                     const unsigned long long free = ~(ua | ub) & (kDone - 1);
                     int batch = free ? __ffsll((long long)free) - 1
-                                     : late_batch(V, make_int2(pa, link.y), make_int2(pb, link.w));
+                                     : late_batch(V.link, V.late, V.slotBatch, link);
                     if (batch >= V.maxBatch) {
                         atomicExch(V.err, 2);
                         batch = -1;
