@@ -56,9 +56,9 @@ int dalloc(T*& p, size_t count) {
 // up (its input, parts of its output, what an earlier sort left) is a valid index
 // at every place.
 template <class T>
-int dalloc_zero(T*& p, size_t count) {
+int dalloc_zero(T*& p, size_t count, cudaStream_t st) {
     B3_TRY(dalloc(p, count));
-    if (p) B3_CUDA(cudaMemset(p, 0, sizeof(T) * count));
+    B3_CUDA(cudaMemsetAsync(p, 0, sizeof(T) * count, st));
     return B3_OK;
 }
 
@@ -626,23 +626,22 @@ extern "C" int b3_register_bodies(b3World w, int n, const float* masses, const f
     return B3_OK;
 }
 
-static int ensure_capacity(b3World w) {
+// New buffers are cleared on st, which b3_write_bodies waits for: not on the default
+// stream, which the caller's streams need not follow.
+static int ensure_capacity(b3World w, cudaStream_t st) {
     const int N = (int)w->bodies.size();
     const int cap = w->cfg.maxPairs;
     auto& d = w->d;
-    bool cleared = false;
     if (!d.cellTable) {
-        cleared = true;
         const size_t cells = (size_t)w->cfg.numWorlds << w->cellBits;
         B3_TRY(dalloc(d.cellTable, cells));
         B3_TRY(dalloc(d.scalars, b3::S_NUM_SCALARS));
         B3_TRY(dalloc(d.counters, 1));
-        B3_CUDA(cudaMemset(d.cellTable, 0, sizeof(uint4) * cells));
-        B3_CUDA(cudaMemset(d.scalars, 0, sizeof(int32_t) * b3::S_NUM_SCALARS));
-        B3_CUDA(cudaMemset(d.counters, 0, sizeof(b3Counters)));
+        B3_CUDA(cudaMemsetAsync(d.cellTable, 0, sizeof(uint4) * cells, st));
+        B3_CUDA(cudaMemsetAsync(d.scalars, 0, sizeof(int32_t) * b3::S_NUM_SCALARS, st));
+        B3_CUDA(cudaMemsetAsync(d.counters, 0, sizeof(b3Counters), st));
     }
     if (w->capBodies < N || !d.pos) {
-        cleared = true;
         const int nb = std::max(N, 1);
         B3_TRY(dalloc(d.pos, nb));
         B3_TRY(dalloc(d.quat, nb));
@@ -666,10 +665,10 @@ static int ensure_capacity(b3World w) {
             B3_TRY(dalloc(d.sapOffset, (size_t)nb + 1));
             B3_TRY(dalloc(d.sapKept, (size_t)nb * b3::kSapKeep));
         }
-        B3_TRY(dalloc_zero(d.keys, nb));
-        B3_TRY(dalloc_zero(d.vals, nb));
-        B3_TRY(dalloc_zero(d.keysAlt, nb));
-        B3_TRY(dalloc_zero(d.valsAlt, nb));
+        B3_TRY(dalloc_zero(d.keys, nb, st));
+        B3_TRY(dalloc_zero(d.vals, nb, st));
+        B3_TRY(dalloc_zero(d.keysAlt, nb, st));
+        B3_TRY(dalloc_zero(d.valsAlt, nb, st));
         d.manifoldScanBytes = (b3::scan_scratch_bytes(std::max<int64_t>(cap, 1)) + 255) / 256 * 256;
         B3_TRY(dalloc(d.manifoldZero, d.manifoldScanBytes + 2 * sizeof(uint32_t) * (size_t)nb));
         d.bodyIncStart = reinterpret_cast<uint32_t*>(d.manifoldZero + d.manifoldScanBytes);
@@ -680,11 +679,10 @@ static int ensure_capacity(b3World w) {
         }
         d.sortScratchBytes = b3::radix_scratch_bytes(nb, w->keyBits);
         B3_TRY(dalloc((unsigned char*&)d.sortScratch, d.sortScratchBytes));
-        B3_CUDA(cudaMemset(d.sortScratch, 0, 16));  // the grid barrier's word; each step leaves it cleared
+        B3_CUDA(cudaMemsetAsync(d.sortScratch, 0, 16, st));  // the grid barrier's word; each step leaves it cleared
         w->capBodies = nb;
     }
     if (!d.pairs) {
-        cleared = true;
         const size_t c = std::max(cap, 1);
         B3_TRY(dalloc(d.pairs, c));
         B3_TRY(dalloc(d.contacts, c));
@@ -698,11 +696,11 @@ static int ensure_capacity(b3World w) {
         B3_TRY(dalloc(d.npCand, (size_t)std::min<size_t>(c, b3::kNpCandSlots) * 32));
         B3_TRY(dalloc(d.manifoldScan, c));
         B3_TRY(dalloc(d.manifoldPair, c));
-        B3_TRY(dalloc_zero(d.incKeys, 2 * c));
-        B3_TRY(dalloc_zero(d.incVals, 2 * c));
-        B3_TRY(dalloc_zero(d.incKeysAlt, 2 * c));
-        B3_TRY(dalloc_zero(d.incValsAlt, 2 * c));
-        B3_TRY(dalloc_zero(d.incPos, 2 * c));
+        B3_TRY(dalloc_zero(d.incKeys, 2 * c, st));
+        B3_TRY(dalloc_zero(d.incVals, 2 * c, st));
+        B3_TRY(dalloc_zero(d.incKeysAlt, 2 * c, st));
+        B3_TRY(dalloc_zero(d.incValsAlt, 2 * c, st));
+        B3_TRY(dalloc_zero(d.incPos, 2 * c, st));
         B3_TRY(dalloc(d.rows, b3::kSolverRowSlots * c));
         B3_TRY(dalloc(d.copies, 8 * c));  // [2 phase buffers][2 sides][capacity][2]
         if (w->gs) {
@@ -725,10 +723,9 @@ static int ensure_capacity(b3World w) {
     const size_t incBytes = std::max(b3::radix_scratch_bytes(2LL * cap, w->bodyBits),
                                      w->gs ? b3::radix_scratch_bytes(cap, 10) : (size_t)0);
     if (incBytes > d.incSortScratchBytes) {
-        cleared = true;
         d.incSortScratchBytes = incBytes;
         B3_TRY(dalloc((unsigned char*&)d.incSortScratch, incBytes));
-        B3_CUDA(cudaMemset(d.incSortScratch, 0, 16));
+        B3_CUDA(cudaMemsetAsync(d.incSortScratch, 0, 16, st));
     }
     if (w->hasSubPairs() && !d.subPairs) {
         const size_t c = std::max(cap, 1);
@@ -741,8 +738,6 @@ static int ensure_capacity(b3World w) {
         B3_TRY(dalloc(d.worldMStart, (size_t)w->cfg.numWorlds));
         B3_TRY(dalloc(d.worldMEnd, (size_t)w->cfg.numWorlds));
     }
-    // the clears are on the default stream, which the caller's need not wait for
-    if (cleared) B3_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     return B3_OK;
 }
 
@@ -874,7 +869,7 @@ extern "C" int b3_write_bodies(b3World w, void* stream) {
     }
     cudaStream_t st = as_stream(stream);
     B3_CUDA(cudaSetDevice(w->ctx->device));
-    B3_TRY(ensure_capacity(w));
+    B3_TRY(ensure_capacity(w, st));
     B3_TRY(upload_shapes(w, st));
     const int N = (int)w->bodies.size();
     std::vector<float4> pos(N), quat(N), lv(N), av(N), ii(N);
