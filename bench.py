@@ -41,7 +41,8 @@ Prints one JSON line on rank 0.
 * scale: the 1,048,576-cube plain step and adjoint.
 --impl reference: the same CPU pipeline on all host cores: one replica per
   core, each one column block of the scene stepped to the settle step and
-  then timed (the 16 blocks tile the whole scene), same metric.
+  then timed (the 16 blocks tile the whole scene), same metric; a line with
+  "unavailable" where that pipeline is not built.
 """
 import argparse
 import json
@@ -769,12 +770,18 @@ def main():
     if args.impl == "reference":
         if rank != 0:
             return
+        import oracle
+        if oracle.bullet_lib() is None:
+            # this build's own port is no reference
+            print(json.dumps({"impl": "reference", "unavailable": "the reference's bullet2 sources are not on this "
+                              "machine and its CPU pipeline (oracle/_ref/libb3bullet.so) is not built"}))
+            return
         procs = max(1, os.cpu_count() or 1)
         r = cpu_baseline_port(args.workload, budget_s=15.0, procs=procs, settle=args.settle)
         cfg["window"] = f"settled: timed from step {args.settle}" if args.workload in LATTICE else "from the start"
         line = {"metric": "body-steps/s", "value": r["value"], "unit": "body-steps/s", "n_gpus": args.gpus,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": None, "higher_is_better": True,
-                "scaling": "weak", "vs_baseline": None, "dtype": "f32" if r["kind"] == "reference" else "f64",
+                "scaling": "weak", "vs_baseline": None, "dtype": "f32",
                 "data": "synthetic (seeded scene generator)", "impl": "reference",
                 "config": cfg, "cpu_baseline": r,
                 "e2e": {"value": r["value"], "unit": "body-steps/s", "h2d_bytes_per_step": 0,
