@@ -101,7 +101,7 @@ __global__ void k_body_ranges(const uint32_t* __restrict__ keys, const uint32_t*
 // Constraint setup (one thread per manifold). The contact is read where it lies:
 // a copy of its 96 bytes, indexed by the point, went through local memory
 // (1,048,576 cubes, 2.85 M manifolds: 602 -> 541 us; the 96 bytes read and 432
-// written of each take 226 at 6.65 TB/s).
+// written of each take 230 at 6.55 TB/s).
 // ---------------------------------------------------------------------------
 struct SetupParams {
     float dt;
@@ -667,7 +667,7 @@ k_jacobi(SolverView V, int iterations, int resident, int most, uint32_t* bar, in
 // per manifold of the body (at 5.4 copies a body, 64 B instead of 350 B of L2
 // reads per manifold and phase); the extra barrier is a few microseconds.
 // 1,048,576 cubes (2.85 M manifolds): 7.22 -> 5.46 ms, of which the streams
-// and copies take 4.3 ms at 6.65 TB/s; 131,072 mixed bodies (395 K): 1.26 -> 0.90 ms.
+// and copies take 4.4 ms at 6.55 TB/s; 131,072 mixed bodies (395 K): 1.26 -> 0.90 ms.
 template <bool TAPE>
 __global__ void __launch_bounds__(256, 2)
 k_jacobi_pass(SolverView V, int iterations, int above, uint32_t* bar, int32_t* err, b3Counters* counters,
