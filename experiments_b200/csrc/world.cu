@@ -1081,6 +1081,7 @@ extern "C" int b3_step(b3World w, int numSteps, void* stream) {
             w->graphValid = true;
         }
         for (int i = done; i < numSteps; ++i) B3_CUDA(cudaGraphLaunch(w->graphExec, st));
+        w->keysInAlt = false;  // a replayed step sorts its keys
         return B3_OK;
     }
     for (int i = 0; i < numSteps; ++i) {

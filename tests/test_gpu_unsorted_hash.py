@@ -30,3 +30,22 @@ def test_keys_before_and_after_the_sort(ctx, n, dims):
         pos[:, :3] += 1.7  # other cells the next time
         w.write_state(pos, quat, lin, ang)
     w.close()
+
+
+def test_keys_after_a_replayed_step(ctx):
+    """A captured step that follows b3_stage_aabbs sorts its own keys."""
+    sc = scenes.random_pile(32, n=9000, box=60.0, hull_frac=0.0)  # cells of all three digits
+    hashes = []
+    for staged in (False, True):
+        w = scenes.build_world(ctx, sc, gridDims=(64, 32, 64), useGraph=1)
+        w.stepSimulation(2)
+        state = w.read_state()
+        if staged:
+            w.stage("aabbs")
+            w.write_state(*state)
+        w.stepSimulation(1)
+        hashes.append(w.sorted_hash())
+        w.close()
+    for a, b in zip(*hashes):
+        assert np.array_equal(a, b)
+    assert np.all(np.diff(hashes[0][0].astype(np.int64)) >= 0)
