@@ -9,7 +9,7 @@ and a written state the world steps like a new one, bit for bit.
 import numpy as np
 import pytest
 
-from experiments_b200 import scenes
+from experiments_b200 import b3, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -37,14 +37,14 @@ def state(sc):
     return pos, np.asarray(sc.quat, np.float32), np.zeros((n, 4), np.float32), np.zeros((n, 4), np.float32)
 
 
-@pytest.mark.parametrize("side", [6, 22, 41])
-def test_steps_after_a_wait_gave_up_stay_in_bounds(ctx, side):
+@pytest.mark.parametrize("side,flags", [(6, 0), (22, 0), (41, 0), (22, b3.B3_WORLD_SAP_BROADPHASE)])
+def test_steps_after_a_wait_gave_up_stay_in_bounds(ctx, side, flags):
     """The solve's barrier gives up while few bodies touch; steps follow with far
     more contacts than any before. 216 and 68,921 bodies: body numbers of one and
     three digits, whose sort ends in the other buffer; 10,648: of two."""
     few, many = cubes(side, 1.05), cubes(side, 0.995)
     cap = max(8192, 16 * few.n)  # sorts of more than one block
-    w = scenes.build_world(ctx, few, maxPairs=cap)
+    w = scenes.build_world(ctx, few, maxPairs=cap, flags=flags)
     t = w.tuning()
     t = [t[0], t[1], 64, t[3], 4, t[5], 0, t[7]]  # many blocks in the solve
     w.set_tuning(t)
@@ -63,7 +63,7 @@ def test_steps_after_a_wait_gave_up_stay_in_bounds(ctx, side):
     w.stepSimulation(2)
     w.set_wait_limits()
     w.reset_counters()
-    fresh = scenes.build_world(ctx, few, maxPairs=cap)
+    fresh = scenes.build_world(ctx, few, maxPairs=cap, flags=flags)
     fresh.set_tuning(t)
     for sc in (many, few):
         for x in (w, fresh):
